@@ -175,12 +175,11 @@ def kernel_bytes(name: str, n: int, p, nleaves: int) -> float | None:
     """Algorithmic bytes per launch of the main kernels (per-unit figures x units)."""
     if name == "k_query_s1":  # read sorted points once, node summaries, one result per window
         return 24.0 * n + 48.0 * nleaves + 8.0 * p.ncells
+    if name == "k_grid_fold":  # x, y, z of every point, read once
+        return 24.0 * n
     if name.startswith("k_gather_leaves"):
-        # the permute step of the whole-step model (read the permutation, gather
-        # xyz, write the permuted points) and 48 B per leaf node.  With the
-        # class fold (the whole-path run) the kernel writes no permuted points:
-        # stage 3 reads its few points through the permutation instead.  The
-        # figure then exceeds what the kernel moves, which `traffic` measures.
+        # the permute step of the tree build (read the permutation, gather xyz,
+        # write the permuted points) and 48 B per leaf node
         return (4 + 24 + 24 + 4) * n + 48.0 * nleaves
     if name == "k_rs_downsweep":
         return 16.0 * n
@@ -190,13 +189,18 @@ def kernel_bytes(name: str, n: int, p, nleaves: int) -> float | None:
 
 
 def path_bytes(n: int, p) -> float:
-    """Compulsory HBM bytes of one whole step (the lower-bound model of the
-    path): build 128 B/pt (read xyz 24, write key 8 and id 8, one sort pass
+    """HBM bytes of one whole step that builds the tree (--stage1-walk): build 128 B/pt (read xyz 24, write key 8 and id 8, one sort pass
     reading and writing 16 each, permute: read id 8, gather xyz 24, write
     permuted xyz 24), stage 1 reading the permuted points once (24 B/pt) plus
     leaf summaries (~2 B/pt) and writing 8 B/window, stage 2 about 32 B/window,
     stage 3 8 B per grid cell: 154 B/pt + 40 B/window + 8 B/cell."""
     return 154.0 * n + 40.0 * p.ncells + 8.0 * p.ngrid
+
+
+def grid_bytes(n: int, p) -> float:
+    """Compulsory HBM bytes of one whole step on the window grid: x, y, z of
+    every point read once (24 B/pt), and per window and cell as path_bytes."""
+    return 24.0 * n + 40.0 * p.ncells + 8.0 * p.ngrid
 
 
 def measured_traffic(name: str, n: int) -> float | None:
@@ -635,13 +639,9 @@ def main():
                 "traffic": round(traffic) if traffic else None,
                 "traffic_gbs": round(traffic / (per_launch_ms / 1e3) / 1e9, 1) if traffic else None,
                 "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch on the 24 M-point "
-                                  "case of the same generator at leaf 256 (profiles/), per point x points"
+                                  "case of the same generator (profiles/), per point x points"
                                   if traffic else None,
                 "ms_per_launch": round(per_launch_ms, 4), "bytes_per_launch": bytes_alg}
-        if name.startswith("k_gather_leaves"):
-            roof["bytes_note"] = ("bytes_per_launch is the whole-step model's permute step (56 B/pt, permuted "
-                                  "points written) + 48 B/leaf; the class-fold gather writes no permuted points "
-                                  "(28 B/pt + 48 B/leaf of its own): `traffic` is what it moves")
     cpu = None
     if rank == 0 and ws == 1 and not args.no_cpu_baseline:
         sspec, sW, sO, sB, smn, sseed = workload(args.config, args.cpu_sample)
@@ -652,9 +652,10 @@ def main():
                "sample": f"{sspec.n} pts, same generator and density ({sspec.x1 - sspec.x0:.0f} m square), "
                          f"W={sW} O={sO} B={sB}, build+OWM once ({t:.2f} s); the reference arm "
                          f"(--impl reference) times the whole workload"}
-    pb = path_bytes(spec.n, p)
+    pb = path_bytes(spec.n, p) if args.stage1_walk else grid_bytes(spec.n, p)
     path_gbs = pb / (ms_max / args.steps / 1e3) / 1e9
-    path_roof = {"model": "compulsory bytes of the whole step: 154 B/pt + 40 B/window + 8 B/cell",
+    path_roof = {"model": "compulsory bytes of the whole step: "
+                          f"{154 if args.stage1_walk else 24} B/pt + 40 B/window + 8 B/cell",
                  "bytes_per_step": pb, "achieved": round(path_gbs, 1), "peak": peak, "peak_kind": peak_kind,
                  "unit": "GB/s", "frac": round(path_gbs / peak, 4)}
     if rank == 0:
@@ -673,9 +674,7 @@ def main():
                 "phases_ms": {"tree": round(phase[0] / args.steps, 4), "stage1": round(phase[1] / args.steps, 4),
                               "stage2": round(phase[2] / args.steps, 4), "stage3": round(phase[3] / args.steps, 4)},
                 "kernel_timing": "second pass over the same K steps with CUDA events around every launch "
-                                 "(the value pass runs without them); k_edges, k_cls_* and k_s2_* run on a side "
-                                 "stream beside the Morton pass, the sort and the hierarchy build, so their event "
-                                 "times include waiting for SMs and the shares sum to more than one step",
+                                 "(the value pass runs without them; each event pair adds about 4 us)",
                 "kernels": {k: {"ms": round(v[0] / args.steps, 4), "share": round(v[0] / tot_k, 4),
                                 "launches_per_step": v[1] / args.steps} for k, v in
                             sorted(ktimes.items(), key=lambda kv: -kv[1][0])},

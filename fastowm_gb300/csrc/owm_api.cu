@@ -222,13 +222,6 @@ int owm_ctx_create(int device, owm_ctx** out) {
   }
   cudaMemset(c->d_small, 0, 4096);
   for (auto& e : c->ev) cudaEventCreate(&e);
-  if (cudaStreamCreateWithFlags(&c->side_stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaEventCreateWithFlags(&c->side_fork, cudaEventDisableTiming) != cudaSuccess ||
-      cudaEventCreateWithFlags(&c->side_join, cudaEventDisableTiming) != cudaSuccess) {
-    cudaGetLastError();
-    owm_ctx_destroy(c);
-    return OWM_ECUDA;
-  }
   cudaStreamSynchronize(c->stream);
   *out = c;
   return OWM_OK;
@@ -255,12 +248,6 @@ int owm_ctx_destroy(owm_ctx* c) {
     cudaStreamSynchronize(c->copy_stream);
     cudaStreamDestroy(c->copy_stream);
   }
-  if (c->side_stream) {
-    cudaStreamSynchronize(c->side_stream);
-    cudaStreamDestroy(c->side_stream);
-  }
-  if (c->side_fork) cudaEventDestroy(c->side_fork);
-  if (c->side_join) cudaEventDestroy(c->side_join);
   c->prof.clear();
   for (cudaEvent_t e : c->prof.pool) cudaEventDestroy(e);
   c->prof.pool.clear();
@@ -774,7 +761,7 @@ int owm_stage3(owm_ctx* c, const owm_tree* tr, const owm_params* p, const int64_
   rc = clear_status(c);
   if (!rc)
     rc = run_stage3(tr->t.view(c->walk_limit, c->tuning.cell_warps), tr->d_xy, kCloudXyStride, *p, l32, d_nllp, n_llp, s3, d_cnt, c->scratch.ptr, c->scratch.cap,
-                    c->d_job, c->d_small + kStatusSlot, c->stream, &c->launches);
+                    c->d_small + kStatusSlot, c->stream, &c->launches);
   if (!rc) rc = check_input_status(c);
   if (rc) return rc;
   OWM_CUDA_TRY(cudaMemcpyAsync(c->h_small + 2, d_cnt, 4, cudaMemcpyDeviceToHost, c->stream));
@@ -901,7 +888,6 @@ int owm_run_submit(owm_ctx* c, const owm_cloud* cl, const owm_run_cfg* cfg, int6
   owm_ctx::AsyncSlot* a = next_slot(c, &rc);
   if (!a) return rc;
   auto fail = [&](int code) {
-    cudaStreamSynchronize(c->side_stream);
     cudaStreamSynchronize(c->stream);
     return code;
   };
@@ -937,7 +923,6 @@ int owm_run_host_submit(owm_ctx* c, const double* xyz, int64_t n, const owm_bbox
   // it before returning, so the caller may free xyz after any return.
   auto fail = [&](int code) {
     cudaStreamSynchronize(c->copy_stream);
-    cudaStreamSynchronize(c->side_stream);
     cudaStreamSynchronize(c->stream);
     return code;
   };

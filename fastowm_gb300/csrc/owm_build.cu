@@ -26,7 +26,6 @@
 #include <cstring>
 
 #include "owm_build.cuh"
-#include "owm_classes.cuh"
 #include "owm_devutil.cuh"
 
 namespace owm {
@@ -140,26 +139,17 @@ __global__ void __launch_bounds__(256) k_morton_counts(const double* __restrict_
 }
 
 // One warp per unit of max(L, 32) sorted positions.  L in {1,2,4,...,256}.
-// Without kCls the sorted points go to the SoA arrays xk, yk, zk, pid.  With
-// kCls (the whole-path run, whose only later reader of points is stage 3's
-// cell walk, which then reads them through the permutation) nothing is
-// stored: 28 bytes a point less to write (100 M points: 2.53 -> 2.39 ms).
-// With kCls, every chunk of 32 gathered points is also folded into the
-// stage-1 window classes while the point is in registers (about 0.45 ms of
-// the kernel's 2.5 ms at 100 M points, nearly all of it the sub-cell lookups
-// and the warp votes; the atomics take about 0.07 ms).
 // At most 40 registers a thread (a few bytes spill): 3 blocks of 512 (48
 // warps) per SM instead of 2 at the 63 registers the compiler would take; the
 // kernel waits on random DRAM reads, and the extra resident warps keep more of
 // them in flight (100 M points: 2.84 -> 2.55 ms; 48 registers 2.69, 36 and 32
 // registers 2.63).  Launched with at most 512 threads.
-template <int L, bool kCls, int kStride>
+template <int L, int kStride>
 __global__ void __maxnreg__(40) k_gather_leaves(const double* __restrict__ xyz, const uint32_t* __restrict__ perm,
                                                        int64_t n, int32_t nleaves, double ox, double oy,
                                                        int64_t* __restrict__ xk, int64_t* __restrict__ yk,
                                                        int64_t* __restrict__ zk, uint32_t* __restrict__ pid,
-                                                       Node* __restrict__ leaves, uint32_t* __restrict__ status,
-                                                       ClassArgs A) {
+                                                       Node* __restrict__ leaves, uint32_t* __restrict__ status) {
   constexpr int kUnit = L < 32 ? 32 : L;
   constexpr int kSeg = L < 32 ? L : 32;
   bool finite = true;
@@ -169,7 +159,7 @@ __global__ void __maxnreg__(40) k_gather_leaves(const double* __restrict__ xyz, 
        u += ((int64_t)gridDim.x * blockDim.x) >> 5) {
     LeafAcc acc;
     acc.init();
-    // the next chunk's permutation entry is in flight while a chunk is folded
+    // the next chunk's permutation entry is in flight while a chunk is reduced
     uint32_t s_nxt = u * kUnit + lane < n ? __ldg(perm + u * kUnit + lane) : 0u;
 #pragma unroll
     for (int c = 0; c < kUnit; c += 32) {
@@ -180,24 +170,11 @@ __global__ void __maxnreg__(40) k_gather_leaves(const double* __restrict__ xyz, 
       if (c + 32 < kUnit) s_nxt = pos + 32 < n ? __ldg(perm + pos + 32) : 0u;
       if (valid) {
         finite &= load_point16<kStride>(xyz, src, x, y, z);
-        if (!kCls) {
-          xk[pos] = x;
-          yk[pos] = y;
-          zk[pos] = z;
-          pid[pos] = src + 1;
-        }
+        xk[pos] = x;
+        yk[pos] = y;
+        zk[pos] = z;
+        pid[pos] = src + 1;
         acc.add(x, y, z, src + 1, (uint32_t)pos);
-      }
-      if (kCls) {
-        if (!__all_sync(0xffffffffu, valid)) {  // ragged tail: idle lanes borrow lane 0's point
-          const int64_t bx = __shfl_sync(0xffffffffu, x, 0), by = __shfl_sync(0xffffffffu, y, 0);
-          if (!valid) {
-            x = bx;
-            y = by;
-            z = 0;
-          }
-        }
-        cls_aggregate_warp(A, valid, x, y, z, src + 1, lane);
       }
     }
     acc.reduce(kSeg);
@@ -405,7 +382,7 @@ int grid_for(int64_t n, int block) {
 
 template <int L, int kStride>
 void launch_gather_leaves(const double* xyz, const uint32_t* perm, int64_t n, int32_t nl, double ox, double oy,
-                          TreeStore* t, uint32_t* status, cudaStream_t s, const ClassArgs* cls) {
+                          TreeStore* t, uint32_t* status, cudaStream_t s) {
   constexpr int kUnit = L < 32 ? 32 : L;
   int64_t nunits = (n + kUnit - 1) / kUnit;
   int64_t warps = nunits;
@@ -414,30 +391,23 @@ void launch_gather_leaves(const double* xyz, const uint32_t* perm, int64_t n, in
   // one warp per unit (no grid-stride reuse): the resident warps then work on
   // neighbouring units, which measured 12-15% faster than 16 blocks per SM
   if (blocks > (int64_t)152 * 1024 * 256 / gb) blocks = (int64_t)152 * 1024 * 256 / gb;
-  if (cls) {
-    OWM_LAUNCH("k_gather_leaves", s, k_gather_leaves<L, true, kStride><<<(unsigned)blocks, gb, 0, s>>>(
-        xyz, perm, n, nl, ox, oy, t->xk, t->yk, t->zk, t->pid, t->nodes + (nl - 1), status, *cls));
-  } else {
-    ClassArgs none;
-    std::memset(&none, 0, sizeof(none));
-    OWM_LAUNCH("k_gather_leaves", s, k_gather_leaves<L, false, kStride><<<(unsigned)blocks, gb, 0, s>>>(
-        xyz, perm, n, nl, ox, oy, t->xk, t->yk, t->zk, t->pid, t->nodes + (nl - 1), status, none));
-  }
+  OWM_LAUNCH("k_gather_leaves", s, k_gather_leaves<L, kStride><<<(unsigned)blocks, gb, 0, s>>>(
+      xyz, perm, n, nl, ox, oy, t->xk, t->yk, t->zk, t->pid, t->nodes + (nl - 1), status));
 }
 
 template <int kStride>
 int gather_leaves_for(int32_t L, const double* xyz, const uint32_t* perm, int64_t n, int32_t nl, double ox, double oy,
-                      TreeStore* t, uint32_t* status, cudaStream_t s, const ClassArgs* cls) {
+                      TreeStore* t, uint32_t* status, cudaStream_t s) {
   switch (L) {
-    case 1: launch_gather_leaves<1, kStride>(xyz, perm, n, nl, ox, oy, t, status, s, cls); break;
-    case 2: launch_gather_leaves<2, kStride>(xyz, perm, n, nl, ox, oy, t, status, s, cls); break;
-    case 4: launch_gather_leaves<4, kStride>(xyz, perm, n, nl, ox, oy, t, status, s, cls); break;
-    case 8: launch_gather_leaves<8, kStride>(xyz, perm, n, nl, ox, oy, t, status, s, cls); break;
-    case 16: launch_gather_leaves<16, kStride>(xyz, perm, n, nl, ox, oy, t, status, s, cls); break;
-    case 32: launch_gather_leaves<32, kStride>(xyz, perm, n, nl, ox, oy, t, status, s, cls); break;
-    case 64: launch_gather_leaves<64, kStride>(xyz, perm, n, nl, ox, oy, t, status, s, cls); break;
-    case 128: launch_gather_leaves<128, kStride>(xyz, perm, n, nl, ox, oy, t, status, s, cls); break;
-    case 256: launch_gather_leaves<256, kStride>(xyz, perm, n, nl, ox, oy, t, status, s, cls); break;
+    case 1: launch_gather_leaves<1, kStride>(xyz, perm, n, nl, ox, oy, t, status, s); break;
+    case 2: launch_gather_leaves<2, kStride>(xyz, perm, n, nl, ox, oy, t, status, s); break;
+    case 4: launch_gather_leaves<4, kStride>(xyz, perm, n, nl, ox, oy, t, status, s); break;
+    case 8: launch_gather_leaves<8, kStride>(xyz, perm, n, nl, ox, oy, t, status, s); break;
+    case 16: launch_gather_leaves<16, kStride>(xyz, perm, n, nl, ox, oy, t, status, s); break;
+    case 32: launch_gather_leaves<32, kStride>(xyz, perm, n, nl, ox, oy, t, status, s); break;
+    case 64: launch_gather_leaves<64, kStride>(xyz, perm, n, nl, ox, oy, t, status, s); break;
+    case 128: launch_gather_leaves<128, kStride>(xyz, perm, n, nl, ox, oy, t, status, s); break;
+    case 256: launch_gather_leaves<256, kStride>(xyz, perm, n, nl, ox, oy, t, status, s); break;
     default:
       return OWM_EINVAL;  // unreachable: leaf_size() gives powers of two up to 256
   }
@@ -504,12 +474,7 @@ size_t tree_scratch_bytes(int64_t n) {
 }
 
 int build_tree(const PointsView& pts, int64_t n, const owm_bbox& bb, const owm_tree_cfg& cfg, TreeStore* t,
-               void* scratch, size_t scratch_bytes, uint32_t* status, cudaStream_t s, int64_t* launches,
-               const ClassArgs* cls, bool* fused, cudaEvent_t cls_ready, cudaEvent_t gather_done) {
-  if (fused) *fused = false;
-  t->perm = nullptr;  // set again below when the gather keeps no point arrays
-  t->rec = nullptr;
-  t->rec_stride = 0;
+               void* scratch, size_t scratch_bytes, uint32_t* status, cudaStream_t s, int64_t* launches) {
   const int stride = pts.rec_stride;
   const double* d_xyz = pts.rec;
   if (n <= 0 || n >= 0x7FFFFFFFLL || (stride != 3 && stride != 4) || (pts.xy_stride != 2 && pts.xy_stride != 3))
@@ -634,18 +599,10 @@ int build_tree(const PointsView& pts, int64_t n, const owm_bbox& bb, const owm_t
   t->root = 0;
 
   if (fixed) {
-    if (cls && cls_ready) OWM_CUDA_TRY(cudaStreamWaitEvent(s, cls_ready, 0));
-    const int grc = stride == 4 ? gather_leaves_for<4>(L, d_xyz, perm, n, nl, t->ox, t->oy, t, status, s, cls)
-                                : gather_leaves_for<3>(L, d_xyz, perm, n, nl, t->ox, t->oy, t, status, s, cls);
+    const int grc = stride == 4 ? gather_leaves_for<4>(L, d_xyz, perm, n, nl, t->ox, t->oy, t, status, s)
+                                : gather_leaves_for<3>(L, d_xyz, perm, n, nl, t->ox, t->oy, t, status, s);
     if (grc) return grc;
     count_launch(launches);
-    if (cls) {  // the class-fold gather keeps no point arrays: points through the permutation
-      t->perm = perm;
-      t->rec = d_xyz;
-      t->rec_stride = stride;
-    }
-    if (fused && cls) *fused = true;
-    if (cls && gather_done) OWM_CUDA_TRY(cudaEventRecord(gather_done, s));
   } else {
     if (stride == 4)
       OWM_LAUNCH("k_gather", s, k_gather<4><<<grid_for(n, 256), 256, 0, s>>>(d_xyz, perm, n, t->xk, t->yk, t->zk, t->pid, status));

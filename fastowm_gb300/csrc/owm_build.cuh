@@ -18,10 +18,6 @@ struct TreeStore {
   int32_t nleaves = 0, root = 0, key_bits = 0, max_leaf = 0;
   int32_t gather_block = 256;  // threads per block of the build's gather (128, 256 or 512)
   double ox = 0, oy = 0;
-  // points through the sort's permutation instead of the arrays (TreeView)
-  const uint32_t* perm = nullptr;
-  const double* rec = nullptr;
-  int32_t rec_stride = 0;
 
   TreeView view(int32_t walk_limit = 0, int32_t cell_warps = 4) const {
     TreeView v;
@@ -36,9 +32,6 @@ struct TreeStore {
     v.root = root;
     v.ox = ox;
     v.oy = oy;
-    v.perm = perm;
-    v.rec = rec;
-    v.rec_stride = rec_stride;
     return v;
   }
 };
@@ -84,18 +77,9 @@ inline PointsView plain_points(const double* xyz) { return PointsView{xyz, 3, xy
 
 // Builds the tree of n device points into t (whose arrays must be allocated
 // with enough capacity).  Scratch is caller-provided.
-// Non-finite input coordinates set bit 0 of *status (device word).  With cls,
-// the fixed-leaf gather also folds every point into the stage-1 window
-// classes (*fused says whether it did; the min-radius build does not); when
-// cls_ready is given, s waits on it right before that gather, so the class
-// tables may be prepared on another stream while the keys are sorted, and
-// gather_done (if given) is recorded on s right after that gather, so the
-// classes may be finished on another stream while the hierarchy is built.
-struct ClassArgs;
+// Non-finite input coordinates set bit 0 of *status (device word).
 int build_tree(const PointsView& pts, int64_t n, const owm_bbox& bbox, const owm_tree_cfg& cfg, TreeStore* t,
-               void* scratch, size_t scratch_bytes, uint32_t* status, cudaStream_t s, int64_t* launches,
-               const ClassArgs* cls = nullptr, bool* fused = nullptr, cudaEvent_t cls_ready = nullptr,
-               cudaEvent_t gather_done = nullptr);
+               void* scratch, size_t scratch_bytes, uint32_t* status, cudaStream_t s, int64_t* launches);
 
 // Structural self-check (checkNumPoints); *h_bad = number of bad nodes.
 int check_tree(const TreeStore* t, int32_t* d_bad, cudaStream_t s, int64_t* launches, int32_t* h_bad);

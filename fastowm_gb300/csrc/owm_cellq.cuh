@@ -28,30 +28,8 @@ constexpr int kS3Stack = 2304;   // node stack entries per warp (the kernels run
 
 __device__ __forceinline__ int64_t cq_shfl64(int64_t v, int src) { return __shfl_sync(0xffffffffu, v, src); }
 
-// Record r of the points a tree without point arrays was built from, as
-// order keys (T.perm set: point p of the sorted order is record T.perm[p]).
-__device__ __forceinline__ void cq_record(const TreeView& T, uint32_t r, int64_t& x, int64_t& y, int64_t& z) {
-  if (T.rec_stride == 4)
-    load_point16<4>(T.rec, r, x, y, z);
-  else
-    load_point16<3>(T.rec, r, x, y, z);
-}
-// x, y of a node's min point: sorted position p, id `id` (its record + 1).
-template <bool kPerm>
-__device__ __forceinline__ void cq_min_point_xy(const TreeView& T, int64_t p, uint32_t id, int64_t& x, int64_t& y) {
-  if (kPerm) {  // the id names the record: no permutation read
-    int64_t z;
-    cq_record(T, id - 1u, x, y, z);
-  } else {
-    x = __ldg(T.xk + p);
-    y = __ldg(T.yk + p);
-  }
-}
-
 // The whole warp answers the cell with edge tables ex, ey over tree T; st is
 // this warp's kS3Stack-entry shared stack.  Returns the result on every lane.
-// kPerm: T keeps no point arrays (T.perm is set).
-template <bool kPerm>
 __device__ __forceinline__ uint32_t cell_min_warp(const TreeView& T, const Edge& ex, const Edge& ey, int32_t* st,
                                                   uint32_t* status, int lane) {
   const uint32_t lt = (1u << lane) - 1u;
@@ -90,8 +68,7 @@ __device__ __forceinline__ uint32_t cell_min_warp(const TreeView& T, const Edge&
       if (inside) {
         cand = true;
       } else if (!outside && (improve || !any)) {
-        int64_t mx, my;
-        cq_min_point_xy<kPerm>(T, npos, nid, mx, my);
+        const int64_t mx = __ldg(T.xk + npos), my = __ldg(T.yk + npos);
         if (mx > ex.lo_k && mx < ex.hi_k && my > ey.lo_k && my < ey.hi_k) {
           cand = true;
         } else if (nodei >= first_leaf) {
@@ -136,46 +113,25 @@ __device__ __forceinline__ uint32_t cell_min_warp(const TreeView& T, const Edge&
       int64_t mz = 0x7FFFFFFFFFFFFFFFll;
       uint32_t mid = 0xFFFFFFFFu;
       bool seen = false;
-      // kU * 32 points per chunk, every load issued before any test: one
-      // memory latency per chunk (with kPerm two, the permutation entries
-      // first; 256 points a chunk, so a leaf of up to 256 points takes one)
-      constexpr int kU = kPerm ? 8 : 4;
+      // 128 points per chunk, every load issued before any test: one memory
+      // latency per chunk
+      constexpr int kU = 4;
       for (uint32_t o = 0; o < c; o += 32 * kU) {
         int64_t x[kU], y[kU], z[kU];
         uint32_t id[kU];
-        if (kPerm) {
-          uint32_t src[kU];
 #pragma unroll
-          for (int u = 0; u < kU; ++u) {
-            const uint32_t k = o + u * 32 + lane;
-            src[u] = k < c ? __ldg(T.perm + (int64_t)first + k) : 0xFFFFFFFFu;  // positions < 2^31
-          }
-#pragma unroll
-          for (int u = 0; u < kU; ++u) {
-            if (src[u] != 0xFFFFFFFFu) {
-              cq_record(T, src[u], x[u], y[u], z[u]);
-              id[u] = src[u] + 1u;
-            } else {
-              x[u] = ex.lo_k;  // fails the strict test
-              y[u] = z[u] = 0;
-              id[u] = 0;
-            }
-          }
-        } else {
-#pragma unroll
-          for (int u = 0; u < kU; ++u) {
-            const uint32_t k = o + u * 32 + lane;
-            if (k < c) {
-              const int64_t q = (int64_t)first + k;
-              x[u] = __ldg(T.xk + q);
-              y[u] = __ldg(T.yk + q);
-              z[u] = __ldg(T.zk + q);
-              id[u] = __ldg(T.pid + q);
-            } else {
-              x[u] = ex.lo_k;  // fails the strict test
-              y[u] = z[u] = 0;
-              id[u] = 0;
-            }
+        for (int u = 0; u < kU; ++u) {
+          const uint32_t k = o + u * 32 + lane;
+          if (k < c) {
+            const int64_t q = (int64_t)first + k;
+            x[u] = __ldg(T.xk + q);
+            y[u] = __ldg(T.yk + q);
+            z[u] = __ldg(T.zk + q);
+            id[u] = __ldg(T.pid + q);
+          } else {
+            x[u] = ex.lo_k;  // fails the strict test
+            y[u] = z[u] = 0;
+            id[u] = 0;
           }
         }
 #pragma unroll

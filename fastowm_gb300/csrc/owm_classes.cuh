@@ -234,23 +234,4 @@ __device__ __forceinline__ int64_t cls_window_slot(const ClassArgs& A, int64_t w
 // exponent); false when no table applies (the per-point search then runs).
 bool cls_table_geometry(double lo, double hi, double step, int64_t* k0, int* sh, int32_t* Q);
 
-size_t classes_scratch_bytes(int64_t n, int32_t ncols, int32_t nrows);
-// Carves the buffers from scratch and enqueues the edge split, s-ranges,
-// class tables and counter resets for the windows of p (edge tables ex/ey).
-int classes_prepare(const owm_params& p, const Edge* ex, const Edge* ey, void* scratch, size_t scratch_bytes,
-                    int64_t n, ClassArgs* A, cudaStream_t s, int64_t* launches);
-// Aggregation as its own pass over sorted points (when it is not fused into
-// the build's gather).
-int classes_aggregate(const ClassArgs& A, const TreeView& t, int64_t n, cudaStream_t s, int64_t* launches);
-// Tie ids, row and window reductions: stage-1 results into d_win.
-int classes_finish(const ClassArgs& A, const TreeView& t, int64_t n, const owm_params& p, uint32_t* d_win,
-                   cudaStream_t s, int64_t* launches);
-// The same, marking stage 2's occupancy bitmaps (zeroed) as each window
-// result is produced (s2_mark_id); stage 2 then only emits the LLPs.
-int classes_finish_marked(const ClassArgs& A, const owm_params& p, uint32_t* d_win, uint32_t* once, uint32_t* twice,
-                          uint32_t max_id, cudaStream_t s, int64_t* launches);
-// prepare + aggregate + finish.
-int run_stage1_classes(const TreeView& t, int64_t n, const owm_params& p, const Edge* ex, const Edge* ey,
-                       uint32_t* d_win, void* scratch, size_t scratch_bytes, cudaStream_t s, int64_t* launches);
-
 }  // namespace owm

@@ -72,8 +72,8 @@ struct owm_ctx {
   uint32_t* h_small = nullptr;  // [1024] pinned host mirror
   owm::QueryJob* d_job = nullptr;
   owm::DeviceBuffer scratch, tree_mem, input, outbuf;
-  owm::TreeStore tree;  // tree of the last owm_run
-  cudaEvent_t ev[8] = {};
+  owm::TreeStore tree;  // tree of the last owm_run that built one
+  cudaEvent_t ev[6] = {};
   // owm_run_host_submit / _wait: two runs in flight, each with its own input
   // buffer and pinned result staging; the host->device copy of one runs on
   // copy_stream while the other computes on `stream`.
@@ -91,13 +91,6 @@ struct owm_ctx {
   };
   cudaStream_t copy_stream = nullptr;
   AsyncSlot aslot[2];
-  // owm_run prepares the stage-1 class tables on side_stream while the tree's
-  // keys are sorted on `stream` (fork and join by the two events).
-  // Then stage 1's last kernels and stage 2 run there too, while the tree's
-  // hierarchy is built on `stream` (stage12_side: the last owm_run did so).
-  cudaStream_t side_stream = nullptr;
-  cudaEvent_t side_fork = nullptr, side_join = nullptr;
-  bool stage12_side = false;
   int64_t next_ticket = 1;
   // > 0: step limit of the bounded tree walks (owm_ctx_set_walk_limit)
   int32_t walk_limit = 0;

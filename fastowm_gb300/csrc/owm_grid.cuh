@@ -1,0 +1,311 @@
+// Window grid: the whole path of one cloud without a spatial hierarchy.
+//
+// Along one axis the stage-1 windows (L_j, R_j) and the stage-3 cells
+// (A_i, B_i) are open intervals whose edges do not decrease with their index.
+// For a coordinate p let
+//     s(p) = #{L_j < p} + #{R_j <= p} + #{A_i < p} + #{B_i <= p}.
+// s does not decrease with p, and an interval (l, r) of either family contains
+// p exactly when s(l+) <= s(p) <= s(r-), with l+ / r- the next double above l /
+// below r.  So every point falls in one (s_x, s_y) sub-cell, and every window
+// and every cell is a rectangle of sub-cells.  The path is then: one pass over
+// the points that keeps each sub-cell's count and (z, id)-minimum (the
+// reference's O3 memo, optim3_func.cpp:255-307, on the sub-cells instead of
+// quadtree nodes), and rectangle reductions for stage 1 and stage 3.
+#pragma once
+
+#include "owm_query.cuh"
+
+namespace owm {
+
+enum GridFamily { kFamL = 0, kFamR = 1, kFamA = 2, kFamB = 3 };
+
+// One axis.  A coordinate's sub-cell is found by arithmetic, not by a table or
+// a search: its position v (32 bits, a fixed-point offset from the axis's
+// origin) times a constant is its place in window (cell) steps, whose integer
+// part is the number of edges passed.  A place within kGridGuard units of an
+// edge's nominal one is settled by comparing with the edge itself.
+struct GridAxis {
+  // Constants of the fold's fast form, for coordinates in [lo, hi] off the edges:
+  // place = mulhi(position above lo, m) + q, count = min((place >> fb) - k, n).
+  int64_t lo0;               // lo's bits (linear) or whole quanta (general)
+  uint64_t span;             // hi's minus lo's
+  uint32_t qw, qr, qc, qb;   // place of lo: L, R, A, B
+  int32_t kl, kr, ka, kb;    // edge counts at place 0
+  int32_t paired;            // R and B places lie where L and A places do: one place for both
+  int32_t lcap, ksum;        // paired: s = min(tl, lcap) + tl + 2 ta - ksum, t = place >> fb
+  int32_t fast;              // that form holds over all of [lo, hi]
+  int64_t f0;                // position 0: a double's bits (linear) or whole quanta (general)
+  uint32_t mw, mc;           // steps per position, times 2^(32 + fb): windows, cells
+  uint32_t c[4];             // place of position 0 by family, bias and guard added
+  int32_t fbw, fbc;          // fraction bits of a place
+  int32_t kw, kc;            // bias: count = (place >> fb) - bias, clamped to [0, n]
+  int32_t n, nc;             // windows, cells
+  int32_t quick;             // 0: no fixed-point form (every coordinate is searched)
+  int32_t linear;            // 1: the range lies in one positive binade, a double's bits are linear in it
+  int32_t sh;                // linear: bits shifted out; general: biased exponent of the quantum + 52
+  int32_t merged;            // s counts the cells' edges too
+  int32_t nclass;            // values of s
+  int32_t par, parmask;      // parmask 1: points off the edges all have s & 1 == par (the main parity)
+  int32_t width[2];          // classes of the main parity, of the other
+  double wbase, step, wr;    // L_j = (wbase + j * step) - wr, R_j = ... + wr
+  double cbase, cr;          // A_i = (cbase + i * bsize) - cr, B_i = ... + cr
+  int32_t bsize, pad;
+  const int64_t* edge[4];    // order keys of the edges, by family (device)
+  int32_t *lo, *hi, *clo, *chi;  // s-range of every window and cell (device; merged cells only)
+};
+
+// Places are compared with nominal ones in units of 2^-fb steps; one position
+// is at most one unit.  An edge's double lies within 2.5 units of the exact
+// arithmetic progression (its roundings after the first edge's: j * step, the
+// sum, the half width, each at most half an ulp, an ulp at most one position),
+// flooring the position and the product adds 2, rounding the constants and
+// the origin 2.  Places further than the guard from an edge's nominal place
+// are therefore on the same side of the edge as the coordinate is.
+constexpr uint32_t kGridGuard = 16;
+constexpr int32_t kGridMinFrac = 8;  // fewest fraction bits of the fixed-point form (4 guards a step)
+
+__host__ __device__ __forceinline__ double grid_add(double a, double b) {
+#ifdef __CUDA_ARCH__
+  return __dadd_rn(a, b);
+#else
+  return a + b;
+#endif
+}
+__host__ __device__ __forceinline__ double grid_mul(double a, double b) {
+#ifdef __CUDA_ARCH__
+  return __dmul_rn(a, b);
+#else
+  return a * b;
+#endif
+}
+
+// Edge j of a family, as an order key; the reference's arithmetic (stage 1:
+// optim3_func.cpp:318-324, 544-555; stage 3: :310-316, 630-651), each
+// operation rounded by itself.
+__host__ __device__ __forceinline__ int64_t grid_edge(const GridAxis& a, int fam, int32_t j) {
+  if (fam < 2) {
+    const double c = grid_add(a.wbase, grid_mul((double)j, a.step));
+    return dkey(grid_add(c, fam == kFamL ? -a.wr : a.wr));
+  }
+  const double c = grid_add(a.cbase, (double)(j * a.bsize));
+  return dkey(grid_add(c, fam == kFamA ? -a.cr : a.cr));
+}
+
+// Whether an edge lies below a coordinate: strictly for the left edges, not
+// above it for the right ones.
+__host__ __device__ __forceinline__ bool grid_passed(int fam, int64_t edge, int64_t key) {
+  return (fam & 1) ? edge <= key : edge < key;
+}
+
+// Position of the double with these bits; false outside the axis's range
+// (also for NaN and infinities).
+__host__ __device__ __forceinline__ bool grid_position(const GridAxis& a, uint64_t bits, uint32_t* v) {
+  uint64_t d;
+  bool ok = a.quick != 0;
+  if (a.linear) {
+    d = (bits - (uint64_t)a.f0) >> a.sh;
+  } else {
+    const int32_t e = (int32_t)((bits >> 52) & 0x7FF);
+    const uint64_t m = (bits & 0xFFFFFFFFFFFFFull) | (e ? 0x10000000000000ull : 0ull);
+    const int32_t s = a.sh - (e ? e : 1);
+    ok = ok && s >= 0 && e != 0x7FF;
+    const int64_t f = s > 63 || s < 0 ? 0 : (int64_t)(m >> s);
+    d = (uint64_t)(((int64_t)bits < 0 ? -f : f) - a.f0);
+  }
+  *v = (uint32_t)d;
+  return ok && (d >> 32) == 0;
+}
+
+__host__ __device__ __forceinline__ uint32_t grid_mulhi(uint32_t a, uint32_t b) {
+#ifdef __CUDA_ARCH__
+  return __umulhi(a, b);
+#else
+  return (uint32_t)(((uint64_t)a * b) >> 32);
+#endif
+}
+
+__host__ __device__ __forceinline__ int32_t grid_clamp(int32_t v, int32_t n) { return v < 0 ? 0 : (v > n ? n : v); }
+
+// Edges of one family passed at position v, and whether the place is near one.
+__host__ __device__ __forceinline__ int32_t grid_count(const GridAxis& a, int fam, uint32_t v, bool* near) {
+  const bool win = fam < 2;
+  const int32_t fb = win ? a.fbw : a.fbc;
+  const uint32_t h = grid_mulhi(v, win ? a.mw : a.mc) + a.c[fam];
+  *near = (h & ((1u << fb) - 1u)) < 2 * kGridGuard;
+  return (int32_t)(h >> fb) - (win ? a.kw : a.kc);
+}
+
+// The four edge counts of a coordinate, exactly.  edge_of(fam, j) gives the
+// edges' order keys.
+template <class EdgeOf>
+__host__ __device__ __forceinline__ void grid_counts_exact(const GridAxis& a, uint64_t bits, int64_t key, EdgeOf edge_of,
+                                                           int32_t cnt[4]) {
+  uint32_t v;
+  const bool ok = grid_position(a, bits, &v);
+  for (int f = 0; f < 4; ++f) {
+    const int32_t n = f < 2 ? a.n : a.nc;
+    if (ok) {
+      bool near;
+      int32_t k = grid_count(a, f, v, &near);
+      if (near && k >= 1 && k <= n) k -= grid_passed(f, edge_of(f, k - 1), key) ? 0 : 1;
+      cnt[f] = grid_clamp(k, n);
+    } else {
+      int32_t lo = 0, hi = n;
+      while (lo < hi) {
+        const int32_t mid = (lo + hi) >> 1;
+        if (grid_passed(f, edge_of(f, mid), key)) lo = mid + 1; else hi = mid;
+      }
+      cnt[f] = lo;
+    }
+  }
+}
+
+// The four edge counts of a coordinate in [lo, hi], not yet clamped to their
+// upper ends.  0: exact.  1: near an edge, each at most one too high
+// (grid_settle).  2: not in [lo, hi], cnt means nothing.
+// Off the edges no count is negative in [lo, hi]: the first edges lie at most
+// one step above lo.  Where windows and cells tile the axis in whole steps one
+// place serves left and right edges.
+__host__ __device__ __forceinline__ int grid_counts_raw(const GridAxis& a, uint64_t bits, int32_t cnt[4]) {
+  uint32_t v;
+  bool in;
+  if (a.linear) {
+    const uint64_t d = bits - (uint64_t)a.lo0;
+    in = d <= a.span;
+    v = (uint32_t)(d >> a.sh);
+  } else {
+    in = grid_position(a, bits, &v);
+    v -= 1u << 30;
+    in = in && v <= (uint32_t)a.span;
+  }
+  const uint32_t hl = grid_mulhi(v, a.mw) + a.qw, ha = grid_mulhi(v, a.mc) + a.qc;
+  const uint32_t mw = (1u << a.fbw) - 1u, mc = (1u << a.fbc) - 1u;
+  bool off = (hl & mw) >= 2 * kGridGuard && (ha & mc) >= 2 * kGridGuard;
+  uint32_t hr = hl, hb = ha;
+  if (!a.paired) {
+    hr = grid_mulhi(v, a.mw) + a.qr;
+    hb = grid_mulhi(v, a.mc) + a.qb;
+    off = off && (hr & mw) >= 2 * kGridGuard && (hb & mc) >= 2 * kGridGuard;
+  }
+  cnt[0] = (int32_t)(hl >> a.fbw) - a.kl;
+  cnt[1] = (int32_t)(hr >> a.fbw) - a.kr;
+  cnt[2] = (int32_t)(ha >> a.fbc) - a.ka;
+  cnt[3] = (int32_t)(hb >> a.fbc) - a.kb;
+  return !in ? 2 : off ? 0 : 1;
+}
+
+// Counts of a coordinate by all of the above.
+template <class EdgeOf>
+__host__ __device__ __forceinline__ int grid_counts(const GridAxis& a, uint64_t bits, EdgeOf edge_of, int32_t cnt[4]) {
+  const int how = grid_counts_raw(a, bits, cnt);
+  if (how == 2) return how;
+#pragma unroll
+  for (int f = 0; f < 4; ++f) cnt[f] = cnt[f] < (f < 2 ? a.n : a.nc) + how ? cnt[f] : (f < 2 ? a.n : a.nc) + how;
+  if (how == 0) return how;
+  double d;
+#ifdef __CUDA_ARCH__
+  d = __longlong_as_double((long long)bits);
+#else
+  __builtin_memcpy(&d, &bits, 8);
+#endif
+  const int64_t key = dkey(d);
+#pragma unroll
+  for (int f = 0; f < 4; ++f) {
+    const int32_t n = f < 2 ? a.n : a.nc, k = cnt[f];
+    if (n > 0)
+      cnt[f] = grid_clamp(k, n) - (k >= 1 && k <= n && !grid_passed(f, edge_of(f, grid_clamp(k - 1, n - 1)), key));
+    else
+      cnt[f] = 0;
+  }
+  return how;
+}
+
+__host__ __device__ __forceinline__ int32_t grid_sum(const GridAxis& a, const int32_t cnt[4]) {
+  return cnt[0] + cnt[1] + (a.merged ? cnt[2] + cnt[3] : 0);
+}
+
+// Class of a coordinate on an axis with the fast form; rare is set where that
+// does not settle it.
+__host__ __device__ __forceinline__ int32_t grid_class_fast(const GridAxis& a, uint64_t bits, bool* rare) {
+  const uint64_t d = bits - (uint64_t)a.lo0;
+  const uint32_t v = (uint32_t)(d >> a.sh);
+  const uint32_t hl = grid_mulhi(v, a.mw) + a.qw, ha = grid_mulhi(v, a.mc) + a.qc;
+  *rare |= (d > a.span) | ((hl & ((1u << a.fbw) - 1u)) < 2 * kGridGuard) | ((ha & ((1u << a.fbc) - 1u)) < 2 * kGridGuard);
+  const int32_t tl = (int32_t)(hl >> a.fbw), ta = (int32_t)(ha >> a.fbc);
+  return (tl < a.lcap ? tl : a.lcap) + tl + 2 * ta - a.ksum;
+}
+
+// Count and (z, id)-minimum of a box, all zero when empty: w is the inverted,
+// sign-flipped order key of z and nid the inverted id, so the lexicographic
+// maximum of (w, nid) is the (z, id)-minimum.
+struct __align__(16) GridRow {
+  unsigned long long w;
+  uint32_t nid, count;
+};
+
+// Sub-cells are stored by quadrants of the two axes' parities (s >> 1 within a
+// quadrant), main parity first: where windows and cells tile the axes in whole
+// steps (overlap 0.8: W = 5 steps), every right edge nearly coincides with a
+// left one and every second class is a few ulps wide and all but empty; apart,
+// the full sub-cells lie side by side, a quarter of the table.
+struct GridJob {
+  GridAxis x, y;
+  uint32_t base[4];      // first sub-cell of quadrant 2 * (y not main) + (x not main)
+  int32_t fast;          // both axes have the fast form
+  ulonglong2* zid;       // [sub-cells] (w, nid)
+  uint32_t* count;       // [sub-cells]
+  ulonglong2* cell_zid;  // [cells] (w, nid), when the cells are not merged
+  GridRow* rows;         // [y.nclass][x.n], main parity first
+  uint32_t* occ;         // [4] words: x main / other, y main / other classes hold points
+  uint8_t* mark;         // [cells] an LLP lies in the cell
+  uint32_t* cellmin;     // [cells] stage-3 id or kNone
+  uint32_t* once;        // stage-2 bitmaps over ids 0..n
+  uint32_t* twice;
+  uint32_t* win;         // [windows] stage-1 ids (kept when overlap is 0)
+  uint32_t thr;
+  int32_t n;
+};
+
+// Stored index of sub-cell (sx, sy).
+__host__ __device__ __forceinline__ uint32_t grid_cell(const GridJob& J, int32_t sx, int32_t sy) {
+  const int qx = (sx ^ J.x.par) & 1, qy = (sy ^ J.y.par) & 1;
+  const uint32_t b = qy ? (qx ? J.base[3] : J.base[2]) : (qx ? J.base[1] : J.base[0]);
+  return b + (uint32_t)(sy >> 1) * (uint32_t)(qx ? J.x.width[1] : J.x.width[0]) + (uint32_t)(sx >> 1);
+}
+
+// Number of sub-cells of a job.
+inline int64_t grid_cells(const GridJob& j) { return (int64_t)j.x.nclass * j.y.nclass; }
+
+// Host set-up of one axis (edge arrays and ranges excepted): windows of half
+// width wsize / 2 at every `step`, cells of half width bsize / 2.
+void grid_axis_setup(double lo, double hi, double step, int32_t whalf, int32_t n, int32_t bsize, int32_t nc, bool merged,
+                     GridAxis* a);
+
+// The pieces of the path, in order, on stream s.  d_words: the context's small
+// words (status, LLP and stage-3 counts).
+struct GridPlan {
+  GridJob job;
+  int64_t n = 0, nwin = 0, ncell = 0, nsub = 0;
+  bool bitmap2 = true;     // stage 2 by occupancy bitmaps (overlap > 0)
+  size_t clear_bytes = 0;  // from the scratch's start
+  size_t bytes = 0;
+  uint32_t *part = nullptr, *llp = nullptr, *s3 = nullptr, *flags = nullptr, *pos = nullptr;
+  int64_t* seeds = nullptr;
+  void *s2_temp = nullptr, *scan_temp = nullptr;
+  size_t s2_bytes = 0, scan_bytes = 0;
+  char* base = nullptr;
+};
+// Sizes the plan (scratch nullptr) or carves it from scratch.
+int grid_plan(const owm_params& p, int64_t n, void* scratch, GridPlan* g);
+// Clears the tables and computes edges and ranges.
+int grid_prepare(const GridPlan& g, uint32_t* status, cudaStream_t s, int64_t* launches);
+// Folds points [first, first + count) of the cloud, ids first + 1 ...
+int grid_fold(const GridPlan& g, const double* rec, int stride, int64_t first, int64_t count, uint32_t* status,
+              cudaStream_t s, int64_t* launches);
+// Stage 1 (rows, windows), stage 2 with stage 3's marks, stage 3 and the seeds.
+int grid_windows(const GridPlan& g, cudaStream_t s, int64_t* launches);
+int grid_stage2(const GridPlan& g, const owm_params& p, const double* xy, int xy_stride, uint32_t* d_nllp,
+                cudaStream_t s, int64_t* launches);
+int grid_stage3(const GridPlan& g, const uint32_t* d_nllp, uint32_t* d_ns3, cudaStream_t s, int64_t* launches);
+
+}  // namespace owm

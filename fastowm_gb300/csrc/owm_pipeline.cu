@@ -1,15 +1,17 @@
 // The whole OWM path of one cloud on the device, as the reference application
 // runs it per loop iteration (CPP-TBB-CPU/application/owm_optim3.cpp:77-230):
-// tree build, stage 1, sort + stage 2, LLP grid + stage 3, and the result
-// (stage-3 ids followed by the LLPs).  Intermediates never leave the device;
-// the host sees two small count words and the final seed list.
+// index, stage 1, sort + stage 2, LLP grid + stage 3, and the result (stage-3
+// ids followed by the LLPs).  The index is the window grid (owm_grid.cuh), or
+// the tree when stage 1 walks it (stage1_walk, or a walk limit is set).
+// Intermediates never leave the device; the host sees two small count words
+// and the final seed list.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cstring>
 
-#include "owm_classes.cuh"
 #include "owm_ctx.cuh"
+#include "owm_grid.cuh"
 
 namespace owm {
 
@@ -146,26 +148,54 @@ int run_stage1(owm_ctx* c, const TreeStore& t, const owm_params& p, Edge* ex, Ed
   return run_query(j, c->d_job, c->stream, &c->launches, "k_query_s1");
 }
 
+namespace {
+// The whole path on the window grid (owm_grid.cuh): no hierarchy is built.
+int run_grid(owm_ctx* c, const PointsView& pts, int64_t n, const owm_params& p, int64_t** d_seeds, int64_t* room) {
+  GridPlan g;
+  int rc = grid_plan(p, n, nullptr, &g);
+  if (!rc) rc = c->scratch.reserve(g.bytes, c->stream);
+  if (!rc) rc = grid_plan(p, n, c->scratch.ptr, &g);
+  if (rc) return rc;
+  cudaStream_t s = c->stream;
+  uint32_t* status = c->d_small + kStatusSlot;
+  uint32_t* d_nllp = c->d_small + kLlpSlot;
+  uint32_t* d_ns3 = c->d_small + kS3Slot;
+  OWM_CUDA_TRY(cudaEventRecord(c->ev[0], s));
+  rc = grid_prepare(g, status, s, &c->launches);
+  if (!rc) rc = grid_fold(g, pts.rec, pts.rec_stride, 0, n, status, s, &c->launches);
+  if (rc) return rc;
+  OWM_CUDA_TRY(cudaEventRecord(c->ev[1], s));
+  rc = grid_windows(g, s, &c->launches);
+  if (rc) return rc;
+  OWM_CUDA_TRY(cudaEventRecord(c->ev[2], s));
+  rc = grid_stage2(g, p, pts.xy, pts.xy_stride, d_nllp, s, &c->launches);
+  if (rc) return rc;
+  OWM_CUDA_TRY(cudaEventRecord(c->ev[3], s));
+  rc = grid_stage3(g, d_nllp, d_ns3, s, &c->launches);
+  if (rc) return rc;
+  OWM_CUDA_TRY(cudaEventRecord(c->ev[4], s));
+  *d_seeds = g.seeds;
+  *room = g.nwin + g.ncell + 1;
+  return OWM_OK;
+}
+}  // namespace
+
 int run_pipeline_enqueue(owm_ctx* c, const PointsView& pts, int64_t n, const owm_bbox& bb, const owm_run_cfg& cfg,
                          owm_params* p_out, int64_t** d_seeds, int64_t* room_out) {
   if (validate_tree_cfg(&cfg.tree) != OWM_OK) return OWM_EINVAL;
   owm_params& p = *p_out;
   int rc = owm_params_compute(&bb, n, cfg.wsize, cfg.overlap, cfg.bsize, &p);
   if (rc) return rc;
+  if (!cfg.stage1_walk && c->walk_limit == 0) return run_grid(c, pts, n, p, d_seeds, room_out);
   const int64_t nc = p.ncells, ng = std::max<int64_t>(p.ngrid, 0);
   rc = tree_alloc(&c->tree, &c->tree_mem, n, cfg.tree, c->stream);
   if (rc) return rc;
-  // scratch = [tree build | window classes | stage 2 | stage 3], disjoint:
-  // the side stream zeroes stage 2's bitmaps and prepares stage 3's edge
-  // tables while the tree is built, and runs stages 1-2 and stage 3's LLP
-  // marks beside the hierarchy build.
+  // scratch = [tree build | stage 2 | stage 3]
   const size_t tbytes = (tree_scratch_bytes(n) + 255) & ~(size_t)255;
-  const size_t cbytes = cfg.stage1_walk ? 0 : (classes_scratch_bytes(n, (int32_t)p.ncols, (int32_t)p.nrows) + 255) &
-                                                  ~(size_t)255;
   const bool bitmap2 = p.overlap > 0.0;
   const size_t s2bytes = bitmap2 ? stage2_bitmap_scratch_bytes(n) : stage2_scratch_bytes(nc);
   const size_t s2al = (s2bytes + 255) & ~(size_t)255;
-  size_t sbytes = tbytes + cbytes + s2al + stage3_scratch_bytes(ng);
+  size_t sbytes = tbytes + s2al + stage3_scratch_bytes(ng);
   rc = c->scratch.reserve(sbytes, c->stream);
   if (rc) return rc;
   size_t obytes = 2 * al(65536 * sizeof(Edge)) + 2 * al((size_t)nc * 4) + al((size_t)std::max<int64_t>(ng, 1) * 4) +
@@ -190,91 +220,23 @@ int run_pipeline_enqueue(owm_ctx* c, const PointsView& pts, int64_t n, const owm
   cudaStream_t s = c->stream;
   OWM_CUDA_TRY(cudaEventRecord(c->ev[0], s));
   rc = clear_status(c);
-  ClassArgs cls;
-  bool forked = false;
-  if (!rc && !cfg.stage1_walk) {
-    // Window edges and class tables, so that the build's gather can fold
-    // every point into its window class on the fly.  They depend on nothing
-    // the build makes before its gather, so they are prepared on the side
-    // stream (forked after everything already queued on s, which may still
-    // use this scratch) while the Morton pass and the sort run.
-    cudaStream_t ss = c->side_stream;
-    OWM_CUDA_TRY(cudaEventRecord(c->side_fork, s));
-    OWM_CUDA_TRY(cudaStreamWaitEvent(ss, c->side_fork, 0));
-    forked = true;
-    rc = compute_edges(p, bb.min_x, bb.min_y, false, ex, ey, ss, &c->launches);
-    if (!rc)
-      rc = classes_prepare(p, ex, ey, static_cast<char*>(c->scratch.ptr) + tbytes, cbytes, n, &cls, ss, &c->launches);
-    if (!rc && bitmap2)
-      rc = stage2_bitmap_clear(static_cast<char*>(c->scratch.ptr) + tbytes + cbytes, s2al, n, ss);
-    if (!rc)
-      rc = run_stage3_prepare(bb.min_x, bb.min_y, p, static_cast<char*>(c->scratch.ptr) + tbytes + cbytes + s2al,
-                              c->scratch.cap - tbytes - cbytes - s2al, ss, &c->launches);
-    OWM_CUDA_TRY(cudaEventRecord(c->side_join, ss));
-  }
-  bool fused = false;
-  c->stage12_side = false;
   c->tree.gather_block = c->tuning.gather_block;
   if (!rc)
-    rc = build_tree(pts, n, bb, cfg.tree, &c->tree, c->scratch.ptr, tbytes, c->d_small + kStatusSlot, s,
-                    &c->launches, cfg.stage1_walk ? nullptr : &cls, &fused, forked ? c->side_join : nullptr,
-                    forked ? c->ev[6] : nullptr);
-  void* s2scratch = static_cast<char*>(c->scratch.ptr) + tbytes + cbytes;
-  const size_t s2cap = s2al;
-  void* s3scratch = static_cast<char*>(c->scratch.ptr) + tbytes + cbytes + s2al;
-  const size_t s3cap = c->scratch.cap - tbytes - cbytes - s2al;
-  auto stage2 = [&](cudaStream_t st) {
-    return bitmap2 ? run_stage2_bitmap(win, nc, n, p.overlap, llp, d_nllp, s2scratch, s2cap, st, &c->launches, forked)
-                   : run_stage2(win, nc, n, p.overlap, llp, d_nllp, s2scratch, s2cap, st, &c->launches);
-  };
-  if (!rc && fused) {
-    // The gather's class fold is all that stage 1 needs: finish stage 1,
-    // run stage 2 and mark stage 3's LLP cells on the side stream (after its
-    // table preparation and the gather) while s builds the hierarchy; join
-    // before stage 3's queries.
-    cudaStream_t ss = c->side_stream;
-    c->stage12_side = true;
-    OWM_CUDA_TRY(cudaStreamWaitEvent(ss, c->ev[6], 0));
-    if (bitmap2) {  // the window kernel marks stage 2's bitmaps (zeroed early, above)
-      uint32_t *once = nullptr, *twice = nullptr;
-      stage2_bitmap_ptrs(s2scratch, n, &once, &twice);
-      rc = classes_finish_marked(cls, p, win, once, twice, (uint32_t)n, ss, &c->launches);
-    } else {
-      rc = classes_finish(cls, c->tree.view(), n, p, win, ss, &c->launches);
-    }
-    if (!rc) OWM_CUDA_TRY(cudaEventRecord(c->ev[2], ss));
-    if (!rc)
-      rc = bitmap2 ? run_stage2_bitmap(win, nc, n, p.overlap, llp, d_nllp, s2scratch, s2cap, ss, &c->launches, true, true)
-                   : stage2(ss);
-    if (!rc) OWM_CUDA_TRY(cudaEventRecord(c->ev[3], ss));
-    if (!rc) rc = run_stage3_mark(pts.xy, pts.xy_stride, p, llp, d_nllp, nc, s3scratch, s3cap, ss, &c->launches);
-    OWM_CUDA_TRY(cudaEventRecord(c->side_join, ss));
-  }
-  // join (again, if the gather already did): nothing queued on s after this
-  // point overtakes the side stream's work, on success or failure
-  if (forked) OWM_CUDA_TRY(cudaEventRecord(c->ev[1], s));
-  if (forked) OWM_CUDA_TRY(cudaStreamWaitEvent(s, c->side_join, 0));
+    rc = build_tree(pts, n, bb, cfg.tree, &c->tree, c->scratch.ptr, tbytes, c->d_small + kStatusSlot, s, &c->launches);
   if (rc) return rc;
-  if (c->stage12_side) {
-    OWM_CUDA_TRY(cudaEventRecord(c->ev[7], s));
-  } else {
-    if (!forked) OWM_CUDA_TRY(cudaEventRecord(c->ev[1], s));
-    if (cfg.stage1_walk) {
-      rc = run_stage1(c, c->tree, p, ex, ey, win);
-    } else {
-      if (!fused) rc = classes_aggregate(cls, c->tree.view(), n, s, &c->launches);
-      if (!rc) rc = classes_finish(cls, c->tree.view(), n, p, win, s, &c->launches);
-    }
-    if (rc) return rc;
-    OWM_CUDA_TRY(cudaEventRecord(c->ev[2], s));
-    rc = stage2(s);
-    if (rc) return rc;
-    OWM_CUDA_TRY(cudaEventRecord(c->ev[3], s));
-  }
-  rc = c->stage12_side
-           ? run_stage3_query(c->tree.view(c->walk_limit, c->tuning.cell_warps), p, s3, d_ns3, s3scratch, s3cap, c->d_small + kStatusSlot, s, &c->launches)
-           : run_stage3(c->tree.view(c->walk_limit, c->tuning.cell_warps), pts.xy, pts.xy_stride, p, llp, d_nllp, nc, s3, d_ns3, s3scratch, s3cap, c->d_job,
-                        c->d_small + kStatusSlot, s, &c->launches);
+  void* s2scratch = static_cast<char*>(c->scratch.ptr) + tbytes;
+  void* s3scratch = static_cast<char*>(c->scratch.ptr) + tbytes + s2al;
+  const size_t s3cap = c->scratch.cap - tbytes - s2al;
+  OWM_CUDA_TRY(cudaEventRecord(c->ev[1], s));
+  rc = run_stage1(c, c->tree, p, ex, ey, win);
+  if (rc) return rc;
+  OWM_CUDA_TRY(cudaEventRecord(c->ev[2], s));
+  rc = bitmap2 ? run_stage2_bitmap(win, nc, n, p.overlap, llp, d_nllp, s2scratch, s2al, s, &c->launches)
+               : run_stage2(win, nc, n, p.overlap, llp, d_nllp, s2scratch, s2al, s, &c->launches);
+  if (rc) return rc;
+  OWM_CUDA_TRY(cudaEventRecord(c->ev[3], s));
+  rc = run_stage3(c->tree.view(c->walk_limit, c->tuning.cell_warps), pts.xy, pts.xy_stride, p, llp, d_nllp, nc, s3, d_ns3,
+                  s3scratch, s3cap, c->d_small + kStatusSlot, s, &c->launches);
   if (rc) return rc;
   OWM_CUDA_TRY(cudaEventRecord(c->ev[4], s));
   const int64_t room = nc + ng + 1;
@@ -314,14 +276,11 @@ int run_pipeline(owm_ctx* c, const PointsView& pts, int64_t n, const owm_bbox& b
   OWM_CUDA_TRY(cudaEventRecord(c->ev[5], s));
   OWM_CUDA_TRY(cudaStreamSynchronize(s));
   if (info) {
-    // With stages 1-2 beside the hierarchy build, stage 1 counts from the
-    // gather's end and stage 3 from the join, so the phases overlap.
     float a = 0, b = 0, d = 0, e = 0, f = 0;
-    const bool side = c->stage12_side;
     cudaEventElapsedTime(&a, c->ev[0], c->ev[1]);
-    cudaEventElapsedTime(&b, side ? c->ev[6] : c->ev[1], c->ev[2]);
+    cudaEventElapsedTime(&b, c->ev[1], c->ev[2]);
     cudaEventElapsedTime(&d, c->ev[2], c->ev[3]);
-    cudaEventElapsedTime(&e, side ? c->ev[7] : c->ev[3], c->ev[4]);
+    cudaEventElapsedTime(&e, c->ev[3], c->ev[4]);
     cudaEventElapsedTime(&f, c->ev[0], c->ev[5]);
     info->ms_tree = a;
     info->ms_stage1 = b;

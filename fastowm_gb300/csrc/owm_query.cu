@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(kQBlock) k_query_persistent(const QueryJob* __
 }
 
 // ---- stage 3: one warp per cell (owm_cellq.cuh) ---------------------------------
-template <int kW, bool kPerm>
+template <int kW>
 __global__ void __launch_bounds__(kW * 32) k_query_cells(TreeView T, const Edge* __restrict__ exs,
                                                            const Edge* __restrict__ eys, int32_t ncols,
                                                            int64_t ncells, const uint8_t* __restrict__ skip,
@@ -293,33 +293,24 @@ __global__ void __launch_bounds__(kW * 32) k_query_cells(TreeView T, const Edge*
     return;
   }
   const uint32_t r =
-      cell_min_warp<kPerm>(T, exs[cell % ncols], eys[cell / ncols], stack_all + wib * kS3Stack, status, lane);
+      cell_min_warp(T, exs[cell % ncols], eys[cell / ncols], stack_all + wib * kS3Stack, status, lane);
   if (lane == 0) out[cell] = r;
 }
 
-template <int kW, bool kPerm>
-cudaError_t launch_query_cells_as(const TreeView& t, const Edge* ex, const Edge* ey, int32_t ncols, int64_t ng,
-                                  const uint8_t* skip, uint32_t* out, uint32_t* status, cudaStream_t s) {
-  static bool configured = false;  // per template instance
-  const size_t smem = (size_t)kW * kS3Stack * sizeof(int32_t);
-  if (!configured) {
-    cudaError_t e =
-        cudaFuncSetAttribute(k_query_cells<kW, kPerm>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
-  OWM_LAUNCH("k_query_s3", s, (k_query_cells<kW, kPerm><<<(unsigned)((ng + kW - 1) / kW), kW * 32, smem, s>>>(
-      t, ex, ey, ncols, ng, skip, out, status)));
-  return cudaGetLastError();
-}
-// Trees without point arrays (t.perm set) read points through the permutation.
 template <int kW>
 cudaError_t launch_query_cells(const TreeView& t, const Edge* ex, const Edge* ey, int32_t ncols, int64_t ng,
                                const uint8_t* skip, uint32_t* out, uint32_t* status, cudaStream_t s) {
-  return t.perm ? launch_query_cells_as<kW, true>(t, ex, ey, ncols, ng, skip, out, status, s)
-                : launch_query_cells_as<kW, false>(t, ex, ey, ncols, ng, skip, out, status, s);
+  static bool configured = false;  // per template instance
+  const size_t smem = (size_t)kW * kS3Stack * sizeof(int32_t);
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(k_query_cells<kW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    configured = true;
+  }
+  OWM_LAUNCH("k_query_s3", s, (k_query_cells<kW><<<(unsigned)((ng + kW - 1) / kW), kW * 32, smem, s>>>(
+      t, ex, ey, ncols, ng, skip, out, status)));
+  return cudaGetLastError();
 }
-
 // ---- stage 2 -----------------------------------------------------------------
 __global__ void k_s2_keys(const uint32_t* __restrict__ win, int64_t n, uint32_t none_key, uint32_t* __restrict__ keys) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -646,23 +637,8 @@ size_t stage2_bitmap_scratch_bytes(int64_t npoints) {
   return 2 * align256((size_t)nw * 4) + align256((size_t)nb * 4) + align256(scan_temp_bytes(nb)) + 1024;
 }
 
-int stage2_bitmap_clear(void* scratch, size_t scratch_bytes, int64_t npoints, cudaStream_t s) {
-  if (npoints < 0 || npoints >= (int64_t)kNone) return OWM_EINVAL;
-  if (scratch_bytes < stage2_bitmap_scratch_bytes(npoints)) return OWM_ENOMEM;
-  const S2Bitmaps B = stage2_bitmap_layout(scratch, npoints);
-  OWM_CUDA_TRY(cudaMemsetAsync(B.once, 0, 2 * align256((size_t)B.nw * 4), s));  // once, then twice
-  return OWM_OK;
-}
-
-void stage2_bitmap_ptrs(void* scratch, int64_t npoints, uint32_t** once, uint32_t** twice) {
-  const S2Bitmaps B = stage2_bitmap_layout(scratch, npoints);
-  *once = B.once;
-  *twice = B.twice;
-}
-
 int run_stage2_bitmap(const uint32_t* d_win, int64_t n, int64_t npoints, double overlap, uint32_t* d_llp,
-                      uint32_t* d_count, void* scratch, size_t scratch_bytes, cudaStream_t s, int64_t* launches,
-                      bool cleared, bool marked) {
+                      uint32_t* d_count, void* scratch, size_t scratch_bytes, cudaStream_t s, int64_t* launches) {
   if (n <= 0) {
     OWM_CUDA_TRY(cudaMemsetAsync(d_count, 0, 4, s));
     return OWM_OK;
@@ -670,11 +646,9 @@ int run_stage2_bitmap(const uint32_t* d_win, int64_t n, int64_t npoints, double 
   if (npoints < 0 || npoints >= (int64_t)kNone || !(overlap > 0.0)) return OWM_EINVAL;
   if (scratch_bytes < stage2_bitmap_scratch_bytes(npoints)) return OWM_ENOMEM;
   const S2Bitmaps B = stage2_bitmap_layout(scratch, npoints);
-  if (!marked) {
-    if (!cleared) OWM_CUDA_TRY(cudaMemsetAsync(B.once, 0, 2 * align256((size_t)B.nw * 4), s));
-    OWM_LAUNCH("k_s2_mark", s, k_s2_mark<<<grid1d(n), 256, 0, s>>>(d_win, n, (uint32_t)npoints, B.once, B.twice));
-    count_launch(launches);
-  }
+  OWM_CUDA_TRY(cudaMemsetAsync(B.once, 0, 2 * align256((size_t)B.nw * 4), s));  // once, then twice
+  OWM_LAUNCH("k_s2_mark", s, k_s2_mark<<<grid1d(n), 256, 0, s>>>(d_win, n, (uint32_t)npoints, B.once, B.twice));
+  count_launch(launches);
   OWM_LAUNCH("k_s2_count", s, k_s2_count<<<(unsigned)B.nblocks, kS2Block, 0, s>>>(B.twice, B.part));
   count_launch(launches);
   OWM_CUDA_TRY(exclusive_scan_u32(B.part, B.part, B.nblocks, d_count, B.ct, B.cb, s, launches));
@@ -748,37 +722,9 @@ S3Layout stage3_layout(void* scratch, int64_t ng) {
 }
 }  // namespace
 
-int run_stage3_prepare(double ox, double oy, const owm_params& p, void* scratch, size_t scratch_bytes,
-                       cudaStream_t s, int64_t* launches) {
-  const int64_t ng = p.ngrid;
-  if (p.bsize == 0 || ng <= 0) return OWM_OK;
-  if (scratch_bytes < stage3_scratch_bytes(ng)) return OWM_ENOMEM;
-  const S3Layout L = stage3_layout(scratch, ng);
-  int rc = compute_edges(p, ox, oy, true, L.ex, L.ey, s, launches);
-  if (rc) return rc;
-  OWM_CUDA_TRY(cudaMemsetAsync(L.mark, 0, (size_t)ng, s));
-  return OWM_OK;
-}
-
-int run_stage3_mark(const double* d_xyz, int stride, const owm_params& p, const uint32_t* d_llp, const uint32_t* d_nllp,
-                    int64_t llp_cap, void* scratch, size_t scratch_bytes, cudaStream_t s, int64_t* launches) {
-  const int64_t ng = p.ngrid;
-  if (p.bsize == 0 || ng <= 0) return OWM_OK;
-  if (scratch_bytes < stage3_scratch_bytes(ng)) return OWM_ENOMEM;
-  const S3Layout L = stage3_layout(scratch, ng);
-  if (llp_cap > 0) {
-    OWM_LAUNCH("k_s3_mark", s, k_s3_mark<<<grid1d(llp_cap), 256, 0, s>>>(d_xyz, stride, d_llp, d_nllp, llp_cap, L.ex, L.ey,
-                                                                       (int32_t)p.ncols_grid, (int32_t)p.nrows_grid,
-                                                                       p.bbox.min_x, p.bbox.min_y, (double)p.bsize,
-                                                                       L.mark));
-    count_launch(launches);
-  }
-  OWM_CUDA_TRY(cudaGetLastError());
-  return OWM_OK;
-}
-
-int run_stage3_query(const TreeView& t, const owm_params& p, uint32_t* d_out, uint32_t* d_count, void* scratch,
-                     size_t scratch_bytes, uint32_t* status, cudaStream_t s, int64_t* launches) {
+int run_stage3(const TreeView& t, const double* d_xyz, int stride, const owm_params& p, const uint32_t* d_llp,
+               const uint32_t* d_nllp, int64_t llp_cap, uint32_t* d_out, uint32_t* d_count, void* scratch,
+               size_t scratch_bytes, uint32_t* status, cudaStream_t s, int64_t* launches) {
   const int64_t ng = p.ngrid;
   if (p.bsize == 0 || ng <= 0) {
     OWM_CUDA_TRY(cudaMemsetAsync(d_count, 0, 4, s));
@@ -786,6 +732,16 @@ int run_stage3_query(const TreeView& t, const owm_params& p, uint32_t* d_out, ui
   }
   if (scratch_bytes < stage3_scratch_bytes(ng)) return OWM_ENOMEM;
   const S3Layout L = stage3_layout(scratch, ng);
+  int rc = compute_edges(p, t.ox, t.oy, true, L.ex, L.ey, s, launches);
+  if (rc) return rc;
+  OWM_CUDA_TRY(cudaMemsetAsync(L.mark, 0, (size_t)ng, s));
+  if (llp_cap > 0) {
+    OWM_LAUNCH("k_s3_mark", s, k_s3_mark<<<grid1d(llp_cap), 256, 0, s>>>(d_xyz, stride, d_llp, d_nllp, llp_cap, L.ex, L.ey,
+                                                                       (int32_t)p.ncols_grid, (int32_t)p.nrows_grid,
+                                                                       p.bbox.min_x, p.bbox.min_y, (double)p.bsize,
+                                                                       L.mark));
+    count_launch(launches);
+  }
   if ((ng + 1) / 2 >= 0x7FFFFFFFll) return OWM_ERANGE;
   OWM_CUDA_TRY(t.cell_warps == 2   ? launch_query_cells<2>(t, L.ex, L.ey, (int32_t)p.ncols_grid, ng, L.mark, L.cellmin, status, s)
                : t.cell_warps == 8 ? launch_query_cells<8>(t, L.ex, L.ey, (int32_t)p.ncols_grid, ng, L.mark, L.cellmin, status, s)
@@ -803,16 +759,6 @@ int run_stage3_query(const TreeView& t, const owm_params& p, uint32_t* d_out, ui
   }
   OWM_CUDA_TRY(cudaGetLastError());
   return OWM_OK;
-}
-
-int run_stage3(const TreeView& t, const double* d_xyz, int stride, const owm_params& p, const uint32_t* d_llp,
-               const uint32_t* d_nllp, int64_t llp_cap, uint32_t* d_out, uint32_t* d_count, void* scratch,
-               size_t scratch_bytes, QueryJob* d_job_slot, uint32_t* status, cudaStream_t s, int64_t* launches) {
-  (void)d_job_slot;
-  int rc = run_stage3_prepare(t.ox, t.oy, p, scratch, scratch_bytes, s, launches);
-  if (!rc) rc = run_stage3_mark(d_xyz, stride, p, d_llp, d_nllp, llp_cap, scratch, scratch_bytes, s, launches);
-  if (rc) return rc;
-  return run_stage3_query(t, p, d_out, d_count, scratch, scratch_bytes, status, s, launches);
 }
 
 int u32_to_i64_ids(const uint32_t* in, const uint32_t* d_count, int64_t cap, int64_t* out, cudaStream_t s,

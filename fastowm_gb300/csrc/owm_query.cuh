@@ -58,17 +58,10 @@ int run_stage2(const uint32_t* d_win, int64_t n, int64_t npoints, double overlap
                uint32_t* d_count, void* scratch, size_t scratch_bytes, cudaStream_t s, int64_t* launches);
 // Same result, for overlap > 0 and ids known to lie in [0, npoints] (window
 // minima of one cloud of npoints points), by occupancy bitmaps instead of a
-// sort: one marking read of the window list, then work per 32 ids.  With
-// cleared, the two bitmaps at the start of scratch were already zeroed by
-// stage2_bitmap_clear (which may run early, on another stream).
+// sort: one marking read of the window list, then work per 32 ids.
 size_t stage2_bitmap_scratch_bytes(int64_t npoints);
-int stage2_bitmap_clear(void* scratch, size_t scratch_bytes, int64_t npoints, cudaStream_t s);
-// With marked, the bitmaps were also marked already (by the stage-1 window
-// kernel, s2_mark_id) and only the ascending emit remains.
 int run_stage2_bitmap(const uint32_t* d_win, int64_t n, int64_t npoints, double overlap, uint32_t* d_llp,
-                      uint32_t* d_count, void* scratch, size_t scratch_bytes, cudaStream_t s, int64_t* launches,
-                      bool cleared = false, bool marked = false);
-void stage2_bitmap_ptrs(void* scratch, int64_t npoints, uint32_t** once, uint32_t** twice);
+                      uint32_t* d_count, void* scratch, size_t scratch_bytes, cudaStream_t s, int64_t* launches);
 
 // Stage 2's occupancy marks of one window result v (ids 0..max_id; kNone is
 // skipped): the first occurrence sets `once`, a later one `twice`.
@@ -91,17 +84,7 @@ int run_stage2_into(const uint32_t* d_win, uint32_t* k0, uint32_t* k1, uint32_t*
 size_t stage3_scratch_bytes(int64_t ngrid);
 int run_stage3(const TreeView& t, const double* d_xyz, int stride, const owm_params& p, const uint32_t* d_llp,
                const uint32_t* d_nllp, int64_t llp_cap, uint32_t* d_out, uint32_t* d_count, void* scratch,
-               size_t scratch_bytes, QueryJob* d_job_slot, uint32_t* status, cudaStream_t s, int64_t* launches);
-// The same in three parts on one scratch layout: the cell edge tables (float
-// offsets from (ox, oy), the tree's origin) and cleared marks (need nothing
-// else), the LLP marks (need stage 2's list), then the queries and the
-// compaction (need the tree hierarchy).
-int run_stage3_prepare(double ox, double oy, const owm_params& p, void* scratch, size_t scratch_bytes,
-                       cudaStream_t s, int64_t* launches);
-int run_stage3_mark(const double* d_xyz, int stride, const owm_params& p, const uint32_t* d_llp, const uint32_t* d_nllp,
-                    int64_t llp_cap, void* scratch, size_t scratch_bytes, cudaStream_t s, int64_t* launches);
-int run_stage3_query(const TreeView& t, const owm_params& p, uint32_t* d_out, uint32_t* d_count, void* scratch,
-                     size_t scratch_bytes, uint32_t* status, cudaStream_t s, int64_t* launches);
+               size_t scratch_bytes, uint32_t* status, cudaStream_t s, int64_t* launches);
 
 // Device kernels used by the API's conversions.
 int u32_to_i64_ids(const uint32_t* in, const uint32_t* d_count, int64_t cap, int64_t* out, cudaStream_t s,

@@ -134,8 +134,8 @@ int64_t owm_ctx_launches(const owm_ctx* ctx);
 /* Device status word: bit 0 non-finite input, bit 1 a bounded tree walk or
  * bounded device wait ran out (the call returned OWM_ETIMEOUT). */
 int owm_ctx_device_status(owm_ctx* ctx, int32_t* status);
-/* Step limit of this context's bounded tree walks: the stage-1 walk
- * (owm_stage1, stage1_walk = 1) stops after `limit` node steps per window and
+/* Step limit of this context's bounded tree walks (owm_run walks the tree
+ * while one is set): the stage-1 walk (owm_stage1, owm_run) stops after `limit` node steps per window and
  * the stage-3 cell walk after `limit` rounds per cell, instead of their
  * structural bounds (which only a corrupt hierarchy can reach).  A walk that
  * stops sets bit 1 of the device status word and its call returns
@@ -276,27 +276,27 @@ typedef struct {
   uint32_t wsize, bsize;
   double overlap;
   owm_tree_cfg tree;
-  /* Stage-1 algorithm of owm_run (same result either way):
-   *  0  exact window classes over the tree's sorted points: every point is
-   *     assigned once to the sub-cell of windows that contain it, O(N);
-   *  1  warp-cooperative stackless tree walk per window with min-z pruning
-   *     (what owm_stage1 runs). */
+  /* Index and algorithm of owm_run (same result either way):
+   *  0  window grid: every point is folded once into the sub-cell of windows
+   *     and cells that contain it (count and minimum), and windows and cells
+   *     are rectangles of sub-cells, O(N); no hierarchy is built (`tree` is
+   *     checked, and the seeds do not depend on it);
+   *  1  tree build, warp-cooperative stackless tree walk per window with min-z
+   *     pruning (what owm_stage1 runs), tree walk per cell.  A context with a
+   *     walk limit (owm_ctx_set_walk_limit) takes this path too. */
   int32_t stage1_walk;
   int32_t _pad;
 } owm_run_cfg;
 
-/* Device time of the run (ms_total) and of its phases.  owm_run overlaps
- * them: with stage 1 by window classes, stages 1-2 run on a second stream
- * while the tree's hierarchy is built, so ms_stage1 counts from the end of
- * the build's gather, ms_stage3 from the end of both streams' work, and the
- * phases may add up to more than ms_total. */
+/* Device time of the run (ms_total) and of its phases; ms_tree is the index:
+ * the window grid's fold or the tree build. */
 typedef struct {
   double ms_tree, ms_stage1, ms_stage2, ms_stage3, ms_total;
   int64_t n_llp, n_stage3, n_seeds;
   owm_params params;
 } owm_run_info;
 
-/* Tree build + stages 1-3 on a device cloud; seeds = stage-3 ids followed
+/* Index + stages 1-3 on a device cloud; seeds = stage-3 ids followed
  * by the LLPs (owm_optim3.cpp:229-230).  cap >= ngrid + ncells is always
  * enough.  info may be NULL. */
 int owm_run(owm_ctx* ctx, const owm_cloud* cloud, const owm_run_cfg* cfg, int64_t* seeds,
