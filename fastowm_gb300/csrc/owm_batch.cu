@@ -1,24 +1,20 @@
 // Batched tiles: many independent clouds (own bbox, Wsize, overlap, Bsize and
-// leaf size) built and queried together with one launch per step instead of
-// one launch sequence per tile.
+// leaf size) run together with one launch per step instead of one launch
+// sequence per tile.  On the window grid (owm_grid.cuh), or, when a tile asks
+// for the tree walk:
 //
 //   * all points are sorted once on a (tile, Morton) key, so every tile's
 //     points stay in their own contiguous range;
 //   * leaves, Karras hierarchies, escape links and refits of all tiles are
 //     built by single launches that find their tile by binary search over
 //     per-tile offsets;
-//   * stage 1 by exact window classes: per-tile class tables built by two
-//     launches, every point folded into its tile's sub-cell counters inside
-//     the gather, then batched row and window reductions (a tile that
-//     asks for the tree walk switches the whole batch to the persistent walk);
-//   * stage 3 (and the stage-1 walk) is one persistent query launch: warps
-//     pull 4 x 8 window patches of any tile from one work counter, which
-//     balances uneven tiles;
-//   * stage 2 sorts all window results on a (tile, id) key;
-//   * the device part can be captured once into a CUDA graph and replayed
-//     while the tile shapes repeat.
-// Results per tile are exactly those of owm_run on that tile alone (ids are
-// 1-based within the tile).
+//   * stage 1 is one persistent query launch: warps pull 4 x 8 window patches
+//     of any tile from one work counter, which balances uneven tiles; stage 3
+//     is one warp per grid cell of any tile;
+//   * stage 2 by occupancy bitmaps, or by sorting (tile, id) keys.
+// The device part can be captured once into a CUDA graph and replayed while
+// the tile shapes repeat.  Results per tile are exactly those of owm_run on
+// that tile alone (ids are 1-based within the tile).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -27,24 +23,12 @@
 
 #include "owm_batch.cuh"
 #include "owm_cellq.cuh"
-#include "owm_classes.cuh"
 #include "owm_devutil.cuh"
+#include "owm_grid.cuh"
 
 namespace owm {
 
 namespace {
-
-// Largest t in [0, ntiles) with off[t] <= x (off has ntiles+1 entries,
-// off[0] = 0, off[ntiles] > x): the tile that owns global index x.
-template <class T>
-__device__ __forceinline__ int tile_of(const T* __restrict__ off, int ntiles, int64_t x) {
-  int lo = 0, hi = ntiles - 1;
-  while (lo < hi) {
-    int mid = (lo + hi + 1) >> 1;
-    if ((int64_t)__ldg(off + mid) <= x) lo = mid; else hi = mid - 1;
-  }
-  return lo;
-}
 
 __global__ void k_b_morton(const double* __restrict__ xyz, int64_t n, const int64_t* __restrict__ pt_off,
                            const TileMeta* __restrict__ meta, int ntiles, int mbits, uint32_t* __restrict__ keys) {
@@ -174,8 +158,7 @@ __global__ void __maxnreg__(40) k_b_gather_leaves(const double* __restrict__ xyz
                                                          int64_t total_leaves, int64_t* __restrict__ xk,
                                                          int64_t* __restrict__ yk, int64_t* __restrict__ zk,
                                                          uint32_t* __restrict__ pid, Node* __restrict__ nodes,
-                                                         uint32_t* __restrict__ status,
-                                                         const ClassArgs* __restrict__ cls) {
+                                                         uint32_t* __restrict__ status) {
   const int lane = threadIdx.x & 31;
   bool finite = true;
   for (int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < total_leaves;
@@ -187,89 +170,23 @@ __global__ void __maxnreg__(40) k_b_gather_leaves(const double* __restrict__ xyz
     const int32_t cnt = min(m.leaf, m.n - first);
     LeafAcc acc;
     acc.init();
-    for (int32_t c0 = 0; c0 < cnt; c0 += 32) {  // warp-uniform: the class fold needs whole warps
-      const int32_t lp = first + c0 + lane;
-      const bool valid = c0 + lane < cnt;
-      int64_t x = 0, y = 0, z = 0;
-      uint32_t id = 0;
-      if (valid) {
-        const int64_t gp = m.pt_off + lp;
-        const uint32_t src = __ldg(perm + gp);
-        finite &= load_point(xyz, src, x, y, z);
-        id = (uint32_t)((int64_t)src - m.pt_off + 1);
-        xk[gp] = x;
-        yk[gp] = y;
-        zk[gp] = z;
-        pid[gp] = id;
-        acc.add(x, y, z, id, (uint32_t)lp);
-      }
-      if (cls) {
-        if (!__all_sync(0xffffffffu, valid)) {  // short leaf: idle lanes borrow lane 0's point
-          const int64_t bx = __shfl_sync(0xffffffffu, x, 0), by = __shfl_sync(0xffffffffu, y, 0);
-          if (!valid) {
-            x = bx;
-            y = by;
-            z = 0;
-          }
-        }
-        cls_aggregate_warp(cls[t], valid, x, y, z, id, lane);
-      }
+    for (int32_t c0 = lane; c0 < cnt; c0 += 32) {
+      const int32_t lp = first + c0;
+      const int64_t gp = m.pt_off + lp;
+      const uint32_t src = __ldg(perm + gp);
+      int64_t x, y, z;
+      finite &= load_point(xyz, src, x, y, z);
+      const uint32_t id = (uint32_t)((int64_t)src - m.pt_off + 1);
+      xk[gp] = x;
+      yk[gp] = y;
+      zk[gp] = z;
+      pid[gp] = id;
+      acc.add(x, y, z, id, (uint32_t)lp);
     }
     acc.reduce(32);
     write_leaf_seg(nodes + m.node_off + (m.nleaves - 1) + j, acc, first, m.ox, m.oy, 32, true);
   }
   if (!finite) atomicOr(status, kStatusNonFinite);
-}
-
-// ---- stage 1 by window classes, all tiles per launch ----------------------
-// Grid y = tile.  Edge keys of the tile's window columns and rows.
-__global__ void k_bc_split(const ClassArgs* __restrict__ cls, const TileMeta* __restrict__ meta,
-                           const Edge* __restrict__ E_wx, const Edge* __restrict__ E_wy) {
-  const ClassArgs& A = cls[blockIdx.y];
-  const TileMeta& m = meta[blockIdx.y];
-  const int32_t nmax = max(A.nx, A.ny);
-  for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nmax; i += gridDim.x * blockDim.x) {
-    if (i < A.nx) {
-      const Edge e = E_wx[m.ex_off + i];
-      const_cast<int64_t*>(A.Lx)[i] = e.lo_k;
-      const_cast<int64_t*>(A.Rx)[i] = e.hi_k;
-    }
-    if (i < A.ny) {
-      const Edge e = E_wy[m.ey_off + i];
-      const_cast<int64_t*>(A.Ly)[i] = e.lo_k;
-      const_cast<int64_t*>(A.Ry)[i] = e.hi_k;
-    }
-  }
-}
-
-// Grid y = tile.  s-ranges of the windows and the class tables.
-__global__ void k_bc_prep(const ClassArgs* __restrict__ cls) {
-  const ClassArgs& A = cls[blockIdx.y];
-  const int32_t nmax = max(max(A.nx, A.ny), max(A.qx, A.qy));
-  for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nmax; i += gridDim.x * blockDim.x) {
-    if (i < A.nx) cls_range_one(A.Lx, A.Rx, A.nx, i, A.sxl + i, A.sxh + i);
-    if (i < A.ny) cls_range_one(A.Ly, A.Ry, A.ny, i, A.syl + i, A.syh + i);
-    if (i < A.qx) const_cast<ClsCell*>(A.tabx)[i] = cls_table_one(A.Lx, A.Rx, A.nx, A.kx0, A.shx, i);
-    if (i < A.qy) const_cast<ClsCell*>(A.taby)[i] = cls_table_one(A.Ly, A.Ry, A.ny, A.ky0, A.shy, i);
-  }
-}
-
-__global__ void k_bc_rows(const ClassArgs* __restrict__ cls, const int64_t* __restrict__ rows_off, int ntiles,
-                          int64_t total) {
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < total; k += (int64_t)gridDim.x * blockDim.x) {
-    const int t = tile_of(rows_off, ntiles, k);
-    cls_row_one(cls[t], k - __ldg(rows_off + t));
-  }
-}
-
-__global__ void k_bc_windows(const ClassArgs* __restrict__ cls, const TileMeta* __restrict__ meta,
-                             const int64_t* __restrict__ win_off, int ntiles, int64_t total,
-                             uint32_t* __restrict__ win) {
-  for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < total; w += (int64_t)gridDim.x * blockDim.x) {
-    const int t = tile_of(win_off, ntiles, w);
-    const int64_t off = __ldg(win_off + t);
-    win[off + cls_window_slot(cls[t], w - off)] = cls_window_one(cls[t], w - off, meta[t].thr);
-  }
 }
 
 // lk: packed leaf keys (k_b_leaf_keys), lk[m.leaf_off + i] for leaf i of tile m.
@@ -623,25 +540,55 @@ struct Plan {
   std::vector<int64_t> bm_off;
   size_t o_bm1 = 0, o_bm2 = 0, o_bmc = 0, o_bmp = 0, o_bmt = 0, o_bmoff = 0;
   std::vector<int32_t> leaf_off, node_off, int_off, ex_off, ey_off, cx_off, cy_off;
-  // stage 1 by window classes (when no tile asks for the tree walk)
-  struct ClsLayout {
-    size_t tabx, taby, Lx, Rx, Ly, Ry, sxl, sxh, syl, syh, rc, rz, ri;  // byte offsets in the misc region
-    int64_t sub_off;                                                   // first sub-cell of the tile
-  };
-  bool classes = false;
-  std::vector<ClassArgs> cls;      // per-tile geometry (pointers are set at launch)
-  std::vector<ClsLayout> clay;
-  std::vector<int64_t> rows_off;   // prefix of (window columns x sub-cell rows)
-  int64_t nsub = 0, rows_total = 0;
-  size_t cls_misc = 0;
-  int32_t cls_grid_x = 1;          // blocks per tile of the class prepare launches
-  size_t o_cls = 0, o_rowsoff = 0, o_ccount = 0, o_czid = 0, o_cmisc = 0;
   // buffer offsets (bytes) inside the batch buffer
   size_t o_xyz, o_k0, o_k1, o_v0, o_v1, o_sort, o_xk, o_yk, o_zk, o_pid, o_nodes, o_parent, o_flags, o_right,
       o_last, o_edges, o_win, o_s2k0, o_s2k1, o_s2f, o_s2p, o_s2t, o_llp, o_mark, o_cmin, o_cf, o_cp, o_ct, o_s3,
       o_meta, o_jobs1, o_jobs3, o_ptoff, o_leafoff, o_nodeoff, o_intoff, o_exoff, o_eyoff, o_cxoff, o_cyoff,
       o_winoff, o_celloff, o_cnt2, o_cnt3, o_llpoff, o_s3off, o_out, o_outoff, o_words, total;
 };
+
+// Checks a tile and derives its parameters (with its bbox).
+int tile_params(const owm_tile_desc& d, owm_params* p) {
+  if (!d.xyz || d.n <= 0 || d.n >= 0x7FFFFFFFLL) return OWM_EINVAL;
+  if (validate_tree_cfg(&d.cfg.tree) != OWM_OK || d.cfg.tree.policy != OWM_TREE_MAX_NUMBER) return OWM_EINVAL;
+  owm_bbox bb = d.bbox;
+  if (!(bb.min_x <= bb.max_x)) {
+    if (is_device_ptr(d.xyz)) return OWM_EINVAL;  // device tiles must carry their bbox
+    owm_bbox_of(d.xyz, d.n, &bb);
+  }
+  return owm_params_compute(&bb, d.n, d.cfg.wsize, d.cfg.overlap, d.cfg.bsize, p);
+}
+
+// Whether a batch runs on the window grid: no tile asks for the tree walk.
+bool on_grid(const owm_tile_desc* td, int32_t ntiles) {
+  for (int32_t t = 0; t < ntiles; ++t)
+    if (td[t].cfg.stage1_walk) return false;
+  return true;
+}
+
+// The batch's parameters and grid layout; the points, when they are copied in,
+// lie before the grid's region.
+struct GridLayout {
+  std::vector<owm_params> p;
+  std::vector<int64_t> n;
+  std::vector<GridSizes> z;
+  int64_t points = 0;
+  size_t point_bytes = 0;
+};
+int grid_layout(const owm_tile_desc* td, int32_t ntiles, GridLayout* L, GridBatch* g) {
+  L->p.resize(ntiles);
+  L->n.resize(ntiles);
+  L->z.resize(ntiles);
+  for (int32_t t = 0; t < ntiles; ++t) {
+    const int rc = tile_params(td[t], &L->p[t]);
+    if (rc) return rc;
+    L->n[t] = td[t].n;
+    L->points += td[t].n;
+  }
+  if (L->points >= 0xFFFFFFFFLL) return OWM_ERANGE;
+  L->point_bytes = ((size_t)L->points * 24 + 255) & ~(size_t)255;
+  return grid_batch_plan(L->p.data(), L->n.data(), ntiles, L->z.data(), nullptr, g);
+}
 
 int make_plan(const owm_tile_desc* td, int32_t ntiles, const BatchRun& br, Plan* P) {
   P->ntiles = ntiles;
@@ -659,27 +606,13 @@ int make_plan(const owm_tile_desc* td, int32_t ntiles, const BatchRun& br, Plan*
   // sort passes) while that leaves at least 7 bits per axis (128 x 128 cells
   // per tile); else use up to 32 bits.  Seeds do not depend on it.
   P->mbits = (24 - P->tile_bits) / 2 >= 7 ? (24 - P->tile_bits) / 2 : std::min(16, (32 - P->tile_bits) / 2);
-  P->classes = true;
-  for (int32_t t = 0; t < ntiles; ++t) P->classes &= td[t].cfg.stage1_walk == 0;
-  if (P->classes) {
-    P->cls.assign(ntiles, ClassArgs{});
-    P->clay.assign(ntiles, Plan::ClsLayout{});
-    P->rows_off.assign(ntiles + 1, 0);
-  }
-  int32_t cls_span = 1;
   int64_t maxn = 0;
   for (int32_t t = 0; t < ntiles; ++t) {
     const owm_tile_desc& d = td[t];
-    if (!d.xyz || d.n <= 0 || d.n >= 0x7FFFFFFFLL) return OWM_EINVAL;
-    if (validate_tree_cfg(&d.cfg.tree) != OWM_OK || d.cfg.tree.policy != OWM_TREE_MAX_NUMBER) return OWM_EINVAL;
-    owm_bbox bb = d.bbox;
-    if (!(bb.min_x <= bb.max_x)) {
-      if (is_device_ptr(d.xyz)) return OWM_EINVAL;  // device tiles must carry their bbox
-      owm_bbox_of(d.xyz, d.n, &bb);
-    }
     owm_params p;
-    int rc = owm_params_compute(&bb, d.n, d.cfg.wsize, d.cfg.overlap, d.cfg.bsize, &p);
+    const int rc = tile_params(d, &p);
     if (rc) return rc;
+    const owm_bbox& bb = p.bbox;
     maxn = std::max<int64_t>(maxn, d.n);
     TileMeta& m = P->meta[t];
     std::memset(&m, 0, sizeof(m));
@@ -745,45 +678,6 @@ int make_plan(const owm_tile_desc* td, int32_t ntiles, const BatchRun& br, Plan*
     P->ey += p.nrows;
     P->cx += p.bsize > 0 ? p.ncols_grid : 0;
     P->cy += p.bsize > 0 ? p.nrows_grid : 0;
-    if (P->classes) {
-      ClassArgs& a = P->cls[t];
-      std::memset(&a, 0, sizeof(a));
-      a.nx = (int32_t)p.ncols;
-      a.ny = (int32_t)p.nrows;
-      a.tx = 2 * a.nx + 1;
-      a.ty = 2 * a.ny + 1;
-      if (!cls_table_geometry(bb.min_x, bb.max_x, p.displace, &a.kx0, &a.shx, &a.qx)) a.qx = 0;
-      if (!cls_table_geometry(bb.min_y, bb.max_y, p.displace, &a.ky0, &a.shy, &a.qy)) a.qy = 0;
-      Plan::ClsLayout& l = P->clay[t];
-      auto piece = [&](size_t bytes) {
-        size_t r = P->cls_misc;
-        P->cls_misc += (bytes + 31) & ~(size_t)31;  // 32-byte table cells
-        return r;
-      };
-      const size_t nx = (size_t)a.nx, ny = (size_t)a.ny, rows = nx * (size_t)a.ty;
-      l.tabx = piece((size_t)a.qx * sizeof(ClsCell));
-      l.taby = piece((size_t)a.qy * sizeof(ClsCell));
-      l.Lx = piece(nx * 8);
-      l.Rx = piece(nx * 8);
-      l.Ly = piece(ny * 8);
-      l.Ry = piece(ny * 8);
-      l.sxl = piece(nx * 4);
-      l.sxh = piece(nx * 4);
-      l.syl = piece(ny * 4);
-      l.syh = piece(ny * 4);
-      l.rc = piece(rows * 4);
-      l.rz = piece(rows * 8);
-      l.ri = piece(rows * 4);
-      l.sub_off = P->nsub;
-      P->nsub += (int64_t)a.tx * a.ty;
-      P->rows_off[t] = P->rows_total;
-      P->rows_total += (int64_t)rows;
-      cls_span = std::max(cls_span, std::max(std::max(a.nx, a.ny), std::max(a.qx, a.qy)));
-    }
-  }
-  if (P->classes) {
-    P->rows_off[ntiles] = P->rows_total;
-    P->cls_grid_x = std::min(64, (cls_span + 255) / 256);
   }
   P->pt_off[ntiles] = P->npts;
   P->bm_off[ntiles] = P->bm_words;
@@ -866,13 +760,6 @@ int make_plan(const owm_tile_desc* td, int32_t ntiles, const BatchRun& br, Plan*
   P->o_out = take((size_t)(NW + NC + 1) * 8);
   P->o_outoff = take((size_t)T1 * 8);
   P->o_words = take(256);
-  if (P->classes) {
-    P->o_cls = take((size_t)ntiles * sizeof(ClassArgs));
-    P->o_rowsoff = take((size_t)T1 * 8);
-    P->o_ccount = take((size_t)std::max<int64_t>(P->nsub, 1) * 4);
-    P->o_czid = take((size_t)std::max<int64_t>(P->nsub, 1) * 16);
-    P->o_cmisc = take(std::max<size_t>(P->cls_misc, 16));
-  }
   P->total = o;
   return OWM_OK;
 }
@@ -889,9 +776,6 @@ int BatchRun::init(int dev, cudaStream_t s) {
     own_stream = true;
   }
   OWM_CUDA_TRY(cudaEventCreateWithFlags(&done, cudaEventDisableTiming));
-  OWM_CUDA_TRY(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
-  for (cudaEvent_t* e : {&ev_fork, &ev_cls, &ev_gather, &ev_join})
-    OWM_CUDA_TRY(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
   return OWM_OK;
 }
 
@@ -909,15 +793,6 @@ void BatchRun::destroy() {
   stage_cap = 0;
   if (done) cudaEventDestroy(done);
   done = nullptr;
-  if (side) {
-    cudaStreamSynchronize(side);
-    cudaStreamDestroy(side);
-  }
-  side = nullptr;
-  for (cudaEvent_t* e : {&ev_fork, &ev_cls, &ev_gather, &ev_join}) {
-    if (*e) cudaEventDestroy(*e);
-    *e = nullptr;
-  }
   if (own_stream && stream) cudaStreamDestroy(stream);
   stream = nullptr;
   cudaGetLastError();
@@ -930,44 +805,141 @@ int BatchRun::leaf_for(int64_t n, int32_t requested) const {
 }
 
 size_t BatchRun::estimate_bytes(const owm_tile_desc* t, int32_t ntiles) {
+  if (on_grid(t, ntiles)) {
+    GridLayout L;
+    GridBatch g;
+    const int rc = grid_layout(t, ntiles, &L, &g);
+    // too many sub-cells to number: more than any budget, not a bad request
+    return rc == OWM_OK ? L.point_bytes + g.bytes : rc == OWM_ERANGE ? (size_t)-2 : (size_t)-1;
+  }
   BatchRun tmp;
   Plan P;
   if (make_plan(t, ntiles, tmp, &P) != OWM_OK) return (size_t)-1;
   return P.total;
 }
 
-int BatchRun::launch(const owm_tile_desc* td, int32_t ntiles) {
-  if (!td || ntiles <= 0) return OWM_EINVAL;
-  OWM_CUDA_TRY(cudaSetDevice(device));
-  Plan P;
-  int rc = make_plan(td, ntiles, *this, &P);
-  if (rc) return rc;
-  bytes_needed = P.total;
-  if (P.total > mem.cap && graph) {  // buffers move: the captured graph is stale
+// Room for a batch: device memory (a captured graph is stale once it moves),
+// the pinned offsets and pinned staging for the per-batch tables (a copy from
+// pageable memory would first wait for this stream's queued point copies,
+// holding the caller, the server's worker, for the whole transfer).
+int BatchRun::room(size_t device_bytes, size_t stage_bytes, int32_t ntiles_) {
+  bytes_needed = device_bytes;
+  if (device_bytes > mem.cap && graph) {
     cudaGraphExecDestroy(graph);
     graph = nullptr;
     graph_sig.clear();
   }
-  rc = mem.reserve(P.total, stream);
+  const int rc = mem.reserve(device_bytes, stream);
   if (rc) return rc;
-  if (cap_tiles < ntiles + 1) {
+  if (cap_tiles < ntiles_ + 1) {
     if (h_off) cudaFreeHost(h_off);
     h_off = nullptr;
-    OWM_CUDA_TRY(cudaMallocHost(&h_off, (size_t)(ntiles + 2) * 8));  // + the status word
-    cap_tiles = ntiles + 1;
+    cap_tiles = 0;
+    OWM_CUDA_TRY(cudaMallocHost(&h_off, (size_t)(ntiles_ + 2) * 8));  // + the status word
+    cap_tiles = ntiles_ + 1;
   }
-  // Per-batch tables go through pinned staging: a copy from pageable memory
-  // would first wait for this stream's queued point copies, holding the
-  // caller (the server's worker) for the whole transfer.
-  const size_t T1 = (size_t)ntiles + 1;
-  const size_t stage_need = 20 * 16 + (size_t)ntiles * (sizeof(TileMeta) + 2 * sizeof(QueryJob) + sizeof(ClassArgs)) +
-                            T1 * (8 * 5 + 4 * 7);
-  if (stage_cap < stage_need) {
+  if (stage_cap < stage_bytes) {
     if (h_stage) cudaFreeHost(h_stage);
     h_stage = nullptr;
-    OWM_CUDA_TRY(cudaMallocHost(&h_stage, stage_need));
-    stage_cap = stage_need;
+    stage_cap = 0;
+    OWM_CUDA_TRY(cudaMallocHost(&h_stage, stage_bytes));
+    stage_cap = stage_bytes;
   }
+  ntiles = ntiles_;
+  return OWM_OK;
+}
+
+// Replays the graph captured under this signature, else runs enqueue(stream)
+// -- with graphs on, into a new graph that is then launched.
+template <class Enqueue>
+int BatchRun::run_or_replay(const std::string& sig, Enqueue enqueue) {
+  if (use_graphs && graph && sig == graph_sig) {
+    OWM_CUDA_TRY(cudaGraphLaunch(graph, stream));
+    count_launch(&launches);
+    return OWM_OK;
+  }
+  if (!use_graphs) return enqueue();
+  ProfScope no_prof(nullptr);
+  OWM_CUDA_TRY(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+  const int rc = enqueue();
+  cudaGraph_t g = nullptr;
+  cudaError_t e = cudaStreamEndCapture(stream, &g);
+  if (rc == OWM_OK && e == cudaSuccess) {
+    if (graph) cudaGraphExecDestroy(graph);
+    graph = nullptr;
+    graph_sig.clear();
+    e = cudaGraphInstantiate(&graph, g, 0);
+    if (e == cudaSuccess) {
+      graph_sig = sig;
+      e = cudaGraphLaunch(graph, stream);
+      count_launch(&launches);
+    }
+  }
+  if (g) cudaGraphDestroy(g);
+  if (e != cudaSuccess) {
+    set_last_cuda_error(e, "batch graph", __FILE__, __LINE__);
+    return OWM_ECUDA;
+  }
+  return rc;
+}
+
+int BatchRun::launch(const owm_tile_desc* td, int32_t n) {
+  if (!td || n <= 0) return OWM_EINVAL;
+  OWM_CUDA_TRY(cudaSetDevice(device));
+  const int rc = on_grid(td, n) ? launch_grid(td, n) : launch_walk(td, n);
+  if (rc) return rc;
+  OWM_CUDA_TRY(cudaEventRecord(done, stream));
+  return OWM_OK;
+}
+
+namespace {
+// Whether the tiles already lie back to back in one buffer of this device.
+bool back_to_back(const owm_tile_desc* td, int32_t ntiles, int device) {
+  if (!device_ptr_on(td[0].xyz, device)) return false;
+  for (int32_t t = 1; t < ntiles; ++t)
+    if (td[t].xyz != td[t - 1].xyz + 3 * td[t - 1].n) return false;
+  return true;
+}
+}  // namespace
+
+int BatchRun::launch_grid(const owm_tile_desc* td, int32_t nt) {
+  GridLayout L;
+  GridBatch g;
+  int rc = grid_layout(td, nt, &L, &g);
+  if (!rc) rc = room(L.point_bytes + g.bytes, g.table_bytes, nt);
+  if (!rc) rc = grid_batch_plan(L.p.data(), L.n.data(), nt, L.z.data(), static_cast<char*>(mem.ptr) + L.point_bytes, &g);
+  if (rc) return rc;
+  const bool in_place = back_to_back(td, nt, device);
+  std::vector<const double*> rec(nt);
+  double* at = static_cast<double*>(mem.ptr);
+  for (int32_t t = 0; t < nt; ++t) {
+    rec[t] = in_place ? td[t].xyz : at;
+    if (!in_place) OWM_CUDA_TRY(cudaMemcpyAsync(at, td[t].xyz, (size_t)td[t].n * 24, cudaMemcpyDefault, stream));
+    at += 3 * td[t].n;
+  }
+  grid_batch_tables(L.p.data(), L.n.data(), L.z.data(), rec.data(), g, h_stage);
+  OWM_CUDA_TRY(cudaMemcpyAsync(g.jobs, h_stage, g.table_bytes, cudaMemcpyHostToDevice, stream));
+  d_out = g.out;
+  // what the launches depend on: sizes and addresses (the jobs are read from
+  // the tables)
+  std::string sig;
+  if (use_graphs) sig.assign(reinterpret_cast<const char*>(&g), sizeof(g));
+  return run_or_replay(sig, [&]() -> int {
+    const int r = grid_batch_run(g, stream, &launches);
+    if (r) return r;
+    OWM_CUDA_TRY(cudaMemcpyAsync(h_off, g.out_off, ((size_t)nt + 1) * 8, cudaMemcpyDeviceToHost, stream));
+    OWM_CUDA_TRY(cudaMemcpyAsync(h_off + nt + 1, g.words, 4, cudaMemcpyDeviceToHost, stream));
+    return OWM_OK;
+  });
+}
+
+int BatchRun::launch_walk(const owm_tile_desc* td, int32_t ntiles) {
+  Plan P;
+  int rc = make_plan(td, ntiles, *this, &P);
+  if (rc) return rc;
+  const size_t T1 = (size_t)ntiles + 1;
+  rc = room(P.total, 20 * 16 + (size_t)ntiles * (sizeof(TileMeta) + 2 * sizeof(QueryJob)) + T1 * (8 * 5 + 4 * 7), ntiles);
+  if (rc) return rc;
   size_t stage_off = 0;
   auto stage_copy = [&](void* dst, const void* src, size_t bytes) -> cudaError_t {
     char* h = h_stage + stage_off;
@@ -975,28 +947,15 @@ int BatchRun::launch(const owm_tile_desc* td, int32_t ntiles) {
     std::memcpy(h, src, bytes);
     return cudaMemcpyAsync(dst, h, bytes, cudaMemcpyHostToDevice, stream);
   };
-  tiles.clear();
   char* B = static_cast<char*>(mem.ptr);
   auto at = [&](size_t off) { return B + off; };
   double* xyz = (double*)at(P.o_xyz);
   const int64_t N = P.npts;
   // tiles already back to back in one device buffer are used in place
-  // (on this device: the kernels read them directly)
-  bool in_place = device_ptr_on(td[0].xyz, device);
-  for (int32_t t = 1; t < ntiles && in_place; ++t) in_place = td[t].xyz == td[0].xyz + 3 * P.pt_off[t];
+  const bool in_place = back_to_back(td, ntiles, device);
   if (in_place) xyz = const_cast<double*>(td[0].xyz);
-  // points in (host or device sources)
-  for (int32_t t = 0; t < ntiles; ++t) {
-    if (!in_place)
-      OWM_CUDA_TRY(cudaMemcpyAsync(xyz + 3 * P.pt_off[t], td[t].xyz, (size_t)td[t].n * 24, cudaMemcpyDefault, stream));
-    TileHost th;
-    th.xyz = td[t].xyz;
-    owm_bbox bb = td[t].bbox;
-    if (!(bb.min_x <= bb.max_x)) owm_bbox_of(td[t].xyz, td[t].n, &bb);
-    owm_params_compute(&bb, td[t].n, td[t].cfg.wsize, td[t].cfg.overlap, td[t].cfg.bsize, &th.p);
-    th.tree = td[t].cfg.tree;
-    tiles.push_back(th);
-  }
+  for (int32_t t = 0; t < ntiles && !in_place; ++t)
+    OWM_CUDA_TRY(cudaMemcpyAsync(xyz + 3 * P.pt_off[t], td[t].xyz, (size_t)td[t].n * 24, cudaMemcpyDefault, stream));
   TileMeta* d_meta = (TileMeta*)at(P.o_meta);
   int64_t* d_ptoff = (int64_t*)at(P.o_ptoff);
   int32_t* d_leafoff = (int32_t*)at(P.o_leafoff);
@@ -1086,40 +1045,9 @@ int BatchRun::launch(const owm_tile_desc* td, int32_t ntiles) {
   QueryJob* d_j3 = (QueryJob*)at(P.o_jobs3);
   OWM_CUDA_TRY(stage_copy(d_j1, j1.data(), (size_t)ntiles * sizeof(QueryJob)));
   OWM_CUDA_TRY(stage_copy(d_j3, j3.data(), (size_t)ntiles * sizeof(QueryJob)));
-  ClassArgs* d_cls = nullptr;
-  int64_t* d_rowsoff = nullptr;
-  if (P.classes) {
-    std::vector<ClassArgs> A(P.cls);
-    char* misc = at(P.o_cmisc);
-    for (int32_t t = 0; t < ntiles; ++t) {
-      const Plan::ClsLayout& l = P.clay[t];
-      ClassArgs& a = A[t];
-      a.tabx = reinterpret_cast<const ClsCell*>(misc + l.tabx);
-      a.taby = reinterpret_cast<const ClsCell*>(misc + l.taby);
-      a.Lx = reinterpret_cast<const int64_t*>(misc + l.Lx);
-      a.Rx = reinterpret_cast<const int64_t*>(misc + l.Rx);
-      a.Ly = reinterpret_cast<const int64_t*>(misc + l.Ly);
-      a.Ry = reinterpret_cast<const int64_t*>(misc + l.Ry);
-      a.sxl = reinterpret_cast<int32_t*>(misc + l.sxl);
-      a.sxh = reinterpret_cast<int32_t*>(misc + l.sxh);
-      a.syl = reinterpret_cast<int32_t*>(misc + l.syl);
-      a.syh = reinterpret_cast<int32_t*>(misc + l.syh);
-      a.rc = reinterpret_cast<uint32_t*>(misc + l.rc);
-      a.rz = reinterpret_cast<unsigned long long*>(misc + l.rz);
-      a.ri = reinterpret_cast<uint32_t*>(misc + l.ri);
-      a.count = reinterpret_cast<uint32_t*>(at(P.o_ccount)) + l.sub_off;
-      a.zid = reinterpret_cast<ulonglong2*>(at(P.o_czid)) + l.sub_off;
-    }
-    d_cls = reinterpret_cast<ClassArgs*>(at(P.o_cls));
-    d_rowsoff = reinterpret_cast<int64_t*>(at(P.o_rowsoff));
-    OWM_CUDA_TRY(stage_copy(d_cls, A.data(), (size_t)ntiles * sizeof(ClassArgs)));
-    OWM_CUDA_TRY(stage_copy(d_rowsoff, P.rows_off.data(), T1 * 8));
-  }
-
   int64_t* d_out = (int64_t*)at(P.o_out);
   int64_t* d_outoff = (int64_t*)at(P.o_outoff);
   this->d_out = d_out;
-  this->d_out_off = d_outoff;
 
   // ---- device work (graph-capturable: no host sync, fixed shapes) ----
   std::string sig;
@@ -1128,18 +1056,10 @@ int BatchRun::launch(const owm_tile_desc* td, int32_t ntiles) {
     sig.append(reinterpret_cast<const char*>(&mem.ptr), sizeof(void*));
     sig.append(reinterpret_cast<const char*>(&xyz), sizeof(void*));
     sig.append(reinterpret_cast<const char*>(&P.total), sizeof(P.total));
-    // the class regions' layout (table sizes follow each tile's bbox, not only its meta)
-    if (P.classes) sig.append(reinterpret_cast<const char*>(P.cls.data()), P.cls.size() * sizeof(ClassArgs));
-    sig.push_back(P.classes ? 'c' : 'w');
+    sig.push_back('w');
     sig.append(reinterpret_cast<const char*>(&tuning), sizeof(tuning));  // launch shapes
   }
-  if (use_graphs && graph && sig == graph_sig) {
-    OWM_CUDA_TRY(cudaGraphLaunch(graph, stream));
-    count_launch(&launches);
-  } else {
-    bool capture = use_graphs;
-    ProfScope no_prof(capture ? nullptr : tls_profiler());
-    if (capture) OWM_CUDA_TRY(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+  return run_or_replay(sig, [&]() -> int {
     cudaStream_t s = stream;
     int64_t* L = &launches;
     uint32_t* k0 = (uint32_t*)at(P.o_k0);
@@ -1157,52 +1077,26 @@ int BatchRun::launch(const owm_tile_desc* td, int32_t ntiles) {
     uint32_t* llp = (uint32_t*)at(P.o_llp);
     uint32_t* s3 = (uint32_t*)at(P.o_s3);
     int rc2 = OWM_OK;
-    // side-stream schedule (stage 1 by classes): ss forks from s, prepares the
-    // tables while s sorts, and finishes stages 1-2 and the LLP marks while s
-    // builds the hierarchies; without classes everything runs on s
-    const bool two = P.classes && side != nullptr;
-    cudaStream_t ss = two ? side : s;
-    bool forked = false;
     const int64_t NW = P.nwin;
     const int64_t NC = P.ncell;
     do {
       if (cudaMemsetAsync(words, 0, 256, s) != cudaSuccess) { rc2 = OWM_ECUDA; break; }
-      if (two) {
-        if (cudaEventRecord(ev_fork, s) != cudaSuccess || cudaStreamWaitEvent(ss, ev_fork, 0) != cudaSuccess) {
-          rc2 = OWM_ECUDA;
-          break;
-        }
-        forked = true;
-      }
-      // edge tables (before the gather: the class fold needs the window edges)
-      if (P.ex) OWM_LAUNCH("k_b_edges", ss, k_b_edges<<<(unsigned)((P.ex + 127) / 128), 128, 0, ss>>>(0, 0, d_meta, d_exoff, ntiles, P.ex, E_wx));
-      if (P.ey) OWM_LAUNCH("k_b_edges", ss, k_b_edges<<<(unsigned)((P.ey + 127) / 128), 128, 0, ss>>>(0, 1, d_meta, d_eyoff, ntiles, P.ey, E_wy));
-      if (P.cx) OWM_LAUNCH("k_b_edges", ss, k_b_edges<<<(unsigned)((P.cx + 127) / 128), 128, 0, ss>>>(1, 0, d_meta, d_cxoff, ntiles, P.cx, E_cx));
-      if (P.cy) OWM_LAUNCH("k_b_edges", ss, k_b_edges<<<(unsigned)((P.cy + 127) / 128), 128, 0, ss>>>(1, 1, d_meta, d_cyoff, ntiles, P.cy, E_cy));
+      if (P.ex) OWM_LAUNCH("k_b_edges", s, k_b_edges<<<(unsigned)((P.ex + 127) / 128), 128, 0, s>>>(0, 0, d_meta, d_exoff, ntiles, P.ex, E_wx));
+      if (P.ey) OWM_LAUNCH("k_b_edges", s, k_b_edges<<<(unsigned)((P.ey + 127) / 128), 128, 0, s>>>(0, 1, d_meta, d_eyoff, ntiles, P.ey, E_wy));
+      if (P.cx) OWM_LAUNCH("k_b_edges", s, k_b_edges<<<(unsigned)((P.cx + 127) / 128), 128, 0, s>>>(1, 0, d_meta, d_cxoff, ntiles, P.cx, E_cx));
+      if (P.cy) OWM_LAUNCH("k_b_edges", s, k_b_edges<<<(unsigned)((P.cy + 127) / 128), 128, 0, s>>>(1, 1, d_meta, d_cyoff, ntiles, P.cy, E_cy));
       count_launch(L, (P.ex > 0) + (P.ey > 0) + (P.cx > 0) + (P.cy > 0));
-      if (P.classes) {
-        const dim3 gp((unsigned)P.cls_grid_x, (unsigned)ntiles);
-        OWM_LAUNCH("k_bc_split", ss, k_bc_split<<<gp, 256, 0, ss>>>(d_cls, d_meta, E_wx, E_wy));
-        OWM_LAUNCH("k_bc_prep", ss, k_bc_prep<<<gp, 256, 0, ss>>>(d_cls));
-        count_launch(L, 2);
-        if (cudaMemsetAsync(at(P.o_ccount), 0, (size_t)P.nsub * 4, ss) != cudaSuccess ||
-            cudaMemsetAsync(at(P.o_czid), 0xFF, (size_t)P.nsub * 16, ss) != cudaSuccess) {
-          rc2 = OWM_ECUDA;
-          break;
-        }
-      }
       // stage 2/3 buffers cleared ahead of time
-      if (cudaMemsetAsync(cnt2, 0, T1 * 4, ss) != cudaSuccess || cudaMemsetAsync(cnt3, 0, T1 * 4, ss) != cudaSuccess) {
+      if (cudaMemsetAsync(cnt2, 0, T1 * 4, s) != cudaSuccess || cudaMemsetAsync(cnt3, 0, T1 * 4, s) != cudaSuccess) {
         rc2 = OWM_ECUDA;
         break;
       }
       if (NW > 0 && P.s2_bitmap &&
-          cudaMemsetAsync(at(P.o_bm1), 0, (size_t)(P.o_bm2 - P.o_bm1) + (size_t)P.bm_words * 4, ss) != cudaSuccess) {
+          cudaMemsetAsync(at(P.o_bm1), 0, (size_t)(P.o_bm2 - P.o_bm1) + (size_t)P.bm_words * 4, s) != cudaSuccess) {
         rc2 = OWM_ECUDA;
         break;
       }
-      if (NC > 0 && cudaMemsetAsync(mark, 0, (size_t)NC, ss) != cudaSuccess) { rc2 = OWM_ECUDA; break; }
-      if (two && cudaEventRecord(ev_cls, ss) != cudaSuccess) { rc2 = OWM_ECUDA; break; }
+      if (NC > 0 && cudaMemsetAsync(mark, 0, (size_t)NC, s) != cudaSuccess) { rc2 = OWM_ECUDA; break; }
 
       const int key_bits = P.tile_bits + 2 * P.mbits;
       const RadixSortPlan sp = radix_sort_plan(N);
@@ -1219,32 +1113,15 @@ int BatchRun::launch(const owm_tile_desc* td, int32_t ntiles) {
                      sp.parts > 0) != cudaSuccess) { rc2 = OWM_ECUDA; break; }
       const uint32_t* mk = alt ? k1 : k0;
       const uint32_t* perm = alt ? v1 : v0;
-      if (two && cudaStreamWaitEvent(s, ev_cls, 0) != cudaSuccess) { rc2 = OWM_ECUDA; break; }
       {
         // one warp per leaf: resident warps then work on neighbouring leaves
         const int gb = tuning.gather_block;
         int64_t blocks = std::min<int64_t>((P.nleaves * 32 + gb - 1) / gb, (int64_t)152 * 1024 * 256 / gb);
         OWM_LAUNCH("k_b_gather_leaves", s, k_b_gather_leaves<<<(unsigned)std::max<int64_t>(blocks, 1), gb, 0, s>>>(
-            xyz, perm, d_meta, d_leafoff, ntiles, P.nleaves, xk, yk, zk, pid, nodes, words, d_cls));
+            xyz, perm, d_meta, d_leafoff, ntiles, P.nleaves, xk, yk, zk, pid, nodes, words));
         count_launch(L);
       }
-      if (two && (cudaEventRecord(ev_gather, s) != cudaSuccess || cudaStreamWaitEvent(ss, ev_gather, 0) != cudaSuccess)) {
-        rc2 = OWM_ECUDA;
-        break;
-      }
-      // stage 1: window classes (rows, windows) on ss, or the persistent walk
-      // (on s, after the hierarchies, below)
-      if (P.classes) {
-        if (P.rows_total > 0) {
-          OWM_LAUNCH("k_bc_rows", ss, k_bc_rows<<<gsz(P.rows_total), 256, 0, ss>>>(d_cls, d_rowsoff, ntiles, P.rows_total));
-          count_launch(L);
-        }
-        if (NW > 0) {
-          OWM_LAUNCH("k_bc_windows", ss, k_bc_windows<<<gsz(NW), 256, 0, ss>>>(d_cls, d_meta, d_winoff, ntiles, NW, win));
-          count_launch(L);
-        }
-      }
-      // hierarchies on s
+      // hierarchies
       if (P.ninternal > 0) {
         uint32_t* lk = alt ? k0 : k1;  // the sort's other key buffer is free now
         OWM_LAUNCH("k_b_leaf_keys", s, k_b_leaf_keys<<<(unsigned)((P.nleaves + 255) / 256), 256, 0, s>>>(
@@ -1256,11 +1133,11 @@ int BatchRun::launch(const owm_tile_desc* td, int32_t ntiles) {
       OWM_LAUNCH("k_b_refit", s, k_b_refit<<<(unsigned)((P.nleaves + 255) / 256), 256, 0, s>>>(
           nodes, parent, flags, right_of, last_of, d_meta, d_leafoff, ntiles, P.nleaves));
       count_launch(L);
-      if (!P.classes && launch_query_persistent(d_j1, ntiles, w1, qnext, 152 * 16, s, L, "k_query_s1_batch")) {
+      if (launch_query_persistent(d_j1, ntiles, w1, qnext, 152 * 16, s, L, "k_query_s1_batch")) {
         rc2 = OWM_ECUDA;
         break;
       }
-      // stage 2 on (tile, id) keys, on ss
+      // stage 2 on (tile, id) keys
       const uint32_t none = (P.idbits >= 32) ? 0xFFFFFFFFu : ((1u << P.idbits) - 1u);
       uint32_t* s2k0 = (uint32_t*)at(P.o_s2k0);
       uint32_t* s2k1 = (uint32_t*)at(P.o_s2k1);
@@ -1273,45 +1150,38 @@ int BatchRun::launch(const owm_tile_desc* td, int32_t ntiles) {
         uint32_t* bm2 = (uint32_t*)at(P.o_bm2);
         uint32_t* bmc = (uint32_t*)at(P.o_bmc);
         uint32_t* bmp = (uint32_t*)at(P.o_bmp);
-        OWM_LAUNCH("k_b_s2_mark", ss, k_b_s2_mark<<<gsz(NW), 256, 0, ss>>>(win, NW, d_winoff, ntiles, d_meta, bm1, bm2));
-        OWM_LAUNCH("k_b_s2_popc", ss, k_b_s2_popc<<<gsz(BW), 256, 0, ss>>>(bm2, BW, bmc));
+        OWM_LAUNCH("k_b_s2_mark", s, k_b_s2_mark<<<gsz(NW), 256, 0, s>>>(win, NW, d_winoff, ntiles, d_meta, bm1, bm2));
+        OWM_LAUNCH("k_b_s2_popc", s, k_b_s2_popc<<<gsz(BW), 256, 0, s>>>(bm2, BW, bmc));
         count_launch(L, 2);
-        if (exclusive_scan_u32(bmc, bmp, BW, words + 1, at(P.o_bmt), scan_temp_bytes(BW) + 256, ss, L) != cudaSuccess) {
+        if (exclusive_scan_u32(bmc, bmp, BW, words + 1, at(P.o_bmt), scan_temp_bytes(BW) + 256, s, L) != cudaSuccess) {
           rc2 = OWM_ECUDA;
           break;
         }
-        OWM_LAUNCH("k_b_s2_emit", ss, k_b_s2_emit<<<gsz(BW), 256, 0, ss>>>(bm2, bmp, BW, d_bmoff, ntiles, P.idbits, llp));
-        OWM_LAUNCH("k_b_s2_tilecount", ss, k_b_s2_tilecount<<<(ntiles + 255) / 256, 256, 0, ss>>>(bmp, d_bmoff, ntiles, BW,
+        OWM_LAUNCH("k_b_s2_emit", s, k_b_s2_emit<<<gsz(BW), 256, 0, s>>>(bm2, bmp, BW, d_bmoff, ntiles, P.idbits, llp));
+        OWM_LAUNCH("k_b_s2_tilecount", s, k_b_s2_tilecount<<<(ntiles + 255) / 256, 256, 0, s>>>(bmp, d_bmoff, ntiles, BW,
                                                                                                words + 1, cnt2));
         count_launch(L, 2);
       } else if (NW > 0) {
-        OWM_LAUNCH("k_b_s2_keys", ss, k_b_s2_keys<<<gsz(NW), 256, 0, ss>>>(win, NW, d_winoff, ntiles, P.idbits, none, s2k0));
+        OWM_LAUNCH("k_b_s2_keys", s, k_b_s2_keys<<<gsz(NW), 256, 0, s>>>(win, NW, d_winoff, ntiles, P.idbits, none, s2k0));
         count_launch(L);
         bool a2 = false;
         size_t sb = radix_sort_temp_bytes(NW);
-        if (radix_sort(s2k0, nullptr, s2k1, nullptr, NW, P.tile_bits + P.idbits, false, s2t, sb, ss, &a2, L) !=
+        if (radix_sort(s2k0, nullptr, s2k1, nullptr, NW, P.tile_bits + P.idbits, false, s2t, sb, s, &a2, L) !=
             cudaSuccess) { rc2 = OWM_ECUDA; break; }
         const uint32_t* sk = a2 ? s2k1 : s2k0;
-        OWM_LAUNCH("k_b_s2_flags", ss, k_b_s2_flags<<<gsz(NW), 256, 0, ss>>>(sk, NW, P.idbits, none, d_meta, s2f, cnt2));
+        OWM_LAUNCH("k_b_s2_flags", s, k_b_s2_flags<<<gsz(NW), 256, 0, s>>>(sk, NW, P.idbits, none, d_meta, s2f, cnt2));
         count_launch(L);
         if (exclusive_scan_u32(s2f, s2p, NW, words + 1, s2t + a256(sb), scan_temp_bytes(std::max<int64_t>(NW, P.ncell)) + 256,
-                               ss, L) != cudaSuccess) { rc2 = OWM_ECUDA; break; }
-        OWM_LAUNCH("k_b_compact", ss, k_b_compact<<<gsz(NW), 256, 0, ss>>>(sk, s2f, s2p, NW, llp));
+                               s, L) != cudaSuccess) { rc2 = OWM_ECUDA; break; }
+        OWM_LAUNCH("k_b_compact", s, k_b_compact<<<gsz(NW), 256, 0, s>>>(sk, s2f, s2p, NW, llp));
         count_launch(L);
       }
-      if (exclusive_scan_u32(cnt2, llp_off, ntiles + 1, nullptr, s2t, scan_temp_bytes(ntiles + 1) + 256, ss, L) !=
+      if (exclusive_scan_u32(cnt2, llp_off, ntiles + 1, nullptr, s2t, scan_temp_bytes(ntiles + 1) + 256, s, L) !=
           cudaSuccess) { rc2 = OWM_ECUDA; break; }
-      // stage 3: LLP marks on ss; queries on s once both streams are done
+      // stage 3: LLP marks, queries
       if (NC > 0 && NW > 0) {
-        OWM_LAUNCH("k_b_s3_mark", ss, k_b_s3_mark<<<gsz(NW), 256, 0, ss>>>(xyz, llp, words + 1, NW, P.idbits, d_meta, E_cx, E_cy, mark));
+        OWM_LAUNCH("k_b_s3_mark", s, k_b_s3_mark<<<gsz(NW), 256, 0, s>>>(xyz, llp, words + 1, NW, P.idbits, d_meta, E_cx, E_cy, mark));
         count_launch(L);
-      }
-      if (two) {
-        if (cudaEventRecord(ev_join, ss) != cudaSuccess || cudaStreamWaitEvent(s, ev_join, 0) != cudaSuccess) {
-          rc2 = OWM_ECUDA;
-          break;
-        }
-        forked = false;
       }
       if (NC > 0) {
         if ((NC + 1) / 2 >= 0x7FFFFFFFll) { rc2 = OWM_ERANGE; break; }
@@ -1338,33 +1208,8 @@ int BatchRun::launch(const owm_tile_desc* td, int32_t ntiles) {
       if (cudaMemcpyAsync(h_off, d_outoff, T1 * 8, cudaMemcpyDeviceToHost, s) != cudaSuccess) { rc2 = OWM_ECUDA; break; }
       if (cudaMemcpyAsync(h_off + T1, words, 4, cudaMemcpyDeviceToHost, s) != cudaSuccess) { rc2 = OWM_ECUDA; break; }
     } while (false);
-    if (forked) {  // an error left the side stream forked: join it (a capture must end joined)
-      cudaEventRecord(ev_join, ss);
-      cudaStreamWaitEvent(s, ev_join, 0);
-    }
-    if (capture) {
-      cudaGraph_t g = nullptr;
-      cudaError_t e = cudaStreamEndCapture(stream, &g);
-      if (rc2 == OWM_OK && e == cudaSuccess) {
-        if (graph) cudaGraphExecDestroy(graph);
-        graph = nullptr;
-        e = cudaGraphInstantiate(&graph, g, 0);
-        if (e == cudaSuccess) {
-          graph_sig = sig;
-          e = cudaGraphLaunch(graph, stream);
-          count_launch(&launches);
-        }
-      }
-      if (g) cudaGraphDestroy(g);
-      if (e != cudaSuccess) {
-        set_last_cuda_error(e, "batch graph", __FILE__, __LINE__);
-        return OWM_ECUDA;
-      }
-    }
-    if (rc2) return rc2;
-  }
-  OWM_CUDA_TRY(cudaEventRecord(done, stream));
-  return OWM_OK;
+    return rc2;
+  });
 }
 
 bool BatchRun::ready() {
@@ -1377,7 +1222,7 @@ bool BatchRun::ready() {
 int BatchRun::finish(int64_t* seeds, int64_t cap, int64_t* offsets, owm_run_info* info) {
   OWM_CUDA_TRY(cudaSetDevice(device));
   OWM_CUDA_TRY(cudaEventSynchronize(done));
-  const int64_t nt = (int64_t)tiles.size();
+  const int64_t nt = ntiles;
   uint32_t st = 0;
   std::memcpy(&st, h_off + nt + 1, 4);  // read back with the offsets at the end of the batch
   if (st & kStatusNonFinite) return OWM_EINVAL;

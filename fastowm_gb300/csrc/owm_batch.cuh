@@ -32,13 +32,6 @@ struct TileMeta {
   int64_t bm_word;  // first 32-bit word of the tile's stage-2 bitmaps (ids 0..n)
 };
 
-// Host-side shape of one tile (what a batch signature is made of).
-struct TileHost {
-  const double* xyz;
-  owm_params p;
-  owm_tree_cfg tree;
-};
-
 // One batch in flight on one stream: device buffers sized for the largest
 // batch seen (kept, so trees stay resident until the next batch reuses them),
 // pinned host words for the per-tile output offsets, an optional CUDA graph.
@@ -60,20 +53,12 @@ struct BatchRun {
   int32_t class_leaf[8] = {};
   owm_tuning tuning = {4, 4, 256, 0};  // launch shapes (a batch takes its context's)
   // results of the last launch
-  std::vector<TileHost> tiles;
+  int32_t ntiles = 0;
   int64_t total_out = 0;
   int64_t* d_out = nullptr;
-  int64_t* d_out_off = nullptr;
   uint32_t* d_status = nullptr;
   size_t bytes_needed = 0;
   cudaEvent_t done = nullptr;
-  // With stage 1 by window classes, a side stream prepares the edge and class
-  // tables and clears the stage-2/3 buffers while the keys are sorted, then
-  // runs stages 1-2 and stage 3's LLP marks while `stream` builds the
-  // hierarchies (fork, tables ready, gather done, join).
-  cudaStream_t side = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_cls = nullptr, ev_gather = nullptr, ev_join = nullptr;
-
   int init(int device, cudaStream_t s);
   void destroy();
   int leaf_for(int64_t n, int32_t requested) const;
@@ -81,6 +66,11 @@ struct BatchRun {
   static size_t estimate_bytes(const owm_tile_desc* t, int32_t ntiles);
   // Enqueue everything (copies in, build, stages, offsets out) on `stream`.
   int launch(const owm_tile_desc* t, int32_t ntiles);
+  int launch_grid(const owm_tile_desc* t, int32_t ntiles);  // window grid
+  int launch_walk(const owm_tile_desc* t, int32_t ntiles);  // trees, persistent stage-1 walk
+  int room(size_t device_bytes, size_t stage_bytes, int32_t ntiles);
+  template <class Enqueue>
+  int run_or_replay(const std::string& sig, Enqueue enqueue);
   // Wait for the launch and copy the seeds / offsets out.
   int finish(int64_t* seeds, int64_t cap, int64_t* offsets, owm_run_info* info);
   bool ready();

@@ -14,6 +14,18 @@ __device__ __forceinline__ uint32_t spread_bits16(uint32_t x) {
   return x;
 }
 
+// Largest t in [0, ntiles) with off[t] <= x (off has ntiles+1 entries,
+// off[0] = 0, off[ntiles] > x): the tile that owns global index x.
+template <class T>
+__device__ __forceinline__ int tile_of(const T* __restrict__ off, int ntiles, int64_t x) {
+  int lo = 0, hi = ntiles - 1;
+  while (lo < hi) {
+    int mid = (lo + hi + 1) >> 1;
+    if ((int64_t)__ldg(off + mid) <= x) lo = mid; else hi = mid - 1;
+  }
+  return lo;
+}
+
 // Per-leaf reduction state: exact int64-key bounding box, count and the
 // (z, id)-minimum with its sorted position.
 struct LeafAcc {

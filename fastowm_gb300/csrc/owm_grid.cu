@@ -24,6 +24,21 @@ namespace {
 
 constexpr int kFoldBlock = 256;
 constexpr int kFoldBlocks = 6;  // resident fold blocks per SM (40 registers a thread)
+// A batch's fold: a block takes a chunk of one tile's points.  Blocks that run
+// together take chunks of kTileStripes stretches of the batch: the blocks of one
+// tile side by side hit the same few thousand sub-cells (72 M points in 128
+// tiles: 1.32 ms in order, 1.18 in 16 stripes, 1.20 in 64, 1.25 in 256).
+constexpr int64_t kTileChunk = 4096;
+constexpr int kTileStripes = 16;
+
+// The job that item *k belongs to; *k becomes the item's number within it.
+template <bool kMulti>
+__device__ __forceinline__ const GridJob& job_at(const GridJob& one, const GridTiles& T, int64_t* k) {
+  if (!kMulti) return one;
+  const int t = tile_of(T.off, T.n, *k);
+  *k -= __ldg(T.off + t);
+  return T.jobs[t];
+}
 
 // ---- prepare ------------------------------------------------------------------
 struct FormulaEdges {
@@ -57,18 +72,25 @@ __device__ void prepare_axis(const GridAxis& a, int32_t i) {
 
 // Bound by the stores of the clear (20 bytes a sub-cell, 2 bits a point);
 // one launch instead of a memset and six small kernels.
-__global__ void __launch_bounds__(256) k_grid_prepare(const __grid_constant__ GridJob J, uint4* __restrict__ clear,
-                                                      int64_t nclear, uint32_t* __restrict__ status) {
+template <bool kMulti>
+__global__ void __launch_bounds__(256) k_grid_prepare(const __grid_constant__ GridJob one, GridTiles T, int64_t items,
+                                                      uint4* __restrict__ clear, int64_t nclear,
+                                                      uint32_t* __restrict__ status) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
-  const int32_t nx = J.x.n + J.x.nc, ny = J.y.n + J.y.nc;
-  for (int64_t i = t; i < nx + ny; i += nt) {
-    if (i < nx) prepare_axis(J.x, (int32_t)i); else prepare_axis(J.y, (int32_t)i - nx);
+  for (int64_t i = t; i < items; i += nt) {
+    int64_t k = i;
+    const GridJob& J = job_at<kMulti>(one, T, &k);
+    const int32_t nx = J.x.n + J.x.nc, ny = J.y.n + J.y.nc;
+    if (k < nx) {
+      prepare_axis(J.x, (int32_t)k);
+    } else if (k < nx + ny) {
+      prepare_axis(J.y, (int32_t)k - nx);
+    } else {
+      const int q = (int)(k - nx - ny);
+      J.occ[q] = !(q < 2 ? J.x : J.y).parmask || (q & 1) == 0;
+    }
   }
-  if (t < 4) {
-    const GridAxis& a = t < 2 ? J.x : J.y;
-    J.occ[t] = !a.parmask || (t & 1) == 0;
-  }
-  if (t == 4) *status = 0;
+  if (t == 0) *status = 0;
   const uint4 z = make_uint4(0, 0, 0, 0);
   for (int64_t i = t; i < nclear; i += nt) clear[i] = z;
 }
@@ -179,30 +201,55 @@ __device__ __noinline__ void raise_own_cells(const GridJob& J, uint64_t x, uint6
     }
 }
 
-// Every point into its sub-cell.  kFast: both axes have the fast form, and
-// whatever it does not settle (an edge, a point outside the box, z zero or not
-// finite) takes the full one in a call.
+// Points [first + b, first + e) of a cloud into their sub-cells, 32 at a time
+// (e a multiple of 32 above b; count: where the cloud or tile ends).  kFast: both axes have the
+// fast form; a point near an edge is settled by the edges its places end at,
+// and one outside the box, or with z zero or not finite, takes the full form in
+// a call.
 //
 // Bound by the L2 requests of points in no order (a read and an add each): 100 M
 // points into 0.9 M sub-cells take 1.04 ms (32 bytes a point: 3.1 TB/s), a bare
-// kernel that does just those two requests 0.87.  The order of the work and the
-// instructions were what cost before: a warp takes a stretch of neighbouring
-// points, so that scan lines side by side are not folded at the same time (40 M
-// points in scan order at 3 a square metre: 1.28 -> 0.53 ms); 144 instructions
-// per 32 points instead of 284 (0.53 -> 0.40); one point a thread at 48 warps
-// an SM (two at 40: 1.05 ms for the 100 M, four at 32: 1.05, and 0.40 -> 0.46
-// for the scan).  A single add whose result carries a filter for the minimum
-// measured 1.40 ms at 100 M.
-template <int kStride, bool kFast>
-__global__ void __launch_bounds__(kFoldBlock, kFoldBlocks)
-    k_grid_fold(const __grid_constant__ GridJob J, const double* __restrict__ rec, int64_t first, int64_t count,
-                uint32_t* __restrict__ status) {
+// kernel that does just those two requests 0.87.  What cost more before:
+// - the order of the work: a warp takes a stretch of neighbouring points, so
+//   that scan lines side by side are not folded at the same time (40 M points in
+//   scan order at 3 a square metre: 1.28 -> 0.53 ms);
+// - instructions: 144 per 32 points instead of 284 (0.53 -> 0.40 ms there);
+// - points on edges (whole centimetres: 1 in 100): two loads side by side in
+//   place of a call (20 M in no order 0.37 -> 0.24 ms, in scan order 0.28 -> 0.23).
+// One point a thread at 48 warps an SM: two at 40 took 1.05 ms for the 100 M,
+// four at 32 1.05, and 0.46 for the scan.  A single add whose result carries a
+// filter for the minimum took 1.40.
+// The fast form's constants where the fold finds them: the kernel's parameters,
+// or (a batch) the tile's job in shared memory, read anew for each group of
+// points in 16-byte words (kept in registers they would halve the warps).
+struct ParamAxes {
+  const GridJob* J;
+  __device__ __forceinline__ const GridAxis& x() const { return J->x; }
+  __device__ __forceinline__ const GridAxis& y() const { return J->y; }
+};
+struct SharedAxes {
+  const GridJob* J;
+  static __device__ __forceinline__ GridFastAxis load(const GridAxis* a) {
+    GridFastAxis f;
+    uint4 w[4];
+    const uint32_t at = (uint32_t)__cvta_generic_to_shared(a);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                   : "=r"(w[k].x), "=r"(w[k].y), "=r"(w[k].z), "=r"(w[k].w)
+                   : "r"(at + 16 * k));
+    memcpy(&f, w, sizeof(f));
+    return f;
+  }
+  __device__ __forceinline__ GridFastAxis x() const { return load(&J->x); }
+  __device__ __forceinline__ GridFastAxis y() const { return load(&J->y); }
+};
+
+template <int kStride, bool kFast, class Axes>
+__device__ __forceinline__ void fold_stretch(const GridJob& J, Axes axes, const double* __restrict__ rec, int64_t first,
+                                             int64_t count, int64_t b, int64_t e, uint32_t& flags) {
   const int lane = threadIdx.x & 31;
-  const int64_t nwarps = ((int64_t)gridDim.x * kFoldBlock) >> 5;
-  uint32_t flags = 0;
-  int64_t t0, t1;
-  chunk_tiles((count + 31) / 32, nwarps, ((int64_t)blockIdx.x * kFoldBlock + threadIdx.x) >> 5, &t0, &t1);
-  for (int64_t b = t0 * 32; b < t1 * 32; b += 32) {
+  for (; b < e; b += 32) {
     // lanes past the end take the last point again, and are not counted
     const int32_t left = (int32_t)min((int64_t)32, count - b);
     const int64_t i = first + b + min(lane, left - 1);
@@ -211,16 +258,29 @@ __global__ void __launch_bounds__(kFoldBlock, kFoldBlocks)
     uint32_t cell, nid = ~(uint32_t)(i + 1);
     unsigned long long w;
     if (kFast) {
-      bool rare = ((uint32_t)(z >> 32) << 1) - 1u >= 0xFFDFFFFFu;  // zero or not finite
-      const int32_t sx = grid_class_fast(J.x, x, &rare), sy = grid_class_fast(J.y, y, &rare);
-      rare |= ((sx ^ J.x.par) | (sy ^ J.y.par)) & 1;
+      int32_t tlx, tax, tly, tay;
+      uint32_t hx, hy, other;
+      const auto& ax = axes.x();
+      int32_t sx = grid_class_fast(ax, x, &hx, &tlx, &tax);
+      other = sx ^ ax.par;
+      const auto& ay = axes.y();
+      int32_t sy = grid_class_fast(ay, y, &hy, &tly, &tay);
+      other |= sy ^ ay.par;
       cell = (uint32_t)(sy >> 1) * (uint32_t)J.x.width[0] + (uint32_t)(sx >> 1);
       w = z ^ (~(uint64_t)((int64_t)z >> 63) & 0x7FFFFFFFFFFFFFFFull);
-      if (rare) {
-        const PointCell p = point_cell_call(J, x, y, z);
-        cell = p.cell;
-        w = p.w;
-        flags |= p.flags;
+      const bool odd_z = ((uint32_t)(z >> 32) << 1) - 1u >= 0xFFDFFFFFu;  // zero or not finite
+      if (odd_z | ((other & 1u) | hx | hy)) {
+        if (odd_z | ((hx | hy) & kGridOutside)) {
+          const PointCell p = point_cell_call(J, x, y, z);
+          cell = p.cell;
+          w = p.w;
+          flags |= p.flags;
+        } else {
+          if (hx) sx = grid_settle_fast(J.x, (int64_t)x, hx, tlx, tax, StoredEdges{&J.x}, sx);
+          if (hy) sy = grid_settle_fast(J.y, (int64_t)y, hy, tly, tay, StoredEdges{&J.y}, sy);
+          cell = grid_cell(J, sx, sy);
+          flags |= (((sx ^ J.x.par) & 1) ? kPointOtherX : 0u) | (((sy ^ J.y.par) & 1) ? kPointOtherY : 0u);
+        }
       }
     } else {
       const PointCell p = point_cell(J, x, y, z);
@@ -255,14 +315,53 @@ __global__ void __launch_bounds__(kFoldBlock, kFoldBlocks)
     }
     if (head) raise_zid(J.zid + cell, cur, w, nid);
   }
-  // one store a warp: a store per point to the one word cost 0.4 ms on 40 M
-  // points in whole centimetres
+}
+
+// What a warp found out, stored once: a store per point to the one word cost
+// 0.4 ms on 40 M points in whole centimetres.
+__device__ __forceinline__ void fold_flags(const GridJob& J, uint32_t flags, uint32_t* __restrict__ status) {
   flags = __reduce_or_sync(0xffffffffu, flags);
-  if (lane == 0 && flags) {
+  if ((threadIdx.x & 31) == 0 && flags) {
     if (flags & kPointNonFinite) atomicOr(status, kStatusNonFinite);
     if (flags & kPointOtherX) J.occ[1] = 1;
     if (flags & kPointOtherY) J.occ[3] = 1;
   }
+}
+
+template <int kStride, bool kFast>
+__global__ void __launch_bounds__(kFoldBlock, kFoldBlocks)
+    k_grid_fold(const __grid_constant__ GridJob J, const double* __restrict__ rec, int64_t first, int64_t count,
+                uint32_t* __restrict__ status) {
+  const int64_t nwarps = ((int64_t)gridDim.x * kFoldBlock) >> 5;
+  uint32_t flags = 0;
+  int64_t t0, t1;
+  chunk_tiles((count + 31) / 32, nwarps, ((int64_t)blockIdx.x * kFoldBlock + threadIdx.x) >> 5, &t0, &t1);
+  fold_stretch<kStride, kFast>(J, ParamAxes{&J}, rec, first, count, t0 * 32, t1 * 32, flags);
+  fold_flags(J, flags, status);
+}
+
+// A batch: block b takes one chunk of its tile's points, with the tile's job in
+// shared memory.
+__global__ void __launch_bounds__(kFoldBlock, kFoldBlocks)
+    k_grid_fold_tiles(GridTiles T, int32_t chunk, uint32_t* __restrict__ status) {
+  __shared__ GridJob J;
+  const int64_t blk = (int64_t)(blockIdx.x % kTileStripes) * (gridDim.x / kTileStripes) + blockIdx.x / kTileStripes;
+  if (blk >= __ldg(T.off + T.n)) return;
+  const int t = tile_of(T.off, T.n, blk);
+  static_assert(sizeof(GridJob) % 16 == 0, "copied in 16-byte words");
+  for (int i = threadIdx.x; i < (int)(sizeof(GridJob) / 16); i += kFoldBlock)
+    reinterpret_cast<uint4*>(&J)[i] = __ldg(reinterpret_cast<const uint4*>(T.jobs + t) + i);
+  __syncthreads();
+  const int64_t c0 = (blk - __ldg(T.off + t)) * (int64_t)chunk;
+  const int64_t n = min((int64_t)chunk, J.n - c0);  // points of this block
+  uint32_t flags = 0;
+  int64_t t0, t1;
+  chunk_tiles((n + 31) / 32, kFoldBlock / 32, threadIdx.x >> 5, &t0, &t1);
+  if (J.fast)
+    fold_stretch<3, true>(J, SharedAxes{&J}, J.rec, 0, J.n, c0 + t0 * 32, c0 + t1 * 32, flags);
+  else
+    fold_stretch<3, false>(J, SharedAxes{&J}, J.rec, 0, J.n, c0 + t0 * 32, c0 + t1 * 32, flags);
+  fold_flags(J, flags, status);
 }
 
 // ---- rectangle reductions ---------------------------------------------------------
@@ -289,9 +388,11 @@ __device__ __forceinline__ bool parity_range(const GridAxis& a, const uint32_t* 
   return true;
 }
 
-__global__ void __launch_bounds__(256) k_grid_rows(const __grid_constant__ GridJob J) {
-  const int64_t total = (int64_t)J.y.nclass * J.x.n;
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < total; k += (int64_t)gridDim.x * blockDim.x) {
+template <bool kMulti>
+__global__ void __launch_bounds__(256) k_grid_rows(const __grid_constant__ GridJob one, GridTiles T, int64_t total) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+    int64_t k = i;
+    const GridJob& J = job_at<kMulti>(one, T, &k);
     const int32_t r = (int32_t)(k / J.x.n), ii = (int32_t)(k % J.x.n);
     const int qy = r >= J.y.width[0];
     if (!J.occ[2 + qy]) continue;
@@ -315,11 +416,13 @@ __global__ void __launch_bounds__(256) k_grid_rows(const __grid_constant__ GridJ
   }
 }
 
-__global__ void __launch_bounds__(256) k_grid_windows(const __grid_constant__ GridJob J) {
+template <bool kMulti>
+__global__ void __launch_bounds__(256) k_grid_windows(const __grid_constant__ GridJob one, GridTiles T, int64_t total) {
   // the search starts from the reference's sentinel point 0 {0, 0, DBL_MAX}
   const unsigned long long sentinel = ~((unsigned long long)kZSentinel ^ 0x8000000000000000ull);
-  const int64_t total = (int64_t)J.x.n * J.y.n;
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < total; k += (int64_t)gridDim.x * blockDim.x) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+    int64_t k = i;
+    const GridJob& J = job_at<kMulti>(one, T, &k);
     const int32_t jj = (int32_t)(k / J.x.n), ii = (int32_t)(k % J.x.n);
     Best m;
     m.w = sentinel;
@@ -393,17 +496,25 @@ __device__ __forceinline__ void mark_cells(const GridJob& J, const double* __res
 
 // The ids marked twice, ascending: block b writes those of its chunk after
 // all chunks before it (whose counts it adds up) and marks their cells.
-__global__ void __launch_bounds__(kSeedBlock) k_grid_seeds(const __grid_constant__ GridJob J, const uint32_t* __restrict__ part,
-                                                           const double* __restrict__ xy, int stride,
-                                                           uint32_t* __restrict__ llp, uint32_t* __restrict__ nllp) {
+// A batch: tile by tile; nllp[t] is tile t's first LLP, nllp[T.n] their number.
+template <bool kMulti>
+__global__ void __launch_bounds__(kSeedBlock) k_grid_seeds(const __grid_constant__ GridJob one, GridTiles T,
+                                                           const uint32_t* __restrict__ part, const double* __restrict__ xy,
+                                                           int stride, uint32_t* __restrict__ llp,
+                                                           uint32_t* __restrict__ nllp) {
+  int64_t chunk = blockIdx.x;
+  const GridJob& J = job_at<kMulti>(one, T, &chunk);
   uint32_t before = 0, total;
   for (uint32_t q = threadIdx.x; q < blockIdx.x; q += kSeedBlock) before += __ldg(part + q);
   block_exclusive_256(before, &before);
-  const int64_t w0 = (int64_t)blockIdx.x * kSeedChunk + (int64_t)threadIdx.x * kSeedWords;
+  const int64_t w0 = chunk * kSeedChunk + (int64_t)threadIdx.x * kSeedWords;
   const uint4 q = __ldg(reinterpret_cast<const uint4*>(J.twice + w0));
   const uint32_t word[4] = {q.x, q.y, q.z, q.w};
   uint32_t at = before + block_exclusive_256((uint32_t)(__popc(q.x) + __popc(q.y) + __popc(q.z) + __popc(q.w)), &total);
-  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *nllp = before + total;
+  if (threadIdx.x == 0) {
+    if (kMulti && chunk == 0) nllp[&J - T.jobs] = before;
+    if (blockIdx.x == gridDim.x - 1) nllp[kMulti ? T.n : 0] = before + total;
+  }
 #pragma unroll
   for (int k = 0; k < kSeedWords; ++k) {
     uint32_t b = word[k];
@@ -411,7 +522,7 @@ __global__ void __launch_bounds__(kSeedBlock) k_grid_seeds(const __grid_constant
       const uint32_t id = (uint32_t)((w0 + k) * 32) + (uint32_t)(__ffs(b) - 1);
       b &= b - 1;
       llp[at++] = id;
-      if (J.x.nc) mark_cells(J, xy, stride, id);
+      if (J.x.nc) mark_cells(J, kMulti ? J.rec : xy, kMulti ? 3 : stride, id);
     }
   }
 }
@@ -432,14 +543,20 @@ __device__ __forceinline__ uint32_t cell_result(unsigned long long w, uint32_t n
   return w == 0 ? kNone : w <= sentinel ? 0u : ~nid;
 }
 
-// One warp per cell: the (z, id)-min of its rectangle of sub-cells.
-__global__ void __launch_bounds__(256) k_grid_cells(const __grid_constant__ GridJob J, int64_t ncell) {
+// One warp per cell: the (z, id)-min of its rectangle of sub-cells, or its own
+// entry.
+template <bool kMulti>
+__global__ void __launch_bounds__(256) k_grid_cells(const __grid_constant__ GridJob one, GridTiles T, int64_t total) {
   const int lane = threadIdx.x & 31;
-  const int64_t c = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (c >= ncell) return;
+  int64_t c = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (c >= total) return;
+  const GridJob& J = job_at<kMulti>(one, T, &c);
   const int32_t ci = (int32_t)(c % J.x.nc), cj = (int32_t)(c / J.x.nc);
   Best m;
-  if (!J.mark[c]) {
+  if (J.cell_zid) {
+    const ulonglong2 e = J.cell_zid[c];
+    if (!J.mark[c]) m.take(e.x, (uint32_t)e.y);
+  } else if (!J.mark[c]) {
     for (int qy = 0; qy < 2; ++qy) {
       int32_t y0, y1;
       if (!parity_range(J.y, J.occ + 2, qy, J.y.clo[cj], J.y.chi[cj], &y0, &y1)) continue;
@@ -459,13 +576,6 @@ __global__ void __launch_bounds__(256) k_grid_cells(const __grid_constant__ Grid
   for (int o = 16; o >= 1; o >>= 1)
     m.take(__shfl_xor_sync(0xffffffffu, m.w, o), __shfl_xor_sync(0xffffffffu, m.nid, o));
   if (lane == 0) J.cellmin[c] = cell_result(m.w, m.nid);
-}
-
-__global__ void __launch_bounds__(256) k_grid_cells_own(const __grid_constant__ GridJob J, int64_t ncell) {
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncell) return;
-  const ulonglong2 e = J.cell_zid[c];
-  J.cellmin[c] = J.mark[c] ? kNone : cell_result(e.x, (uint32_t)e.y);
 }
 
 // seeds = the valid entries of cellmin in order, then the LLPs.  Every block
@@ -509,6 +619,75 @@ __global__ void k_grid_output_scanned(const uint32_t* __restrict__ cellmin, cons
     if (cellmin[i] != kNone) seeds[pos[i]] = cellmin[i];
   const int64_t n = *nllp, base = *ns3;
   for (int64_t i = t; i < n; i += nt) seeds[base + i] = llp[i];
+}
+
+// ---- batches: overlap 0 in some tile, and the output ------------------------------
+// Stage 2 by sorting (tile, id) keys: the tiles' windows, then the first of
+// every run of two or more (overlap > 0) or every valid one.
+__global__ void k_gridb_keys(const uint32_t* __restrict__ win, GridTiles T, int64_t n, int id_bits, uint32_t none,
+                             uint32_t* __restrict__ keys) {
+  for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < n; w += (int64_t)gridDim.x * blockDim.x) {
+    const uint32_t v = win[w];
+    keys[w] = ((uint32_t)tile_of(T.off, T.n, w) << id_bits) | (v == kNone ? none : v);
+  }
+}
+__global__ void k_gridb_flags(const uint32_t* __restrict__ keys, int64_t n, int id_bits, uint32_t none, GridTiles T,
+                              uint32_t* __restrict__ flags, uint32_t* __restrict__ tile_count) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const uint32_t k = keys[i], t = k >> id_bits;
+    bool f = (k & none) != none;
+    if (T.jobs[t].need_dup) f = f && (i == 0 || keys[i - 1] != k) && (i + 1 < n && keys[i + 1] == k);
+    flags[i] = f ? 1u : 0u;
+    if (f) atomicAdd(tile_count + t, 1u);
+  }
+}
+__global__ void k_gridb_ids(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ flags,
+                            const uint32_t* __restrict__ pos, int64_t n, int id_bits, GridTiles T, uint32_t* __restrict__ llp) {
+  const uint32_t mask = (1u << id_bits) - 1u;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    if (!flags[i]) continue;
+    const uint32_t id = keys[i] & mask;
+    const GridJob& J = T.jobs[keys[i] >> id_bits];
+    llp[pos[i]] = id;
+    if (J.x.nc) mark_cells(J, J.rec, 3, id);
+  }
+}
+
+// Block t: the number of tile t's cells with a result.
+__global__ void __launch_bounds__(kSeedBlock) k_gridb_count(GridTiles T, uint32_t* __restrict__ s3cnt) {
+  const GridJob& J = T.jobs[blockIdx.x];
+  const int64_t n = (int64_t)J.x.nc * J.y.nc;
+  uint32_t c = 0;
+  for (int64_t i = threadIdx.x; i < n; i += kSeedBlock) c += J.cellmin[i] != kNone ? 1u : 0u;
+  block_exclusive_256(c, &c);
+  if (threadIdx.x == 0) s3cnt[blockIdx.x] = c;
+}
+
+// Block t: tile t's stage-3 ids in cell order, then its LLPs, after those of
+// the tiles before it.
+__global__ void __launch_bounds__(kSeedBlock) k_gridb_output(GridTiles T, const uint32_t* __restrict__ s3cnt,
+                                                             const uint32_t* __restrict__ llp, const uint32_t* __restrict__ llp_off,
+                                                             int64_t* __restrict__ out, int64_t* __restrict__ out_off) {
+  const int t = blockIdx.x;
+  const GridJob& J = T.jobs[t];
+  uint32_t c = 0, s3_before;
+  for (int q = threadIdx.x; q < t; q += kSeedBlock) c += __ldg(s3cnt + q);
+  block_exclusive_256(c, &s3_before);
+  const uint32_t l0 = llp_off[t], l1 = llp_off[t + 1], mine = s3cnt[t];
+  int64_t at = (int64_t)s3_before + l0;
+  if (threadIdx.x == 0) {
+    out_off[t] = at;
+    if (t == T.n - 1) out_off[T.n] = at + mine + (l1 - l0);
+  }
+  for (uint32_t k = threadIdx.x; k < l1 - l0; k += kSeedBlock) out[at + mine + k] = llp[l0 + k];
+  const int64_t n = (int64_t)J.x.nc * J.y.nc;
+  for (int64_t i = 0; i < n && mine; i += kSeedBlock) {
+    const uint32_t v = i + threadIdx.x < n ? J.cellmin[i + threadIdx.x] : kNone;
+    uint32_t got;
+    const uint32_t p = block_exclusive_256(v != kNone ? 1u : 0u, &got);
+    if (v != kNone) out[at + p] = v;
+    at += got;
+  }
 }
 
 unsigned blocks_for(int64_t n, int64_t most, int block = 256) {
@@ -608,6 +787,8 @@ void grid_axis_setup(double lo, double hi, double step, int32_t whalf, int32_t n
                           &a->fbc, &a->kc);
   }
   a->quick = quick ? 1 : 0;
+  a->fmw = (1u << a->fbw) - 1u;
+  a->fmc = (1u << a->fbc) - 1u;
   // the fast form, from lo; an empty range (span 0 above the greatest position) without one
   a->lo0 = linear ? bits_of(lo) : 0;
   a->span = 0;
@@ -675,84 +856,279 @@ void grid_axis_setup(double lo, double hi, double step, int32_t whalf, int32_t n
   }
 }
 
-int grid_plan(const owm_params& p, int64_t n, void* scratch, GridPlan* g) {
-  *g = GridPlan{};
-  GridJob& J = g->job;
-  std::memset(&J, 0, sizeof(J));
-  const int32_t nc = (int32_t)p.ncols, nr = (int32_t)p.nrows;
-  if (nc <= 0 || nr <= 0) return OWM_EINVAL;
-  const int64_t tx = 2 * (int64_t)nc + 1, ty = 2 * (int64_t)nr + 1;
+int grid_sizes(const owm_params& p, int64_t n, GridSizes* z) {
+  const int64_t nc = p.ncols, nr = p.nrows;
+  const int64_t tx = 2 * nc + 1, ty = 2 * nr + 1;
   if (tx * ty >= 0xFFFFFFFFll) return OWM_ERANGE;
   const bool cells = p.bsize > 0 && p.ngrid > 0;
-  const int32_t ncg = cells ? (int32_t)p.ncols_grid : 0, nrg = cells ? (int32_t)p.nrows_grid : 0;
-  const bool merged = cells && (tx + 2 * ncg) * (ty + 2 * nrg) <= std::min<int64_t>(std::max<int64_t>(4 * tx * ty, 1 << 20), 1 << 28);
-  const int32_t whalf = (uint16_t)p.wsize / 2, bsize = (uint16_t)p.bsize;
-  grid_axis_setup(p.bbox.min_x, p.bbox.max_x, p.displace, whalf, nc, bsize, ncg, merged, &J.x);
-  grid_axis_setup(p.bbox.min_y, p.bbox.max_y, p.displace, whalf, nr, bsize, nrg, merged, &J.y);
-  J.thr = p.min_num_points;
-  J.n = (int32_t)n;
-  g->n = n;
-  g->nwin = (int64_t)nc * nr;
-  g->ncell = (int64_t)ncg * nrg;
-  g->nsub = grid_cells(J);
-  J.base[1] = (uint32_t)J.x.width[0] * (uint32_t)J.y.width[0];
-  J.base[2] = J.base[1] + (uint32_t)J.x.width[1] * (uint32_t)J.y.width[0];
-  J.base[3] = J.base[2] + (uint32_t)J.x.width[0] * (uint32_t)J.y.width[1];
-  J.fast = J.x.fast && J.y.fast && (!cells || merged);
-  g->bitmap2 = p.overlap > 0.0;
-  char* b = static_cast<char*>(scratch);
-  size_t o = 0;
-  auto take = [&](size_t bytes) -> char* {
-    char* q = b ? b + o : nullptr;
-    o += up256(bytes);
-    return q;
-  };
-  // cleared
-  J.zid = (ulonglong2*)take((size_t)g->nsub * 16);
-  J.count = (uint32_t*)take((size_t)g->nsub * 4);
-  if (cells && !merged) J.cell_zid = (ulonglong2*)take((size_t)g->ncell * 16);
-  const int64_t chunks = ((n + 1 + 31) / 32 + kSeedChunk - 1) / kSeedChunk;
-  if (g->bitmap2) {
-    J.once = (uint32_t*)take((size_t)(chunks * kSeedChunk) * 4);
-    J.twice = (uint32_t*)take((size_t)(chunks * kSeedChunk) * 4);
-  }
-  J.mark = (uint8_t*)take((size_t)g->ncell);
-  g->clear_bytes = o;
-  // written by the kernels
-  for (int ax = 0; ax < 2; ++ax) {
-    GridAxis& a = ax ? J.y : J.x;
-    for (int f = 0; f < 4; ++f) a.edge[f] = (int64_t*)take((size_t)(f < 2 ? a.n : a.nc) * 8);
-    a.lo = (int32_t*)take((size_t)a.n * 4);
-    a.hi = (int32_t*)take((size_t)a.n * 4);
-    a.clo = (int32_t*)take((size_t)a.nc * 4);
-    a.chi = (int32_t*)take((size_t)a.nc * 4);
-  }
-  J.occ = (uint32_t*)take(16);
-  J.rows = (GridRow*)take((size_t)J.y.nclass * nc * sizeof(GridRow));
-  J.cellmin = (uint32_t*)take((size_t)g->ncell * 4);
-  g->llp = (uint32_t*)take((size_t)g->nwin * 4);
-  g->seeds = (int64_t*)take((size_t)(g->nwin + g->ncell + 1) * 8);
-  if (g->bitmap2) {
-    g->part = (uint32_t*)take((size_t)chunks * 4);
-  } else {
-    J.win = (uint32_t*)take((size_t)g->nwin * 4);
-    g->s2_bytes = stage2_scratch_bytes(g->nwin);
-    g->s2_temp = take(g->s2_bytes);
-  }
-  if (g->ncell > kOutputCells) {
-    g->flags = (uint32_t*)take((size_t)g->ncell * 4);
-    g->pos = (uint32_t*)take((size_t)g->ncell * 4);
-    g->scan_bytes = scan_temp_bytes(g->ncell);
-    g->scan_temp = take(g->scan_bytes);
-  }
-  g->bytes = o;
-  g->base = b;
+  const int64_t ncg = cells ? p.ncols_grid : 0, nrg = cells ? p.nrows_grid : 0;
+  // The cells' edges go with the windows' while they do not multiply the
+  // sub-cells: a point then costs nothing for stage 3.  Beyond that the cells
+  // get a table of their own, which no point count or window size can blow up.
+  z->merged = cells && (tx + 2 * ncg) * (ty + 2 * nrg) <= std::min<int64_t>(std::max<int64_t>(4 * tx * ty, 1 << 20), 1 << 28);
+  const int64_t sx = tx + (z->merged ? 2 * ncg : 0), sy = ty + (z->merged ? 2 * nrg : 0);
+  z->nsub = sx * sy;
+  z->nwin = nc * nr;
+  z->ncell = ncg * nrg;
+  z->rows = sy * nc;
+  z->edges = 24 * (nc + ncg + nr + nrg) + 16;  // keys and s-ranges, and the occupancy words
+  z->chunks = ((n + 1 + 31) / 32 + kSeedChunk - 1) / kSeedChunk;
   return OWM_OK;
 }
 
-int grid_prepare(const GridPlan& g, uint32_t* status, cudaStream_t s, int64_t* launches) {
+void grid_job(const owm_params& p, int64_t n, const GridSizes& z, GridJob* j) {
+  GridJob& J = *j;
+  std::memset(&J, 0, sizeof(J));
+  const int32_t ncg = z.ncell ? (int32_t)p.ncols_grid : 0, nrg = z.ncell ? (int32_t)p.nrows_grid : 0;
+  const int32_t whalf = (uint16_t)p.wsize / 2, bsize = (uint16_t)p.bsize;
+  grid_axis_setup(p.bbox.min_x, p.bbox.max_x, p.displace, whalf, (int32_t)p.ncols, bsize, ncg, z.merged, &J.x);
+  grid_axis_setup(p.bbox.min_y, p.bbox.max_y, p.displace, whalf, (int32_t)p.nrows, bsize, nrg, z.merged, &J.y);
+  J.thr = p.min_num_points;
+  J.n = (int32_t)n;
+  J.need_dup = p.overlap > 0.0;
+  J.base[1] = (uint32_t)J.x.width[0] * (uint32_t)J.y.width[0];
+  J.base[2] = J.base[1] + (uint32_t)J.x.width[1] * (uint32_t)J.y.width[0];
+  J.base[3] = J.base[2] + (uint32_t)J.x.width[0] * (uint32_t)J.y.width[1];
+  J.fast = J.x.fast && J.y.fast && (z.merged || z.ncell == 0);
+}
+
+namespace {
+// Hands out 256-byte aligned pieces of a region, or their sizes alone.
+struct Carver {
+  char* base;
+  size_t at = 0;
+  template <class T>
+  T* take(int64_t count) {
+    char* q = base ? base + at : nullptr;
+    at += up256((size_t)count * sizeof(T));
+    return reinterpret_cast<T*>(q);
+  }
+};
+// The edge arrays, occupancy words and ranges of a job, from a piece of
+// GridSizes::edges bytes.
+void carve_edges(GridJob& J, char* b) {
+  auto take = [&](size_t bytes) {
+    char* q = b;
+    b += bytes;
+    return q;
+  };
+  for (GridAxis* a : {&J.x, &J.y})
+    for (int f = 0; f < 4; ++f) a->edge[f] = (int64_t*)take((size_t)(f < 2 ? a->n : a->nc) * 8);
+  J.occ = (uint32_t*)take(16);
+  for (GridAxis* a : {&J.x, &J.y}) {
+    a->lo = (int32_t*)take((size_t)a->n * 4);
+    a->hi = (int32_t*)take((size_t)a->n * 4);
+    a->clo = (int32_t*)take((size_t)a->nc * 4);
+    a->chi = (int32_t*)take((size_t)a->nc * 4);
+  }
+}
+// Threads' items of k_grid_prepare: windows and cells per axis, occupancy words.
+int64_t prepare_items(const owm_params& p, const GridSizes& z) {
+  return (int64_t)p.ncols + p.nrows + (z.ncell ? (int64_t)p.ncols_grid + p.nrows_grid : 0) + 4;
+}
+}  // namespace
+
+int grid_plan(const owm_params& p, int64_t n, void* scratch, GridPlan* g) {
+  *g = GridPlan{};
+  GridJob& J = g->job;
+  if (p.ncells <= 0) return OWM_EINVAL;
+  const int rc = grid_sizes(p, n, &g->z);
+  if (rc) return rc;
+  const GridSizes& z = g->z;
+  if (scratch) grid_job(p, n, z, &J);
+  g->n = n;
+  g->bitmap2 = p.overlap > 0.0;
+  Carver c{static_cast<char*>(scratch)};
+  // cleared
+  J.zid = c.take<ulonglong2>(z.nsub);
+  J.count = c.take<uint32_t>(z.nsub);
+  if (!z.merged && z.ncell) J.cell_zid = c.take<ulonglong2>(z.ncell);
+  if (g->bitmap2) {
+    J.once = c.take<uint32_t>(z.chunks * kSeedChunk);
+    J.twice = c.take<uint32_t>(z.chunks * kSeedChunk);
+  }
+  J.mark = c.take<uint8_t>(z.ncell);
+  g->clear_bytes = c.at;
+  // written by the kernels
+  char* edges = c.take<char>(z.edges);
+  if (edges) carve_edges(J, edges);
+  J.rows = c.take<GridRow>(z.rows);
+  J.cellmin = c.take<uint32_t>(z.ncell);
+  g->llp = c.take<uint32_t>(z.nwin);
+  g->seeds = c.take<int64_t>(z.nwin + z.ncell + 1);
+  if (g->bitmap2) {
+    g->part = c.take<uint32_t>(z.chunks);
+  } else {
+    J.win = c.take<uint32_t>(z.nwin);
+    g->s2_bytes = stage2_scratch_bytes(z.nwin);
+    g->s2_temp = c.take<char>((int64_t)g->s2_bytes);
+  }
+  if (z.ncell > kOutputCells) {
+    g->flags = c.take<uint32_t>(z.ncell);
+    g->pos = c.take<uint32_t>(z.ncell);
+    g->scan_bytes = scan_temp_bytes(z.ncell);
+    g->scan_temp = c.take<char>((int64_t)g->scan_bytes);
+  }
+  g->bytes = c.at;
+  g->base = c.base;
+  return OWM_OK;
+}
+
+int grid_batch_plan(const owm_params* p, const int64_t* n, int32_t ntiles, GridSizes* z, char* base, GridBatch* g) {
+  std::memset(static_cast<void*>(g), 0, sizeof(*g));  // padding too: a batch's bytes name its graph
+  g->ntiles = ntiles;
+  g->bitmap2 = 1;
+  g->tile_bits = g->id_bits = 1;
+  int64_t points = 0, nsub = 0, own = 0, edges = 0, maxn = 0;
+  for (int32_t k = 0; k < ntiles; ++k) {
+    const int rc = grid_sizes(p[k], n[k], &z[k]);
+    if (rc) return rc;
+    if (!(p[k].overlap > 0.0)) g->bitmap2 = 0;
+    points += n[k];
+    maxn = std::max(maxn, n[k]);
+    nsub += z[k].nsub;
+    own += z[k].merged ? 0 : z[k].ncell;
+    edges += (z[k].edges + 15) & ~(int64_t)15;
+    g->items += prepare_items(p[k], z[k]);
+    g->rows += z[k].rows;
+    g->wins += z[k].nwin;
+    g->chunks += z[k].chunks;
+    g->cells += z[k].ncell;
+  }
+  // enough fold blocks to fill the chip twice, of 256 to 4096 points
+  g->chunk = (int32_t)std::min<int64_t>(kTileChunk, std::max<int64_t>(256, (points / (152 * kFoldBlocks * 2) + 255) / 256 * 256));
+  for (int32_t k = 0; k < ntiles; ++k) g->folds += (n[k] + g->chunk - 1) / g->chunk;
+  if (g->folds >= 0x7FFFFFFFll || g->chunks >= 0x7FFFFFFFll || g->cells >= 0x7FFFFFFFll * 8) return OWM_ERANGE;
+  while (((uint64_t)1 << g->tile_bits) < (uint64_t)ntiles) ++g->tile_bits;
+  while (((uint64_t)1 << g->id_bits) <= (uint64_t)maxn + 1) ++g->id_bits;
+  if (g->tile_bits + g->id_bits > 32) return OWM_ERANGE;  // split the batch
+
+  Carver c{base};
+  g->zid = c.take<char>(nsub * 16);
+  g->count = c.take<char>(nsub * 4);
+  g->cell_zid = c.take<char>(own * 16);
+  g->bitmap = g->bitmap2 ? c.take<uint32_t>(2 * g->chunks * kSeedChunk) : nullptr;
+  g->mark = c.take<char>(g->cells);
+  g->cnt2 = c.take<uint32_t>(ntiles + 1);
+  g->words = c.take<uint32_t>(64);
+  g->clear_bytes = c.at;
+  g->jobs = c.take<GridJob>(ntiles);
+  for (auto** v : {&g->item_off, &g->fold_off, &g->row_off, &g->win_off, &g->chunk_off, &g->cell_off})
+    *v = c.take<int64_t>(ntiles + 1);
+  g->table_bytes = c.at - g->clear_bytes;
+  g->edges = c.take<char>(edges);
+  g->row_mem = c.take<char>(g->rows * (int64_t)sizeof(GridRow));
+  g->cellmin = c.take<char>(g->cells * 4);
+  g->llp = c.take<uint32_t>(g->wins);
+  g->llp_off = c.take<uint32_t>(ntiles + 1);
+  g->s3cnt = c.take<uint32_t>(ntiles + 1);
+  g->out = c.take<int64_t>(g->wins + g->cells + 1);
+  g->out_off = c.take<int64_t>(ntiles + 1);
+  if (g->bitmap2) {
+    g->part = c.take<uint32_t>(g->chunks);
+  } else {
+    g->win = c.take<uint32_t>(g->wins);
+    g->k0 = c.take<uint32_t>(g->wins);
+    g->k1 = c.take<uint32_t>(g->wins);
+    g->flags = c.take<uint32_t>(g->wins);
+    g->pos = c.take<uint32_t>(g->wins);
+    g->sort_bytes = radix_sort_temp_bytes(g->wins);
+    g->sort_temp = c.take<char>((int64_t)g->sort_bytes);
+    g->scan_bytes = scan_temp_bytes(std::max<int64_t>(g->wins, ntiles + 1));
+    g->scan_temp = c.take<char>((int64_t)g->scan_bytes);
+  }
+  g->bytes = c.at;
+  g->base = base;
+  return OWM_OK;
+}
+
+void grid_batch_tables(const owm_params* p, const int64_t* n, const GridSizes* z, const double* const* rec, const GridBatch& g,
+                       char* host) {
+  auto at = [&](const void* device) { return host + (static_cast<const char*>(device) - reinterpret_cast<const char*>(g.jobs)); };
+  GridJob* jobs = reinterpret_cast<GridJob*>(host);
+  int64_t *items = (int64_t*)at(g.item_off), *folds = (int64_t*)at(g.fold_off), *rows = (int64_t*)at(g.row_off),
+          *wins = (int64_t*)at(g.win_off), *chunks = (int64_t*)at(g.chunk_off), *cells = (int64_t*)at(g.cell_off);
+  items[0] = folds[0] = rows[0] = wins[0] = chunks[0] = cells[0] = 0;
+  int64_t sub = 0, own = 0, edges = 0;
+  for (int32_t k = 0; k < g.ntiles; ++k) {
+    GridJob& J = jobs[k];
+    grid_job(p[k], n[k], z[k], &J);
+    J.rec = rec[k];
+    J.zid = (ulonglong2*)g.zid + sub;
+    J.count = (uint32_t*)g.count + sub;
+    sub += z[k].nsub;
+    if (!z[k].merged && z[k].ncell) {
+      J.cell_zid = (ulonglong2*)g.cell_zid + own;
+      own += z[k].ncell;
+    }
+    if (g.bitmap2) {
+      J.once = g.bitmap + chunks[k] * kSeedChunk;
+      J.twice = g.bitmap + (g.chunks + chunks[k]) * kSeedChunk;
+    } else {
+      J.win = g.win + wins[k];
+    }
+    J.mark = (uint8_t*)g.mark + cells[k];
+    carve_edges(J, g.edges + edges);
+    edges += (z[k].edges + 15) & ~(int64_t)15;
+    J.rows = (GridRow*)g.row_mem + rows[k];
+    J.cellmin = (uint32_t*)g.cellmin + cells[k];
+    items[k + 1] = items[k] + prepare_items(p[k], z[k]);
+    folds[k + 1] = folds[k] + (n[k] + g.chunk - 1) / g.chunk;
+    rows[k + 1] = rows[k] + z[k].rows;
+    wins[k + 1] = wins[k] + z[k].nwin;
+    chunks[k + 1] = chunks[k] + z[k].chunks;
+    cells[k + 1] = cells[k] + z[k].ncell;
+  }
+}
+
+int grid_batch_run(const GridBatch& g, cudaStream_t s, int64_t* launches) {
+  GridJob none;
+  std::memset(&none, 0, sizeof(none));
+  auto tiles = [&](const int64_t* off) { return GridTiles{g.jobs, off, g.ntiles}; };
   const int64_t n16 = (int64_t)(g.clear_bytes / 16);
-  OWM_LAUNCH("k_grid_prepare", s, k_grid_prepare<<<blocks_for(n16, 152 * 8), 256, 0, s>>>(g.job, (uint4*)g.base, n16, status));
+  OWM_LAUNCH("k_grid_prepare", s, k_grid_prepare<true><<<blocks_for(std::max(n16, g.items), 152 * 8), 256, 0, s>>>(
+      none, tiles(g.item_off), g.items, (uint4*)g.base, n16, g.words));
+  OWM_LAUNCH("k_grid_fold_tiles", s, k_grid_fold_tiles<<<(unsigned)((g.folds + kTileStripes - 1) / kTileStripes * kTileStripes), kFoldBlock, 0, s>>>(tiles(g.fold_off), g.chunk, g.words));
+  OWM_LAUNCH("k_grid_rows", s, k_grid_rows<true><<<blocks_for(g.rows, 152 * 32), 256, 0, s>>>(none, tiles(g.row_off), g.rows));
+  OWM_LAUNCH("k_grid_windows", s, k_grid_windows<true><<<blocks_for(g.wins, 152 * 32), 256, 0, s>>>(none, tiles(g.win_off), g.wins));
+  count_launch(launches, 4);
+  if (g.bitmap2) {
+    OWM_LAUNCH("k_grid_seed_count", s, k_grid_seed_count<<<(unsigned)g.chunks, kSeedBlock, 0, s>>>(
+        g.bitmap + g.chunks * kSeedChunk, g.part));
+    OWM_LAUNCH("k_grid_seeds", s, k_grid_seeds<true><<<(unsigned)g.chunks, kSeedBlock, 0, s>>>(
+        none, tiles(g.chunk_off), g.part, nullptr, 3, g.llp, g.llp_off));
+    count_launch(launches, 2);
+  } else {
+    const uint32_t ids = (1u << g.id_bits) - 1u;
+    const unsigned nb = blocks_for(g.wins, 152 * 32);
+    OWM_LAUNCH("k_gridb_keys", s, k_gridb_keys<<<nb, 256, 0, s>>>(g.win, tiles(g.win_off), g.wins, g.id_bits, ids, g.k0));
+    bool alt = false;
+    if (g.wins > 0)
+      OWM_CUDA_TRY(radix_sort(g.k0, nullptr, g.k1, nullptr, g.wins, g.tile_bits + g.id_bits, false, g.sort_temp, g.sort_bytes, s,
+                            &alt, launches));
+    const uint32_t* keys = alt ? g.k1 : g.k0;
+    OWM_LAUNCH("k_gridb_flags", s, k_gridb_flags<<<nb, 256, 0, s>>>(keys, g.wins, g.id_bits, ids, tiles(g.win_off), g.flags, g.cnt2));
+    if (g.wins > 0) OWM_CUDA_TRY(exclusive_scan_u32(g.flags, g.pos, g.wins, nullptr, g.scan_temp, g.scan_bytes, s, launches));
+    OWM_LAUNCH("k_gridb_ids", s, k_gridb_ids<<<nb, 256, 0, s>>>(keys, g.flags, g.pos, g.wins, g.id_bits, tiles(g.win_off), g.llp));
+    OWM_CUDA_TRY(exclusive_scan_u32(g.cnt2, g.llp_off, g.ntiles + 1, nullptr, g.scan_temp, g.scan_bytes, s, launches));
+    count_launch(launches, 3);
+  }
+  if (g.cells > 0) {
+    OWM_LAUNCH("k_grid_cells", s, k_grid_cells<true><<<(unsigned)((g.cells + 7) / 8), 256, 0, s>>>(none, tiles(g.cell_off), g.cells));
+    count_launch(launches);
+  }
+  OWM_LAUNCH("k_gridb_count", s, k_gridb_count<<<(unsigned)g.ntiles, kSeedBlock, 0, s>>>(tiles(g.cell_off), g.s3cnt));
+  OWM_LAUNCH("k_gridb_output", s, k_gridb_output<<<(unsigned)g.ntiles, kSeedBlock, 0, s>>>(tiles(g.cell_off), g.s3cnt, g.llp, g.llp_off,
+                                                                                     g.out, g.out_off));
+  count_launch(launches, 2);
+  OWM_CUDA_TRY(cudaGetLastError());
+  return OWM_OK;
+}
+
+int grid_prepare(const GridPlan& g, const owm_params& p, uint32_t* status, cudaStream_t s, int64_t* launches) {
+  const int64_t n16 = (int64_t)(g.clear_bytes / 16);
+  OWM_LAUNCH("k_grid_prepare", s, k_grid_prepare<false><<<blocks_for(n16, 152 * 8), 256, 0, s>>>(
+      g.job, GridTiles{}, prepare_items(p, g.z), (uint4*)g.base, n16, status));
   count_launch(launches);
   OWM_CUDA_TRY(cudaGetLastError());
   return OWM_OK;
@@ -773,8 +1149,8 @@ int grid_fold(const GridPlan& g, const double* rec, int stride, int64_t first, i
 
 int grid_windows(const GridPlan& g, cudaStream_t s, int64_t* launches) {
   const GridJob& J = g.job;
-  OWM_LAUNCH("k_grid_rows", s, k_grid_rows<<<blocks_for((int64_t)J.y.nclass * J.x.n, 152 * 32), 256, 0, s>>>(J));
-  OWM_LAUNCH("k_grid_windows", s, k_grid_windows<<<blocks_for(g.nwin, 152 * 32), 256, 0, s>>>(J));
+  OWM_LAUNCH("k_grid_rows", s, k_grid_rows<false><<<blocks_for(g.z.rows, 152 * 32), 256, 0, s>>>(J, GridTiles{}, g.z.rows));
+  OWM_LAUNCH("k_grid_windows", s, k_grid_windows<false><<<blocks_for(g.z.nwin, 152 * 32), 256, 0, s>>>(J, GridTiles{}, g.z.nwin));
   count_launch(launches, 2);
   OWM_CUDA_TRY(cudaGetLastError());
   return OWM_OK;
@@ -784,16 +1160,17 @@ int grid_stage2(const GridPlan& g, const owm_params& p, const double* xy, int xy
                 cudaStream_t s, int64_t* launches) {
   const GridJob& J = g.job;
   if (g.bitmap2) {
-    const unsigned chunks = (unsigned)(((g.n + 1 + 31) / 32 + kSeedChunk - 1) / kSeedChunk);
+    const unsigned chunks = (unsigned)g.z.chunks;
     OWM_LAUNCH("k_grid_seed_count", s, k_grid_seed_count<<<chunks, kSeedBlock, 0, s>>>(J.twice, g.part));
-    OWM_LAUNCH("k_grid_seeds", s, k_grid_seeds<<<chunks, kSeedBlock, 0, s>>>(J, g.part, xy, xy_stride, g.llp, d_nllp));
+    OWM_LAUNCH("k_grid_seeds", s, k_grid_seeds<false><<<chunks, kSeedBlock, 0, s>>>(J, GridTiles{}, g.part, xy, xy_stride, g.llp,
+                                                                                      d_nllp));
     count_launch(launches, 2);
   } else {
     // overlap 0 keeps every valid minimum, repeated sentinel ids included: by sorting
-    const int rc = run_stage2(J.win, g.nwin, g.n, p.overlap, g.llp, d_nllp, g.s2_temp, g.s2_bytes, s, launches);
+    const int rc = run_stage2(J.win, g.z.nwin, g.n, p.overlap, g.llp, d_nllp, g.s2_temp, g.s2_bytes, s, launches);
     if (rc) return rc;
-    if (g.ncell) {
-      OWM_LAUNCH("k_grid_mark", s, k_grid_mark<<<blocks_for(g.nwin, 152 * 8), 256, 0, s>>>(J, xy, xy_stride, g.llp, d_nllp));
+    if (g.z.ncell) {
+      OWM_LAUNCH("k_grid_mark", s, k_grid_mark<<<blocks_for(g.z.nwin, 152 * 8), 256, 0, s>>>(J, xy, xy_stride, g.llp, d_nllp));
       count_launch(launches);
     }
   }
@@ -803,23 +1180,20 @@ int grid_stage2(const GridPlan& g, const owm_params& p, const double* xy, int xy
 
 int grid_stage3(const GridPlan& g, const uint32_t* d_nllp, uint32_t* d_ns3, cudaStream_t s, int64_t* launches) {
   const GridJob& J = g.job;
-  if (g.ncell > 0) {
-    if (J.cell_zid)
-      OWM_LAUNCH("k_grid_cells", s, k_grid_cells_own<<<(unsigned)((g.ncell + 255) / 256), 256, 0, s>>>(J, g.ncell));
-    else
-      OWM_LAUNCH("k_grid_cells", s, k_grid_cells<<<(unsigned)((g.ncell + 7) / 8), 256, 0, s>>>(J, g.ncell));
+  if (g.z.ncell > 0) {
+    OWM_LAUNCH("k_grid_cells", s, k_grid_cells<false><<<(unsigned)((g.z.ncell + 7) / 8), 256, 0, s>>>(J, GridTiles{}, g.z.ncell));
     count_launch(launches);
   }
-  if (g.ncell <= kOutputCells) {
-    OWM_LAUNCH("k_grid_output", s, k_grid_output<<<blocks_for(g.nwin / 4 + g.ncell, 64), kSeedBlock, 0, s>>>(
-        J.cellmin, g.ncell, g.llp, d_nllp, g.seeds, d_ns3));
+  if (g.z.ncell <= kOutputCells) {
+    OWM_LAUNCH("k_grid_output", s, k_grid_output<<<blocks_for(g.z.nwin / 4 + g.z.ncell, 64), kSeedBlock, 0, s>>>(
+        J.cellmin, g.z.ncell, g.llp, d_nllp, g.seeds, d_ns3));
     count_launch(launches);
   } else {
-    OWM_LAUNCH("k_grid_flags", s, k_grid_flags<<<blocks_for(g.ncell, 152 * 8), 256, 0, s>>>(J.cellmin, g.ncell, g.flags));
+    OWM_LAUNCH("k_grid_flags", s, k_grid_flags<<<blocks_for(g.z.ncell, 152 * 8), 256, 0, s>>>(J.cellmin, g.z.ncell, g.flags));
     count_launch(launches);
-    OWM_CUDA_TRY(exclusive_scan_u32(g.flags, g.pos, g.ncell, d_ns3, g.scan_temp, g.scan_bytes, s, launches));
-    OWM_LAUNCH("k_grid_output", s, k_grid_output_scanned<<<blocks_for(g.nwin + g.ncell, 152 * 8), 256, 0, s>>>(
-        J.cellmin, g.pos, g.ncell, g.llp, d_nllp, d_ns3, g.seeds));
+    OWM_CUDA_TRY(exclusive_scan_u32(g.flags, g.pos, g.z.ncell, d_ns3, g.scan_temp, g.scan_bytes, s, launches));
+    OWM_LAUNCH("k_grid_output", s, k_grid_output_scanned<<<blocks_for(g.z.nwin + g.z.ncell, 152 * 8), 256, 0, s>>>(
+        J.cellmin, g.pos, g.z.ncell, g.llp, d_nllp, d_ns3, g.seeds));
     count_launch(launches);
   }
   OWM_CUDA_TRY(cudaGetLastError());
@@ -850,9 +1224,15 @@ extern "C" int owm_grid_classify_host(double lo, double hi, double step, int32_t
     const int how = grid_counts(a, b, FormulaEdges{&a}, counts + 4 * i);
     if (how == 2) grid_counts_exact(a, b, dkey(p[i]), FormulaEdges{&a}, counts + 4 * i);
     mode[3] += how == 0;
-    bool rare = false;
-    const int32_t cls = grid_class_fast(a, b, &rare);
-    if (a.fast && (rare ? how == 0 : how != 0 || cls != grid_sum(a, counts + 4 * i))) return 1;
+    if (!a.fast) continue;
+    uint32_t h;
+    int32_t tl, ta;
+    const int32_t cls = grid_class_fast(a, b, &h, &tl, &ta);
+    if (h & kGridOutside) {
+      if (how != 2) return 1;
+    } else if (grid_settle_fast(a, dkey(p[i]), h, tl, ta, FormulaEdges{&a}, cls) != grid_sum(a, counts + 4 * i)) {
+      return 1;
+    }
   }
   return 0;
 }

@@ -24,32 +24,39 @@ enum GridFamily { kFamL = 0, kFamR = 1, kFamA = 2, kFamB = 3 };
 // origin) times a constant is its place in window (cell) steps, whose integer
 // part is the number of edges passed.  A place within kGridGuard units of an
 // edge's nominal one is settled by comparing with the edge itself.
-struct GridAxis {
-  // Constants of the fold's fast form, for coordinates in [lo, hi] off the edges:
-  // place = mulhi(position above lo, m) + q, count = min((place >> fb) - k, n).
+struct __align__(16) GridAxis {
+  // The fast form's constants (grid_class_fast), for coordinates in [lo, hi] off
+  // the edges: place = mulhi(position above lo, m) + q, t = place >> fb,
+  // s = min(tl, lcap) + tl + 2 ta - ksum.  64 bytes that a batch's fold reads in
+  // four 16-byte words.
   int64_t lo0;               // lo's bits (linear) or whole quanta (general)
   uint64_t span;             // hi's minus lo's
-  uint32_t qw, qr, qc, qb;   // place of lo: L, R, A, B
+  int32_t sh;                // linear: bits shifted out; general: biased exponent of the quantum + 52
+  uint32_t mw, mc;           // steps per position, times 2^(32 + fb): windows, cells
+  uint32_t qw;               // place of lo: L
+  uint32_t qc;               // place of lo: A
+  int32_t fbw, fbc;          // fraction bits of a place
+  int32_t lcap;
+  int32_t ksum, par;         // par: the main parity of s
+  uint32_t fmw, fmc;         // masks of a place's fraction
+  // the rest of the form for [lo, hi]
+  uint32_t qr, qb;           // places of lo: R, B
   int32_t kl, kr, ka, kb;    // edge counts at place 0
   int32_t paired;            // R and B places lie where L and A places do: one place for both
-  int32_t lcap, ksum;        // paired: s = min(tl, lcap) + tl + 2 ta - ksum, t = place >> fb
-  int32_t fast;              // that form holds over all of [lo, hi]
+  int32_t fast;              // the fast form holds over all of [lo, hi]
   int64_t f0;                // position 0: a double's bits (linear) or whole quanta (general)
-  uint32_t mw, mc;           // steps per position, times 2^(32 + fb): windows, cells
   uint32_t c[4];             // place of position 0 by family, bias and guard added
-  int32_t fbw, fbc;          // fraction bits of a place
   int32_t kw, kc;            // bias: count = (place >> fb) - bias, clamped to [0, n]
   int32_t n, nc;             // windows, cells
   int32_t quick;             // 0: no fixed-point form (every coordinate is searched)
   int32_t linear;            // 1: the range lies in one positive binade, a double's bits are linear in it
-  int32_t sh;                // linear: bits shifted out; general: biased exponent of the quantum + 52
   int32_t merged;            // s counts the cells' edges too
   int32_t nclass;            // values of s
-  int32_t par, parmask;      // parmask 1: points off the edges all have s & 1 == par (the main parity)
+  int32_t parmask;           // 1: points off the edges all have s & 1 == par
   int32_t width[2];          // classes of the main parity, of the other
   double wbase, step, wr;    // L_j = (wbase + j * step) - wr, R_j = ... + wr
   double cbase, cr;          // A_i = (cbase + i * bsize) - cr, B_i = ... + cr
-  int32_t bsize, pad;
+  int32_t bsize;
   const int64_t* edge[4];    // order keys of the edges, by family (device)
   int32_t *lo, *hi, *clo, *chi;  // s-range of every window and cell (device; merged cells only)
 };
@@ -179,13 +186,12 @@ __host__ __device__ __forceinline__ int grid_counts_raw(const GridAxis& a, uint6
     in = in && v <= (uint32_t)a.span;
   }
   const uint32_t hl = grid_mulhi(v, a.mw) + a.qw, ha = grid_mulhi(v, a.mc) + a.qc;
-  const uint32_t mw = (1u << a.fbw) - 1u, mc = (1u << a.fbc) - 1u;
-  bool off = (hl & mw) >= 2 * kGridGuard && (ha & mc) >= 2 * kGridGuard;
+  bool off = (hl & a.fmw) >= 2 * kGridGuard && (ha & a.fmc) >= 2 * kGridGuard;
   uint32_t hr = hl, hb = ha;
   if (!a.paired) {
     hr = grid_mulhi(v, a.mw) + a.qr;
     hb = grid_mulhi(v, a.mc) + a.qb;
-    off = off && (hr & mw) >= 2 * kGridGuard && (hb & mc) >= 2 * kGridGuard;
+    off = off && (hr & a.fmw) >= 2 * kGridGuard && (hb & a.fmc) >= 2 * kGridGuard;
   }
   cnt[0] = (int32_t)(hl >> a.fbw) - a.kl;
   cnt[1] = (int32_t)(hr >> a.fbw) - a.kr;
@@ -224,16 +230,53 @@ __host__ __device__ __forceinline__ int32_t grid_sum(const GridAxis& a, const in
   return cnt[0] + cnt[1] + (a.merged ? cnt[2] + cnt[3] : 0);
 }
 
-// Class of a coordinate on an axis with the fast form; rare is set where that
-// does not settle it.
-__host__ __device__ __forceinline__ int32_t grid_class_fast(const GridAxis& a, uint64_t bits, bool* rare) {
+// Class of a coordinate on an axis with the fast form, where *how is 0.  Near a
+// window edge (kGridNearWindow), a cell edge (kGridNearCell) or both, the edges
+// that its places end at still have to be looked at (grid_settle_fast);
+// kGridOutside: not in [lo, hi].  a: a GridAxis or a copy of its first 64 bytes.
+constexpr uint32_t kGridNearWindow = 1, kGridNearCell = 2, kGridOutside = 4;
+template <class Axis>
+__host__ __device__ __forceinline__ int32_t grid_class_fast(const Axis& a, uint64_t bits, uint32_t* how, int32_t* tl,
+                                                            int32_t* ta) {
   const uint64_t d = bits - (uint64_t)a.lo0;
   const uint32_t v = (uint32_t)(d >> a.sh);
   const uint32_t hl = grid_mulhi(v, a.mw) + a.qw, ha = grid_mulhi(v, a.mc) + a.qc;
-  *rare |= (d > a.span) | ((hl & ((1u << a.fbw) - 1u)) < 2 * kGridGuard) | ((ha & ((1u << a.fbc) - 1u)) < 2 * kGridGuard);
-  const int32_t tl = (int32_t)(hl >> a.fbw), ta = (int32_t)(ha >> a.fbc);
-  return (tl < a.lcap ? tl : a.lcap) + tl + 2 * ta - a.ksum;
+  *how = (d > a.span ? kGridOutside : 0u) | ((hl & a.fmw) < 2 * kGridGuard ? kGridNearWindow : 0u) |
+         ((ha & a.fmc) < 2 * kGridGuard ? kGridNearCell : 0u);
+  *tl = (int32_t)(hl >> a.fbw);
+  *ta = (int32_t)(ha >> a.fbc);
+  return (*tl < a.lcap ? *tl : a.lcap) + *tl + 2 * *ta - a.ksum;
 }
+
+// The class s that the fast form gave near an edge counts the edges of both
+// families at that place as passed: takes back those that are not.  (Linear
+// axes: a coordinate's bits are its order key.)
+template <class EdgeOf>
+__host__ __device__ __forceinline__ int32_t grid_settle_fast(const GridAxis& a, int64_t key, uint32_t how, int32_t tl, int32_t ta,
+                                                             EdgeOf edge_of, int32_t s) {
+  if (how & kGridNearWindow) {
+    const int32_t l = tl - a.kl - 1, r = tl - a.kr - 1;
+    const bool has_l = l >= 0 && l < a.n, has_r = r >= 0 && r < a.n;
+    const int64_t el = has_l ? edge_of(kFamL, l) : 0, er = has_r ? edge_of(kFamR, r) : 0;
+    s -= (has_l && !(el < key)) + (has_r && !(er <= key));
+  }
+  if (how & kGridNearCell) {
+    const int32_t l = ta - a.ka - 1, r = ta - a.kb - 1;
+    const bool has_l = l >= 0 && l < a.nc, has_r = r >= 0 && r < a.nc;
+    const int64_t el = has_l ? edge_of(kFamA, l) : 0, er = has_r ? edge_of(kFamB, r) : 0;
+    s -= (has_l && !(el < key)) + (has_r && !(er <= key));
+  }
+  return s;
+}
+struct GridFastAxis {
+  int64_t lo0;
+  uint64_t span;
+  int32_t sh;
+  uint32_t mw, mc, qw, qc;
+  int32_t fbw, fbc, lcap, ksum, par;
+  uint32_t fmw, fmc;
+};
+static_assert(sizeof(GridFastAxis) == 64, "the first four 16-byte words of a GridAxis");
 
 // Count and (z, id)-minimum of a box, all zero when empty: w is the inverted,
 // sign-flipped order key of z and nid the inverted id, so the lexicographic
@@ -248,7 +291,7 @@ struct __align__(16) GridRow {
 // steps (overlap 0.8: W = 5 steps), every right edge nearly coincides with a
 // left one and every second class is a few ulps wide and all but empty; apart,
 // the full sub-cells lie side by side, a quarter of the table.
-struct GridJob {
+struct __align__(16) GridJob {
   GridAxis x, y;
   uint32_t base[4];      // first sub-cell of quadrant 2 * (y not main) + (x not main)
   int32_t fast;          // both axes have the fast form
@@ -264,6 +307,16 @@ struct GridJob {
   uint32_t* win;         // [windows] stage-1 ids (kept when overlap is 0)
   uint32_t thr;
   int32_t n;
+  const double* rec;     // batches: the tile's points (plain x, y, z)
+  int32_t need_dup;      // overlap > 0: LLPs are ids of two or more windows
+  int32_t pad;
+};
+
+// The tiles of a batch as a kernel sees them: off[t] is tile t's first item.
+struct GridTiles {
+  const GridJob* jobs = nullptr;
+  const int64_t* off = nullptr;
+  int32_t n = 0;
 };
 
 // Stored index of sub-cell (sx, sy).
@@ -281,11 +334,21 @@ inline int64_t grid_cells(const GridJob& j) { return (int64_t)j.x.nclass * j.y.n
 void grid_axis_setup(double lo, double hi, double step, int32_t whalf, int32_t n, int32_t bsize, int32_t nc, bool merged,
                      GridAxis* a);
 
-// The pieces of the path, in order, on stream s.  d_words: the context's small
-// words (status, LLP and stage-3 counts).
+// How many entries the tables of one cloud take (OWM_ERANGE when its sub-cells
+// cannot be numbered in 32 bits), and its job, pointers excepted.
+struct GridSizes {
+  int64_t nsub = 0, nwin = 0, ncell = 0, rows = 0, edges = 0;
+  int64_t chunks = 0;  // of a stage-2 bitmap
+  bool merged = false;  // cells share the windows' sub-cells
+};
+int grid_sizes(const owm_params& p, int64_t n, GridSizes* z);
+void grid_job(const owm_params& p, int64_t n, const GridSizes& z, GridJob* j);
+
+// The pieces of the path, in order, on stream s.
 struct GridPlan {
   GridJob job;
-  int64_t n = 0, nwin = 0, ncell = 0, nsub = 0;
+  GridSizes z;
+  int64_t n = 0;
   bool bitmap2 = true;     // stage 2 by occupancy bitmaps (overlap > 0)
   size_t clear_bytes = 0;  // from the scratch's start
   size_t bytes = 0;
@@ -298,7 +361,7 @@ struct GridPlan {
 // Sizes the plan (scratch nullptr) or carves it from scratch.
 int grid_plan(const owm_params& p, int64_t n, void* scratch, GridPlan* g);
 // Clears the tables and computes edges and ranges.
-int grid_prepare(const GridPlan& g, uint32_t* status, cudaStream_t s, int64_t* launches);
+int grid_prepare(const GridPlan& g, const owm_params& p, uint32_t* status, cudaStream_t s, int64_t* launches);
 // Folds points [first, first + count) of the cloud, ids first + 1 ...
 int grid_fold(const GridPlan& g, const double* rec, int stride, int64_t first, int64_t count, uint32_t* status,
               cudaStream_t s, int64_t* launches);
@@ -307,5 +370,37 @@ int grid_windows(const GridPlan& g, cudaStream_t s, int64_t* launches);
 int grid_stage2(const GridPlan& g, const owm_params& p, const double* xy, int xy_stride, uint32_t* d_nllp,
                 cudaStream_t s, int64_t* launches);
 int grid_stage3(const GridPlan& g, const uint32_t* d_nllp, uint32_t* d_ns3, cudaStream_t s, int64_t* launches);
+
+// Many tiles at once: one launch per step, every tile with its own job.
+struct GridBatch {
+  int32_t ntiles = 0, chunk = 0;  // chunk: points per fold block
+  int32_t bitmap2 = 1;            // every tile has overlap > 0
+  int32_t tile_bits = 1, id_bits = 1;
+  int64_t items = 0, folds = 0, rows = 0, wins = 0, chunks = 0, cells = 0;  // totals over the tiles
+  size_t clear_bytes = 0, table_bytes = 0, bytes = 0;
+  char* base = nullptr;
+  char *zid = nullptr, *count = nullptr, *cell_zid = nullptr, *mark = nullptr, *edges = nullptr, *row_mem = nullptr,
+       *cellmin = nullptr;
+  // device tables, written by the host for each batch: the jobs and, per kind
+  // of item, the tiles' first ones
+  GridJob* jobs = nullptr;
+  int64_t *item_off = nullptr, *fold_off = nullptr, *row_off = nullptr, *win_off = nullptr, *chunk_off = nullptr,
+          *cell_off = nullptr;
+  uint32_t *bitmap = nullptr, *part = nullptr, *llp = nullptr, *llp_off = nullptr, *s3cnt = nullptr, *words = nullptr;
+  int64_t *out = nullptr, *out_off = nullptr;
+  uint32_t *win = nullptr, *k0 = nullptr, *k1 = nullptr, *flags = nullptr, *pos = nullptr, *cnt2 = nullptr;
+  void *sort_temp = nullptr, *scan_temp = nullptr;
+  size_t sort_bytes = 0, scan_bytes = 0;
+};
+// Sizes and lays out a batch (base nullptr: sizes only; else 256-byte aligned).
+// p[t], n[t]: parameters and points per tile; z[t] gets the tile's sizes.
+int grid_batch_plan(const owm_params* p, const int64_t* n, int32_t ntiles, GridSizes* z, char* base, GridBatch* g);
+// The tables of a batch that was laid out, as they go to the device: table_bytes
+// from g.jobs on.  rec[t]: the tile's points on the device.
+void grid_batch_tables(const owm_params* p, const int64_t* n, const GridSizes* z, const double* const* rec, const GridBatch& g,
+                       char* host);
+// All device work of a batch whose tables are on the device; words[0] is the
+// status word.  out and out_off hold the seeds.  Capturable.
+int grid_batch_run(const GridBatch& g, cudaStream_t s, int64_t* launches);
 
 }  // namespace owm

@@ -161,7 +161,7 @@ int run_grid(owm_ctx* c, const PointsView& pts, int64_t n, const owm_params& p, 
   uint32_t* d_nllp = c->d_small + kLlpSlot;
   uint32_t* d_ns3 = c->d_small + kS3Slot;
   OWM_CUDA_TRY(cudaEventRecord(c->ev[0], s));
-  rc = grid_prepare(g, status, s, &c->launches);
+  rc = grid_prepare(g, p, status, s, &c->launches);
   if (!rc) rc = grid_fold(g, pts.rec, pts.rec_stride, 0, n, status, s, &c->launches);
   if (rc) return rc;
   OWM_CUDA_TRY(cudaEventRecord(c->ev[1], s));
@@ -175,7 +175,7 @@ int run_grid(owm_ctx* c, const PointsView& pts, int64_t n, const owm_params& p, 
   if (rc) return rc;
   OWM_CUDA_TRY(cudaEventRecord(c->ev[4], s));
   *d_seeds = g.seeds;
-  *room = g.nwin + g.ncell + 1;
+  *room = g.z.nwin + g.z.ncell + 1;
   return OWM_OK;
 }
 }  // namespace
