@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(256) k_grid_prepare(const __grid_constant__ Gr
       prepare_axis(J.y, (int32_t)k - nx);
     } else {
       const int q = (int)(k - nx - ny);
-      J.occ[q] = !(q < 2 ? J.x : J.y).parmask || (q & 1) == 0;
+      J.occ[q] = (q & 1) == 0;  // the other parity: when a point says so
     }
   }
   if (t == 0) *status = 0;
@@ -150,18 +150,26 @@ __device__ __forceinline__ void raise_zid(ulonglong2* p, ulonglong2 cur, unsigne
   }
 }
 
-// Point i as raw bits, read once: 32-byte records or plain 24-byte points.
+// Point i as raw bits, and its inverted id; every point is read once.
 template <int kStride>
-__device__ __forceinline__ void load_raw(const double* __restrict__ rec, int64_t i, uint64_t& x, uint64_t& y, uint64_t& z) {
+__device__ __forceinline__ void load_raw(const GridPoints& pts, int64_t i, uint64_t& x, uint64_t& y, uint64_t& z,
+                                         uint32_t& nid) {
   if (kStride == 4) {
     asm("ld.global.nc.L1::no_allocate.L2::evict_first.v4.b64 {%0, %1, %2, _}, [%3];"
         : "=l"(x), "=l"(y), "=l"(z)
-        : "l"(rec + 4 * i));
-  } else {
-    const uint64_t* p = reinterpret_cast<const uint64_t*>(rec) + 3 * i;
+        : "l"(pts.rec + 4 * i));
+    nid = ~(uint32_t)(i + 1);
+  } else if (kStride == 3) {
+    const uint64_t* p = reinterpret_cast<const uint64_t*>(pts.rec) + 3 * i;
     x = __ldg(p);
     y = __ldg(p + 1);
     z = __ldg(p + 2);
+    nid = ~(uint32_t)(i + 1);
+  } else {
+    x = (uint64_t)__double_as_longlong(dkey_inv(__ldg(pts.xk + i)));
+    y = (uint64_t)__double_as_longlong(dkey_inv(__ldg(pts.yk + i)));
+    z = (uint64_t)__double_as_longlong(dkey_inv(__ldg(pts.zk + i)));
+    nid = ~__ldg(pts.id + i);
   }
 }
 
@@ -231,10 +239,10 @@ struct SharedAxes {
   const GridJob* J;
   static __device__ __forceinline__ GridFastAxis load(const GridAxis* a) {
     GridFastAxis f;
-    uint4 w[4];
+    uint4 w[5];
     const uint32_t at = (uint32_t)__cvta_generic_to_shared(a);
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
+    for (int k = 0; k < 5; ++k)
       asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
                    : "=r"(w[k].x), "=r"(w[k].y), "=r"(w[k].z), "=r"(w[k].w)
                    : "r"(at + 16 * k));
@@ -245,8 +253,8 @@ struct SharedAxes {
   __device__ __forceinline__ GridFastAxis y() const { return load(&J->y); }
 };
 
-template <int kStride, bool kFast, class Axes>
-__device__ __forceinline__ void fold_stretch(const GridJob& J, Axes axes, const double* __restrict__ rec, int64_t first,
+template <int kStride, int kFast, class Axes>
+__device__ __forceinline__ void fold_stretch(const GridJob& J, Axes axes, const GridPoints& pts, int64_t first,
                                              int64_t count, int64_t b, int64_t e, uint32_t& flags) {
   const int lane = threadIdx.x & 31;
   for (; b < e; b += 32) {
@@ -254,32 +262,33 @@ __device__ __forceinline__ void fold_stretch(const GridJob& J, Axes axes, const 
     const int32_t left = (int32_t)min((int64_t)32, count - b);
     const int64_t i = first + b + min(lane, left - 1);
     uint64_t x, y, z;
-    load_raw<kStride>(rec, i, x, y, z);
-    uint32_t cell, nid = ~(uint32_t)(i + 1);
+    uint32_t cell, nid;
+    load_raw<kStride>(pts, i, x, y, z, nid);
     unsigned long long w;
     if (kFast) {
-      int32_t tlx, tax, tly, tay;
+      int32_t tx[4], ty[4];
       uint32_t hx, hy, other;
       const auto& ax = axes.x();
-      int32_t sx = grid_class_fast(ax, x, &hx, &tlx, &tax);
-      other = sx ^ ax.par;
+      int32_t sx = grid_class_fast<kFast == 2>(ax, x, &hx, tx);
+      other = (sx ^ ax.par) & ax.parmask;
+      const uint32_t ix = (uint32_t)(sx >> ax.parmask);
       const auto& ay = axes.y();
-      int32_t sy = grid_class_fast(ay, y, &hy, &tly, &tay);
-      other |= sy ^ ay.par;
-      cell = (uint32_t)(sy >> 1) * (uint32_t)J.x.width[0] + (uint32_t)(sx >> 1);
+      int32_t sy = grid_class_fast<kFast == 2>(ay, y, &hy, ty);
+      other |= (sy ^ ay.par) & ay.parmask;
+      cell = (uint32_t)(sy >> ay.parmask) * (uint32_t)J.x.width[0] + ix;
       w = z ^ (~(uint64_t)((int64_t)z >> 63) & 0x7FFFFFFFFFFFFFFFull);
       const bool odd_z = ((uint32_t)(z >> 32) << 1) - 1u >= 0xFFDFFFFFu;  // zero or not finite
-      if (odd_z | ((other & 1u) | hx | hy)) {
+      if (odd_z | (other | hx | hy)) {
         if (odd_z | ((hx | hy) & kGridOutside)) {
           const PointCell p = point_cell_call(J, x, y, z);
           cell = p.cell;
           w = p.w;
           flags |= p.flags;
         } else {
-          if (hx) sx = grid_settle_fast(J.x, (int64_t)x, hx, tlx, tax, StoredEdges{&J.x}, sx);
-          if (hy) sy = grid_settle_fast(J.y, (int64_t)y, hy, tly, tay, StoredEdges{&J.y}, sy);
+          if (hx) sx = grid_settle_fast(J.x, (int64_t)x, hx, tx, StoredEdges{&J.x}, sx);
+          if (hy) sy = grid_settle_fast(J.y, (int64_t)y, hy, ty, StoredEdges{&J.y}, sy);
           cell = grid_cell(J, sx, sy);
-          flags |= (((sx ^ J.x.par) & 1) ? kPointOtherX : 0u) | (((sy ^ J.y.par) & 1) ? kPointOtherY : 0u);
+          flags |= (((sx ^ J.x.par) & J.x.parmask) ? kPointOtherX : 0u) | (((sy ^ J.y.par) & J.y.parmask) ? kPointOtherY : 0u);
         }
       }
     } else {
@@ -294,7 +303,7 @@ __device__ __forceinline__ void fold_stretch(const GridJob& J, Axes axes, const 
     const uint32_t before = __shfl_up_sync(0xffffffffu, cell, 1);
     const uint32_t heads = __ballot_sync(0xffffffffu, before != cell) | 1u;
     if (heads == 0xFFFFFFFFu) {  // none (a lane past the end would repeat its neighbour)
-      atomicAdd(J.count + cell, 1u);
+      atomicAdd(J.count + grid_count_slot(J, cell), 1u);
       if (w >= cur.x) raise_zid(J.zid + cell, cur, w, nid);
       continue;
     }
@@ -302,7 +311,7 @@ __device__ __forceinline__ void fold_stretch(const GridJob& J, Axes axes, const 
     const int end = after ? __ffs(after) - 1 : 32;
     const bool head = (heads >> lane) & 1u;
     const int run = min(end, left) - lane;
-    if (head && run > 0) atomicAdd(J.count + cell, (uint32_t)run);
+    if (head && run > 0) atomicAdd(J.count + grid_count_slot(J, cell), (uint32_t)run);
     if (!__any_sync(0xffffffffu, w >= cur.x)) continue;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {  // the run's minimum, to its head
@@ -328,15 +337,15 @@ __device__ __forceinline__ void fold_flags(const GridJob& J, uint32_t flags, uin
   }
 }
 
-template <int kStride, bool kFast>
+template <int kStride, int kFast>
 __global__ void __launch_bounds__(kFoldBlock, kFoldBlocks)
-    k_grid_fold(const __grid_constant__ GridJob J, const double* __restrict__ rec, int64_t first, int64_t count,
+    k_grid_fold(const __grid_constant__ GridJob J, const __grid_constant__ GridPoints pts, int64_t first, int64_t count,
                 uint32_t* __restrict__ status) {
   const int64_t nwarps = ((int64_t)gridDim.x * kFoldBlock) >> 5;
   uint32_t flags = 0;
   int64_t t0, t1;
   chunk_tiles((count + 31) / 32, nwarps, ((int64_t)blockIdx.x * kFoldBlock + threadIdx.x) >> 5, &t0, &t1);
-  fold_stretch<kStride, kFast>(J, ParamAxes{&J}, rec, first, count, t0 * 32, t1 * 32, flags);
+  fold_stretch<kStride, kFast>(J, ParamAxes{&J}, pts, first, count, t0 * 32, t1 * 32, flags);
   fold_flags(J, flags, status);
 }
 
@@ -354,13 +363,17 @@ __global__ void __launch_bounds__(kFoldBlock, kFoldBlocks)
   __syncthreads();
   const int64_t c0 = (blk - __ldg(T.off + t)) * (int64_t)chunk;
   const int64_t n = min((int64_t)chunk, J.n - c0);  // points of this block
+  GridPoints pts;
+  pts.rec = J.rec;
   uint32_t flags = 0;
   int64_t t0, t1;
   chunk_tiles((n + 31) / 32, kFoldBlock / 32, threadIdx.x >> 5, &t0, &t1);
-  if (J.fast)
-    fold_stretch<3, true>(J, SharedAxes{&J}, J.rec, 0, J.n, c0 + t0 * 32, c0 + t1 * 32, flags);
+  if (J.fast == 2)
+    fold_stretch<3, 2>(J, SharedAxes{&J}, pts, 0, J.n, c0 + t0 * 32, c0 + t1 * 32, flags);
+  else if (J.fast)
+    fold_stretch<3, 1>(J, SharedAxes{&J}, pts, 0, J.n, c0 + t0 * 32, c0 + t1 * 32, flags);
   else
-    fold_stretch<3, false>(J, SharedAxes{&J}, J.rec, 0, J.n, c0 + t0 * 32, c0 + t1 * 32, flags);
+    fold_stretch<3, 0>(J, SharedAxes{&J}, pts, 0, J.n, c0 + t0 * 32, c0 + t1 * 32, flags);
   fold_flags(J, flags, status);
 }
 
@@ -376,16 +389,19 @@ struct Best {
   }
 };
 
-// First and last s >> 1 of the classes lo..hi of the main (q = 0) or the other
-// parity; false when there are none or they hold no point.
+// First and last stored index of the classes lo..hi of the main (q = 0) or the
+// other parity; false when there are none or they hold no point.
 __device__ __forceinline__ bool parity_range(const GridAxis& a, const uint32_t* occ, int q, int32_t lo, int32_t hi,
                                              int32_t* i0, int32_t* i1) {
   if (!occ[q]) return false;
-  const int32_t par = a.par ^ q, s0 = lo + ((lo ^ par) & 1), s1 = hi - ((hi ^ par) & 1);
-  if (s0 > s1) return false;
-  *i0 = s0 >> 1;
-  *i1 = s1 >> 1;
-  return true;
+  if (a.parmask) {
+    const int32_t par = a.par ^ q;
+    lo += (lo ^ par) & 1;
+    hi -= (hi ^ par) & 1;
+  }
+  *i0 = lo >> a.parmask;
+  *i1 = hi >> a.parmask;
+  return lo <= hi;
 }
 
 template <bool kMulti>
@@ -404,7 +420,7 @@ __global__ void __launch_bounds__(256) k_grid_rows(const __grid_constant__ GridJ
       const int64_t at = J.base[2 * qy + q] + (int64_t)iy * J.x.width[q];
       for (int64_t c = at + i0; c <= at + i1; ++c) {
         const ulonglong2 e = J.zid[c];
-        m.count += J.count[c];
+        m.count += J.count[grid_count_slot(J, (uint32_t)c)];
         m.take(e.x, (uint32_t)e.y);
       }
     }
@@ -731,6 +747,13 @@ bool place_setup(double origin, double qv, double l0, double r0, double step, ui
 
 }  // namespace
 
+// Whether windows (and cells whose edges count too) tile an axis in whole
+// steps, so that every right edge nominally coincides with a left one.
+static bool steps_tile(int32_t whalf, double step, int32_t bsize, bool cells) {
+  const double steps = 2.0 * whalf / step;
+  return std::fabs(steps - std::round(steps)) < 1e-6 && (!cells || bsize % 2 == 0);
+}
+
 void grid_axis_setup(double lo, double hi, double step, int32_t whalf, int32_t n, int32_t bsize, int32_t nc, bool merged,
                      GridAxis* a) {
   std::memset(a, 0, sizeof(*a));
@@ -831,22 +854,22 @@ void grid_axis_setup(double lo, double hi, double step, int32_t whalf, int32_t n
     a->lo0 = (int64_t)0xFFFFFFFFFFFFFFFFull;
     a->sh = 0;
   }
-  // Whether every right edge nominally coincides with a left one (and the
-  // cells' edges with one another): then the classes off the edges are all of
-  // one parity, which is read off the middle of the axis.  Only a hint: a
-  // point of the other parity says so in J.occ.
-  const double steps = 2.0 * whalf / step;
-  if (std::fabs(steps - std::round(steps)) < 1e-6 && (!merged || nc == 0 || bsize % 2 == 0)) {
+  // Where every right edge nominally coincides with a left one, the classes off
+  // the edges are all of one parity, read off the middle of the axis.  Only a
+  // hint: a point of the other parity says so in J.occ.
+  if (steps_tile(whalf, step, bsize, merged && nc > 0)) {
     int32_t cnt[4];
     const double mid = lo + 0.4637 * span;
     grid_counts_exact(*a, (uint64_t)bits_of(mid), dkey(mid), FormulaEdges{a}, cnt);
     a->par = grid_sum(*a, cnt) & 1;
     a->parmask = 1;
+    const int32_t even = (a->nclass + 1) / 2;
+    a->width[0] = a->par ? a->nclass - even : even;
+    a->width[1] = a->nclass - a->width[0];
+  } else {
+    a->width[0] = a->nclass;
   }
-  const int32_t even = (a->nclass + 1) / 2;
-  a->width[0] = a->par ? a->nclass - even : even;
-  a->width[1] = a->nclass - a->width[0];
-  if (a->paired && a->linear && a->parmask && (merged || nc == 0)) {
+  if (a->quick && a->linear && (merged || nc == 0)) {
     a->lcap = n + a->kl;
     a->ksum = a->kl + a->kr + a->ka + a->kb;
     int32_t at_lo[4], at_hi[4];  // no clamps but the left windows' upper one
@@ -868,6 +891,10 @@ int grid_sizes(const owm_params& p, int64_t n, GridSizes* z) {
   z->merged = cells && (tx + 2 * ncg) * (ty + 2 * nrg) <= std::min<int64_t>(std::max<int64_t>(4 * tx * ty, 1 << 20), 1 << 28);
   const int64_t sx = tx + (z->merged ? 2 * ncg : 0), sy = ty + (z->merged ? 2 * nrg : 0);
   z->nsub = sx * sy;
+  // the sub-cells that points in no order spread over: all, or one quadrant
+  const bool tile = steps_tile((uint16_t)p.wsize / 2, p.displace, (uint16_t)p.bsize, z->merged);
+  const int64_t main = tile ? ((sx + 1) / 2) * ((sy + 1) / 2) : z->nsub;
+  z->counts = z->nsub + (main <= kGridSpreadMax ? 3 * main : 0);
   z->nwin = nc * nr;
   z->ncell = ncg * nrg;
   z->rows = sy * nc;
@@ -889,7 +916,8 @@ void grid_job(const owm_params& p, int64_t n, const GridSizes& z, GridJob* j) {
   J.base[1] = (uint32_t)J.x.width[0] * (uint32_t)J.y.width[0];
   J.base[2] = J.base[1] + (uint32_t)J.x.width[1] * (uint32_t)J.y.width[0];
   J.base[3] = J.base[2] + (uint32_t)J.x.width[0] * (uint32_t)J.y.width[1];
-  J.fast = J.x.fast && J.y.fast && (z.merged || z.ncell == 0);
+  if (z.counts > z.nsub) J.spread = J.x.parmask ? J.base[1] : (uint32_t)z.nsub;
+  J.fast = J.x.fast && J.y.fast && (z.merged || z.ncell == 0) ? (J.x.paired && J.y.paired ? 2 : 1) : 0;
 }
 
 namespace {
@@ -928,20 +956,22 @@ int64_t prepare_items(const owm_params& p, const GridSizes& z) {
 }
 }  // namespace
 
-int grid_plan(const owm_params& p, int64_t n, void* scratch, GridPlan* g) {
+int grid_plan(const owm_params& p_in, int64_t n, void* scratch, GridPlan* g, bool stage1_only) {
   *g = GridPlan{};
   GridJob& J = g->job;
+  owm_params p = p_in;
+  if (stage1_only) p.bsize = 0;  // no cells
   if (p.ncells <= 0) return OWM_EINVAL;
   const int rc = grid_sizes(p, n, &g->z);
   if (rc) return rc;
   const GridSizes& z = g->z;
   if (scratch) grid_job(p, n, z, &J);
   g->n = n;
-  g->bitmap2 = p.overlap > 0.0;
+  g->bitmap2 = p.overlap > 0.0 && !stage1_only;
   Carver c{static_cast<char*>(scratch)};
   // cleared
   J.zid = c.take<ulonglong2>(z.nsub);
-  J.count = c.take<uint32_t>(z.nsub);
+  J.count = c.take<uint32_t>(z.counts);
   if (!z.merged && z.ncell) J.cell_zid = c.take<ulonglong2>(z.ncell);
   if (g->bitmap2) {
     J.once = c.take<uint32_t>(z.chunks * kSeedChunk);
@@ -953,6 +983,12 @@ int grid_plan(const owm_params& p, int64_t n, void* scratch, GridPlan* g) {
   char* edges = c.take<char>(z.edges);
   if (edges) carve_edges(J, edges);
   J.rows = c.take<GridRow>(z.rows);
+  if (stage1_only) {
+    J.win = c.take<uint32_t>(z.nwin);
+    g->bytes = c.at;
+    g->base = c.base;
+    return OWM_OK;
+  }
   J.cellmin = c.take<uint32_t>(z.ncell);
   g->llp = c.take<uint32_t>(z.nwin);
   g->seeds = c.take<int64_t>(z.nwin + z.ncell + 1);
@@ -979,7 +1015,7 @@ int grid_batch_plan(const owm_params* p, const int64_t* n, int32_t ntiles, GridS
   g->ntiles = ntiles;
   g->bitmap2 = 1;
   g->tile_bits = g->id_bits = 1;
-  int64_t points = 0, nsub = 0, own = 0, edges = 0, maxn = 0;
+  int64_t points = 0, nsub = 0, counts = 0, own = 0, edges = 0, maxn = 0;
   for (int32_t k = 0; k < ntiles; ++k) {
     const int rc = grid_sizes(p[k], n[k], &z[k]);
     if (rc) return rc;
@@ -987,6 +1023,7 @@ int grid_batch_plan(const owm_params* p, const int64_t* n, int32_t ntiles, GridS
     points += n[k];
     maxn = std::max(maxn, n[k]);
     nsub += z[k].nsub;
+    counts += z[k].counts;
     own += z[k].merged ? 0 : z[k].ncell;
     edges += (z[k].edges + 15) & ~(int64_t)15;
     g->items += prepare_items(p[k], z[k]);
@@ -1005,7 +1042,7 @@ int grid_batch_plan(const owm_params* p, const int64_t* n, int32_t ntiles, GridS
 
   Carver c{base};
   g->zid = c.take<char>(nsub * 16);
-  g->count = c.take<char>(nsub * 4);
+  g->count = c.take<char>(counts * 4);
   g->cell_zid = c.take<char>(own * 16);
   g->bitmap = g->bitmap2 ? c.take<uint32_t>(2 * g->chunks * kSeedChunk) : nullptr;
   g->mark = c.take<char>(g->cells);
@@ -1049,14 +1086,15 @@ void grid_batch_tables(const owm_params* p, const int64_t* n, const GridSizes* z
   int64_t *items = (int64_t*)at(g.item_off), *folds = (int64_t*)at(g.fold_off), *rows = (int64_t*)at(g.row_off),
           *wins = (int64_t*)at(g.win_off), *chunks = (int64_t*)at(g.chunk_off), *cells = (int64_t*)at(g.cell_off);
   items[0] = folds[0] = rows[0] = wins[0] = chunks[0] = cells[0] = 0;
-  int64_t sub = 0, own = 0, edges = 0;
+  int64_t sub = 0, counts = 0, own = 0, edges = 0;
   for (int32_t k = 0; k < g.ntiles; ++k) {
     GridJob& J = jobs[k];
     grid_job(p[k], n[k], z[k], &J);
     J.rec = rec[k];
     J.zid = (ulonglong2*)g.zid + sub;
-    J.count = (uint32_t*)g.count + sub;
+    J.count = (uint32_t*)g.count + counts;
     sub += z[k].nsub;
+    counts += z[k].counts;
     if (!z[k].merged && z[k].ncell) {
       J.cell_zid = (ulonglong2*)g.cell_zid + own;
       own += z[k].ncell;
@@ -1134,14 +1172,17 @@ int grid_prepare(const GridPlan& g, const owm_params& p, uint32_t* status, cudaS
   return OWM_OK;
 }
 
-int grid_fold(const GridPlan& g, const double* rec, int stride, int64_t first, int64_t count, uint32_t* status,
-              cudaStream_t s, int64_t* launches) {
+int grid_fold(const GridPlan& g, const GridPoints& pts, int64_t first, int64_t count, uint32_t* status, cudaStream_t s,
+              int64_t* launches) {
   if (count <= 0) return OWM_OK;
   const GridJob& J = g.job;
   const unsigned nb = blocks_for(count, 152 * kFoldBlocks, kFoldBlock);
-  auto kernel = J.fast ? (stride == 4 ? k_grid_fold<4, true> : k_grid_fold<3, true>)
-                       : (stride == 4 ? k_grid_fold<4, false> : k_grid_fold<3, false>);
-  OWM_LAUNCH("k_grid_fold", s, kernel<<<nb, kFoldBlock, 0, s>>>(J, rec, first, count, status));
+  using Kernel = void (*)(GridJob, GridPoints, int64_t, int64_t, uint32_t*);
+  static const Kernel kernels[3][3] = {{k_grid_fold<0, 0>, k_grid_fold<0, 1>, k_grid_fold<0, 2>},
+                                       {k_grid_fold<3, 0>, k_grid_fold<3, 1>, k_grid_fold<3, 2>},
+                                       {k_grid_fold<4, 0>, k_grid_fold<4, 1>, k_grid_fold<4, 2>}};
+  const Kernel kernel = kernels[pts.stride == 4 ? 2 : pts.stride == 3 ? 1 : 0][J.fast];
+  OWM_LAUNCH("k_grid_fold", s, kernel<<<nb, kFoldBlock, 0, s>>>(J, pts, first, count, status));
   count_launch(launches);
   OWM_CUDA_TRY(cudaGetLastError());
   return OWM_OK;
@@ -1226,11 +1267,11 @@ extern "C" int owm_grid_classify_host(double lo, double hi, double step, int32_t
     mode[3] += how == 0;
     if (!a.fast) continue;
     uint32_t h;
-    int32_t tl, ta;
-    const int32_t cls = grid_class_fast(a, b, &h, &tl, &ta);
+    int32_t t[4];
+    const int32_t cls = a.paired ? grid_class_fast<true>(a, b, &h, t) : grid_class_fast<false>(a, b, &h, t);
     if (h & kGridOutside) {
       if (how != 2) return 1;
-    } else if (grid_settle_fast(a, dkey(p[i]), h, tl, ta, FormulaEdges{&a}, cls) != grid_sum(a, counts + 4 * i)) {
+    } else if (grid_settle_fast(a, dkey(p[i]), h, t, FormulaEdges{&a}, cls) != grid_sum(a, counts + 4 * i)) {
       return 1;
     }
   }

@@ -26,9 +26,9 @@ enum GridFamily { kFamL = 0, kFamR = 1, kFamA = 2, kFamB = 3 };
 // edge's nominal one is settled by comparing with the edge itself.
 struct __align__(16) GridAxis {
   // The fast form's constants (grid_class_fast), for coordinates in [lo, hi] off
-  // the edges: place = mulhi(position above lo, m) + q, t = place >> fb,
-  // s = min(tl, lcap) + tl + 2 ta - ksum.  64 bytes that a batch's fold reads in
-  // four 16-byte words.
+  // the edges: place = mulhi(position above lo, m) + q by family, t = place >> fb,
+  // s = min(tl, lcap) + tr + ta + tb - ksum.  80 bytes that a batch's fold reads
+  // in five 16-byte words.
   int64_t lo0;               // lo's bits (linear) or whole quanta (general)
   uint64_t span;             // hi's minus lo's
   int32_t sh;                // linear: bits shifted out; general: biased exponent of the quantum + 52
@@ -39,8 +39,9 @@ struct __align__(16) GridAxis {
   int32_t lcap;
   int32_t ksum, par;         // par: the main parity of s
   uint32_t fmw, fmc;         // masks of a place's fraction
-  // the rest of the form for [lo, hi]
   uint32_t qr, qb;           // places of lo: R, B
+  int32_t parmask, pad;      // 1: points off the edges all have s & 1 == par
+  // the rest of the form for [lo, hi]
   int32_t kl, kr, ka, kb;    // edge counts at place 0
   int32_t paired;            // R and B places lie where L and A places do: one place for both
   int32_t fast;              // the fast form holds over all of [lo, hi]
@@ -52,8 +53,7 @@ struct __align__(16) GridAxis {
   int32_t linear;            // 1: the range lies in one positive binade, a double's bits are linear in it
   int32_t merged;            // s counts the cells' edges too
   int32_t nclass;            // values of s
-  int32_t parmask;           // 1: points off the edges all have s & 1 == par
-  int32_t width[2];          // classes of the main parity, of the other
+  int32_t width[2];          // stored classes: of the main parity, of the other; all, none (parmask 0)
   double wbase, step, wr;    // L_j = (wbase + j * step) - wr, R_j = ... + wr
   double cbase, cr;          // A_i = (cbase + i * bsize) - cr, B_i = ... + cr
   int32_t bsize;
@@ -232,36 +232,45 @@ __host__ __device__ __forceinline__ int32_t grid_sum(const GridAxis& a, const in
 
 // Class of a coordinate on an axis with the fast form, where *how is 0.  Near a
 // window edge (kGridNearWindow), a cell edge (kGridNearCell) or both, the edges
-// that its places end at still have to be looked at (grid_settle_fast);
-// kGridOutside: not in [lo, hi].  a: a GridAxis or a copy of its first 64 bytes.
+// that its places t (by family) end at still have to be looked at
+// (grid_settle_fast); kGridOutside: not in [lo, hi].  kPaired: the axis is
+// (R shares L's place, B shares A's).  a: a GridAxis or a copy of its first 80
+// bytes.
 constexpr uint32_t kGridNearWindow = 1, kGridNearCell = 2, kGridOutside = 4;
-template <class Axis>
-__host__ __device__ __forceinline__ int32_t grid_class_fast(const Axis& a, uint64_t bits, uint32_t* how, int32_t* tl,
-                                                            int32_t* ta) {
+template <bool kPaired, class Axis>
+__host__ __device__ __forceinline__ int32_t grid_class_fast(const Axis& a, uint64_t bits, uint32_t* how, int32_t t[4]) {
   const uint64_t d = bits - (uint64_t)a.lo0;
   const uint32_t v = (uint32_t)(d >> a.sh);
-  const uint32_t hl = grid_mulhi(v, a.mw) + a.qw, ha = grid_mulhi(v, a.mc) + a.qc;
-  *how = (d > a.span ? kGridOutside : 0u) | ((hl & a.fmw) < 2 * kGridGuard ? kGridNearWindow : 0u) |
-         ((ha & a.fmc) < 2 * kGridGuard ? kGridNearCell : 0u);
-  *tl = (int32_t)(hl >> a.fbw);
-  *ta = (int32_t)(ha >> a.fbc);
-  return (*tl < a.lcap ? *tl : a.lcap) + *tl + 2 * *ta - a.ksum;
+  const uint32_t mw = grid_mulhi(v, a.mw), mc = grid_mulhi(v, a.mc);
+  const uint32_t hl = mw + a.qw, ha = mc + a.qc;
+  bool nw = (hl & a.fmw) < 2 * kGridGuard, nc = (ha & a.fmc) < 2 * kGridGuard;
+  t[0] = t[1] = (int32_t)(hl >> a.fbw);
+  t[2] = t[3] = (int32_t)(ha >> a.fbc);
+  if (!kPaired) {
+    const uint32_t hr = mw + a.qr, hb = mc + a.qb;
+    nw |= (hr & a.fmw) < 2 * kGridGuard;
+    nc |= (hb & a.fmc) < 2 * kGridGuard;
+    t[1] = (int32_t)(hr >> a.fbw);
+    t[3] = (int32_t)(hb >> a.fbc);
+  }
+  *how = (d > a.span ? kGridOutside : 0u) | (nw ? kGridNearWindow : 0u) | (nc ? kGridNearCell : 0u);
+  return (t[0] < a.lcap ? t[0] : a.lcap) + t[1] + t[2] + t[3] - a.ksum;
 }
 
-// The class s that the fast form gave near an edge counts the edges of both
-// families at that place as passed: takes back those that are not.  (Linear
-// axes: a coordinate's bits are its order key.)
+// The class s that the fast form gave near an edge counts the edges at its
+// places as passed: takes back those that are not.  (Linear axes: a
+// coordinate's bits are its order key.)
 template <class EdgeOf>
-__host__ __device__ __forceinline__ int32_t grid_settle_fast(const GridAxis& a, int64_t key, uint32_t how, int32_t tl, int32_t ta,
+__host__ __device__ __forceinline__ int32_t grid_settle_fast(const GridAxis& a, int64_t key, uint32_t how, const int32_t t[4],
                                                              EdgeOf edge_of, int32_t s) {
   if (how & kGridNearWindow) {
-    const int32_t l = tl - a.kl - 1, r = tl - a.kr - 1;
+    const int32_t l = t[0] - a.kl - 1, r = t[1] - a.kr - 1;
     const bool has_l = l >= 0 && l < a.n, has_r = r >= 0 && r < a.n;
     const int64_t el = has_l ? edge_of(kFamL, l) : 0, er = has_r ? edge_of(kFamR, r) : 0;
     s -= (has_l && !(el < key)) + (has_r && !(er <= key));
   }
   if (how & kGridNearCell) {
-    const int32_t l = ta - a.ka - 1, r = ta - a.kb - 1;
+    const int32_t l = t[2] - a.ka - 1, r = t[3] - a.kb - 1;
     const bool has_l = l >= 0 && l < a.nc, has_r = r >= 0 && r < a.nc;
     const int64_t el = has_l ? edge_of(kFamA, l) : 0, er = has_r ? edge_of(kFamB, r) : 0;
     s -= (has_l && !(el < key)) + (has_r && !(er <= key));
@@ -274,9 +283,10 @@ struct GridFastAxis {
   int32_t sh;
   uint32_t mw, mc, qw, qc;
   int32_t fbw, fbc, lcap, ksum, par;
-  uint32_t fmw, fmc;
+  uint32_t fmw, fmc, qr, qb;
+  int32_t parmask, pad;
 };
-static_assert(sizeof(GridFastAxis) == 64, "the first four 16-byte words of a GridAxis");
+static_assert(sizeof(GridFastAxis) == 80, "the first five 16-byte words of a GridAxis");
 
 // Count and (z, id)-minimum of a box, all zero when empty: w is the inverted,
 // sign-flipped order key of z and nid the inverted id, so the lexicographic
@@ -286,17 +296,18 @@ struct __align__(16) GridRow {
   uint32_t nid, count;
 };
 
-// Sub-cells are stored by quadrants of the two axes' parities (s >> 1 within a
-// quadrant), main parity first: where windows and cells tile the axes in whole
-// steps (overlap 0.8: W = 5 steps), every right edge nearly coincides with a
-// left one and every second class is a few ulps wide and all but empty; apart,
-// the full sub-cells lie side by side, a quarter of the table.
+// Where windows and cells tile the axes in whole steps (overlap 0.8: W = 5
+// steps), every right edge nearly coincides with a left one and every second
+// class is a few ulps wide and all but empty.  Sub-cells of such an axis
+// (parmask) are stored by parity, the main one first, s >> 1 within it: the
+// full sub-cells of two such axes lie side by side, a quarter of the table.
 struct __align__(16) GridJob {
   GridAxis x, y;
   uint32_t base[4];      // first sub-cell of quadrant 2 * (y not main) + (x not main)
-  int32_t fast;          // both axes have the fast form
+  int32_t fast;          // both axes have the fast form: 2 paired, 1 not
+  uint32_t spread;       // the first sub-cells, whose counts lie 16 bytes apart
   ulonglong2* zid;       // [sub-cells] (w, nid)
-  uint32_t* count;       // [sub-cells]
+  uint32_t* count;       // [sub-cells], at grid_count_slot
   ulonglong2* cell_zid;  // [cells] (w, nid), when the cells are not merged
   GridRow* rows;         // [y.nclass][x.n], main parity first
   uint32_t* occ;         // [4] words: x main / other, y main / other classes hold points
@@ -309,7 +320,16 @@ struct __align__(16) GridJob {
   int32_t n;
   const double* rec;     // batches: the tile's points (plain x, y, z)
   int32_t need_dup;      // overlap > 0: LLPs are ids of two or more windows
-  int32_t pad;
+};
+
+// Points as the fold reads them: records of `stride` doubles (4: 32-byte records
+// x, y, z, pad; 3: plain x, y, z), point i with id i + 1; or (stride 0) a tree's
+// sorted order keys and ids.
+struct GridPoints {
+  const double* rec = nullptr;
+  int stride = 0;
+  const int64_t *xk = nullptr, *yk = nullptr, *zk = nullptr;
+  const uint32_t* id = nullptr;
 };
 
 // The tiles of a batch as a kernel sees them: off[t] is tile t's first item.
@@ -321,9 +341,20 @@ struct GridTiles {
 
 // Stored index of sub-cell (sx, sy).
 __host__ __device__ __forceinline__ uint32_t grid_cell(const GridJob& J, int32_t sx, int32_t sy) {
-  const int qx = (sx ^ J.x.par) & 1, qy = (sy ^ J.y.par) & 1;
+  const int qx = (sx ^ J.x.par) & J.x.parmask, qy = (sy ^ J.y.par) & J.y.parmask;
   const uint32_t b = qy ? (qx ? J.base[3] : J.base[2]) : (qx ? J.base[1] : J.base[0]);
-  return b + (uint32_t)(sy >> 1) * (uint32_t)(qx ? J.x.width[1] : J.x.width[0]) + (uint32_t)(sx >> 1);
+  return b + (uint32_t)(sy >> J.y.parmask) * (uint32_t)(qx ? J.x.width[1] : J.x.width[0]) + (uint32_t)(sx >> J.x.parmask);
+}
+
+// Where a sub-cell's count lies.  Four counts a sector would have the adds of
+// points in no order wait for one another where the sub-cells are few: a bare
+// kernel's read and add for each of 100 M points take 1.21 ms with counts 4
+// bytes apart and 0.93 with 16 at 25,600 sub-cells, 0.95 and 0.76 at 100,000,
+// 0.76 and 0.73 at 700,000; 0.73 and 0.83 at 3 M, past which the counts would
+// leave L2.
+constexpr int64_t kGridSpreadMax = (int64_t)1 << 20;
+__host__ __device__ __forceinline__ int64_t grid_count_slot(const GridJob& J, uint32_t cell) {
+  return (int64_t)cell + 3 * (int64_t)(cell < J.spread ? cell : J.spread);
 }
 
 // Number of sub-cells of a job.
@@ -338,6 +369,7 @@ void grid_axis_setup(double lo, double hi, double step, int32_t whalf, int32_t n
 // cannot be numbered in 32 bits), and its job, pointers excepted.
 struct GridSizes {
   int64_t nsub = 0, nwin = 0, ncell = 0, rows = 0, edges = 0;
+  int64_t counts = 0;  // words of the counts
   int64_t chunks = 0;  // of a stage-2 bitmap
   bool merged = false;  // cells share the windows' sub-cells
 };
@@ -358,13 +390,14 @@ struct GridPlan {
   size_t s2_bytes = 0, scan_bytes = 0;
   char* base = nullptr;
 };
-// Sizes the plan (scratch nullptr) or carves it from scratch.
-int grid_plan(const owm_params& p, int64_t n, void* scratch, GridPlan* g);
+// Sizes the plan (scratch nullptr) or carves it from scratch.  stage1_only: the
+// window results alone, in g->job.win.
+int grid_plan(const owm_params& p, int64_t n, void* scratch, GridPlan* g, bool stage1_only = false);
 // Clears the tables and computes edges and ranges.
 int grid_prepare(const GridPlan& g, const owm_params& p, uint32_t* status, cudaStream_t s, int64_t* launches);
-// Folds points [first, first + count) of the cloud, ids first + 1 ...
-int grid_fold(const GridPlan& g, const double* rec, int stride, int64_t first, int64_t count, uint32_t* status,
-              cudaStream_t s, int64_t* launches);
+// Folds points [first, first + count) of the cloud.
+int grid_fold(const GridPlan& g, const GridPoints& pts, int64_t first, int64_t count, uint32_t* status, cudaStream_t s,
+              int64_t* launches);
 // Stage 1 (rows, windows), stage 2 with stage 3's marks, stage 3 and the seeds.
 int grid_windows(const GridPlan& g, cudaStream_t s, int64_t* launches);
 int grid_stage2(const GridPlan& g, const owm_params& p, const double* xy, int xy_stride, uint32_t* d_nllp,

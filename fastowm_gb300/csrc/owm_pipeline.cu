@@ -162,7 +162,10 @@ int run_grid(owm_ctx* c, const PointsView& pts, int64_t n, const owm_params& p, 
   uint32_t* d_ns3 = c->d_small + kS3Slot;
   OWM_CUDA_TRY(cudaEventRecord(c->ev[0], s));
   rc = grid_prepare(g, p, status, s, &c->launches);
-  if (!rc) rc = grid_fold(g, pts.rec, pts.rec_stride, 0, n, status, s, &c->launches);
+  GridPoints gp;
+  gp.rec = pts.rec;
+  gp.stride = pts.rec_stride;
+  if (!rc) rc = grid_fold(g, gp, 0, n, status, s, &c->launches);
   if (rc) return rc;
   OWM_CUDA_TRY(cudaEventRecord(c->ev[1], s));
   rc = grid_windows(g, s, &c->launches);
