@@ -235,7 +235,9 @@ int owm_tree_destroy(owm_tree* tree);
 /* ---- OWM stages -------------------------------------------------------- */
 /* Replaces stage1 (optim3_func.cpp:541-561): win_min[ii*nrows + jj] = id of
  * the (z, id)-minimum point strictly inside window (ii, jj) if at least
- * min_num_points points are strictly inside, else -1.  [ncells] entries. */
+ * min_num_points points are strictly inside, else -1.  [ncells] entries.  By
+ * the tree walk, or by folding the tree's points into a window grid where that
+ * is faster (never while a walk limit is set). */
 int owm_stage1(owm_ctx* ctx, const owm_tree* tree, const owm_params* params, int64_t* win_min);
 
 /* Replaces std::sort + stage2 (owm_optim3.cpp:160-188, optim3_func.cpp:
@@ -282,7 +284,7 @@ typedef struct {
    *     are rectangles of sub-cells, O(N); no hierarchy is built (`tree` is
    *     checked, and the seeds do not depend on it);
    *  1  tree build, warp-cooperative stackless tree walk per window with min-z
-   *     pruning (what owm_stage1 runs), tree walk per cell.  A context with a
+   *     pruning, tree walk per cell.  A context with a
    *     walk limit (owm_ctx_set_walk_limit) takes this path too. */
   int32_t stage1_walk;
   int32_t _pad;

@@ -76,3 +76,22 @@ def test_zero_and_sentinel_heights_outside_points(owm, oracle, ctx):
     xyz[19_999, 0] = np.inf
     with pytest.raises(owm.OwmError):
         ctx.run_host(xyz, bb, owm.run_cfg(7, 0.5, 6, 32))
+
+
+@pytest.mark.parametrize("W,Ov,policy", [(10, 0.8, 1), (9, 0.3, 1), (10, 0.5, 0), (60, 0.0, 1)])
+@pytest.mark.parametrize("x0", [500000.0, -40.0])
+def test_stage1_of_a_tree(owm, oracle, x0, W, Ov, policy):
+    """owm_stage1 folds the tree's sorted points into a window grid or walks the
+    tree, by the number of windows; a walk limit above every walk's steps gives
+    the walk's answer."""
+    ctx = owm.Context(0)
+    xyz = _cloud(np.random.default_rng(8), 60_000, x0, 1000.0, 80.0, 0.01)
+    bb = owm.Bbox(x0, 1000.0, x0 + 80.0, 1080.0)
+    cloud = ctx.cloud(xyz, bb)
+    tree = ctx.tree(cloud, policy, 32, 0.5)
+    p = owm.params(bb, xyz.shape[0], W, Ov, 20)
+    got = ctx.stage1(tree, p)
+    ctx.set_walk_limit(1 << 30)
+    np.testing.assert_array_equal(ctx.stage1(tree, p), got)
+    np.testing.assert_array_equal(got, oracle.stage1(xyz, oracle.params(bb, xyz.shape[0], W, Ov, 20)))
+    ctx.close()
