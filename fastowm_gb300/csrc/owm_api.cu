@@ -241,9 +241,9 @@ int owm_ctx_destroy(owm_ctx* c) {
     a.input.release(c->copy_stream ? c->copy_stream : c->stream);
     if (a.ready) cudaEventDestroy(a.ready);
     if (a.done) cudaEventDestroy(a.done);
-    if (a.h_seeds) cudaFreeHost(a.h_seeds);
-    if (a.h_words) cudaFreeHost(a.h_words);
+    a.result.release();
   }
+  c->result.release();
   if (c->stream) cudaStreamSynchronize(c->stream);
   if (c->copy_stream) {
     cudaStreamSynchronize(c->copy_stream);
@@ -868,32 +868,17 @@ int owm_run_host(owm_ctx* c, const double* xyz, int64_t n, const owm_bbox* bbox,
 namespace {
 
 // Queues the run of slot a on the context's stream (after whatever is queued
-// there: a copy-stream event for host input), then the device->host copy of
-// its status words and of the whole seed buffer into the slot's pinned
-// staging, and hands out the ticket.  On failure the caller's fail() waits
-// for everything queued so far.
+// there: a copy-stream event for host input), whose result lands in the slot's
+// pinned buffer, and hands out the ticket.  On failure the caller's fail()
+// waits for everything queued so far.
 template <class Fail>
 int submit_slot(owm_ctx* c, owm_ctx::AsyncSlot& a, const PointsView& pts, int64_t n, const owm_bbox& bb,
                 const owm_run_cfg& cfg, int64_t* seeds, int64_t cap, int64_t* ticket, const char* fn, Fail fail) {
   int64_t* d_seeds = nullptr;
   int64_t room = 0;
-  int rc = run_pipeline_enqueue(c, pts, n, bb, cfg, &a.p, &d_seeds, &room);
+  const int rc = run_pipeline_enqueue(c, pts, n, bb, cfg, &a.result, INT64_MAX, &a.p, &d_seeds, &room);
   if (rc) return fail(rc);
-  if (a.h_cap < room) {
-    // growth only: the old staging may still be a copy target
-    if (cudaStreamSynchronize(c->stream) != cudaSuccess) return fail(OWM_ECUDA);
-    if (a.h_seeds) cudaFreeHost(a.h_seeds);
-    a.h_seeds = nullptr;
-    a.h_cap = 0;
-    if (cudaMallocHost(&a.h_seeds, (size_t)room * 8) != cudaSuccess) {
-      cudaGetLastError();
-      return fail(OWM_ENOMEM);
-    }
-    a.h_cap = room;
-  }
-  cudaError_t e = cudaMemcpyAsync(a.h_words, c->d_small, 32, cudaMemcpyDeviceToHost, c->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(a.h_seeds, d_seeds, (size_t)room * 8, cudaMemcpyDeviceToHost, c->stream);
-  if (e == cudaSuccess) e = cudaEventRecord(a.done, c->stream);
+  const cudaError_t e = cudaEventRecord(a.done, c->stream);
   if (e != cudaSuccess) {
     set_last_cuda_error(e, fn, __FILE__, __LINE__);
     return fail(OWM_ECUDA);
@@ -906,8 +891,7 @@ int submit_slot(owm_ctx* c, owm_ctx::AsyncSlot& a, const PointsView& pts, int64_
   return OWM_OK;
 }
 
-// The slot the next ticket uses, with its events and pinned status words
-// created; nullptr (and *rc) when both runs are still in flight or creation
+// The slot the next ticket uses, with its events created; nullptr (and *rc) when both runs are still in flight or creation
 // failed.
 owm_ctx::AsyncSlot* next_slot(owm_ctx* c, int* rc) {
   owm_ctx::AsyncSlot& a = c->aslot[c->next_ticket & 1];
@@ -919,7 +903,6 @@ owm_ctx::AsyncSlot* next_slot(owm_ctx* c, int* rc) {
   cudaError_t e = cudaSuccess;
   if (!a.ready) e = cudaEventCreateWithFlags(&a.ready, cudaEventDisableTiming);
   if (e == cudaSuccess && !a.done) e = cudaEventCreateWithFlags(&a.done, cudaEventDisableTiming);
-  if (e == cudaSuccess && !a.h_words) e = cudaMallocHost(&a.h_words, 32);
   if (e != cudaSuccess) {
     set_last_cuda_error(e, "owm_run_submit", __FILE__, __LINE__);
     *rc = OWM_ECUDA;
@@ -1004,10 +987,11 @@ int owm_run_host_wait(owm_ctx* c, int64_t ticket, int64_t* n_seeds, owm_run_info
     set_last_cuda_error(e, "owm_run_host_wait", __FILE__, __LINE__);
     return OWM_ECUDA;
   }
-  const uint32_t st = a.h_words[kStatusSlot];
+  const uint32_t* words = a.result.words;
+  const uint32_t st = words[kStatusSlot];
   if (st & kStatusNonFinite) return OWM_EINVAL;
   if (st & kStatusWalkBound) return OWM_ETIMEOUT;
-  const int64_t nllp = a.h_words[kLlpSlot], ns3 = a.h_words[kS3Slot];
+  const int64_t nllp = words[kLlpSlot], ns3 = words[kS3Slot];
   const int64_t total = nllp + ns3;
   *n_seeds = total;
   if (info) {
@@ -1018,7 +1002,7 @@ int owm_run_host_wait(owm_ctx* c, int64_t ticket, int64_t* n_seeds, owm_run_info
     info->params = a.p;
   }
   if (total > a.cap || total > a.room) return OWM_ERANGE;
-  if (total > 0) std::memcpy(a.seeds, a.h_seeds, (size_t)total * 8);
+  if (total > 0) std::memcpy(a.seeds, a.result.seeds, (size_t)total * 8);
   return OWM_OK;
 }
 

@@ -22,6 +22,7 @@ constexpr int kCountSlot = 2;
 constexpr int kLlpSlot = 3;
 constexpr int kS3Slot = 4;
 constexpr int kBboxSlot = 8;  // 4 x int64 (8-byte aligned)
+constexpr int kStampSlot = 128;  // kGridStamps x uint64
 
 bool is_device_ptr(const void* p);
 // Device memory of the given device (or managed memory), which that device's
@@ -61,6 +62,22 @@ struct ProfScope {
 };
 }  // namespace owm
 
+namespace owm {
+// Pinned memory that a run's last kernel writes its result to (no copy to
+// queue, no second wait): the words of d_small, the phase stamps, the seeds.
+struct ResultBuffer {
+  int64_t* seeds = nullptr;
+  int64_t cap = 0;
+  uint32_t* words = nullptr;  // [64]: 0..7 as in d_small; 8: stamps are set; 16..: the stamps
+  // Room for that many seeds; waits for s before it frees anything.
+  int reserve(int64_t room, cudaStream_t s);
+  void release();
+};
+// Synchronous runs of more windows and cells than this copy exactly their seeds
+// from the device instead (32 MB of pinned memory).
+constexpr int64_t kDirectSeeds = (int64_t)1 << 22;
+}  // namespace owm
+
 struct owm_ctx {
   owm::Profiler prof;
   bool profiling = false;
@@ -72,6 +89,7 @@ struct owm_ctx {
   uint32_t* h_small = nullptr;  // [1024] pinned host mirror
   owm::QueryJob* d_job = nullptr;
   owm::DeviceBuffer scratch, tree_mem, input, outbuf;
+  owm::ResultBuffer result;  // of synchronous runs
   owm::TreeStore tree;  // tree of the last owm_run that built one
   cudaEvent_t ev[6] = {};
   // owm_run_host_submit / _wait: two runs in flight, each with its own input
@@ -81,9 +99,7 @@ struct owm_ctx {
     int64_t ticket = 0;  // 0 = free
     owm::DeviceBuffer input;
     cudaEvent_t ready = nullptr, done = nullptr;
-    int64_t* h_seeds = nullptr;  // pinned [h_cap]
-    int64_t h_cap = 0;
-    uint32_t* h_words = nullptr;  // pinned [8]: status, counts
+    owm::ResultBuffer result;
     int64_t* seeds = nullptr;     // caller's output
     int64_t cap = 0, room = 0;
     owm_params p{};
@@ -118,10 +134,11 @@ int device_bbox(owm_ctx* c, const double* d_xy, int stride, int64_t n, owm_bbox*
 int run_stage1(owm_ctx* c, const TreeStore& t, const owm_params& p, Edge* ex, Edge* ey, uint32_t* d_win);
 int run_pipeline(owm_ctx* c, const PointsView& pts, int64_t n, const owm_bbox& bb, const owm_run_cfg& cfg,
                  int64_t* seeds, int64_t cap, int64_t* n_seeds, owm_run_info* info);
-// The device part of run_pipeline: enqueues the whole run on c->stream and
-// leaves the status words in c->d_small and the assembled seeds (room slots)
-// at *d_seeds; no host sync (except inside the min-radius build).
+// The device part of run_pipeline: enqueues the whole run on c->stream; the
+// result lands in rb, but for more than direct_max room slots the seeds stay
+// on the device, at *d_seeds (else null).  No host sync (except inside the
+// min-radius build).
 int run_pipeline_enqueue(owm_ctx* c, const PointsView& pts, int64_t n, const owm_bbox& bb, const owm_run_cfg& cfg,
-                         owm_params* p, int64_t** d_seeds, int64_t* room);
+                         ResultBuffer* rb, int64_t direct_max, owm_params* p, int64_t** d_seeds, int64_t* room);
 
 }  // namespace owm

@@ -31,6 +31,40 @@ constexpr int kFoldBlocks = 6;  // resident fold blocks per SM (40 registers a t
 constexpr int64_t kTileChunk = 4096;
 constexpr int kTileStripes = 16;
 
+// Start of a kernel of a chain: lets the next one be set up while this one runs
+// (its launch latency then overlaps this kernel), and waits until everything
+// before this one is done.  Without the launch attribute both do nothing.
+// What earlier kernels of the chain write is read by plain loads only: the
+// read-only path may be used for data that nothing writes while a kernel
+// exists, and it exists before they end.
+__device__ __forceinline__ void chain_start() {
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// Launch of a kernel that starts with chain_start.
+template <class... P, class... A>
+cudaError_t chain(void (*kernel)(P...), unsigned grid, int block, cudaStream_t s, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.stream = s;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+__device__ __forceinline__ void stamp(const GridJob& J, int phase) {
+  if (J.stamps && blockIdx.x == 0 && threadIdx.x == 0) {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    J.stamps[phase] = t;
+  }
+}
+
 // The job that item *k belongs to; *k becomes the item's number within it.
 template <bool kMulti>
 __device__ __forceinline__ const GridJob& job_at(const GridJob& one, const GridTiles& T, int64_t* k) {
@@ -47,7 +81,7 @@ struct FormulaEdges {
 };
 struct StoredEdges {
   const GridAxis* a;
-  __device__ __forceinline__ int64_t operator()(int f, int32_t j) const { return __ldg(a->edge[f] + j); }
+  __device__ __forceinline__ int64_t operator()(int f, int32_t j) const { return a->edge[f][j]; }
 };
 
 __device__ int32_t class_of_key(const GridAxis& a, int64_t key) {
@@ -76,6 +110,8 @@ template <bool kMulti>
 __global__ void __launch_bounds__(256) k_grid_prepare(const __grid_constant__ GridJob one, GridTiles T, int64_t items,
                                                       uint4* __restrict__ clear, int64_t nclear,
                                                       uint32_t* __restrict__ status) {
+  if (one.stamps && blockIdx.x == 0 && threadIdx.x == 0) one.stamps[1] = one.stamps[2] = one.stamps[3] = 0;
+  stamp(one, 0);
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = t; i < items; i += nt) {
     int64_t k = i;
@@ -341,6 +377,7 @@ template <int kStride, int kFast>
 __global__ void __launch_bounds__(kFoldBlock, kFoldBlocks)
     k_grid_fold(const __grid_constant__ GridJob J, const __grid_constant__ GridPoints pts, int64_t first, int64_t count,
                 uint32_t* __restrict__ status) {
+  chain_start();
   const int64_t nwarps = ((int64_t)gridDim.x * kFoldBlock) >> 5;
   uint32_t flags = 0;
   int64_t t0, t1;
@@ -406,6 +443,8 @@ __device__ __forceinline__ bool parity_range(const GridAxis& a, const uint32_t* 
 
 template <bool kMulti>
 __global__ void __launch_bounds__(256) k_grid_rows(const __grid_constant__ GridJob one, GridTiles T, int64_t total) {
+  chain_start();
+  stamp(one, 1);
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     int64_t k = i;
     const GridJob& J = job_at<kMulti>(one, T, &k);
@@ -434,6 +473,7 @@ __global__ void __launch_bounds__(256) k_grid_rows(const __grid_constant__ GridJ
 
 template <bool kMulti>
 __global__ void __launch_bounds__(256) k_grid_windows(const __grid_constant__ GridJob one, GridTiles T, int64_t total) {
+  chain_start();
   // the search starts from the reference's sentinel point 0 {0, 0, DBL_MAX}
   const unsigned long long sentinel = ~((unsigned long long)kZSentinel ^ 0x8000000000000000ull);
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -489,8 +529,9 @@ __device__ __forceinline__ uint32_t block_exclusive_256(uint32_t v, uint32_t* to
   return before + inc - v;
 }
 
-__global__ void __launch_bounds__(kSeedBlock) k_grid_seed_count(const uint32_t* __restrict__ bm, uint32_t* __restrict__ part) {
-  const uint4 q = __ldg(reinterpret_cast<const uint4*>(bm) + (int64_t)blockIdx.x * kSeedBlock + threadIdx.x);
+__global__ void __launch_bounds__(kSeedBlock) k_grid_seed_count(const uint32_t* bm, uint32_t* __restrict__ part) {
+  chain_start();
+  const uint4 q = reinterpret_cast<const uint4*>(bm)[(int64_t)blockIdx.x * kSeedBlock + threadIdx.x];
   uint32_t total;
   block_exclusive_256((uint32_t)(__popc(q.x) + __popc(q.y) + __popc(q.z) + __popc(q.w)), &total);
   if (threadIdx.x == 0) part[blockIdx.x] = total;
@@ -511,20 +552,30 @@ __device__ __forceinline__ void mark_cells(const GridJob& J, const double* __res
 }
 
 // The ids marked twice, ascending: block b writes those of its chunk after
-// all chunks before it (whose counts it adds up) and marks their cells.
+// all chunks before it (whose counts, or words when part is null, it adds up)
+// and marks their cells.
 // A batch: tile by tile; nllp[t] is tile t's first LLP, nllp[T.n] their number.
 template <bool kMulti>
 __global__ void __launch_bounds__(kSeedBlock) k_grid_seeds(const __grid_constant__ GridJob one, GridTiles T,
-                                                           const uint32_t* __restrict__ part, const double* __restrict__ xy,
-                                                           int stride, uint32_t* __restrict__ llp,
-                                                           uint32_t* __restrict__ nllp) {
+                                                           const uint32_t* part, const double* __restrict__ xy, int stride,
+                                                           uint32_t* llp, uint32_t* nllp) {
+  chain_start();
+  stamp(one, 2);
   int64_t chunk = blockIdx.x;
   const GridJob& J = job_at<kMulti>(one, T, &chunk);
   uint32_t before = 0, total;
-  for (uint32_t q = threadIdx.x; q < blockIdx.x; q += kSeedBlock) before += __ldg(part + q);
+  if (part) {
+    for (uint32_t q = threadIdx.x; q < blockIdx.x; q += kSeedBlock) before += part[q];
+  } else {  // few chunks: their words themselves
+    const uint4* w = reinterpret_cast<const uint4*>(J.twice);
+    for (uint32_t q = threadIdx.x; q < blockIdx.x * kSeedBlock; q += kSeedBlock) {
+      const uint4 v = w[q];
+      before += (uint32_t)(__popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w));
+    }
+  }
   block_exclusive_256(before, &before);
   const int64_t w0 = chunk * kSeedChunk + (int64_t)threadIdx.x * kSeedWords;
-  const uint4 q = __ldg(reinterpret_cast<const uint4*>(J.twice + w0));
+  const uint4 q = *reinterpret_cast<const uint4*>(J.twice + w0);
   const uint32_t word[4] = {q.x, q.y, q.z, q.w};
   uint32_t at = before + block_exclusive_256((uint32_t)(__popc(q.x) + __popc(q.y) + __popc(q.z) + __popc(q.w)), &total);
   if (threadIdx.x == 0) {
@@ -546,6 +597,7 @@ __global__ void __launch_bounds__(kSeedBlock) k_grid_seeds(const __grid_constant
 // The cells of LLPs that another kernel listed.
 __global__ void __launch_bounds__(256) k_grid_mark(const __grid_constant__ GridJob J, const double* __restrict__ xy, int stride,
                                                    const uint32_t* __restrict__ llp, const uint32_t* __restrict__ nllp) {
+  stamp(J, 2);
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < *nllp; k += gridDim.x * blockDim.x)
     mark_cells(J, xy, stride, llp[k]);
 }
@@ -563,6 +615,8 @@ __device__ __forceinline__ uint32_t cell_result(unsigned long long w, uint32_t n
 // entry.
 template <bool kMulti>
 __global__ void __launch_bounds__(256) k_grid_cells(const __grid_constant__ GridJob one, GridTiles T, int64_t total) {
+  chain_start();
+  stamp(one, 3);
   const int lane = threadIdx.x & 31;
   int64_t c = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (c >= total) return;
@@ -594,47 +648,61 @@ __global__ void __launch_bounds__(256) k_grid_cells(const __grid_constant__ Grid
   if (lane == 0) J.cellmin[c] = cell_result(m.w, m.nid);
 }
 
+// The result's words (ResultBuffer), by one thread once the counts are known.
+__device__ __forceinline__ void write_words(const GridJob& J, const GridResult& R, uint32_t nllp, uint32_t ns3) {
+  *R.ns3 = ns3;
+  R.words[kResultStatus] = *R.status;
+  R.words[kResultLlp] = nllp;
+  R.words[kResultS3] = ns3;
+  unsigned long long* to = reinterpret_cast<unsigned long long*>(R.words + 16);
+  unsigned long long t = 0;
+  for (int k = 0; k < kGridStamps - 1; ++k) to[k] = t = J.stamps[k] ? J.stamps[k] : t;  // a phase without a kernel: 0 long
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  to[kGridStamps - 1] = t;
+  R.words[8] = 1;
+}
+
 // seeds = the valid entries of cellmin in order, then the LLPs.  Every block
 // counts all cells (at most kOutputCells) for the total and its own start.
 constexpr int64_t kOutputCells = 32768;
-__global__ void __launch_bounds__(kSeedBlock) k_grid_output(const uint32_t* __restrict__ cellmin, int64_t ncell,
-                                                            const uint32_t* __restrict__ llp, const uint32_t* __restrict__ nllp,
-                                                            int64_t* __restrict__ seeds, uint32_t* __restrict__ ns3) {
+__global__ void __launch_bounds__(kSeedBlock) k_grid_output(const __grid_constant__ GridJob J, int64_t ncell, const uint32_t* llp,
+                                                            GridResult R) {
+  chain_start();
   const int64_t per = (ncell + gridDim.x - 1) / gridDim.x;
   const int64_t b0 = per * blockIdx.x, b1 = min(b0 + per, ncell);
   uint32_t before = 0, all = 0;
   for (int64_t i = threadIdx.x; i < ncell; i += kSeedBlock) {
-    const uint32_t v = __ldg(cellmin + i) != kNone ? 1u : 0u;
+    const uint32_t v = J.cellmin[i] != kNone ? 1u : 0u;
     all += v;
     if (i < b0) before += v;
   }
   block_exclusive_256(before, &before);
   block_exclusive_256(all, &all);
-  if (blockIdx.x == 0 && threadIdx.x == 0) *ns3 = all;
   uint32_t at = before;
   for (int64_t t = b0; t < b1; t += kSeedBlock) {
-    const uint32_t v = t + threadIdx.x < b1 ? __ldg(cellmin + t + threadIdx.x) : kNone;
+    const uint32_t v = t + threadIdx.x < b1 ? J.cellmin[t + threadIdx.x] : kNone;
     uint32_t got;
     const uint32_t p = block_exclusive_256(v != kNone ? 1u : 0u, &got);
-    if (v != kNone) seeds[at + p] = v;
+    if (v != kNone) R.seeds[at + p] = v;
     at += got;
   }
-  const uint32_t n = *nllp;
-  for (uint32_t k = blockIdx.x * kSeedBlock + threadIdx.x; k < n; k += gridDim.x * kSeedBlock) seeds[all + k] = llp[k];
+  const uint32_t n = *R.nllp;
+  for (uint32_t k = blockIdx.x * kSeedBlock + threadIdx.x; k < n; k += gridDim.x * kSeedBlock) R.seeds[all + k] = llp[k];
+  if (blockIdx.x == 0 && threadIdx.x == 0) write_words(J, R, n, all);
 }
 
 __global__ void k_grid_flags(const uint32_t* __restrict__ v, int64_t n, uint32_t* __restrict__ flags) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     flags[i] = v[i] != kNone ? 1u : 0u;
 }
-__global__ void k_grid_output_scanned(const uint32_t* __restrict__ cellmin, const uint32_t* __restrict__ pos, int64_t ncell,
-                                      const uint32_t* __restrict__ llp, const uint32_t* __restrict__ nllp,
-                                      const uint32_t* __restrict__ ns3, int64_t* __restrict__ seeds) {
+__global__ void k_grid_output_scanned(const __grid_constant__ GridJob J, const uint32_t* __restrict__ pos, int64_t ncell,
+                                      const uint32_t* __restrict__ llp, GridResult R) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = t; i < ncell; i += nt)
-    if (cellmin[i] != kNone) seeds[pos[i]] = cellmin[i];
-  const int64_t n = *nllp, base = *ns3;
-  for (int64_t i = t; i < n; i += nt) seeds[base + i] = llp[i];
+    if (J.cellmin[i] != kNone) R.seeds[pos[i]] = J.cellmin[i];
+  const uint32_t n = *R.nllp, base = *R.ns3;
+  for (int64_t i = t; i < n; i += nt) R.seeds[base + i] = llp[i];
+  if (t == 0) write_words(J, R, n, base);
 }
 
 // ---- batches: overlap 0 in some tile, and the output ------------------------------
@@ -1182,7 +1250,7 @@ int grid_fold(const GridPlan& g, const GridPoints& pts, int64_t first, int64_t c
                                        {k_grid_fold<3, 0>, k_grid_fold<3, 1>, k_grid_fold<3, 2>},
                                        {k_grid_fold<4, 0>, k_grid_fold<4, 1>, k_grid_fold<4, 2>}};
   const Kernel kernel = kernels[pts.stride == 4 ? 2 : pts.stride == 3 ? 1 : 0][J.fast];
-  OWM_LAUNCH("k_grid_fold", s, kernel<<<nb, kFoldBlock, 0, s>>>(J, pts, first, count, status));
+  OWM_LAUNCH("k_grid_fold", s, OWM_CUDA_TRY(chain(kernel, nb, kFoldBlock, s, J, pts, first, count, status)));
   count_launch(launches);
   OWM_CUDA_TRY(cudaGetLastError());
   return OWM_OK;
@@ -1190,8 +1258,10 @@ int grid_fold(const GridPlan& g, const GridPoints& pts, int64_t first, int64_t c
 
 int grid_windows(const GridPlan& g, cudaStream_t s, int64_t* launches) {
   const GridJob& J = g.job;
-  OWM_LAUNCH("k_grid_rows", s, k_grid_rows<false><<<blocks_for(g.z.rows, 152 * 32), 256, 0, s>>>(J, GridTiles{}, g.z.rows));
-  OWM_LAUNCH("k_grid_windows", s, k_grid_windows<false><<<blocks_for(g.z.nwin, 152 * 32), 256, 0, s>>>(J, GridTiles{}, g.z.nwin));
+  OWM_LAUNCH("k_grid_rows", s, OWM_CUDA_TRY(chain(k_grid_rows<false>, blocks_for(g.z.rows, 152 * 32), 256, s, J, GridTiles{},
+                                                  g.z.rows)));
+  OWM_LAUNCH("k_grid_windows", s, OWM_CUDA_TRY(chain(k_grid_windows<false>, blocks_for(g.z.nwin, 152 * 32), 256, s, J,
+                                                     GridTiles{}, g.z.nwin)));
   count_launch(launches, 2);
   OWM_CUDA_TRY(cudaGetLastError());
   return OWM_OK;
@@ -1201,11 +1271,15 @@ int grid_stage2(const GridPlan& g, const owm_params& p, const double* xy, int xy
                 cudaStream_t s, int64_t* launches) {
   const GridJob& J = g.job;
   if (g.bitmap2) {
+    // up to 32 chunks (1 M ids) each block counts the words before its own: one
+    // launch less
     const unsigned chunks = (unsigned)g.z.chunks;
-    OWM_LAUNCH("k_grid_seed_count", s, k_grid_seed_count<<<chunks, kSeedBlock, 0, s>>>(J.twice, g.part));
-    OWM_LAUNCH("k_grid_seeds", s, k_grid_seeds<false><<<chunks, kSeedBlock, 0, s>>>(J, GridTiles{}, g.part, xy, xy_stride, g.llp,
-                                                                                      d_nllp));
-    count_launch(launches, 2);
+    const bool count = chunks > 32;
+    if (count)
+      OWM_LAUNCH("k_grid_seed_count", s, OWM_CUDA_TRY(chain(k_grid_seed_count, chunks, kSeedBlock, s, J.twice, g.part)));
+    OWM_LAUNCH("k_grid_seeds", s, OWM_CUDA_TRY(chain(k_grid_seeds<false>, chunks, kSeedBlock, s, J, GridTiles{},
+                                                     count ? g.part : nullptr, xy, xy_stride, g.llp, d_nllp)));
+    count_launch(launches, 1 + count);
   } else {
     // overlap 0 keeps every valid minimum, repeated sentinel ids included: by sorting
     const int rc = run_stage2(J.win, g.z.nwin, g.n, p.overlap, g.llp, d_nllp, g.s2_temp, g.s2_bytes, s, launches);
@@ -1219,22 +1293,23 @@ int grid_stage2(const GridPlan& g, const owm_params& p, const double* xy, int xy
   return OWM_OK;
 }
 
-int grid_stage3(const GridPlan& g, const uint32_t* d_nllp, uint32_t* d_ns3, cudaStream_t s, int64_t* launches) {
+int grid_stage3(const GridPlan& g, const GridResult& out, cudaStream_t s, int64_t* launches) {
   const GridJob& J = g.job;
   if (g.z.ncell > 0) {
-    OWM_LAUNCH("k_grid_cells", s, k_grid_cells<false><<<(unsigned)((g.z.ncell + 7) / 8), 256, 0, s>>>(J, GridTiles{}, g.z.ncell));
+    OWM_LAUNCH("k_grid_cells", s, OWM_CUDA_TRY(chain(k_grid_cells<false>, (unsigned)((g.z.ncell + 7) / 8), 256, s, J, GridTiles{},
+                                                     g.z.ncell)));
     count_launch(launches);
   }
   if (g.z.ncell <= kOutputCells) {
-    OWM_LAUNCH("k_grid_output", s, k_grid_output<<<blocks_for(g.z.nwin / 4 + g.z.ncell, 64), kSeedBlock, 0, s>>>(
-        J.cellmin, g.z.ncell, g.llp, d_nllp, g.seeds, d_ns3));
+    OWM_LAUNCH("k_grid_output", s, OWM_CUDA_TRY(chain(k_grid_output, blocks_for(g.z.nwin / 4 + g.z.ncell, 64), kSeedBlock, s, J,
+                                                      g.z.ncell, g.llp, out)));
     count_launch(launches);
   } else {
     OWM_LAUNCH("k_grid_flags", s, k_grid_flags<<<blocks_for(g.z.ncell, 152 * 8), 256, 0, s>>>(J.cellmin, g.z.ncell, g.flags));
     count_launch(launches);
-    OWM_CUDA_TRY(exclusive_scan_u32(g.flags, g.pos, g.z.ncell, d_ns3, g.scan_temp, g.scan_bytes, s, launches));
+    OWM_CUDA_TRY(exclusive_scan_u32(g.flags, g.pos, g.z.ncell, out.ns3, g.scan_temp, g.scan_bytes, s, launches));
     OWM_LAUNCH("k_grid_output", s, k_grid_output_scanned<<<blocks_for(g.z.nwin + g.z.ncell, 152 * 8), 256, 0, s>>>(
-        J.cellmin, g.pos, g.z.ncell, g.llp, d_nllp, d_ns3, g.seeds));
+        J, g.pos, g.z.ncell, g.llp, out));
     count_launch(launches);
   }
   OWM_CUDA_TRY(cudaGetLastError());

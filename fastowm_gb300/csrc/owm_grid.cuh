@@ -320,7 +320,10 @@ struct __align__(16) GridJob {
   int32_t n;
   const double* rec;     // batches: the tile's points (plain x, y, z)
   int32_t need_dup;      // overlap > 0: LLPs are ids of two or more windows
+  unsigned long long* stamps;  // [kGridStamps] nanoseconds at the phases' ends, or null
 };
+// Phase stamps: start, index done, stage 1, stage 2, stage 3 and output done.
+constexpr int kGridStamps = 5;
 
 // Points as the fold reads them: records of `stride` doubles (4: 32-byte records
 // x, y, z, pad; 3: plain x, y, z), point i with id i + 1; or (stride 0) a tree's
@@ -402,7 +405,15 @@ int grid_fold(const GridPlan& g, const GridPoints& pts, int64_t first, int64_t c
 int grid_windows(const GridPlan& g, cudaStream_t s, int64_t* launches);
 int grid_stage2(const GridPlan& g, const owm_params& p, const double* xy, int xy_stride, uint32_t* d_nllp,
                 cudaStream_t s, int64_t* launches);
-int grid_stage3(const GridPlan& g, const uint32_t* d_nllp, uint32_t* d_ns3, cudaStream_t s, int64_t* launches);
+// Where a run's result goes: status, nllp, ns3 are device words; seeds and words
+// (ResultBuffer's) may be pinned host memory.
+constexpr int kResultStatus = 0, kResultLlp = 3, kResultS3 = 4;  // words, as kStatusSlot, kLlpSlot, kS3Slot
+struct GridResult {
+  uint32_t *status = nullptr, *nllp = nullptr, *ns3 = nullptr;
+  int64_t* seeds = nullptr;
+  uint32_t* words = nullptr;
+};
+int grid_stage3(const GridPlan& g, const GridResult& out, cudaStream_t s, int64_t* launches);
 
 // Many tiles at once: one launch per step, every tile with its own job.
 struct GridBatch {

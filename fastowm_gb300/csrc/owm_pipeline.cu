@@ -148,48 +148,78 @@ int run_stage1(owm_ctx* c, const TreeStore& t, const owm_params& p, Edge* ex, Ed
   return run_query(j, c->d_job, c->stream, &c->launches, "k_query_s1");
 }
 
+int ResultBuffer::reserve(int64_t room, cudaStream_t s) {
+  if (!words) {
+    OWM_CUDA_TRY(cudaMallocHost(&words, 256));
+    std::memset(words, 0, 256);
+  }
+  if (room <= cap) return OWM_OK;
+  OWM_CUDA_TRY(cudaStreamSynchronize(s));  // an earlier run may still write there
+  if (seeds) cudaFreeHost(seeds);
+  seeds = nullptr;
+  cap = 0;
+  const int64_t want = std::max<int64_t>(room + room / 4, 1 << 16);  // fewer steps for clouds that grow
+  if (cudaMallocHost(&seeds, (size_t)want * 8) != cudaSuccess) {
+    cudaGetLastError();
+    seeds = nullptr;
+    return OWM_ENOMEM;
+  }
+  cap = want;
+  return OWM_OK;
+}
+
+void ResultBuffer::release() {
+  if (seeds) cudaFreeHost(seeds);
+  if (words) cudaFreeHost(words);
+  seeds = nullptr;
+  words = nullptr;
+  cap = 0;
+}
+
 namespace {
 // The whole path on the window grid (owm_grid.cuh): no hierarchy is built.
-int run_grid(owm_ctx* c, const PointsView& pts, int64_t n, const owm_params& p, int64_t** d_seeds, int64_t* room) {
+int run_grid(owm_ctx* c, const PointsView& pts, int64_t n, const owm_params& p, ResultBuffer* rb, int64_t direct_max,
+             int64_t** d_seeds) {
   GridPlan g;
   int rc = grid_plan(p, n, nullptr, &g);
   if (!rc) rc = c->scratch.reserve(g.bytes, c->stream);
   if (!rc) rc = grid_plan(p, n, c->scratch.ptr, &g);
   if (rc) return rc;
   cudaStream_t s = c->stream;
-  uint32_t* status = c->d_small + kStatusSlot;
-  uint32_t* d_nllp = c->d_small + kLlpSlot;
-  uint32_t* d_ns3 = c->d_small + kS3Slot;
-  OWM_CUDA_TRY(cudaEventRecord(c->ev[0], s));
-  rc = grid_prepare(g, p, status, s, &c->launches);
+  g.job.stamps = reinterpret_cast<unsigned long long*>(c->d_small + kStampSlot);
+  GridResult out;
+  out.status = c->d_small + kStatusSlot;
+  out.nllp = c->d_small + kLlpSlot;
+  out.ns3 = c->d_small + kS3Slot;
+  const bool direct = g.z.nwin + g.z.ncell + 1 <= direct_max;
+  out.seeds = direct ? rb->seeds : g.seeds;
+  out.words = rb->words;
+  *d_seeds = direct ? nullptr : g.seeds;
   GridPoints gp;
   gp.rec = pts.rec;
   gp.stride = pts.rec_stride;
-  if (!rc) rc = grid_fold(g, gp, 0, n, status, s, &c->launches);
-  if (rc) return rc;
-  OWM_CUDA_TRY(cudaEventRecord(c->ev[1], s));
-  rc = grid_windows(g, s, &c->launches);
-  if (rc) return rc;
-  OWM_CUDA_TRY(cudaEventRecord(c->ev[2], s));
-  rc = grid_stage2(g, p, pts.xy, pts.xy_stride, d_nllp, s, &c->launches);
-  if (rc) return rc;
-  OWM_CUDA_TRY(cudaEventRecord(c->ev[3], s));
-  rc = grid_stage3(g, d_nllp, d_ns3, s, &c->launches);
-  if (rc) return rc;
-  OWM_CUDA_TRY(cudaEventRecord(c->ev[4], s));
-  *d_seeds = g.seeds;
-  *room = g.z.nwin + g.z.ncell + 1;
-  return OWM_OK;
+  OWM_CUDA_TRY(cudaEventRecord(c->ev[0], s));
+  rc = grid_prepare(g, p, out.status, s, &c->launches);
+  if (!rc) rc = grid_fold(g, gp, 0, n, out.status, s, &c->launches);
+  if (!rc) rc = grid_windows(g, s, &c->launches);
+  if (!rc) rc = grid_stage2(g, p, pts.xy, pts.xy_stride, out.nllp, s, &c->launches);
+  if (!rc) rc = grid_stage3(g, out, s, &c->launches);
+  return rc;
 }
 }  // namespace
 
 int run_pipeline_enqueue(owm_ctx* c, const PointsView& pts, int64_t n, const owm_bbox& bb, const owm_run_cfg& cfg,
-                         owm_params* p_out, int64_t** d_seeds, int64_t* room_out) {
+                         ResultBuffer* rb, int64_t direct_max, owm_params* p_out, int64_t** d_seeds, int64_t* room_out) {
   if (validate_tree_cfg(&cfg.tree) != OWM_OK) return OWM_EINVAL;
   owm_params& p = *p_out;
   int rc = owm_params_compute(&bb, n, cfg.wsize, cfg.overlap, cfg.bsize, &p);
   if (rc) return rc;
-  if (!cfg.stage1_walk && c->walk_limit == 0) return run_grid(c, pts, n, p, d_seeds, room_out);
+  const int64_t room = p.ncells + std::max<int64_t>(p.ngrid, 0) + 1;
+  *room_out = room;
+  rc = rb->reserve(room <= direct_max ? room : 0, c->stream);
+  if (rc) return rc;
+  rb->words[8] = 0;
+  if (!cfg.stage1_walk && c->walk_limit == 0) return run_grid(c, pts, n, p, rb, direct_max, d_seeds);
   const int64_t nc = p.ncells, ng = std::max<int64_t>(p.ngrid, 0);
   rc = tree_alloc(&c->tree, &c->tree_mem, n, cfg.tree, c->stream);
   if (rc) return rc;
@@ -242,13 +272,14 @@ int run_pipeline_enqueue(owm_ctx* c, const PointsView& pts, int64_t n, const owm
                   s3scratch, s3cap, c->d_small + kStatusSlot, s, &c->launches);
   if (rc) return rc;
   OWM_CUDA_TRY(cudaEventRecord(c->ev[4], s));
-  const int64_t room = nc + ng + 1;
   const unsigned ga = (unsigned)std::min<int64_t>((room + 255) / 256, 152 * 8);
   OWM_LAUNCH("k_assemble", s, k_assemble<<<ga, 256, 0, s>>>(s3, d_ns3, llp, d_nllp, room, s64));
   count_launch(&c->launches);
   OWM_CUDA_TRY(cudaGetLastError());
-  *d_seeds = s64;
-  *room_out = room;
+  OWM_CUDA_TRY(cudaMemcpyAsync(rb->words, c->d_small, 32, cudaMemcpyDeviceToHost, s));
+  const bool direct = room <= direct_max;
+  if (direct) OWM_CUDA_TRY(cudaMemcpyAsync(rb->seeds, s64, (size_t)room * 8, cudaMemcpyDeviceToHost, s));
+  *d_seeds = direct ? nullptr : s64;
   return OWM_OK;
 }
 
@@ -257,14 +288,15 @@ int run_pipeline(owm_ctx* c, const PointsView& pts, int64_t n, const owm_bbox& b
   owm_params p;
   int64_t* s64 = nullptr;
   int64_t room = 0;
-  int rc = run_pipeline_enqueue(c, pts, n, bb, cfg, &p, &s64, &room);
+  ResultBuffer& rb = c->result;
+  int rc = run_pipeline_enqueue(c, pts, n, bb, cfg, &rb, kDirectSeeds, &p, &s64, &room);
   if (rc) return rc;
   cudaStream_t s = c->stream;
-  OWM_CUDA_TRY(cudaMemcpyAsync(c->h_small, c->d_small, 32, cudaMemcpyDeviceToHost, s));
+  OWM_CUDA_TRY(cudaEventRecord(c->ev[5], s));
   OWM_CUDA_TRY(cudaStreamSynchronize(s));
-  if (c->h_small[kStatusSlot] & kStatusNonFinite) return OWM_EINVAL;
-  if (c->h_small[kStatusSlot] & kStatusWalkBound) return OWM_ETIMEOUT;
-  const int64_t nllp = c->h_small[kLlpSlot], ns3 = c->h_small[kS3Slot];
+  if (rb.words[kStatusSlot] & kStatusNonFinite) return OWM_EINVAL;
+  if (rb.words[kStatusSlot] & kStatusWalkBound) return OWM_ETIMEOUT;
+  const int64_t nllp = rb.words[kLlpSlot], ns3 = rb.words[kS3Slot];
   const int64_t total = nllp + ns3;
   *n_seeds = total;
   if (info) {
@@ -274,22 +306,33 @@ int run_pipeline(owm_ctx* c, const PointsView& pts, int64_t n, const owm_bbox& b
     info->n_seeds = total;
     info->params = p;
   }
-  if (total > cap) return OWM_ERANGE;
-  if (total > 0) OWM_CUDA_TRY(cudaMemcpyAsync(seeds, s64, (size_t)total * 8, cudaMemcpyDefault, s));
-  OWM_CUDA_TRY(cudaEventRecord(c->ev[5], s));
-  OWM_CUDA_TRY(cudaStreamSynchronize(s));
   if (info) {
-    float a = 0, b = 0, d = 0, e = 0, f = 0;
-    cudaEventElapsedTime(&a, c->ev[0], c->ev[1]);
-    cudaEventElapsedTime(&b, c->ev[1], c->ev[2]);
-    cudaEventElapsedTime(&d, c->ev[2], c->ev[3]);
-    cudaEventElapsedTime(&e, c->ev[3], c->ev[4]);
+    if (rb.words[8]) {
+      unsigned long long t[kGridStamps];
+      std::memcpy(t, rb.words + 16, sizeof(t));
+      double* ms[4] = {&info->ms_tree, &info->ms_stage1, &info->ms_stage2, &info->ms_stage3};
+      for (int k = 0; k < 4; ++k) *ms[k] = 1e-6 * (double)(t[k + 1] - t[k]);
+    } else {
+      float a = 0, b = 0, d = 0, e = 0;
+      cudaEventElapsedTime(&a, c->ev[0], c->ev[1]);
+      cudaEventElapsedTime(&b, c->ev[1], c->ev[2]);
+      cudaEventElapsedTime(&d, c->ev[2], c->ev[3]);
+      cudaEventElapsedTime(&e, c->ev[3], c->ev[4]);
+      info->ms_tree = a;
+      info->ms_stage1 = b;
+      info->ms_stage2 = d;
+      info->ms_stage3 = e;
+    }
+    float f = 0;
     cudaEventElapsedTime(&f, c->ev[0], c->ev[5]);
-    info->ms_tree = a;
-    info->ms_stage1 = b;
-    info->ms_stage2 = d;
-    info->ms_stage3 = e;
     info->ms_total = f;
+  }
+  if (total > cap) return OWM_ERANGE;
+  if (total > 0 && !s64 && !is_device_ptr(seeds)) {
+    std::memcpy(seeds, rb.seeds, (size_t)total * 8);
+  } else if (total > 0) {
+    OWM_CUDA_TRY(cudaMemcpyAsync(seeds, s64 ? s64 : rb.seeds, (size_t)total * 8, cudaMemcpyDefault, s));
+    OWM_CUDA_TRY(cudaStreamSynchronize(s));
   }
   return OWM_OK;
 }
