@@ -76,7 +76,7 @@ struct ResultBuffer {
 // Synchronous runs of more windows and cells than this copy their seeds from
 // the device to the caller instead: one core reads pinned memory at about 20
 // GB/s, so that 120 K seeds cost more than a second wait (40.7 M points, 0.9 M
-// windows: 640 against 622 us), and 4 K seeds less (1 M points: 71 against 88).
+// windows: 640 against 589 us), and 4 K seeds less (1 M points: 71 against 88).
 constexpr int64_t kDirectSeeds = (int64_t)1 << 17;
 }  // namespace owm
 
