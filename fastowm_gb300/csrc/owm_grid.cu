@@ -74,6 +74,28 @@ __device__ __forceinline__ const GridJob& job_at(const GridJob& one, const GridT
   return T.jobs[t];
 }
 
+// The job of a block that works on one tile of a batch, in shared memory, and
+// the tile; *blk becomes the block's number within it.  Every thread of the
+// block calls it.  Found per thread instead (a search of log2(tiles) loads one
+// after the other, then the job's fields from global memory wherever they are
+// used) stage 1's reductions for 72 M points in 128 tiles took 220 us, not 185.
+struct BlockJob {
+  int tile;
+  GridJob job;
+};
+__device__ __forceinline__ void block_job(const GridTiles& T, BlockJob& S, int64_t* blk) {
+  int below = 0;
+  for (int j = threadIdx.x; j - (int)threadIdx.x < T.n; j += blockDim.x)
+    below += __syncthreads_count(j < T.n && __ldg(T.off + j) <= *blk);
+  const int t = below - 1;
+  *blk -= __ldg(T.off + t);
+  static_assert(sizeof(GridJob) % 16 == 0, "copied in 16-byte words");
+  for (int i = threadIdx.x; i < (int)(sizeof(GridJob) / 16); i += blockDim.x)
+    reinterpret_cast<uint4*>(&S.job)[i] = __ldg(reinterpret_cast<const uint4*>(T.jobs + t) + i);
+  if (threadIdx.x == 0) S.tile = t;
+  __syncthreads();
+}
+
 // ---- prepare ------------------------------------------------------------------
 struct FormulaEdges {
   const GridAxis* a;
@@ -390,15 +412,12 @@ __global__ void __launch_bounds__(kFoldBlock, kFoldBlocks)
 // shared memory.
 __global__ void __launch_bounds__(kFoldBlock, kFoldBlocks)
     k_grid_fold_tiles(GridTiles T, int32_t chunk, uint32_t* __restrict__ status) {
-  __shared__ GridJob J;
-  const int64_t blk = (int64_t)(blockIdx.x % kTileStripes) * (gridDim.x / kTileStripes) + blockIdx.x / kTileStripes;
+  __shared__ __align__(16) BlockJob S;
+  int64_t blk = (int64_t)(blockIdx.x % kTileStripes) * (gridDim.x / kTileStripes) + blockIdx.x / kTileStripes;
   if (blk >= __ldg(T.off + T.n)) return;
-  const int t = tile_of(T.off, T.n, blk);
-  static_assert(sizeof(GridJob) % 16 == 0, "copied in 16-byte words");
-  for (int i = threadIdx.x; i < (int)(sizeof(GridJob) / 16); i += kFoldBlock)
-    reinterpret_cast<uint4*>(&J)[i] = __ldg(reinterpret_cast<const uint4*>(T.jobs + t) + i);
-  __syncthreads();
-  const int64_t c0 = (blk - __ldg(T.off + t)) * (int64_t)chunk;
+  block_job(T, S, &blk);
+  const GridJob& J = S.job;
+  const int64_t c0 = blk * (int64_t)chunk;
   const int64_t n = min((int64_t)chunk, J.n - c0);  // points of this block
   GridPoints pts;
   pts.rec = J.rec;
@@ -441,63 +460,83 @@ __device__ __forceinline__ bool parity_range(const GridAxis& a, const uint32_t* 
   return lo <= hi;
 }
 
-template <bool kMulti>
-__global__ void __launch_bounds__(256) k_grid_rows(const __grid_constant__ GridJob one, GridTiles T, int64_t total) {
-  chain_start();
-  stamp(one, 1);
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    int64_t k = i;
-    const GridJob& J = job_at<kMulti>(one, T, &k);
-    const int32_t r = (int32_t)(k / J.x.n), ii = (int32_t)(k % J.x.n);
-    const int qy = r >= J.y.width[0];
-    if (!J.occ[2 + qy]) continue;
-    const int32_t iy = r - (qy ? J.y.width[0] : 0), lo = J.x.lo[ii], hi = J.x.hi[ii];
-    Best m;
-    for (int q = 0; q < 2; ++q) {
-      int32_t i0, i1;
-      if (!parity_range(J.x, J.occ, q, lo, hi, &i0, &i1)) continue;
-      const int64_t at = J.base[2 * qy + q] + (int64_t)iy * J.x.width[q];
-      for (int64_t c = at + i0; c <= at + i1; ++c) {
-        const ulonglong2 e = J.zid[c];
-        m.count += J.count[grid_count_slot(J, (uint32_t)c)];
-        m.take(e.x, (uint32_t)e.y);
-      }
+// A thread per sub-cell row and window column.  A batch's block takes rows of
+// one tile.
+__device__ __forceinline__ void rows_of(const GridJob& J, int64_t item) {
+  if (item >= (int64_t)J.y.nclass * J.x.n) return;
+  const uint32_t k = (uint32_t)item;  // below 2^32, as the sub-cells are
+  const int32_t r = (int32_t)(k / (uint32_t)J.x.n), ii = (int32_t)(k % (uint32_t)J.x.n);
+  const int qy = r >= J.y.width[0];
+  if (!J.occ[2 + qy]) return;
+  const int32_t iy = r - (qy ? J.y.width[0] : 0), lo = J.x.lo[ii], hi = J.x.hi[ii];
+  Best m;
+  for (int q = 0; q < 2; ++q) {
+    int32_t i0, i1;
+    if (!parity_range(J.x, J.occ, q, lo, hi, &i0, &i1)) continue;
+    const int64_t at = J.base[2 * qy + q] + (int64_t)iy * J.x.width[q];
+    for (int64_t c = at + i0; c <= at + i1; ++c) {
+      const ulonglong2 e = J.zid[c];
+      m.count += J.count[grid_count_slot(J, (uint32_t)c)];
+      m.take(e.x, (uint32_t)e.y);
     }
-    GridRow o;
-    o.w = m.w;
-    o.nid = m.nid;
-    o.count = m.count;
-    J.rows[k] = o;
   }
+  GridRow o;
+  o.w = m.w;
+  o.nid = m.nid;
+  o.count = m.count;
+  J.rows[k] = o;
 }
 
 template <bool kMulti>
-__global__ void __launch_bounds__(256) k_grid_windows(const __grid_constant__ GridJob one, GridTiles T, int64_t total) {
+__global__ void __launch_bounds__(256) k_grid_rows(const __grid_constant__ GridJob one, GridTiles T) {
   chain_start();
+  stamp(one, 1);
+  int64_t blk = blockIdx.x;
+  if (kMulti) {
+    __shared__ __align__(16) BlockJob S;
+    block_job(T, S, &blk);
+    rows_of(S.job, blk * 256 + threadIdx.x);
+  } else {
+    rows_of(one, blk * 256 + threadIdx.x);
+  }
+}
+
+__device__ __forceinline__ void window_of(const GridJob& J, int64_t item) {
+  if (item >= (int64_t)J.y.n * J.x.n) return;
   // the search starts from the reference's sentinel point 0 {0, 0, DBL_MAX}
   const unsigned long long sentinel = ~((unsigned long long)kZSentinel ^ 0x8000000000000000ull);
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    int64_t k = i;
-    const GridJob& J = job_at<kMulti>(one, T, &k);
-    const int32_t jj = (int32_t)(k / J.x.n), ii = (int32_t)(k % J.x.n);
-    Best m;
-    m.w = sentinel;
-    m.nid = ~0u;
-    for (int q = 0; q < 2; ++q) {
-      int32_t i0, i1;
-      if (!parity_range(J.y, J.occ + 2, q, J.y.lo[jj], J.y.hi[jj], &i0, &i1)) continue;
-      const int64_t at = q ? J.y.width[0] : 0;
-      for (int32_t r = i0; r <= i1; ++r) {
-        const GridRow e = J.rows[(at + r) * J.x.n + ii];
-        m.count += e.count;
-        m.take(e.w, e.nid);
-      }
+  const uint32_t k = (uint32_t)item;
+  const int32_t jj = (int32_t)(k / (uint32_t)J.x.n), ii = (int32_t)(k % (uint32_t)J.x.n);
+  Best m;
+  m.w = sentinel;
+  m.nid = ~0u;
+  for (int q = 0; q < 2; ++q) {
+    int32_t i0, i1;
+    if (!parity_range(J.y, J.occ + 2, q, J.y.lo[jj], J.y.hi[jj], &i0, &i1)) continue;
+    const int64_t at = q ? J.y.width[0] : 0;
+    for (int32_t r = i0; r <= i1; ++r) {
+      const GridRow e = J.rows[(at + r) * J.x.n + ii];
+      m.count += e.count;
+      m.take(e.w, e.nid);
     }
-    const uint32_t id = m.count >= J.thr ? ~m.nid : kNone;
-    if (J.win)
-      J.win[(int64_t)ii * J.y.n + jj] = id;
-    else
-      s2_mark_id(J.once, J.twice, (uint32_t)J.n, id);
+  }
+  const uint32_t id = m.count >= J.thr ? ~m.nid : kNone;
+  if (J.win)
+    J.win[(int64_t)ii * J.y.n + jj] = id;
+  else
+    s2_mark_id(J.once, J.twice, (uint32_t)J.n, id);
+}
+
+template <bool kMulti>
+__global__ void __launch_bounds__(256) k_grid_windows(const __grid_constant__ GridJob one, GridTiles T) {
+  chain_start();
+  int64_t blk = blockIdx.x;
+  if (kMulti) {
+    __shared__ __align__(16) BlockJob S;
+    block_job(T, S, &blk);
+    window_of(S.job, blk * 256 + threadIdx.x);
+  } else {
+    window_of(one, blk * 256 + threadIdx.x);
   }
 }
 
@@ -555,14 +594,13 @@ __device__ __forceinline__ void mark_cells(const GridJob& J, const double* __res
 // all chunks before it (whose counts, or words when part is null, it adds up)
 // and marks their cells.
 // A batch: tile by tile; nllp[t] is tile t's first LLP, nllp[T.n] their number.
+// The ids are listed first and then taken a thread each: the points' loads and
+// the marks of a chunk are in flight together (in the loop over a thread's
+// words they came one after the other: 24 us for 100 M points, now 18; 87 for 72
+// M in 128 tiles, now 50).
 template <bool kMulti>
-__global__ void __launch_bounds__(kSeedBlock) k_grid_seeds(const __grid_constant__ GridJob one, GridTiles T,
-                                                           const uint32_t* part, const double* __restrict__ xy, int stride,
-                                                           uint32_t* llp, uint32_t* nllp) {
-  chain_start();
-  stamp(one, 2);
-  int64_t chunk = blockIdx.x;
-  const GridJob& J = job_at<kMulti>(one, T, &chunk);
+__device__ __forceinline__ void write_seeds(const GridJob& J, const GridTiles& T, int tile, int64_t chunk, const uint32_t* part,
+                                            const double* __restrict__ xy, int stride, uint32_t* llp, uint32_t* nllp) {
   uint32_t before = 0, total;
   if (part) {
     for (uint32_t q = threadIdx.x; q < blockIdx.x; q += kSeedBlock) before += part[q];
@@ -579,18 +617,36 @@ __global__ void __launch_bounds__(kSeedBlock) k_grid_seeds(const __grid_constant
   const uint32_t word[4] = {q.x, q.y, q.z, q.w};
   uint32_t at = before + block_exclusive_256((uint32_t)(__popc(q.x) + __popc(q.y) + __popc(q.z) + __popc(q.w)), &total);
   if (threadIdx.x == 0) {
-    if (kMulti && chunk == 0) nllp[&J - T.jobs] = before;
+    if (kMulti && chunk == 0) nllp[tile] = before;
     if (blockIdx.x == gridDim.x - 1) nllp[kMulti ? T.n : 0] = before + total;
   }
 #pragma unroll
   for (int k = 0; k < kSeedWords; ++k) {
     uint32_t b = word[k];
     while (b) {
-      const uint32_t id = (uint32_t)((w0 + k) * 32) + (uint32_t)(__ffs(b) - 1);
+      llp[at++] = (uint32_t)((w0 + k) * 32) + (uint32_t)(__ffs(b) - 1);
       b &= b - 1;
-      llp[at++] = id;
-      if (J.x.nc) mark_cells(J, kMulti ? J.rec : xy, kMulti ? 3 : stride, id);
     }
+  }
+  if (!J.x.nc) return;
+  __syncthreads();  // the whole block's list
+  for (uint32_t k = before + threadIdx.x; k < before + total; k += kSeedBlock)
+    mark_cells(J, kMulti ? J.rec : xy, kMulti ? 3 : stride, llp[k]);
+}
+
+template <bool kMulti>
+__global__ void __launch_bounds__(kSeedBlock) k_grid_seeds(const __grid_constant__ GridJob one, GridTiles T,
+                                                           const uint32_t* part, const double* __restrict__ xy, int stride,
+                                                           uint32_t* llp, uint32_t* nllp) {
+  chain_start();
+  stamp(one, 2);
+  int64_t chunk = blockIdx.x;
+  if (kMulti) {
+    __shared__ __align__(16) BlockJob S;
+    block_job(T, S, &chunk);
+    write_seeds<true>(S.job, T, S.tile, chunk, part, xy, stride, llp, nllp);
+  } else {
+    write_seeds<false>(one, T, 0, chunk, part, xy, stride, llp, nllp);
   }
 }
 
@@ -1097,6 +1153,8 @@ int grid_batch_plan(const owm_params* p, const int64_t* n, int32_t ntiles, GridS
     g->items += prepare_items(p[k], z[k]);
     g->rows += z[k].rows;
     g->wins += z[k].nwin;
+    g->row_blocks += (z[k].rows + 255) / 256;
+    g->win_blocks += (z[k].nwin + 255) / 256;
     g->chunks += z[k].chunks;
     g->cells += z[k].ncell;
   }
@@ -1118,7 +1176,7 @@ int grid_batch_plan(const owm_params* p, const int64_t* n, int32_t ntiles, GridS
   g->words = c.take<uint32_t>(64);
   g->clear_bytes = c.at;
   g->jobs = c.take<GridJob>(ntiles);
-  for (auto** v : {&g->item_off, &g->fold_off, &g->row_off, &g->win_off, &g->chunk_off, &g->cell_off})
+  for (auto** v : {&g->item_off, &g->fold_off, &g->row_off, &g->win_off, &g->winb_off, &g->chunk_off, &g->cell_off})
     *v = c.take<int64_t>(ntiles + 1);
   g->table_bytes = c.at - g->clear_bytes;
   g->edges = c.take<char>(edges);
@@ -1152,9 +1210,9 @@ void grid_batch_tables(const owm_params* p, const int64_t* n, const GridSizes* z
   auto at = [&](const void* device) { return host + (static_cast<const char*>(device) - reinterpret_cast<const char*>(g.jobs)); };
   GridJob* jobs = reinterpret_cast<GridJob*>(host);
   int64_t *items = (int64_t*)at(g.item_off), *folds = (int64_t*)at(g.fold_off), *rows = (int64_t*)at(g.row_off),
-          *wins = (int64_t*)at(g.win_off), *chunks = (int64_t*)at(g.chunk_off), *cells = (int64_t*)at(g.cell_off);
-  items[0] = folds[0] = rows[0] = wins[0] = chunks[0] = cells[0] = 0;
-  int64_t sub = 0, counts = 0, own = 0, edges = 0;
+          *wins = (int64_t*)at(g.win_off), *winb = (int64_t*)at(g.winb_off), *chunks = (int64_t*)at(g.chunk_off), *cells = (int64_t*)at(g.cell_off);
+  items[0] = folds[0] = rows[0] = wins[0] = winb[0] = chunks[0] = cells[0] = 0;
+  int64_t sub = 0, counts = 0, own = 0, edges = 0, row_mem = 0;
   for (int32_t k = 0; k < g.ntiles; ++k) {
     GridJob& J = jobs[k];
     grid_job(p[k], n[k], z[k], &J);
@@ -1176,12 +1234,14 @@ void grid_batch_tables(const owm_params* p, const int64_t* n, const GridSizes* z
     J.mark = (uint8_t*)g.mark + cells[k];
     carve_edges(J, g.edges + edges);
     edges += (z[k].edges + 15) & ~(int64_t)15;
-    J.rows = (GridRow*)g.row_mem + rows[k];
+    J.rows = (GridRow*)g.row_mem + row_mem;
+    row_mem += z[k].rows;
     J.cellmin = (uint32_t*)g.cellmin + cells[k];
     items[k + 1] = items[k] + prepare_items(p[k], z[k]);
     folds[k + 1] = folds[k] + (n[k] + g.chunk - 1) / g.chunk;
-    rows[k + 1] = rows[k] + z[k].rows;
+    rows[k + 1] = rows[k] + (z[k].rows + 255) / 256;
     wins[k + 1] = wins[k] + z[k].nwin;
+    winb[k + 1] = winb[k] + (z[k].nwin + 255) / 256;
     chunks[k + 1] = chunks[k] + z[k].chunks;
     cells[k + 1] = cells[k] + z[k].ncell;
   }
@@ -1195,9 +1255,12 @@ int grid_batch_run(const GridBatch& g, cudaStream_t s, int64_t* launches) {
   OWM_LAUNCH("k_grid_prepare", s, k_grid_prepare<true><<<blocks_for(std::max(n16, g.items), 152 * 8), 256, 0, s>>>(
       none, tiles(g.item_off), g.items, (uint4*)g.base, n16, g.words));
   OWM_LAUNCH("k_grid_fold_tiles", s, k_grid_fold_tiles<<<(unsigned)((g.folds + kTileStripes - 1) / kTileStripes * kTileStripes), kFoldBlock, 0, s>>>(tiles(g.fold_off), g.chunk, g.words));
-  OWM_LAUNCH("k_grid_rows", s, k_grid_rows<true><<<blocks_for(g.rows, 152 * 32), 256, 0, s>>>(none, tiles(g.row_off), g.rows));
-  OWM_LAUNCH("k_grid_windows", s, k_grid_windows<true><<<blocks_for(g.wins, 152 * 32), 256, 0, s>>>(none, tiles(g.win_off), g.wins));
-  count_launch(launches, 4);
+  count_launch(launches, 2);
+  if (g.wins > 0) {
+    OWM_LAUNCH("k_grid_rows", s, k_grid_rows<true><<<(unsigned)g.row_blocks, 256, 0, s>>>(none, tiles(g.row_off)));
+    OWM_LAUNCH("k_grid_windows", s, k_grid_windows<true><<<(unsigned)g.win_blocks, 256, 0, s>>>(none, tiles(g.winb_off)));
+    count_launch(launches, 2);
+  }
   if (g.bitmap2) {
     OWM_LAUNCH("k_grid_seed_count", s, k_grid_seed_count<<<(unsigned)g.chunks, kSeedBlock, 0, s>>>(
         g.bitmap + g.chunks * kSeedChunk, g.part));
@@ -1258,10 +1321,8 @@ int grid_fold(const GridPlan& g, const GridPoints& pts, int64_t first, int64_t c
 
 int grid_windows(const GridPlan& g, cudaStream_t s, int64_t* launches) {
   const GridJob& J = g.job;
-  OWM_LAUNCH("k_grid_rows", s, OWM_CUDA_TRY(chain(k_grid_rows<false>, blocks_for(g.z.rows, 152 * 32), 256, s, J, GridTiles{},
-                                                  g.z.rows)));
-  OWM_LAUNCH("k_grid_windows", s, OWM_CUDA_TRY(chain(k_grid_windows<false>, blocks_for(g.z.nwin, 152 * 32), 256, s, J,
-                                                     GridTiles{}, g.z.nwin)));
+  OWM_LAUNCH("k_grid_rows", s, OWM_CUDA_TRY(chain(k_grid_rows<false>, (unsigned)((g.z.rows + 255) / 256), 256, s, J, GridTiles{})));
+  OWM_LAUNCH("k_grid_windows", s, OWM_CUDA_TRY(chain(k_grid_windows<false>, (unsigned)((g.z.nwin + 255) / 256), 256, s, J, GridTiles{})));
   count_launch(launches, 2);
   OWM_CUDA_TRY(cudaGetLastError());
   return OWM_OK;

@@ -421,6 +421,7 @@ struct GridBatch {
   int32_t bitmap2 = 1;            // every tile has overlap > 0
   int32_t tile_bits = 1, id_bits = 1;
   int64_t items = 0, folds = 0, rows = 0, wins = 0, chunks = 0, cells = 0;  // totals over the tiles
+  int64_t row_blocks = 0, win_blocks = 0;  // of 256 rows (windows) of one tile
   size_t clear_bytes = 0, table_bytes = 0, bytes = 0;
   char* base = nullptr;
   char *zid = nullptr, *count = nullptr, *cell_zid = nullptr, *mark = nullptr, *edges = nullptr, *row_mem = nullptr,
@@ -428,7 +429,8 @@ struct GridBatch {
   // device tables, written by the host for each batch: the jobs and, per kind
   // of item, the tiles' first ones
   GridJob* jobs = nullptr;
-  int64_t *item_off = nullptr, *fold_off = nullptr, *row_off = nullptr, *win_off = nullptr, *chunk_off = nullptr,
+  int64_t *item_off = nullptr, *fold_off = nullptr, *row_off = nullptr, *win_off = nullptr, *winb_off = nullptr,
+          *chunk_off = nullptr,
           *cell_off = nullptr;
   uint32_t *bitmap = nullptr, *part = nullptr, *llp = nullptr, *llp_off = nullptr, *s3cnt = nullptr, *words = nullptr;
   int64_t *out = nullptr, *out_off = nullptr;
