@@ -1,6 +1,6 @@
 // The window-grid path of one cloud (owm_grid.cuh): stage 1
 // (optim3_func.cpp:541-561), stage 2 (:610-625) and stage 3 (:627-662) with
-// their decisions on exact order keys, in seven launches:
+// their decisions on exact order keys, in seven launches (small clouds: k_grid_small, the same steps in one):
 //   k_grid_prepare   clears the tables, edge keys, s-ranges
 //   k_grid_fold      every point into its sub-cell (count, (z, id)-min)
 //   k_grid_rows      per sub-cell row and window column: reduce along x
@@ -14,6 +14,8 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <cstddef>
+#include <type_traits>
 
 #include "owm_devutil.cuh"
 #include "owm_grid.cuh"
@@ -106,51 +108,79 @@ struct StoredEdges {
   __device__ __forceinline__ int64_t operator()(int f, int32_t j) const { return a->edge[f][j]; }
 };
 
-__device__ int32_t class_of_key(const GridAxis& a, int64_t key) {
-  int32_t cnt[4];
-  grid_counts_exact(a, (uint64_t)__double_as_longlong(dkey_inv(key)), key, FormulaEdges{&a}, cnt);
-  return grid_sum(a, cnt);
-}
-
-// Edge keys and s-ranges of item i of one axis (windows, then cells).
-__device__ void prepare_axis(const GridAxis& a, int32_t i) {
+// Edge keys and s-range of item i of one axis (windows, then cells), by one
+// lane, or by eight neighbouring ones: lanes 0-3 the left edge, 4-7 the right
+// one, each counting the edges of one family passed just inside it.  (The
+// double-precision sums are a chain of slow operations: one cloud's edges, at
+// 10 K points, take 2.1 us by eight lanes an item and 4.7 by one.)
+template <int kLanes>
+__device__ __forceinline__ void prepare_axis(const GridAxis& a, int32_t i) {
   const bool win = i < a.n;
   const int32_t j = win ? i : i - a.n;
   const int f = win ? kFamL : kFamA;
-  const int64_t l = grid_edge(a, f, j), r = grid_edge(a, f + 1, j);
+  auto passed = [&](int q, int64_t key) {
+    uint32_t v;
+    const bool ok = grid_position(a, (uint64_t)__double_as_longlong(dkey_inv(key)), &v);
+    return q < 2 || a.merged ? grid_count_exact(a, q, ok, v, key, FormulaEdges{&a}) : 0;
+  };
+  int32_t lo = 0, hi = 0;
+  int64_t l, r;
+  if (kLanes == 8) {
+    const int lane = threadIdx.x & 7, q = lane & 3, side = lane >> 2;
+    const uint32_t group = 0xFFu << (threadIdx.x & 24);
+    const int64_t e = grid_edge(a, f + side, j), other = __shfl_xor_sync(group, e, 4);
+    l = side ? other : e;
+    r = side ? e : other;
+    int32_t c = passed(q, side ? r - 1 : l + 1);
+    __syncwarp(group);
+    c += __shfl_xor_sync(group, c, 1);
+    c += __shfl_xor_sync(group, c, 2);
+    lo = c;
+    hi = __shfl_xor_sync(group, c, 4);
+    if (lane) return;
+  } else {
+    l = grid_edge(a, f, j);
+    r = grid_edge(a, f + 1, j);
+    for (int q = 0; q < 4; ++q) lo += passed(q, l + 1);
+    for (int q = 0; q < 4; ++q) hi += passed(q, r - 1);
+  }
   const_cast<int64_t*>(a.edge[f])[j] = l;
   const_cast<int64_t*>(a.edge[f + 1])[j] = r;
   if (!win && !a.merged) return;
-  // no double lies between l and r when they touch: an empty range
-  (win ? a.lo : a.clo)[j] = class_of_key(a, l + 1);
-  (win ? a.hi : a.chi)[j] = l + 1 <= r - 1 ? class_of_key(a, r - 1) : -1;
+  (win ? a.lo : a.clo)[j] = lo;
+  (win ? a.hi : a.chi)[j] = l + 1 <= r - 1 ? hi : -1;  // no double lies between edges that touch: an empty range
 }
 
 // Bound by the stores of the clear (20 bytes a sub-cell, 2 bits a point);
 // one launch instead of a memset and six small kernels.
 template <bool kMulti>
-__global__ void __launch_bounds__(256) k_grid_prepare(const __grid_constant__ GridJob one, GridTiles T, int64_t items,
-                                                      uint4* __restrict__ clear, int64_t nclear,
-                                                      uint32_t* __restrict__ status) {
+__device__ __forceinline__ void prepare(const GridJob& one, const GridTiles& T, int64_t items, uint4* clear, int64_t nclear,
+                                        int64_t t, int64_t nt) {
   if (one.stamps && blockIdx.x == 0 && threadIdx.x == 0) one.stamps[1] = one.stamps[2] = one.stamps[3] = 0;
   stamp(one, 0);
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = t; i < items; i += nt) {
-    int64_t k = i;
+  const uint4 z = make_uint4(0, 0, 0, 0);  // the stores drain under the edges' arithmetic
+  for (int64_t i = t; i < nclear; i += nt) clear[i] = z;
+  constexpr int kLanes = kMulti ? 1 : 8;  // 128 tiles' items fill the chip by themselves (68 us; 72 by eight lanes)
+  for (int64_t i = t; i < kLanes * items; i += nt) {  // nt: whole warps
+    int64_t k = i / kLanes;
     const GridJob& J = job_at<kMulti>(one, T, &k);
     const int32_t nx = J.x.n + J.x.nc, ny = J.y.n + J.y.nc;
     if (k < nx) {
-      prepare_axis(J.x, (int32_t)k);
+      prepare_axis<kLanes>(J.x, (int32_t)k);
     } else if (k < nx + ny) {
-      prepare_axis(J.y, (int32_t)k - nx);
-    } else {
+      prepare_axis<kLanes>(J.y, (int32_t)k - nx);
+    } else if (t % kLanes == 0) {
       const int q = (int)(k - nx - ny);
       J.occ[q] = (q & 1) == 0;  // the other parity: when a point says so
     }
   }
+}
+template <bool kMulti>
+__global__ void __launch_bounds__(256) k_grid_prepare(const __grid_constant__ GridJob one, GridTiles T, int64_t items,
+                                                      uint4* clear, int64_t nclear, uint32_t* status) {
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t == 0) *status = 0;
-  const uint4 z = make_uint4(0, 0, 0, 0);
-  for (int64_t i = t; i < nclear; i += nt) clear[i] = z;
+  prepare<kMulti>(one, T, items, clear, nclear, t, (int64_t)gridDim.x * blockDim.x);
 }
 
 // ---- fold -----------------------------------------------------------------------
@@ -311,6 +341,37 @@ struct SharedAxes {
   __device__ __forceinline__ GridFastAxis y() const { return load(&J->y); }
 };
 
+// A point's sub-cell and z on axes with the fast form.
+template <bool kPaired, class Axes>
+__device__ __forceinline__ void fast_cell(const GridJob& J, Axes axes, uint64_t x, uint64_t y, uint64_t z, uint32_t& cell,
+                                          unsigned long long& w, uint32_t& flags) {
+  int32_t tx[4], ty[4];
+  uint32_t hx, hy, other;
+  const auto& ax = axes.x();
+  int32_t sx = grid_class_fast<kPaired>(ax, x, &hx, tx);
+  other = (sx ^ ax.par) & ax.parmask;
+  const uint32_t ix = (uint32_t)(sx >> ax.parmask);
+  const auto& ay = axes.y();
+  int32_t sy = grid_class_fast<kPaired>(ay, y, &hy, ty);
+  other |= (sy ^ ay.par) & ay.parmask;
+  cell = (uint32_t)(sy >> ay.parmask) * (uint32_t)J.x.width[0] + ix;
+  w = z ^ (~(uint64_t)((int64_t)z >> 63) & 0x7FFFFFFFFFFFFFFFull);
+  const bool odd_z = ((uint32_t)(z >> 32) << 1) - 1u >= 0xFFDFFFFFu;  // zero or not finite
+  if (odd_z | (other | hx | hy)) {
+    if (odd_z | ((hx | hy) & kGridOutside)) {
+      const PointCell p = point_cell_call(J, x, y, z);
+      cell = p.cell;
+      w = p.w;
+      flags |= p.flags;
+    } else {
+      if (hx) sx = grid_settle_fast(J.x, (int64_t)x, hx, tx, StoredEdges{&J.x}, sx);
+      if (hy) sy = grid_settle_fast(J.y, (int64_t)y, hy, ty, StoredEdges{&J.y}, sy);
+      cell = grid_cell(J, sx, sy);
+      flags |= (((sx ^ J.x.par) & J.x.parmask) ? kPointOtherX : 0u) | (((sy ^ J.y.par) & J.y.parmask) ? kPointOtherY : 0u);
+    }
+  }
+}
+
 template <int kStride, int kFast, class Axes>
 __device__ __forceinline__ void fold_stretch(const GridJob& J, Axes axes, const GridPoints& pts, int64_t first,
                                              int64_t count, int64_t b, int64_t e, uint32_t& flags) {
@@ -324,31 +385,7 @@ __device__ __forceinline__ void fold_stretch(const GridJob& J, Axes axes, const 
     load_raw<kStride>(pts, i, x, y, z, nid);
     unsigned long long w;
     if (kFast) {
-      int32_t tx[4], ty[4];
-      uint32_t hx, hy, other;
-      const auto& ax = axes.x();
-      int32_t sx = grid_class_fast<kFast == 2>(ax, x, &hx, tx);
-      other = (sx ^ ax.par) & ax.parmask;
-      const uint32_t ix = (uint32_t)(sx >> ax.parmask);
-      const auto& ay = axes.y();
-      int32_t sy = grid_class_fast<kFast == 2>(ay, y, &hy, ty);
-      other |= (sy ^ ay.par) & ay.parmask;
-      cell = (uint32_t)(sy >> ay.parmask) * (uint32_t)J.x.width[0] + ix;
-      w = z ^ (~(uint64_t)((int64_t)z >> 63) & 0x7FFFFFFFFFFFFFFFull);
-      const bool odd_z = ((uint32_t)(z >> 32) << 1) - 1u >= 0xFFDFFFFFu;  // zero or not finite
-      if (odd_z | (other | hx | hy)) {
-        if (odd_z | ((hx | hy) & kGridOutside)) {
-          const PointCell p = point_cell_call(J, x, y, z);
-          cell = p.cell;
-          w = p.w;
-          flags |= p.flags;
-        } else {
-          if (hx) sx = grid_settle_fast(J.x, (int64_t)x, hx, tx, StoredEdges{&J.x}, sx);
-          if (hy) sy = grid_settle_fast(J.y, (int64_t)y, hy, ty, StoredEdges{&J.y}, sy);
-          cell = grid_cell(J, sx, sy);
-          flags |= (((sx ^ J.x.par) & J.x.parmask) ? kPointOtherX : 0u) | (((sy ^ J.y.par) & J.y.parmask) ? kPointOtherY : 0u);
-        }
-      }
+      fast_cell<kFast == 2>(J, axes, x, y, z, cell, w, flags);
     } else {
       const PointCell p = point_cell(J, x, y, z);
       cell = p.cell;
@@ -542,11 +579,11 @@ __global__ void __launch_bounds__(256) k_grid_windows(const __grid_constant__ Gr
 
 // ---- stage 2 ------------------------------------------------------------------
 constexpr int kSeedBlock = 256;
-constexpr int kSeedWords = 4;
-constexpr int64_t kSeedChunk = (int64_t)kSeedBlock * kSeedWords;  // bitmap words a block takes
+constexpr int64_t kSeedChunk = 4 * (int64_t)kSeedBlock;  // bitmap words a block takes
 
-__device__ __forceinline__ uint32_t block_exclusive_256(uint32_t v, uint32_t* total) {
-  __shared__ uint32_t ws[kSeedBlock / 32];
+template <int kBlock = kSeedBlock>
+__device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t* total) {
+  __shared__ uint32_t ws[kBlock / 32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   uint32_t inc = v;
 #pragma unroll
@@ -557,14 +594,26 @@ __device__ __forceinline__ uint32_t block_exclusive_256(uint32_t v, uint32_t* to
   __syncthreads();  // the last call's readers of ws are done
   if (lane == 31) ws[w] = inc;
   __syncthreads();
-  uint32_t before = 0, all = 0;
+  uint32_t before = 0;
+  if (kBlock > 256) {
+    uint32_t sum = ws[lane % (kBlock / 32)];
 #pragma unroll
-  for (int q = 0; q < kSeedBlock / 32; ++q) {
-    const uint32_t x = ws[q];
-    before += q < w ? x : 0u;
-    all += x;
+    for (int o = 1; o < kBlock / 32; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, sum, o);
+      if (lane >= o) sum += t;
+    }
+    *total = __shfl_sync(0xffffffffu, sum, kBlock / 32 - 1);
+    if (w) before = __shfl_sync(0xffffffffu, sum, w - 1);
+  } else {
+    uint32_t all = 0;
+#pragma unroll
+    for (int q = 0; q < kBlock / 32; ++q) {
+      const uint32_t x = ws[q];
+      before += q < w ? x : 0u;
+      all += x;
+    }
+    *total = all;
   }
-  *total = all;
   return before + inc - v;
 }
 
@@ -572,7 +621,7 @@ __global__ void __launch_bounds__(kSeedBlock) k_grid_seed_count(const uint32_t* 
   chain_start();
   const uint4 q = reinterpret_cast<const uint4*>(bm)[(int64_t)blockIdx.x * kSeedBlock + threadIdx.x];
   uint32_t total;
-  block_exclusive_256((uint32_t)(__popc(q.x) + __popc(q.y) + __popc(q.z) + __popc(q.w)), &total);
+  block_exclusive((uint32_t)(__popc(q.x) + __popc(q.y) + __popc(q.z) + __popc(q.w)), &total);
   if (threadIdx.x == 0) part[blockIdx.x] = total;
 }
 
@@ -598,30 +647,33 @@ __device__ __forceinline__ void mark_cells(const GridJob& J, const double* __res
 // the marks of a chunk are in flight together (in the loop over a thread's
 // words they came one after the other: 24 us for 100 M points, now 18; 87 for 72
 // M in 128 tiles, now 50).
-template <bool kMulti>
-__device__ __forceinline__ void write_seeds(const GridJob& J, const GridTiles& T, int tile, int64_t chunk, const uint32_t* part,
+template <bool kMulti, int kBlock = kSeedBlock>
+__device__ __forceinline__ void write_seeds(const GridJob& J, const GridTiles& T, int tile, int64_t chunk, uint32_t blocks, const uint32_t* part,
                                             const double* __restrict__ xy, int stride, uint32_t* llp, uint32_t* nllp) {
   uint32_t before = 0, total;
   if (part) {
-    for (uint32_t q = threadIdx.x; q < blockIdx.x; q += kSeedBlock) before += part[q];
+    for (uint32_t q = threadIdx.x; q < blockIdx.x; q += kBlock) before += part[q];
   } else {  // few chunks: their words themselves
     const uint4* w = reinterpret_cast<const uint4*>(J.twice);
-    for (uint32_t q = threadIdx.x; q < blockIdx.x * kSeedBlock; q += kSeedBlock) {
+    const uint32_t words = blockIdx.x * (uint32_t)(kSeedChunk / 4);
+    for (uint32_t q = threadIdx.x; q < words; q += kBlock) {
       const uint4 v = w[q];
       before += (uint32_t)(__popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w));
     }
   }
-  block_exclusive_256(before, &before);
-  const int64_t w0 = chunk * kSeedChunk + (int64_t)threadIdx.x * kSeedWords;
-  const uint4 q = *reinterpret_cast<const uint4*>(J.twice + w0);
+  block_exclusive<kBlock>(before, &before);
+  constexpr int kWords = (int)(kSeedChunk / kBlock);  // of a thread
+  static_assert(kWords == 4 || kWords == 1, "one load");
+  const int64_t w0 = chunk * kSeedChunk + (int64_t)threadIdx.x * kWords;
+  const uint4 q = kWords == 4 ? *reinterpret_cast<const uint4*>(J.twice + w0) : make_uint4(J.twice[w0], 0, 0, 0);
   const uint32_t word[4] = {q.x, q.y, q.z, q.w};
-  uint32_t at = before + block_exclusive_256((uint32_t)(__popc(q.x) + __popc(q.y) + __popc(q.z) + __popc(q.w)), &total);
+  uint32_t at = before + block_exclusive<kBlock>((uint32_t)(__popc(q.x) + __popc(q.y) + __popc(q.z) + __popc(q.w)), &total);
   if (threadIdx.x == 0) {
     if (kMulti && chunk == 0) nllp[tile] = before;
-    if (blockIdx.x == gridDim.x - 1) nllp[kMulti ? T.n : 0] = before + total;
+    if (blockIdx.x == blocks - 1) nllp[kMulti ? T.n : 0] = before + total;
   }
 #pragma unroll
-  for (int k = 0; k < kSeedWords; ++k) {
+  for (int k = 0; k < kWords; ++k) {
     uint32_t b = word[k];
     while (b) {
       llp[at++] = (uint32_t)((w0 + k) * 32) + (uint32_t)(__ffs(b) - 1);
@@ -630,7 +682,7 @@ __device__ __forceinline__ void write_seeds(const GridJob& J, const GridTiles& T
   }
   if (!J.x.nc) return;
   __syncthreads();  // the whole block's list
-  for (uint32_t k = before + threadIdx.x; k < before + total; k += kSeedBlock)
+  for (uint32_t k = before + threadIdx.x; k < before + total; k += kBlock)
     mark_cells(J, kMulti ? J.rec : xy, kMulti ? 3 : stride, llp[k]);
 }
 
@@ -644,9 +696,9 @@ __global__ void __launch_bounds__(kSeedBlock) k_grid_seeds(const __grid_constant
   if (kMulti) {
     __shared__ __align__(16) BlockJob S;
     block_job(T, S, &chunk);
-    write_seeds<true>(S.job, T, S.tile, chunk, part, xy, stride, llp, nllp);
+    write_seeds<true>(S.job, T, S.tile, chunk, gridDim.x, part, xy, stride, llp, nllp);
   } else {
-    write_seeds<false>(one, T, 0, chunk, part, xy, stride, llp, nllp);
+    write_seeds<false>(one, T, 0, chunk, gridDim.x, part, xy, stride, llp, nllp);
   }
 }
 
@@ -669,14 +721,8 @@ __device__ __forceinline__ uint32_t cell_result(unsigned long long w, uint32_t n
 
 // One warp per cell: the (z, id)-min of its rectangle of sub-cells, or its own
 // entry.
-template <bool kMulti>
-__global__ void __launch_bounds__(256) k_grid_cells(const __grid_constant__ GridJob one, GridTiles T, int64_t total) {
-  chain_start();
-  stamp(one, 3);
+__device__ __forceinline__ void cell_of(const GridJob& J, int64_t c) {
   const int lane = threadIdx.x & 31;
-  int64_t c = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (c >= total) return;
-  const GridJob& J = job_at<kMulti>(one, T, &c);
   const int32_t ci = (int32_t)(c % J.x.nc), cj = (int32_t)(c / J.x.nc);
   Best m;
   if (J.cell_zid) {
@@ -704,6 +750,16 @@ __global__ void __launch_bounds__(256) k_grid_cells(const __grid_constant__ Grid
   if (lane == 0) J.cellmin[c] = cell_result(m.w, m.nid);
 }
 
+template <bool kMulti>
+__global__ void __launch_bounds__(256) k_grid_cells(const __grid_constant__ GridJob one, GridTiles T, int64_t total) {
+  chain_start();
+  stamp(one, 3);
+  int64_t c = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (c >= total) return;
+  const GridJob& J = job_at<kMulti>(one, T, &c);
+  cell_of(J, c);
+}
+
 // The result's words (ResultBuffer), by one thread once the counts are known.
 __device__ __forceinline__ void write_words(const GridJob& J, const GridResult& R, uint32_t nllp, uint32_t ns3) {
   *R.ns3 = ns3;
@@ -721,30 +777,181 @@ __device__ __forceinline__ void write_words(const GridJob& J, const GridResult& 
 // seeds = the valid entries of cellmin in order, then the LLPs.  Every block
 // counts all cells (at most kOutputCells) for the total and its own start.
 constexpr int64_t kOutputCells = 32768;
-__global__ void __launch_bounds__(kSeedBlock) k_grid_output(const __grid_constant__ GridJob J, int64_t ncell, const uint32_t* llp,
-                                                            GridResult R) {
-  chain_start();
-  const int64_t per = (ncell + gridDim.x - 1) / gridDim.x;
-  const int64_t b0 = per * blockIdx.x, b1 = min(b0 + per, ncell);
+template <int kBlock>
+__device__ __forceinline__ void write_output(const GridJob& J, int64_t ncell, const uint32_t* llp, const GridResult& R, int64_t blk,
+                                             int64_t blocks) {
+  const int64_t per = (ncell + blocks - 1) / blocks;
+  const int64_t b0 = per * blk, b1 = min(b0 + per, ncell);
   uint32_t before = 0, all = 0;
-  for (int64_t i = threadIdx.x; i < ncell; i += kSeedBlock) {
+  for (int64_t i = threadIdx.x; i < ncell; i += kBlock) {
     const uint32_t v = J.cellmin[i] != kNone ? 1u : 0u;
     all += v;
     if (i < b0) before += v;
   }
-  block_exclusive_256(before, &before);
-  block_exclusive_256(all, &all);
+  block_exclusive<kBlock>(before, &before);
+  block_exclusive<kBlock>(all, &all);
   uint32_t at = before;
-  for (int64_t t = b0; t < b1; t += kSeedBlock) {
+  for (int64_t t = b0; t < b1; t += kBlock) {
     const uint32_t v = t + threadIdx.x < b1 ? J.cellmin[t + threadIdx.x] : kNone;
     uint32_t got;
-    const uint32_t p = block_exclusive_256(v != kNone ? 1u : 0u, &got);
+    const uint32_t p = block_exclusive<kBlock>(v != kNone ? 1u : 0u, &got);
     if (v != kNone) R.seeds[at + p] = v;
     at += got;
   }
   const uint32_t n = *R.nllp;
-  for (uint32_t k = blockIdx.x * kSeedBlock + threadIdx.x; k < n; k += gridDim.x * kSeedBlock) R.seeds[all + k] = llp[k];
-  if (blockIdx.x == 0 && threadIdx.x == 0) write_words(J, R, n, all);
+  for (uint32_t k = (uint32_t)blk * kBlock + threadIdx.x; k < n; k += (uint32_t)blocks * kBlock) R.seeds[all + k] = llp[k];
+  if (blk == 0 && threadIdx.x == 0) write_words(J, R, n, all);
+}
+
+__global__ void __launch_bounds__(kSeedBlock) k_grid_output(const __grid_constant__ GridJob J, int64_t ncell, const uint32_t* llp,
+                                                            GridResult R) {
+  chain_start();
+  write_output<kSeedBlock>(J, ncell, llp, R, blockIdx.x, gridDim.x);
+}
+
+// ---- small clouds: all of it in one launch -----------------------------------------
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// This block's address of p (in shared memory) in the block of that rank.
+template <class T>
+__device__ __forceinline__ T* in_block(T* p, int rank) {
+  T* q;
+  asm("mapa.u64 %0, %1, %2;" : "=l"(q) : "l"(p), "r"(rank));
+  return q;
+}
+
+constexpr int kSmallCluster = 8, kSmallBlock = 1024, kSmallPer = 4;
+// Points: at most kSmallPer a thread, and ids in one chunk of the bitmaps.
+constexpr int64_t kSmallPoints = (int64_t)kSmallCluster * kSmallBlock * kSmallPer - 1;
+static_assert((kSmallPoints + 1 + 31) / 32 <= kSeedChunk, "one chunk");
+
+// The 8-byte words of a GridJob that are addresses of its tables.
+struct JobTables {
+  uint64_t m[2];
+};
+constexpr JobTables job_tables() {
+  JobTables w{};
+  constexpr size_t x = offsetof(GridJob, x), y = offsetof(GridJob, y);
+  const size_t at[] = {offsetof(GridJob, zid), offsetof(GridJob, count), offsetof(GridJob, rows), offsetof(GridJob, occ),
+                       offsetof(GridJob, mark), offsetof(GridJob, cellmin), offsetof(GridJob, once), offsetof(GridJob, twice)};
+  for (size_t a : at) w.m[a / 512] |= 1ull << (a / 8 % 64);
+  for (size_t axis : {x, y}) {
+    for (size_t k = 0; k < 4; ++k) {
+      const size_t a = axis + offsetof(GridAxis, edge) + 8 * k;
+      w.m[a / 512] |= 1ull << (a / 8 % 64);
+    }
+    for (size_t f : {offsetof(GridAxis, lo), offsetof(GridAxis, hi), offsetof(GridAxis, clo), offsetof(GridAxis, chi)})
+      w.m[(axis + f) / 512] |= 1ull << ((axis + f) / 8 % 64);
+  }
+  return w;
+}
+constexpr uint64_t kJobTables0 = job_tables().m[0], kJobTables1 = job_tables().m[1];
+static_assert(sizeof(GridJob) <= 1024 && sizeof(GridJob) % 8 == 0, "two words of 64 bits");
+
+// The whole path of a small cloud by one cluster, with every table of the plan
+// in shared memory: each block folds an eighth of the points into tables of its
+// own (minimum of z first, then of the ids that have it), the blocks merge a
+// slice of the sub-cells each into the first one's, and that one does the rest.
+// Bound by latency, about 2 us each for the edges, the fold, the merge, the
+// reductions, the seeds and the output.  10 K points take 34 us a call and as a
+// chain of seven kernels, which meet in L2, 46 (the launches hide behind the
+// kernels: the same steps in one launch on global tables took 43).
+// base: where the plan's tables would lie.
+template <int kStride>
+__global__ void __cluster_dims__(kSmallCluster) __launch_bounds__(kSmallBlock)
+    k_grid_small(const __grid_constant__ GridJob G, const __grid_constant__ GridPoints pts, const char* base, int64_t items,
+                 int64_t nclear, uint32_t nsub, const double* __restrict__ xy, int xy_stride, int32_t ncell,
+                 int64_t llp_at, const __grid_constant__ GridResult R) {
+  extern __shared__ __align__(256) char mem[];
+  __shared__ __align__(16) GridJob J;
+  __shared__ uint32_t words[4];
+  __shared__ unsigned long long stamps[kGridStamps];
+  const int t = threadIdx.x, rank = blockIdx.x;
+  const int64_t delta = (int64_t)mem - (int64_t)base;  // whole numbers: an address made from a parameter's is taken for global memory
+  uint32_t* llp = reinterpret_cast<uint32_t*>(mem + llp_at);
+  if (t < (int)(sizeof(GridJob) / 8)) {  // the job, its tables' addresses moved here
+    int64_t v = reinterpret_cast<const int64_t*>(&G)[t];
+    if ((((t < 64 ? kJobTables0 : kJobTables1) >> (t & 63)) & 1) && v) v += delta;
+    if (t == (int)(offsetof(GridJob, stamps) / 8)) v = (int64_t)stamps;
+    reinterpret_cast<int64_t*>(&J)[t] = v;
+  }
+  GridResult out = R;  // the words that it reads again itself
+  out.status = &words[0];
+  out.nllp = &words[1];
+  out.ns3 = &words[2];
+  if (t < 4) words[t] = 0;
+  const int per = (G.n + kSmallCluster - 1) / kSmallCluster, first = rank * per + t, last = min(G.n, (rank + 1) * per);
+  // the points' loads go out before the tables are ready
+  uint64_t x[kSmallPer], y[kSmallPer], z[kSmallPer];
+  uint32_t nid[kSmallPer], cell[kSmallPer];
+#pragma unroll
+  for (int k = 0; k < kSmallPer; ++k) {
+    const int i = first + k * kSmallBlock;
+    if (i < last) load_raw<kStride>(pts, i, x[k], y[k], z[k], nid[k]);
+  }
+  __syncthreads();
+  prepare<false>(J, GridTiles{}, items, reinterpret_cast<uint4*>(mem), nclear, t, kSmallBlock);
+  __syncthreads();
+  uint32_t flags = 0;
+#pragma unroll
+  for (int k = 0; k < kSmallPer; ++k) {
+    if (first + k * kSmallBlock >= last) break;
+    if (J.fast == 2) {
+      unsigned long long w;
+      fast_cell<true>(J, ParamAxes{&J}, x[k], y[k], z[k], cell[k], w, flags);
+      z[k] = w;
+    } else {
+      const PointCell p = point_cell_call(J, x[k], y[k], z[k]);
+      cell[k] = p.cell;
+      z[k] = p.w;
+      flags |= p.flags;
+    }
+    atomicAdd(J.count + grid_count_slot(J, cell[k]), 1u);
+    atomicMax(&J.zid[cell[k]].x, (unsigned long long)z[k]);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kSmallPer; ++k) {
+    if (first + k * kSmallBlock >= last) break;
+    ulonglong2* e = J.zid + cell[k];
+    if (e->x == z[k]) atomicMax(&e->y, (unsigned long long)nid[k]);
+  }
+  flags = __reduce_or_sync(0xffffffffu, flags);
+  cluster_barrier();  // all folded; the first block's words are set up
+  if ((t & 31) == 0 && flags) {
+    uint32_t* occ = in_block(J.occ, 0);
+    if (flags & kPointNonFinite) atomicOr(in_block(&words[0], 0), kStatusNonFinite);
+    if (flags & kPointOtherX) occ[1] = 1;
+    if (flags & kPointOtherY) occ[3] = 1;
+  }
+  const uint32_t slice = (nsub + kSmallCluster - 1) / kSmallCluster, end = min(nsub, (rank + 1) * slice);
+  for (uint32_t c = rank * slice + t; c < end; c += kSmallBlock) {
+    Best m;
+#pragma unroll
+    for (int k = 0; k < kSmallCluster; ++k) {
+      const ulonglong2 e = *in_block(J.zid + c, k);
+      m.count += *in_block(J.count + grid_count_slot(J, c), k);
+      m.take(e.x, (uint32_t)e.y);
+    }
+    *in_block(J.zid + c, 0) = make_ulonglong2(m.w, m.nid);
+    *in_block(J.count + grid_count_slot(J, c), 0) = m.count;
+  }
+  cluster_barrier();
+  if (rank) return;
+  stamp(J, 1);
+  for (int64_t i = t; i < (int64_t)J.y.nclass * J.x.n; i += kSmallBlock) rows_of(J, i);
+  __syncthreads();
+  for (int64_t i = t; i < (int64_t)J.y.n * J.x.n; i += kSmallBlock) window_of(J, i);
+  __syncthreads();
+  stamp(J, 2);
+  write_seeds<false, kSmallBlock>(J, GridTiles{}, 0, 0, 1, nullptr, xy, xy_stride, llp, out.nllp);
+  __syncthreads();
+  stamp(J, 3);
+  for (int32_t c = t >> 5; c < ncell; c += kSmallBlock / 32) cell_of(J, c);
+  __syncthreads();
+  write_output<kSmallBlock>(J, ncell, llp, out, 0, 1);
 }
 
 __global__ void k_grid_flags(const uint32_t* __restrict__ v, int64_t n, uint32_t* __restrict__ flags) {
@@ -799,7 +1006,7 @@ __global__ void __launch_bounds__(kSeedBlock) k_gridb_count(GridTiles T, uint32_
   const int64_t n = (int64_t)J.x.nc * J.y.nc;
   uint32_t c = 0;
   for (int64_t i = threadIdx.x; i < n; i += kSeedBlock) c += J.cellmin[i] != kNone ? 1u : 0u;
-  block_exclusive_256(c, &c);
+  block_exclusive(c, &c);
   if (threadIdx.x == 0) s3cnt[blockIdx.x] = c;
 }
 
@@ -812,7 +1019,7 @@ __global__ void __launch_bounds__(kSeedBlock) k_gridb_output(GridTiles T, const 
   const GridJob& J = T.jobs[t];
   uint32_t c = 0, s3_before;
   for (int q = threadIdx.x; q < t; q += kSeedBlock) c += __ldg(s3cnt + q);
-  block_exclusive_256(c, &s3_before);
+  block_exclusive(c, &s3_before);
   const uint32_t l0 = llp_off[t], l1 = llp_off[t + 1], mine = s3cnt[t];
   int64_t at = (int64_t)s3_before + l0;
   if (threadIdx.x == 0) {
@@ -824,7 +1031,7 @@ __global__ void __launch_bounds__(kSeedBlock) k_gridb_output(GridTiles T, const 
   for (int64_t i = 0; i < n && mine; i += kSeedBlock) {
     const uint32_t v = i + threadIdx.x < n ? J.cellmin[i + threadIdx.x] : kNone;
     uint32_t got;
-    const uint32_t p = block_exclusive_256(v != kNone ? 1u : 0u, &got);
+    const uint32_t p = block_exclusive(v != kNone ? 1u : 0u, &got);
     if (v != kNone) out[at + p] = v;
     at += got;
   }
@@ -1074,6 +1281,9 @@ void carve_edges(GridJob& J, char* b) {
     a->chi = (int32_t*)take((size_t)a->nc * 4);
   }
 }
+// What k_grid_small's tables take: the plan's pieces before the seeds.
+constexpr size_t kSmallBytes = 224 * 1024;  // of a block's 227 K
+size_t small_bytes(const GridPlan& g) { return (size_t)(reinterpret_cast<const char*>(g.seeds) - g.base); }
 // Threads' items of k_grid_prepare: windows and cells per axis, occupancy words.
 int64_t prepare_items(const owm_params& p, const GridSizes& z) {
   return (int64_t)p.ncols + p.nrows + (z.ncell ? (int64_t)p.ncols_grid + p.nrows_grid : 0) + 4;
@@ -1314,6 +1524,25 @@ int grid_fold(const GridPlan& g, const GridPoints& pts, int64_t first, int64_t c
                                        {k_grid_fold<4, 0>, k_grid_fold<4, 1>, k_grid_fold<4, 2>}};
   const Kernel kernel = kernels[pts.stride == 4 ? 2 : pts.stride == 3 ? 1 : 0][J.fast];
   OWM_LAUNCH("k_grid_fold", s, OWM_CUDA_TRY(chain(kernel, nb, kFoldBlock, s, J, pts, first, count, status)));
+  count_launch(launches);
+  OWM_CUDA_TRY(cudaGetLastError());
+  return OWM_OK;
+}
+
+// 32 K points take 39 us a call this way and 43 as a chain, 20 K 34 and 40, 1 K
+// 28 and 36; 10 K more points add 4 us here and 1 there.  Cells with a table of
+// their own, and stage 2 by sorting, go by the chain.
+bool grid_is_small(const GridPlan& g) {
+  return g.bitmap2 && g.n <= kSmallPoints && (g.z.merged || g.z.ncell == 0) && small_bytes(g) <= kSmallBytes;
+}
+
+int grid_small(const GridPlan& g, const owm_params& p, const GridPoints& pts, const double* xy, int xy_stride,
+               const GridResult& out, cudaStream_t s, int64_t* launches) {
+  const auto kernel = pts.stride == 4 ? k_grid_small<4> : k_grid_small<3>;
+  OWM_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallBytes));
+  OWM_LAUNCH("k_grid_small", s, kernel<<<kSmallCluster, kSmallBlock, small_bytes(g), s>>>(
+      g.job, pts, g.base, prepare_items(p, g.z), (int64_t)(g.clear_bytes / 16), (uint32_t)g.z.nsub, xy, xy_stride,
+      (int32_t)g.z.ncell, reinterpret_cast<const char*>(g.llp) - g.base, out));
   count_launch(launches);
   OWM_CUDA_TRY(cudaGetLastError());
   return OWM_OK;

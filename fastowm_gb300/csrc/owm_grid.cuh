@@ -142,29 +142,33 @@ __host__ __device__ __forceinline__ int32_t grid_count(const GridAxis& a, int fa
   return (int32_t)(h >> fb) - (win ? a.kw : a.kc);
 }
 
-// The four edge counts of a coordinate, exactly.  edge_of(fam, j) gives the
-// edges' order keys.
+// Edge count of family f at an order key, exactly.  v: the key's position, where
+// it has one (ok).  edge_of(fam, j) gives the edges' order keys.
+template <class EdgeOf>
+__host__ __device__ __forceinline__ int32_t grid_count_exact(const GridAxis& a, int f, bool ok, uint32_t v, int64_t key,
+                                                             EdgeOf edge_of) {
+  const int32_t n = f < 2 ? a.n : a.nc;
+  if (ok) {
+    bool near;
+    int32_t k = grid_count(a, f, v, &near);
+    if (near && k >= 1 && k <= n) k -= grid_passed(f, edge_of(f, k - 1), key) ? 0 : 1;
+    return grid_clamp(k, n);
+  }
+  int32_t lo = 0, hi = n;
+  while (lo < hi) {
+    const int32_t mid = (lo + hi) >> 1;
+    if (grid_passed(f, edge_of(f, mid), key)) lo = mid + 1; else hi = mid;
+  }
+  return lo;
+}
+
+// All four of a coordinate.
 template <class EdgeOf>
 __host__ __device__ __forceinline__ void grid_counts_exact(const GridAxis& a, uint64_t bits, int64_t key, EdgeOf edge_of,
                                                            int32_t cnt[4]) {
   uint32_t v;
   const bool ok = grid_position(a, bits, &v);
-  for (int f = 0; f < 4; ++f) {
-    const int32_t n = f < 2 ? a.n : a.nc;
-    if (ok) {
-      bool near;
-      int32_t k = grid_count(a, f, v, &near);
-      if (near && k >= 1 && k <= n) k -= grid_passed(f, edge_of(f, k - 1), key) ? 0 : 1;
-      cnt[f] = grid_clamp(k, n);
-    } else {
-      int32_t lo = 0, hi = n;
-      while (lo < hi) {
-        const int32_t mid = (lo + hi) >> 1;
-        if (grid_passed(f, edge_of(f, mid), key)) lo = mid + 1; else hi = mid;
-      }
-      cnt[f] = lo;
-    }
-  }
+  for (int f = 0; f < 4; ++f) cnt[f] = grid_count_exact(a, f, ok, v, key, edge_of);
 }
 
 // The four edge counts of a coordinate in [lo, hi], not yet clamped to their
@@ -413,6 +417,10 @@ struct GridResult {
   int64_t* seeds = nullptr;
   uint32_t* words = nullptr;
 };
+// Whether a run takes one launch (grid_small) in place of all of these.
+bool grid_is_small(const GridPlan& g);
+int grid_small(const GridPlan& g, const owm_params& p, const GridPoints& pts, const double* xy, int xy_stride,
+               const GridResult& out, cudaStream_t s, int64_t* launches);
 int grid_stage3(const GridPlan& g, const GridResult& out, cudaStream_t s, int64_t* launches);
 
 // Many tiles at once: one launch per step, every tile with its own job.

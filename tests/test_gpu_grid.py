@@ -95,3 +95,28 @@ def test_stage1_of_a_tree(owm, oracle, x0, W, Ov, policy):
     np.testing.assert_array_equal(ctx.stage1(tree, p), got)
     np.testing.assert_array_equal(got, oracle.stage1(xyz, oracle.params(bb, xyz.shape[0], W, Ov, 20)))
     ctx.close()
+
+
+@pytest.mark.parametrize("n", [7, 1025, 8192, 8193, 32767, 32768])
+@pytest.mark.parametrize("x0,quantum,W,Ov,B,fits", [(500000.0, 0.01, 10, 0.8, 20, True), (500000.0, 0.5, 10, 0.5, 15, True),
+                                                    (-31.0, 0.01, 9, 0.6, 6, True), (500000.0, 0.0, 8, 0.8, 0, False),
+                                                    (500000.0, 0.01, 6, 0.0, 5, False)])
+def test_one_launch(owm, oracle, x0, quantum, W, Ov, B, fits, n):
+    """Small clouds by one launch (up to 32767 points whose tables fit a block's
+    shared memory, overlap above 0), at the ends of its blocks' shares, and the
+    first that goes by the chain; the same seeds again in the context's used
+    scratch."""
+    ctx = owm.Context(0)
+    side = 60.0
+    xyz = _cloud(np.random.default_rng(n), n, x0, 4700000.0, side, quantum)
+    bb = owm.Bbox(x0, 4700000.0, x0 + side, 4700000.0 + side)
+    want = _check(owm, oracle, ctx, xyz, bb, W, Ov, B)
+    cloud = ctx.cloud(xyz, bb)
+    l0 = ctx.launches
+    np.testing.assert_array_equal(ctx.run(cloud, owm.run_cfg(W, Ov, B, 32)), want)
+    assert (ctx.launches - l0 == 1) == (n < 32768 and fits)
+    xyz[n // 2, 1] = np.nan
+    with pytest.raises(owm.OwmError):
+        ctx.run_host(xyz, bb, owm.run_cfg(W, Ov, B, 32))
+    cloud.close()
+    ctx.close()
