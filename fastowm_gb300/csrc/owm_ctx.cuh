@@ -21,6 +21,7 @@ constexpr int kCheckSlot = 1;
 constexpr int kCountSlot = 2;
 constexpr int kLlpSlot = 3;
 constexpr int kS3Slot = 4;
+constexpr int kTopSlot = 5;
 constexpr int kBboxSlot = 8;  // 4 x int64 (8-byte aligned)
 constexpr int kStampSlot = 128;  // kGridStamps x uint64
 

@@ -341,7 +341,8 @@ __global__ void k_s2_flags(const uint32_t* __restrict__ keys, int64_t n, uint32_
 // first id of every run of length >= 2 gives (owm_optim3.cpp:160-173,
 // stage2 in optim3_func.cpp:609-625).
 __global__ void k_s2_mark(const uint32_t* __restrict__ win, int64_t n, uint32_t max_id,
-                          uint32_t* __restrict__ once, uint32_t* __restrict__ twice) {
+                          uint32_t* __restrict__ once, uint32_t* __restrict__ twice, const uint32_t* __restrict__ top) {
+  if (top && *top > max_id) return;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     s2_mark_id(once, twice, max_id, win[i]);  // kNone (and nothing else: ids are <= max_id) is skipped
   }
@@ -378,7 +379,28 @@ __device__ __forceinline__ uint32_t block_sum_excl_256(uint32_t v, uint32_t* tot
   return before + inc - v;
 }
 
-__global__ void __launch_bounds__(kS2Block) k_s2_count(const uint32_t* __restrict__ bm, uint32_t* __restrict__ part) {
+// Whether a chunk lies beyond the highest id, or that one beyond all chunks
+// (then none is worked on); top null: neither.
+__device__ __forceinline__ bool s2_beyond(const uint32_t* top) {
+  const int64_t ids = kS2Chunk * 32;
+  return top && ((int64_t)blockIdx.x * ids > (int64_t)*top || (int64_t)gridDim.x * ids <= (int64_t)*top);
+}
+
+// The chunks of both bitmaps up to the highest id.
+__global__ void __launch_bounds__(kS2Block) k_s2_clear(uint32_t* __restrict__ once, uint32_t* __restrict__ twice,
+                                                       const uint32_t* __restrict__ top) {
+  if (s2_beyond(top)) return;
+  const int64_t at = (int64_t)blockIdx.x * kS2Block + threadIdx.x;
+  reinterpret_cast<uint4*>(once)[at] = make_uint4(0, 0, 0, 0);
+  reinterpret_cast<uint4*>(twice)[at] = make_uint4(0, 0, 0, 0);
+}
+
+__global__ void __launch_bounds__(kS2Block) k_s2_count(const uint32_t* __restrict__ bm, uint32_t* __restrict__ part,
+                                                       const uint32_t* __restrict__ top) {
+  if (s2_beyond(top)) {
+    if (threadIdx.x == 0) part[blockIdx.x] = 0;
+    return;
+  }
   const uint4 q = __ldg(reinterpret_cast<const uint4*>(bm) + (int64_t)blockIdx.x * kS2Block + threadIdx.x);
   const uint32_t c = (uint32_t)(__popc(q.x) + __popc(q.y) + __popc(q.z) + __popc(q.w));
   uint32_t tot;
@@ -387,8 +409,9 @@ __global__ void __launch_bounds__(kS2Block) k_s2_count(const uint32_t* __restric
 }
 
 __global__ void __launch_bounds__(kS2Block) k_s2_emit_chunk(const uint32_t* __restrict__ bm,
-                                                            const uint32_t* __restrict__ part,
-                                                            uint32_t* __restrict__ out) {
+                                                            const uint32_t* __restrict__ part, uint32_t* __restrict__ out,
+                                                            const uint32_t* __restrict__ top) {
+  if (s2_beyond(top)) return;
   const int64_t w0 = (int64_t)blockIdx.x * kS2Chunk + (int64_t)threadIdx.x * kS2Words;
   const uint4 q = __ldg(reinterpret_cast<const uint4*>(bm + w0));
   const uint32_t word[4] = {q.x, q.y, q.z, q.w};
@@ -499,6 +522,19 @@ __global__ void k_i64_to_u32(const int64_t* __restrict__ in, int64_t n, uint32_t
     int64_t v = in[i];
     out[i] = (v < 0 || v >= (int64_t)kNone) ? kNone : (uint32_t)v;
   }
+}
+
+// The same, and the highest id below kNone, raised in *top (0 at first).
+__global__ void k_i64_to_u32_top(const int64_t* __restrict__ in, int64_t n, uint32_t* __restrict__ out, uint32_t* top) {
+  uint32_t m = 0;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t v = in[i];
+    const bool none = v < 0 || v >= (int64_t)kNone;
+    out[i] = none ? kNone : (uint32_t)v;
+    if (!none) m = max(m, (uint32_t)v);
+  }
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0 && m > 0) atomicMax(top, m);
 }
 
 int grid1d(int64_t n, int block = 256) {
@@ -638,7 +674,8 @@ size_t stage2_bitmap_scratch_bytes(int64_t npoints) {
 }
 
 int run_stage2_bitmap(const uint32_t* d_win, int64_t n, int64_t npoints, double overlap, uint32_t* d_llp,
-                      uint32_t* d_count, void* scratch, size_t scratch_bytes, cudaStream_t s, int64_t* launches) {
+                      uint32_t* d_count, void* scratch, size_t scratch_bytes, cudaStream_t s, int64_t* launches,
+                      const uint32_t* top) {
   if (n <= 0) {
     OWM_CUDA_TRY(cudaMemsetAsync(d_count, 0, 4, s));
     return OWM_OK;
@@ -646,13 +683,18 @@ int run_stage2_bitmap(const uint32_t* d_win, int64_t n, int64_t npoints, double 
   if (npoints < 0 || npoints >= (int64_t)kNone || !(overlap > 0.0)) return OWM_EINVAL;
   if (scratch_bytes < stage2_bitmap_scratch_bytes(npoints)) return OWM_ENOMEM;
   const S2Bitmaps B = stage2_bitmap_layout(scratch, npoints);
-  OWM_CUDA_TRY(cudaMemsetAsync(B.once, 0, 2 * align256((size_t)B.nw * 4), s));  // once, then twice
-  OWM_LAUNCH("k_s2_mark", s, k_s2_mark<<<grid1d(n), 256, 0, s>>>(d_win, n, (uint32_t)npoints, B.once, B.twice));
+  if (top) {
+    OWM_LAUNCH("k_s2_clear", s, k_s2_clear<<<(unsigned)B.nblocks, kS2Block, 0, s>>>(B.once, B.twice, top));
+    count_launch(launches);
+  } else {
+    OWM_CUDA_TRY(cudaMemsetAsync(B.once, 0, 2 * align256((size_t)B.nw * 4), s));  // once, then twice
+  }
+  OWM_LAUNCH("k_s2_mark", s, k_s2_mark<<<grid1d(n), 256, 0, s>>>(d_win, n, (uint32_t)npoints, B.once, B.twice, top));
   count_launch(launches);
-  OWM_LAUNCH("k_s2_count", s, k_s2_count<<<(unsigned)B.nblocks, kS2Block, 0, s>>>(B.twice, B.part));
+  OWM_LAUNCH("k_s2_count", s, k_s2_count<<<(unsigned)B.nblocks, kS2Block, 0, s>>>(B.twice, B.part, top));
   count_launch(launches);
   OWM_CUDA_TRY(exclusive_scan_u32(B.part, B.part, B.nblocks, d_count, B.ct, B.cb, s, launches));
-  OWM_LAUNCH("k_s2_emit", s, k_s2_emit_chunk<<<(unsigned)B.nblocks, kS2Block, 0, s>>>(B.twice, B.part, d_llp));
+  OWM_LAUNCH("k_s2_emit", s, k_s2_emit_chunk<<<(unsigned)B.nblocks, kS2Block, 0, s>>>(B.twice, B.part, d_llp, top));
   count_launch(launches);
   OWM_CUDA_TRY(cudaGetLastError());
   return OWM_OK;
@@ -770,9 +812,13 @@ int u32_to_i64_ids(const uint32_t* in, const uint32_t* d_count, int64_t cap, int
   return OWM_OK;
 }
 
-int i64_to_u32_ids(const int64_t* in, int64_t n, uint32_t* out, cudaStream_t s, int64_t* launches) {
+int i64_to_u32_ids(const int64_t* in, int64_t n, uint32_t* out, cudaStream_t s, int64_t* launches, uint32_t* top) {
+  if (top) OWM_CUDA_TRY(cudaMemsetAsync(top, 0, 4, s));
   if (n <= 0) return OWM_OK;
-  OWM_LAUNCH("k_i64_to_u32", s, k_i64_to_u32<<<grid1d(n), 256, 0, s>>>(in, n, out));
+  if (top)
+    OWM_LAUNCH("k_i64_to_u32", s, k_i64_to_u32_top<<<grid1d(n), 256, 0, s>>>(in, n, out, top));
+  else
+    OWM_LAUNCH("k_i64_to_u32", s, k_i64_to_u32<<<grid1d(n), 256, 0, s>>>(in, n, out));
   count_launch(launches);
   OWM_CUDA_TRY(cudaGetLastError());
   return OWM_OK;

@@ -61,7 +61,8 @@ int run_stage2(const uint32_t* d_win, int64_t n, int64_t npoints, double overlap
 // sort: one marking read of the window list, then work per 32 ids.
 size_t stage2_bitmap_scratch_bytes(int64_t npoints);
 int run_stage2_bitmap(const uint32_t* d_win, int64_t n, int64_t npoints, double overlap, uint32_t* d_llp,
-                      uint32_t* d_count, void* scratch, size_t scratch_bytes, cudaStream_t s, int64_t* launches);
+                      uint32_t* d_count, void* scratch, size_t scratch_bytes, cudaStream_t s, int64_t* launches,
+                      const uint32_t* top = nullptr);
 
 // Stage 2's occupancy marks of one window result v (ids 0..max_id; kNone is
 // skipped): the first occurrence sets `once`, a later one `twice`.
@@ -89,6 +90,7 @@ int run_stage3(const TreeView& t, const double* d_xyz, int stride, const owm_par
 // Device kernels used by the API's conversions.
 int u32_to_i64_ids(const uint32_t* in, const uint32_t* d_count, int64_t cap, int64_t* out, cudaStream_t s,
                    int64_t* launches);
-int i64_to_u32_ids(const int64_t* in, int64_t n, uint32_t* out, cudaStream_t s, int64_t* launches);
+// top (may be null): gets the highest id below kNone, 0 when there is none.
+int i64_to_u32_ids(const int64_t* in, int64_t n, uint32_t* out, cudaStream_t s, int64_t* launches, uint32_t* top = nullptr);
 
 }  // namespace owm
