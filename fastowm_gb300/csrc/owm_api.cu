@@ -709,7 +709,7 @@ int stage1_grid(owm_ctx* c, const TreeStore& t, const owm_params& p, uint32_t** 
   pts.zk = t.zk;
   pts.id = t.pid;
   rc = grid_prepare(g, p, status, c->stream, &c->launches);
-  if (!rc) rc = grid_fold(g, pts, 0, t.n, status, c->stream, &c->launches);
+  if (!rc) rc = grid_fold(g, pts, status, c->stream, &c->launches);
   if (!rc) rc = grid_windows(g, c->stream, &c->launches);
   *win = g.job.win;
   return rc;

@@ -240,19 +240,19 @@ __device__ __forceinline__ void raise_zid(ulonglong2* p, ulonglong2 cur, unsigne
 
 // Point i as raw bits, and its inverted id; every point is read once.
 template <int kStride>
-__device__ __forceinline__ void load_raw(const GridPoints& pts, int64_t i, uint64_t& x, uint64_t& y, uint64_t& z,
+__device__ __forceinline__ void load_raw(const GridPoints& pts, uint32_t i, uint64_t& x, uint64_t& y, uint64_t& z,
                                          uint32_t& nid) {
   if (kStride == 4) {
     asm("ld.global.nc.L1::no_allocate.L2::evict_first.v4.b64 {%0, %1, %2, _}, [%3];"
         : "=l"(x), "=l"(y), "=l"(z)
-        : "l"(pts.rec + 4 * i));
-    nid = ~(uint32_t)(i + 1);
+        : "l"(pts.rec + 4 * (uint64_t)i));
+    nid = ~(i + 1);
   } else if (kStride == 3) {
-    const uint64_t* p = reinterpret_cast<const uint64_t*>(pts.rec) + 3 * i;
+    const uint64_t* p = reinterpret_cast<const uint64_t*>(pts.rec) + 3 * (uint64_t)i;
     x = __ldg(p);
     y = __ldg(p + 1);
     z = __ldg(p + 2);
-    nid = ~(uint32_t)(i + 1);
+    nid = ~(i + 1);
   } else {
     x = (uint64_t)__double_as_longlong(dkey_inv(__ldg(pts.xk + i)));
     y = (uint64_t)__double_as_longlong(dkey_inv(__ldg(pts.yk + i)));
@@ -297,8 +297,8 @@ __device__ __noinline__ void raise_own_cells(const GridJob& J, uint64_t x, uint6
     }
 }
 
-// Points [first + b, first + e) of a cloud into their sub-cells, 32 at a time
-// (e a multiple of 32 above b; count: where the cloud or tile ends).  kFast: both axes have the
+// Points [b, e) of a cloud or tile into their sub-cells, 32 at a time (e a
+// multiple of 32 above b).  kFast: both axes have the
 // fast form; a point near an edge is settled by the edges its places end at,
 // and one outside the box, or with z zero or not finite, takes the full form in
 // a call.
@@ -373,13 +373,13 @@ __device__ __forceinline__ void fast_cell(const GridJob& J, Axes axes, uint64_t 
 }
 
 template <int kStride, int kFast, class Axes>
-__device__ __forceinline__ void fold_stretch(const GridJob& J, Axes axes, const GridPoints& pts, int64_t first,
-                                             int64_t count, int64_t b, int64_t e, uint32_t& flags) {
+__device__ __forceinline__ void fold_stretch(const GridJob& J, Axes axes, const GridPoints& pts, uint32_t b, uint32_t e,
+                                             uint32_t& flags) {
   const int lane = threadIdx.x & 31;
   for (; b < e; b += 32) {
     // lanes past the end take the last point again, and are not counted
-    const int32_t left = (int32_t)min((int64_t)32, count - b);
-    const int64_t i = first + b + min(lane, left - 1);
+    const int32_t left = (int32_t)min(32u, (uint32_t)J.n - b);
+    const uint32_t i = b + (uint32_t)min(lane, left - 1);
     uint64_t x, y, z;
     uint32_t cell, nid;
     load_raw<kStride>(pts, i, x, y, z, nid);
@@ -408,16 +408,34 @@ __device__ __forceinline__ void fold_stretch(const GridJob& J, Axes axes, const 
     const int run = min(end, left) - lane;
     if (head && run > 0) atomicAdd(J.count + grid_count_slot(J, cell), (uint32_t)run);
     if (!__any_sync(0xffffffffu, w >= cur.x)) continue;
+    // the highest top half of w in the run, to its head and from there to all
+    // its lanes; the lane that has it raises the entry
+    uint32_t top = (uint32_t)(w >> 32);
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {  // the run's minimum, to its head
-      const unsigned long long ow = __shfl_down_sync(0xffffffffu, w, o);
-      const uint32_t on = __shfl_down_sync(0xffffffffu, nid, o);
-      if (lane + o < end && (ow > w || (ow == w && on > nid))) {
-        w = ow;
-        nid = on;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t other = __shfl_down_sync(0xffffffffu, top, o);
+      if (lane + o < end) top = max(top, other);
+    }
+    const int start = 31 - __clz(heads & (0xFFFFFFFFu >> (31 - lane)));
+    top = __shfl_sync(0xffffffffu, top, start);
+    bool raise = (uint32_t)(w >> 32) == top && w >= cur.x;
+    const uint32_t several = __ballot_sync(0xffffffffu, raise) & (0xFFFFFFFFu << start) & (0xFFFFFFFFu >> (32 - end));
+    if (__any_sync(0xffffffffu, (several & (several - 1)) != 0)) {
+      raise = raise && zid_above(w, nid, cur);
+      if (__any_sync(0xffffffffu, raise)) {  // none on flat ground: its ids rise
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {  // the run's minimum, to its head
+          const unsigned long long ow = __shfl_down_sync(0xffffffffu, w, o);
+          const uint32_t on = __shfl_down_sync(0xffffffffu, nid, o);
+          if (lane + o < end && (ow > w || (ow == w && on > nid))) {
+            w = ow;
+            nid = on;
+          }
+        }
+        raise = head;
       }
     }
-    if (head) raise_zid(J.zid + cell, cur, w, nid);
+    if (raise) raise_zid(J.zid + cell, cur, w, nid);
   }
 }
 
@@ -434,14 +452,13 @@ __device__ __forceinline__ void fold_flags(const GridJob& J, uint32_t flags, uin
 
 template <int kStride, int kFast>
 __global__ void __launch_bounds__(kFoldBlock, kFoldBlocks)
-    k_grid_fold(const __grid_constant__ GridJob J, const __grid_constant__ GridPoints pts, int64_t first, int64_t count,
-                uint32_t* __restrict__ status) {
+    k_grid_fold(const __grid_constant__ GridJob J, const __grid_constant__ GridPoints pts, uint32_t* __restrict__ status) {
   chain_start();
   const int64_t nwarps = ((int64_t)gridDim.x * kFoldBlock) >> 5;
   uint32_t flags = 0;
   int64_t t0, t1;
-  chunk_tiles((count + 31) / 32, nwarps, ((int64_t)blockIdx.x * kFoldBlock + threadIdx.x) >> 5, &t0, &t1);
-  fold_stretch<kStride, kFast>(J, ParamAxes{&J}, pts, first, count, t0 * 32, t1 * 32, flags);
+  chunk_tiles(((int64_t)J.n + 31) / 32, nwarps, ((int64_t)blockIdx.x * kFoldBlock + threadIdx.x) >> 5, &t0, &t1);
+  fold_stretch<kStride, kFast>(J, ParamAxes{&J}, pts, (uint32_t)(t0 * 32), (uint32_t)(t1 * 32), flags);
   fold_flags(J, flags, status);
 }
 
@@ -462,11 +479,11 @@ __global__ void __launch_bounds__(kFoldBlock, kFoldBlocks)
   int64_t t0, t1;
   chunk_tiles((n + 31) / 32, kFoldBlock / 32, threadIdx.x >> 5, &t0, &t1);
   if (J.fast == 2)
-    fold_stretch<3, 2>(J, SharedAxes{&J}, pts, 0, J.n, c0 + t0 * 32, c0 + t1 * 32, flags);
+    fold_stretch<3, 2>(J, SharedAxes{&J}, pts, (uint32_t)(c0 + t0 * 32), (uint32_t)(c0 + t1 * 32), flags);
   else if (J.fast)
-    fold_stretch<3, 1>(J, SharedAxes{&J}, pts, 0, J.n, c0 + t0 * 32, c0 + t1 * 32, flags);
+    fold_stretch<3, 1>(J, SharedAxes{&J}, pts, (uint32_t)(c0 + t0 * 32), (uint32_t)(c0 + t1 * 32), flags);
   else
-    fold_stretch<3, 0>(J, SharedAxes{&J}, pts, 0, J.n, c0 + t0 * 32, c0 + t1 * 32, flags);
+    fold_stretch<3, 0>(J, SharedAxes{&J}, pts, (uint32_t)(c0 + t0 * 32), (uint32_t)(c0 + t1 * 32), flags);
   fold_flags(J, flags, status);
 }
 
@@ -1513,17 +1530,15 @@ int grid_prepare(const GridPlan& g, const owm_params& p, uint32_t* status, cudaS
   return OWM_OK;
 }
 
-int grid_fold(const GridPlan& g, const GridPoints& pts, int64_t first, int64_t count, uint32_t* status, cudaStream_t s,
-              int64_t* launches) {
-  if (count <= 0) return OWM_OK;
+int grid_fold(const GridPlan& g, const GridPoints& pts, uint32_t* status, cudaStream_t s, int64_t* launches) {
   const GridJob& J = g.job;
-  const unsigned nb = blocks_for(count, 152 * kFoldBlocks, kFoldBlock);
-  using Kernel = void (*)(GridJob, GridPoints, int64_t, int64_t, uint32_t*);
+  const unsigned nb = blocks_for(J.n, 152 * kFoldBlocks, kFoldBlock);
+  using Kernel = void (*)(GridJob, GridPoints, uint32_t*);
   static const Kernel kernels[3][3] = {{k_grid_fold<0, 0>, k_grid_fold<0, 1>, k_grid_fold<0, 2>},
                                        {k_grid_fold<3, 0>, k_grid_fold<3, 1>, k_grid_fold<3, 2>},
                                        {k_grid_fold<4, 0>, k_grid_fold<4, 1>, k_grid_fold<4, 2>}};
   const Kernel kernel = kernels[pts.stride == 4 ? 2 : pts.stride == 3 ? 1 : 0][J.fast];
-  OWM_LAUNCH("k_grid_fold", s, OWM_CUDA_TRY(chain(kernel, nb, kFoldBlock, s, J, pts, first, count, status)));
+  OWM_LAUNCH("k_grid_fold", s, OWM_CUDA_TRY(chain(kernel, nb, kFoldBlock, s, J, pts, status)));
   count_launch(launches);
   OWM_CUDA_TRY(cudaGetLastError());
   return OWM_OK;

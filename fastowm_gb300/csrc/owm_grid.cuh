@@ -402,9 +402,8 @@ struct GridPlan {
 int grid_plan(const owm_params& p, int64_t n, void* scratch, GridPlan* g, bool stage1_only = false);
 // Clears the tables and computes edges and ranges.
 int grid_prepare(const GridPlan& g, const owm_params& p, uint32_t* status, cudaStream_t s, int64_t* launches);
-// Folds points [first, first + count) of the cloud.
-int grid_fold(const GridPlan& g, const GridPoints& pts, int64_t first, int64_t count, uint32_t* status, cudaStream_t s,
-              int64_t* launches);
+// Folds the cloud's points.
+int grid_fold(const GridPlan& g, const GridPoints& pts, uint32_t* status, cudaStream_t s, int64_t* launches);
 // Stage 1 (rows, windows), stage 2 with stage 3's marks, stage 3 and the seeds.
 int grid_windows(const GridPlan& g, cudaStream_t s, int64_t* launches);
 int grid_stage2(const GridPlan& g, const owm_params& p, const double* xy, int xy_stride, uint32_t* d_nllp,

@@ -201,7 +201,7 @@ int run_grid(owm_ctx* c, const PointsView& pts, int64_t n, const owm_params& p, 
   OWM_CUDA_TRY(cudaEventRecord(c->ev[0], s));
   if (grid_is_small(g)) return grid_small(g, p, gp, pts.xy, pts.xy_stride, out, s, &c->launches);
   rc = grid_prepare(g, p, out.status, s, &c->launches);
-  if (!rc) rc = grid_fold(g, gp, 0, n, out.status, s, &c->launches);
+  if (!rc) rc = grid_fold(g, gp, out.status, s, &c->launches);
   if (!rc) rc = grid_windows(g, s, &c->launches);
   if (!rc) rc = grid_stage2(g, p, pts.xy, pts.xy_stride, out.nllp, s, &c->launches);
   if (!rc) rc = grid_stage3(g, out, s, &c->launches);
