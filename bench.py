@@ -452,7 +452,7 @@ def main():
                          "-1 = the workload's configured value")
     ap.add_argument("--no-ingest", action="store_true")
     ap.add_argument("--stage1-walk", action="store_true",
-                    help="stage 1 by the per-window tree walk instead of window classes (profiling runs)")
+                    help="stage 1 by the per-window tree walk instead of the window grid (profiling runs)")
     ap.add_argument("--ingest-n", type=int, default=20_000_000, help="points of the ingest leg's text")
     ap.add_argument("--only", choices=["batched", "served", "ingest"], default=None,
                     help="run that leg alone and print its JSON (profiling and tuning runs)")

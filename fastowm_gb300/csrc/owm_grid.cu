@@ -304,12 +304,15 @@ __device__ __noinline__ void raise_own_cells(const GridJob& J, uint64_t x, uint6
 // a call.
 //
 // Bound by the L2 requests of points in no order (a read and an add each): 100 M
-// points into 0.9 M sub-cells take 1.04 ms (32 bytes a point: 3.1 TB/s), a bare
-// kernel that does just those two requests 0.87.  What cost more before:
+// points into 0.9 M sub-cells take 0.97 ms (32 bytes a point: 3.3 TB/s), a bare
+// kernel that does just those two requests 0.87.  In scan order it is bound by
+// latency and instructions (issue 51 %).  What cost more before:
 // - the order of the work: a warp takes a stretch of neighbouring points, so
 //   that scan lines side by side are not folded at the same time (40 M points in
 //   scan order at 3 a square metre: 1.28 -> 0.53 ms);
 // - instructions: 144 per 32 points instead of 284 (0.53 -> 0.40 ms there);
+// - runs of points reduced on 96 bits where the top half of their heights tells
+//   them apart (0.45 -> 0.41 ms there, in whole centimetres);
 // - points on edges (whole centimetres: 1 in 100): two loads side by side in
 //   place of a call (20 M in no order 0.37 -> 0.24 ms, in scan order 0.28 -> 0.23).
 // One point a thread at 48 warps an SM: two at 40 took 1.05 ms for the 100 M,
