@@ -120,3 +120,27 @@ def test_one_launch(owm, oracle, x0, quantum, W, Ov, B, fits, n):
         ctx.run_host(xyz, bb, owm.run_cfg(W, Ov, B, 32))
     cloud.close()
     ctx.close()
+
+
+@pytest.mark.parametrize("n", [40_960, 40_961, 622_593])
+@pytest.mark.parametrize("heights", ["tied", "falling"])
+@pytest.mark.parametrize("x0,side,W,Ov,B,quantum", [(500000.0, 90.0, 16, 0.5, 20, 0.5), (500000.0, 90.0, 16, 0.5, 25, 0.01),
+                                                    (-31.0, 60.0, 15, 0.6, 0, 0.01), (500000.0, 1200.0, 200, 0.5, 2, 0.25)])
+def test_few_sub_cells(owm, oracle, ctx, x0, side, W, Ov, B, quantum, heights, n):
+    """Many points on few sub-cells: blocks fold into tables in shared memory,
+    some in more than one group of points; equal heights keep the lowest id,
+    and heights that fall with the id replace the entry in every group."""
+    rng = np.random.default_rng(n)
+    xyz = _cloud(rng, n, x0, 4700000.0, side, quantum)
+    xyz[:, 2] = np.round(xyz[:, 2]) if heights == "tied" else 500.0 - np.arange(n) * 1e-4
+    bb = owm.Bbox(x0, 4700000.0, x0 + side, 4700000.0 + side)
+    _check(owm, oracle, ctx, xyz, bb, W, Ov, B)
+    cloud = ctx.cloud(xyz, bb)
+    tree = ctx.tree(cloud, 1, 32)
+    p = owm.params(bb, n, W, Ov, B)
+    np.testing.assert_array_equal(ctx.stage1(tree, p), oracle.stage1(xyz, oracle.params(bb, n, W, Ov, B)))
+    tree.close()
+    cloud.close()
+    xyz[n - 1, 2] = np.inf
+    with pytest.raises(owm.OwmError):
+        ctx.run_host(xyz, bb, owm.run_cfg(W, Ov, B, 32))
