@@ -1058,6 +1058,11 @@ __global__ void __cluster_dims__(kSmallCluster) __launch_bounds__(kSmallBlock)
   for (int32_t c = t >> 5; c < ncell; c += kSmallBlock / 32) cell_of(J, c);
   __syncthreads();
   write_output<kSmallBlock>(J, ncell, llp, out, 0, 1);
+  if (t == 0) {  // the context's words, as the chain leaves them
+    *R.status = words[0];
+    *R.nllp = words[1];
+    *R.ns3 = words[2];
+  }
 }
 
 __global__ void k_grid_flags(const uint32_t* __restrict__ v, int64_t n, uint32_t* __restrict__ flags) {
