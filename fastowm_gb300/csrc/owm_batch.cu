@@ -818,20 +818,24 @@ size_t BatchRun::estimate_bytes(const owm_tile_desc* t, int32_t ntiles) {
   return P.total;
 }
 
-// Room for a batch: device memory (a captured graph is stale once it moves),
-// the pinned offsets and pinned staging for the per-batch tables (a copy from
-// pageable memory would first wait for this stream's queued point copies,
-// holding the caller, the server's worker, for the whole transfer).
+void BatchRun::drop_graph() {
+  if (graph) cudaGraphExecDestroy(graph);
+  graph = nullptr;
+  graph_sig.clear();
+}
+
+// Room for a batch: device memory, the pinned offsets (a captured graph holds
+// the addresses of both and goes when either moves) and pinned staging for the
+// per-batch tables (a copy from pageable memory would first wait for this
+// stream's queued point copies, holding the caller, the server's worker, for the
+// whole transfer).
 int BatchRun::room(size_t device_bytes, size_t stage_bytes, int32_t ntiles_) {
   bytes_needed = device_bytes;
-  if (device_bytes > mem.cap && graph) {
-    cudaGraphExecDestroy(graph);
-    graph = nullptr;
-    graph_sig.clear();
-  }
+  if (device_bytes > mem.cap) drop_graph();
   const int rc = mem.reserve(device_bytes, stream);
   if (rc) return rc;
   if (cap_tiles < ntiles_ + 1) {
+    drop_graph();
     if (h_off) cudaFreeHost(h_off);
     h_off = nullptr;
     cap_tiles = 0;
@@ -865,9 +869,7 @@ int BatchRun::run_or_replay(const std::string& sig, Enqueue enqueue) {
   cudaGraph_t g = nullptr;
   cudaError_t e = cudaStreamEndCapture(stream, &g);
   if (rc == OWM_OK && e == cudaSuccess) {
-    if (graph) cudaGraphExecDestroy(graph);
-    graph = nullptr;
-    graph_sig.clear();
+    drop_graph();
     e = cudaGraphInstantiate(&graph, g, 0);
     if (e == cudaSuccess) {
       graph_sig = sig;

@@ -68,6 +68,7 @@ struct BatchRun {
   int launch(const owm_tile_desc* t, int32_t ntiles);
   int launch_grid(const owm_tile_desc* t, int32_t ntiles);  // window grid
   int launch_walk(const owm_tile_desc* t, int32_t ntiles);  // trees, persistent stage-1 walk
+  void drop_graph();
   int room(size_t device_bytes, size_t stage_bytes, int32_t ntiles);
   template <class Enqueue>
   int run_or_replay(const std::string& sig, Enqueue enqueue);
