@@ -112,6 +112,7 @@ int DeviceBuffer::reserve(size_t bytes, cudaStream_t s) {
     ptr = nullptr;
     cap = 0;
   }
+  if (bytes > most) return OWM_ENOMEM;
   size_t want = bytes + bytes / 8 + 4096;
   cudaError_t e = cudaMallocAsync(&ptr, want, s);
   if (e != cudaSuccess) {
@@ -685,33 +686,37 @@ namespace {
 // (73 K windows) 90 / 376 us, leaf 256 82 / 670; W 16, overlap 0.5 70 / 175;
 // 100 M points, W 10, overlap 0.8 1.42 / 6.80 ms; but W 16, overlap 0.5 1.00 /
 // 0.54 ms, at 20 M 0.25 / 0.21.  A handful of windows: 57 / 41 us (one).
-bool stage1_on_grid(const TreeStore& t, const owm_params& p) {
+// The grid counts windows whose edges rise with their index.
+bool stage1_on_grid(int64_t points, int32_t nleaves, const owm_params& p) {
   if (p.ncells <= 16 || p.ncells != (int64_t)p.ncols * p.nrows) return false;
-  const double n = (double)t.n, leaf = n / t.nleaves;
+  const double n = (double)points, leaf = n / nleaves;
   const double area = (p.bbox.max_x - p.bbox.min_x) * (p.bbox.max_y - p.bbox.min_y);
+  if (!(area > 0.0) || !std::isfinite(area) || !(p.displace > 0.0)) return false;
   const double sides = 4.0 * p.wsize / std::sqrt(leaf * area / n);  // leaves along a window's sides
   const double walk_us = 1e-4 * (double)p.ncells * sides * std::max(1.0, leaf / 32.0);
   const double grid_us = 50.0 + 9.5e-6 * n + 1.2e-4 * (double)p.ncells;
-  return grid_us < std::max(150.0, walk_us);  // false for a box without an area
+  return grid_us < std::max(150.0, walk_us);
 }
 
-// Stage 1 over a tree's sorted points on the window grid; *win: the results.
-int stage1_grid(owm_ctx* c, const TreeStore& t, const owm_params& p, uint32_t** win) {
-  GridPlan g;
-  int rc = grid_plan(p, t.n, nullptr, &g, true);
-  if (!rc) rc = c->scratch.reserve(g.bytes, c->stream);
-  if (!rc) rc = grid_plan(p, t.n, c->scratch.ptr, &g, true);
-  if (rc) return rc;
+// Plans stage 1 on the window grid in the context's scratch; false where the
+// walk answers sooner, or where the tables (about 100 bytes a window, 12 for the
+// walk) cannot be numbered or do not fit.
+bool stage1_plan(owm_ctx* c, const TreeStore& t, const owm_params& p, GridPlan* g) {
+  return c->walk_limit == 0 && stage1_on_grid(t.n, t.nleaves, p) && grid_plan(p, t.n, nullptr, g, true) == OWM_OK &&
+         c->scratch.reserve(g->bytes, c->stream) == OWM_OK && grid_plan(p, t.n, c->scratch.ptr, g, true) == OWM_OK;
+}
+
+// Stage 1 over a tree's sorted points; the results are in g.job.win.
+int stage1_grid(owm_ctx* c, const TreeStore& t, const owm_params& p, const GridPlan& g) {
   uint32_t* status = c->d_small + kStatusSlot;
   GridPoints pts;
   pts.xk = t.xk;
   pts.yk = t.yk;
   pts.zk = t.zk;
   pts.id = t.pid;
-  rc = grid_prepare(g, p, status, c->stream, &c->launches);
+  int rc = grid_prepare(g, p, status, c->stream, &c->launches);
   if (!rc) rc = grid_fold(g, pts, status, c->stream, &c->launches);
   if (!rc) rc = grid_windows(g, c->stream, &c->launches);
-  *win = g.job.win;
   return rc;
 }
 }  // namespace
@@ -740,8 +745,10 @@ int owm_stage1(owm_ctx* c, const owm_tree* tr, const owm_params* p, int64_t* win
   Edge* ey = ex + 65536;
   uint32_t* win = (uint32_t*)(ey + 65536);
   int64_t* w64 = (int64_t*)(((uintptr_t)(win + nc) + 255) & ~(uintptr_t)255);
-  if (c->walk_limit == 0 && stage1_on_grid(tr->t, *p)) {
-    rc = stage1_grid(c, tr->t, *p, &win);
+  GridPlan g;
+  if (stage1_plan(c, tr->t, *p, &g)) {
+    win = g.job.win;
+    rc = stage1_grid(c, tr->t, *p, g);
   } else {
     rc = clear_status(c);
     if (!rc) rc = run_stage1(c, tr->t, *p, ex, ey, win);
@@ -1035,5 +1042,14 @@ int owm_run_host_wait(owm_ctx* c, int64_t ticket, int64_t* n_seeds, owm_run_info
 int owm_run_wait(owm_ctx* c, int64_t ticket, int64_t* n_seeds, owm_run_info* info) {
   return owm_run_host_wait(c, ticket, n_seeds, info);
 }
+
+// For tests: whether owm_stage1 would plan the window grid for these parameters
+// and a tree of n points in nleaves leaves; a context whose scratch cannot grow
+// past that many bytes (0: no limit).
+int owm_stage1_route_host(const owm_params* p, int64_t n, int32_t nleaves) {
+  GridPlan g;
+  return stage1_on_grid(n, nleaves, *p) && grid_plan(*p, n, nullptr, &g, true) == OWM_OK;
+}
+void owm_ctx_limit_scratch(owm_ctx* c, int64_t bytes) { c->scratch.most = bytes > 0 ? (size_t)bytes : SIZE_MAX; }
 
 }  // extern "C"

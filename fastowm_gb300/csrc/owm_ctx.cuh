@@ -1,6 +1,7 @@
 // Context object and the whole-path pipeline shared by API, batch and server.
 #pragma once
 
+#include <cstdint>
 #include <vector>
 
 #include "owm_query.cuh"
@@ -11,6 +12,7 @@ namespace owm {
 struct DeviceBuffer {
   void* ptr = nullptr;
   size_t cap = 0;
+  size_t most = SIZE_MAX;  // a larger reservation fails (tests)
   int reserve(size_t bytes, cudaStream_t s);
   void release(cudaStream_t s);
 };
