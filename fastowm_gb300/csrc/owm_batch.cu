@@ -804,18 +804,23 @@ int BatchRun::leaf_for(int64_t n, int32_t requested) const {
   return requested;
 }
 
-size_t BatchRun::estimate_bytes(const owm_tile_desc* t, int32_t ntiles) {
-  if (on_grid(t, ntiles)) {
+int BatchRun::route(const owm_tile_desc* td, int32_t nt, size_t most, bool* grid, size_t* bytes) const {
+  int grc = OWM_ERANGE;
+  if (on_grid(td, nt)) {
     GridLayout L;
     GridBatch g;
-    const int rc = grid_layout(t, ntiles, &L, &g);
-    // too many sub-cells to number: more than any budget, not a bad request
-    return rc == OWM_OK ? L.point_bytes + g.bytes : rc == OWM_ERANGE ? (size_t)-2 : (size_t)-1;
+    grc = grid_layout(td, nt, &L, &g);
+    *grid = true;
+    if (!grc) *bytes = L.point_bytes + g.bytes;
+    if (grc ? grc != OWM_ERANGE : *bytes <= most) return grc;
   }
-  BatchRun tmp;
   Plan P;
-  if (make_plan(t, ntiles, tmp, &P) != OWM_OK) return (size_t)-1;
-  return P.total;
+  const int rc = make_plan(td, nt, *this, &P);
+  if (!grc && (rc || P.total > most)) return OWM_OK;  // over `most` either way
+  if (rc) return rc;
+  *grid = false;
+  *bytes = P.total;
+  return OWM_OK;
 }
 
 void BatchRun::drop_graph() {
@@ -885,10 +890,12 @@ int BatchRun::run_or_replay(const std::string& sig, Enqueue enqueue) {
   return rc;
 }
 
-int BatchRun::launch(const owm_tile_desc* td, int32_t n) {
+int BatchRun::launch(const owm_tile_desc* td, int32_t n, size_t most) {
   if (!td || n <= 0) return OWM_EINVAL;
   OWM_CUDA_TRY(cudaSetDevice(device));
-  const int rc = on_grid(td, n) ? launch_grid(td, n) : launch_walk(td, n);
+  int rc = on_grid(td, n) ? launch_grid(td, n, most) : OWM_ERANGE;
+  // tables that cannot be numbered or held: nothing is queued yet
+  if (rc == OWM_ERANGE || rc == OWM_ENOMEM) rc = launch_walk(td, n);
   if (rc) return rc;
   OWM_CUDA_TRY(cudaEventRecord(done, stream));
   return OWM_OK;
@@ -904,10 +911,11 @@ bool back_to_back(const owm_tile_desc* td, int32_t ntiles, int device) {
 }
 }  // namespace
 
-int BatchRun::launch_grid(const owm_tile_desc* td, int32_t nt) {
+int BatchRun::launch_grid(const owm_tile_desc* td, int32_t nt, size_t most) {
   GridLayout L;
   GridBatch g;
   int rc = grid_layout(td, nt, &L, &g);
+  if (!rc && L.point_bytes + g.bytes > most) rc = OWM_ENOMEM;
   if (!rc) rc = room(L.point_bytes + g.bytes, g.table_bytes, nt);
   if (!rc) rc = grid_batch_plan(L.p.data(), L.n.data(), nt, L.z.data(), static_cast<char*>(mem.ptr) + L.point_bytes, &g);
   if (rc) return rc;
@@ -1300,6 +1308,19 @@ int owm_batch_set_leaf_classes(owm_batch* b, int32_t nclass, const int64_t* boun
   }
   return OWM_OK;
 }
+
+// For tests: device bytes that a batch of these tiles takes (0 on_grid: by its
+// trees) where it should take at most `most`; a batch whose buffer cannot grow
+// past that many bytes (0: no limit).
+int owm_batch_route_host(const owm_tile_desc* tiles, int32_t ntiles, int64_t most, int32_t* on_grid, int64_t* bytes) {
+  bool grid = false;
+  size_t n = 0;
+  const int rc = BatchRun().route(tiles, ntiles, (size_t)most, &grid, &n);
+  *on_grid = grid;
+  *bytes = (int64_t)n;
+  return rc;
+}
+void owm_batch_limit_memory(owm_batch* b, int64_t bytes) { b->run.mem.most = bytes > 0 ? (size_t)bytes : SIZE_MAX; }
 
 int owm_batch_run(owm_batch* b, const owm_tile_desc* tiles, int32_t ntiles, int64_t* seeds, int64_t cap,
                   int64_t* offsets, owm_run_info* info) {

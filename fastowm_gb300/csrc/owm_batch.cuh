@@ -62,11 +62,13 @@ struct BatchRun {
   int init(int device, cudaStream_t s);
   void destroy();
   int leaf_for(int64_t n, int32_t requested) const;
-  // Estimated device bytes for these tiles (admission control).
-  static size_t estimate_bytes(const owm_tile_desc* t, int32_t ntiles);
+  // Whether these tiles run on the window grid, and the device bytes they take:
+  // the grid unless a tile asks for the tree walk, or the grid's tables cannot be
+  // numbered or take more than `most` bytes where the trees take less.
+  int route(const owm_tile_desc* t, int32_t ntiles, size_t most, bool* grid, size_t* bytes) const;
   // Enqueue everything (copies in, build, stages, offsets out) on `stream`.
-  int launch(const owm_tile_desc* t, int32_t ntiles);
-  int launch_grid(const owm_tile_desc* t, int32_t ntiles);  // window grid
+  int launch(const owm_tile_desc* t, int32_t ntiles, size_t most = SIZE_MAX);
+  int launch_grid(const owm_tile_desc* t, int32_t ntiles, size_t most);  // window grid
   int launch_walk(const owm_tile_desc* t, int32_t ntiles);  // trees, persistent stage-1 walk
   void drop_graph();
   int room(size_t device_bytes, size_t stage_bytes, int32_t ntiles);

@@ -177,8 +177,10 @@ struct owm_server {
     }
     scratch_descs.clear();
     for (Request* r : take) scratch_descs.push_back(r->desc);
-    size_t need = BatchRun::estimate_bytes(scratch_descs.data(), (int32_t)scratch_descs.size());
-    if (need == (size_t)-1) {  // malformed request: fail it alone
+    size_t need = 0;
+    bool grid = false;
+    const int bad = free_slot->run.route(scratch_descs.data(), (int32_t)scratch_descs.size(), (size_t)cfg.hbm_budget_bytes, &grid, &need);
+    if (bad) {  // malformed request: fail it alone
       Request* r = take.front();
       pending.erase(std::find(pending.begin(), pending.end(), r));
       r->status = OWM_EINVAL;
@@ -212,7 +214,7 @@ struct owm_server {
     free_slot->reqs = take;
     free_slot->busy = true;
     free_slot->t_launch = now_ms();
-    int rc = free_slot->run.launch(scratch_descs.data(), (int32_t)scratch_descs.size());
+    int rc = free_slot->run.launch(scratch_descs.data(), (int32_t)scratch_descs.size(), (size_t)cfg.hbm_budget_bytes);
     st.batches++;
     st.bytes_in_use = (int64_t)slot_bytes();
     st.peak_bytes = std::max(st.peak_bytes, st.bytes_in_use);
@@ -314,8 +316,8 @@ int owm_server_submit(owm_server* s, const owm_tile_desc* tile, int64_t* ticket)
     delete r;
     return OWM_EINVAL;
   }
-  r->est_bytes = BatchRun::estimate_bytes(&r->desc, 1);
-  if (r->est_bytes == (size_t)-1) {
+  bool grid = false;
+  if (BatchRun().route(&r->desc, 1, (size_t)s->cfg.hbm_budget_bytes, &grid, &r->est_bytes) != OWM_OK) {
     delete r;
     return OWM_EINVAL;
   }
