@@ -81,6 +81,29 @@ struct Request {
   size_t est_bytes = 0;
 };
 
+// How many of the first tiles go into one batch within the budget, and the bytes
+// they take: halved until their batch can be laid out and fits.  rc: what a tile
+// that is refused alone is refused with.
+struct Admission {
+  int rc = OWM_OK;
+  int32_t tiles = 0;
+  size_t bytes = 0;
+};
+Admission admissible(const owm_tile_desc* td, int32_t n, size_t budget) {
+  Admission a;
+  const BatchRun run;
+  for (a.tiles = n;; a.tiles = (a.tiles + 1) / 2) {
+    bool grid = false;
+    a.rc = run.route(td, a.tiles, budget, &grid, &a.bytes);
+    if (!a.rc && a.bytes > budget) a.rc = OWM_ENOMEM;
+    if (!a.rc || a.tiles <= 1) return a;
+  }
+}
+
+// Whether a slot may hold `mine` bytes beside the others' (the sum may not be
+// representable).
+bool within(size_t others, size_t mine, size_t budget) { return others <= budget && mine <= budget - others; }
+
 struct Slot {
   BatchRun run;
   std::vector<Request*> reqs;
@@ -177,23 +200,25 @@ struct owm_server {
     }
     scratch_descs.clear();
     for (Request* r : take) scratch_descs.push_back(r->desc);
-    size_t need = 0;
-    bool grid = false;
-    const int bad = free_slot->run.route(scratch_descs.data(), (int32_t)scratch_descs.size(), (size_t)cfg.hbm_budget_bytes, &grid, &need);
-    if (bad) {  // malformed request: fail it alone
+    const size_t budget = (size_t)cfg.hbm_budget_bytes;
+    const Admission adm = admissible(scratch_descs.data(), (int32_t)scratch_descs.size(), budget);
+    if (adm.rc) {  // a request that no batch can take: fail it alone
       Request* r = take.front();
       pending.erase(std::find(pending.begin(), pending.end(), r));
-      r->status = OWM_EINVAL;
+      r->status = adm.rc;
       r->t_done = now_ms();
       pinned.put(r->pts, r->pts_cls);
       r->pts = nullptr;
       cv_done.notify_all();
       return true;
     }
+    take.resize((size_t)adm.tiles);
+    scratch_descs.resize((size_t)adm.tiles);
+    const size_t need = adm.bytes;
     // budget: other slots' resident buffers + this slot's (grown) buffer
     size_t others = slot_bytes() - free_slot->run.mem.cap;
     size_t mine = std::max(need, free_slot->run.mem.cap);
-    if (others + mine > (size_t)cfg.hbm_budget_bytes) {
+    if (!within(others, mine, budget)) {
       // evict idle slots' resident trees
       for (auto& sp : slots)
         if (!sp->busy && sp.get() != free_slot && sp->run.mem.ptr) {
@@ -201,20 +226,20 @@ struct owm_server {
           sp->run.mem.release(sp->run.stream);
         }
       others = slot_bytes() - free_slot->run.mem.cap;
-      if (others + mine > (size_t)cfg.hbm_budget_bytes) {
+      if (!within(others, mine, budget)) {
         if (free_slot->run.mem.cap > need) {
           // shrink this slot to what the batch needs
           free_slot->run.mem.release(free_slot->run.stream);
           mine = need;
         }
-        if (others + mine > (size_t)cfg.hbm_budget_bytes) return false;  // wait for a slot to finish
+        if (!within(others, mine, budget)) return false;  // wait for a slot to finish
       }
     }
     for (Request* r : take) pending.erase(std::find(pending.begin(), pending.end(), r));
     free_slot->reqs = take;
     free_slot->busy = true;
     free_slot->t_launch = now_ms();
-    int rc = free_slot->run.launch(scratch_descs.data(), (int32_t)scratch_descs.size(), (size_t)cfg.hbm_budget_bytes);
+    int rc = free_slot->run.launch(scratch_descs.data(), (int32_t)scratch_descs.size(), budget);
     st.batches++;
     st.bytes_in_use = (int64_t)slot_bytes();
     st.peak_bytes = std::max(st.peak_bytes, st.bytes_in_use);
@@ -401,5 +426,16 @@ int owm_server_get_stats(owm_server* s, owm_server_stats* out) {
   *out = s->st;
   return OWM_OK;
 }
+
+// For tests: how many of these tiles a server admits as one batch within the
+// budget (0: none, *rc says why) and the bytes it counts for them; whether a slot
+// may hold `mine` bytes beside the others'.
+int owm_server_admissible_host(const owm_tile_desc* tiles, int32_t ntiles, int64_t budget, int64_t* bytes, int32_t* rc) {
+  const Admission a = admissible(tiles, ntiles, (size_t)budget);
+  *bytes = (int64_t)a.bytes;
+  *rc = a.rc;
+  return a.rc ? 0 : a.tiles;
+}
+int owm_server_within_host(uint64_t others, uint64_t mine, uint64_t budget) { return within(others, mine, budget); }
 
 }  // extern "C"
