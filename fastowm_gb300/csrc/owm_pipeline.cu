@@ -2,7 +2,7 @@
 // runs it per loop iteration (CPP-TBB-CPU/application/owm_optim3.cpp:77-230):
 // index, stage 1, sort + stage 2, LLP grid + stage 3, and the result (stage-3
 // ids followed by the LLPs).  The index is the window grid (owm_grid.cuh), or
-// the tree when stage 1 walks it (stage1_walk, or a walk limit is set).
+// the tree: with stage1_walk, and for stage 3 while a walk limit is set.
 // Intermediates never leave the device; the host sees two small count words
 // and the final seed list.
 #include <cuda_runtime.h>
@@ -224,8 +224,14 @@ int run_pipeline_enqueue(owm_ctx* c, const PointsView& pts, int64_t n, const owm
   const int64_t nc = p.ncells, ng = std::max<int64_t>(p.ngrid, 0);
   rc = tree_alloc(&c->tree, &c->tree_mem, n, cfg.tree, c->stream);
   if (rc) return rc;
-  // scratch = [tree build | stage 2 | stage 3]
-  const size_t tbytes = (tree_scratch_bytes(n) + 255) & ~(size_t)255;
+  // With a walk limit alone, stage 1 counts on the window grid, which needs no
+  // walk: the limit acts on the cells.
+  GridPlan g1;
+  if (!cfg.stage1_walk) rc = grid_plan(p, n, nullptr, &g1, true);
+  if (rc) return rc;
+  // scratch = [tree build | stage 1's grid | stage 2 | stage 3]
+  const size_t bbytes = (tree_scratch_bytes(n) + 255) & ~(size_t)255;
+  const size_t tbytes = bbytes + ((g1.bytes + 255) & ~(size_t)255);
   const bool bitmap2 = p.overlap > 0.0;
   const size_t s2bytes = bitmap2 ? stage2_bitmap_scratch_bytes(n) : stage2_scratch_bytes(nc);
   const size_t s2al = (s2bytes + 255) & ~(size_t)255;
@@ -256,13 +262,24 @@ int run_pipeline_enqueue(owm_ctx* c, const PointsView& pts, int64_t n, const owm
   rc = clear_status(c);
   c->tree.gather_block = c->tuning.gather_block;
   if (!rc)
-    rc = build_tree(pts, n, bb, cfg.tree, &c->tree, c->scratch.ptr, tbytes, c->d_small + kStatusSlot, s, &c->launches);
+    rc = build_tree(pts, n, bb, cfg.tree, &c->tree, c->scratch.ptr, bbytes, c->d_small + kStatusSlot, s, &c->launches);
   if (rc) return rc;
   void* s2scratch = static_cast<char*>(c->scratch.ptr) + tbytes;
   void* s3scratch = static_cast<char*>(c->scratch.ptr) + tbytes + s2al;
   const size_t s3cap = c->scratch.cap - tbytes - s2al;
   OWM_CUDA_TRY(cudaEventRecord(c->ev[1], s));
-  rc = run_stage1(c, c->tree, p, ex, ey, win);
+  if (cfg.stage1_walk) {
+    rc = run_stage1(c, c->tree, p, ex, ey, win);
+  } else {
+    GridPoints gp;
+    gp.rec = pts.rec;
+    gp.stride = pts.rec_stride;
+    rc = grid_plan(p, n, static_cast<char*>(c->scratch.ptr) + bbytes, &g1, true);
+    if (!rc) rc = grid_prepare(g1, p, c->d_small + kStatusSlot, s, &c->launches);
+    if (!rc) rc = grid_fold(g1, gp, c->d_small + kStatusSlot, s, &c->launches);
+    if (!rc) rc = grid_windows(g1, s, &c->launches);
+    win = g1.job.win;
+  }
   if (rc) return rc;
   OWM_CUDA_TRY(cudaEventRecord(c->ev[2], s));
   rc = bitmap2 ? run_stage2_bitmap(win, nc, n, p.overlap, llp, d_nllp, s2scratch, s2al, s, &c->launches)

@@ -134,9 +134,10 @@ int64_t owm_ctx_launches(const owm_ctx* ctx);
 /* Device status word: bit 0 non-finite input, bit 1 a bounded tree walk or
  * bounded device wait ran out (the call returned OWM_ETIMEOUT). */
 int owm_ctx_device_status(owm_ctx* ctx, int32_t* status);
-/* Step limit of this context's bounded tree walks (owm_run walks the tree
- * while one is set): the stage-1 walk (owm_stage1, owm_run) stops after `limit` node steps per window and
- * the stage-3 cell walk after `limit` rounds per cell, instead of their
+/* Step limit of this context's bounded tree walks: the stage-1 walk
+ * (owm_stage1, stage1_walk = 1) stops after `limit` node steps per window and
+ * the stage-3 cell walk (owm_stage3, owm_run while a limit is set) after `limit`
+ * rounds per cell, instead of their
  * structural bounds (which only a corrupt hierarchy can reach).  A walk that
  * stops sets bit 1 of the device status word and its call returns
  * OWM_ETIMEOUT; the context stays usable.  0 restores the structural bounds.
@@ -284,8 +285,9 @@ typedef struct {
    *     are rectangles of sub-cells, O(N); no hierarchy is built (`tree` is
    *     checked, and the seeds do not depend on it);
    *  1  tree build, warp-cooperative stackless tree walk per window with min-z
-   *     pruning, tree walk per cell.  A context with a
-   *     walk limit (owm_ctx_set_walk_limit) takes this path too. */
+   *     pruning, tree walk per cell.  In a context with a walk limit
+   *     (owm_ctx_set_walk_limit) 0 walks the tree for the cells too, with
+   *     stage 1 on the grid. */
   int32_t stage1_walk;
   int32_t _pad;
 } owm_run_cfg;
