@@ -278,6 +278,7 @@ struct PointCell {
   uint32_t cell, flags;
 };
 constexpr uint32_t kPointOtherX = 1, kPointOtherY = 2, kPointNonFinite = 4;
+constexpr uint32_t kCrowded = 8;  // of a lane of the fold: shared its sub-cell with lanes further off
 
 // A point's sub-cell and z, in full: any coordinate, any axes.
 __device__ __forceinline__ PointCell point_cell(const GridJob& J, uint64_t x, uint64_t y, uint64_t z) {
@@ -317,8 +318,13 @@ __device__ __noinline__ void raise_own_cells(const GridJob& J, uint64_t x, uint6
 //   that scan lines side by side are not folded at the same time (40 M points in
 //   scan order at 3 a square metre: 1.28 -> 0.53 ms);
 // - instructions: 144 per 32 points instead of 284 (0.53 -> 0.40 ms there);
-// - runs of points reduced on 96 bits where the top half of their heights tells
-//   them apart (0.45 -> 0.41 ms there, in whole centimetres);
+// - lanes of one sub-cell reduced on 96 bits where the top half of their heights
+//   tells them apart (0.45 -> 0.41 ms there, in whole centimetres);
+// - an add for each run of neighbours where the lanes of one sub-cell lie apart:
+//   its adds queue in L2 (a cloud crowded in a few places, in no order: 20 M
+//   points, half of them within a metre, 3.4 -> 0.6 to 1.0 ms; 1 / r^2 around one
+//   place 1.7 -> 1.0).  Such lanes are found where neighbours share a sub-cell,
+//   and looked for in every group once a warp has met some;
 // - points on edges (whole centimetres: 1 in 100): two loads side by side in
 //   place of a call (20 M in no order 0.37 -> 0.24 ms, in scan order 0.28 -> 0.23).
 // One point a thread at 48 warps an SM: two at 40 took 1.05 ms for the 100 M,
@@ -403,45 +409,30 @@ __device__ __forceinline__ void fold_stretch(const GridJob& J, Axes axes, const 
       if (J.cell_zid) raise_own_cells(J, x, y, w, nid);
     }
     const ulonglong2 cur = load_zid(J.zid + cell);
-    // runs of neighbouring lanes in one sub-cell (a cloud in scan order)
+    // neighbouring lanes in one sub-cell (a cloud in scan order)
     const uint32_t before = __shfl_up_sync(0xffffffffu, cell, 1);
-    const uint32_t heads = __ballot_sync(0xffffffffu, before != cell) | 1u;
-    if (heads == 0xFFFFFFFFu) {  // none (a lane past the end would repeat its neighbour)
+    if (!__any_sync(0xffffffffu, (lane && before == cell) || (flags & kCrowded))) {  // none (a lane past the end would repeat its neighbour)
       atomicAdd(J.count + grid_count_slot(J, cell), 1u);
       if (w >= cur.x) raise_zid(J.zid + cell, cur, w, nid);
       continue;
     }
-    const uint32_t after = heads & (0xFFFFFFFEu << lane);
-    const int end = after ? __ffs(after) - 1 : 32;
-    const bool head = (heads >> lane) & 1u;
-    const int run = min(end, left) - lane;
-    if (head && run > 0) atomicAdd(J.count + grid_count_slot(J, cell), (uint32_t)run);
+    const uint32_t group = __match_any_sync(0xffffffffu, cell);
+    if ((group & (0u - group)) == 1u << lane)
+      atomicAdd(J.count + grid_count_slot(J, cell), (uint32_t)__popc(group & (0xFFFFFFFFu >> (32 - left))));
+    const uint32_t from = group >> lane;
+    if (from & (from + 1)) flags |= kCrowded;
     if (!__any_sync(0xffffffffu, w >= cur.x)) continue;
-    // the highest top half of w in the run, to its head and from there to all
-    // its lanes; the lane that has it raises the entry
-    uint32_t top = (uint32_t)(w >> 32);
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t other = __shfl_down_sync(0xffffffffu, top, o);
-      if (lane + o < end) top = max(top, other);
-    }
-    const int start = 31 - __clz(heads & (0xFFFFFFFFu >> (31 - lane)));
-    top = __shfl_sync(0xffffffffu, top, start);
-    bool raise = (uint32_t)(w >> 32) == top && w >= cur.x;
-    const uint32_t several = __ballot_sync(0xffffffffu, raise) & (0xFFFFFFFFu << start) & (0xFFFFFFFFu >> (32 - end));
+    // the lane with the highest top half of w in the group raises the entry
+    const uint32_t top = (uint32_t)(w >> 32);
+    bool raise = __reduce_max_sync(group, top) == top && w >= cur.x;
+    const uint32_t several = __ballot_sync(0xffffffffu, raise) & group;
     if (__any_sync(0xffffffffu, (several & (several - 1)) != 0)) {
       raise = raise && zid_above(w, nid, cur);
       if (__any_sync(0xffffffffu, raise)) {  // none on flat ground: its ids rise
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {  // the run's minimum, to its head
-          const unsigned long long ow = __shfl_down_sync(0xffffffffu, w, o);
-          const uint32_t on = __shfl_down_sync(0xffffffffu, nid, o);
-          if (lane + o < end && (ow > w || (ow == w && on > nid))) {
-            w = ow;
-            nid = on;
-          }
-        }
-        raise = head;
+        const uint32_t low = __reduce_max_sync(group, raise ? (uint32_t)w : 0u);
+        raise = raise && (uint32_t)w == low;
+        const uint32_t best = __reduce_max_sync(group, raise ? nid : 0u);
+        raise = raise && nid == best;
       }
     }
     if (raise) raise_zid(J.zid + cell, cur, w, nid);

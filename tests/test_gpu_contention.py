@@ -58,3 +58,67 @@ def test_sparse_cloud_under_many_windows(owm, oracle):
     us = _kernel_us(owm, ctx, lambda: ctx.run(cloud, cfg))
     assert us["k_grid_windows"] < 20 * us["k_grid_rows"], us
     ctx.close()
+
+
+def _crowded(n, side, part, spots, seed, order):
+    """part of the points within half a metre of some places, in no order or by places."""
+    rng = np.random.default_rng(seed)
+    xy = rng.random((n, 2)) * side
+    m = int(n * part)
+    if spots:
+        at = (0.1 + 0.8 * rng.random((spots, 2))) * side
+        xy[:m] = at[rng.integers(0, spots, m)] + rng.random((m, 2)) - 0.5
+    else:  # as seen from one place: density falls with the square of the distance
+        r, a = np.exp(rng.uniform(np.log(0.5), np.log(side / 2), n)), rng.uniform(0, 2 * np.pi, n)
+        xy = side / 2 + np.column_stack([r * np.cos(a), r * np.sin(a)])
+    xy = xy[rng.permutation(n)] if order == "none" else xy[np.lexsort((xy[:, 0], np.floor(xy[:, 1] * 2)))]
+    xyz = np.column_stack([500000.0 + xy[:, 0], 4700000.0 + xy[:, 1], np.round(50 + 4 * rng.random(n), 2)])
+    return xyz, (500000.0, 4700000.0, 500000.0 + side, 4700000.0 + side)
+
+
+@pytest.mark.parametrize("n", [40_001, 300_007])
+@pytest.mark.parametrize("part,spots,heights", [(0.9, 1, "rough"), (0.5, 3, "rough"), (0.0, 0, "rough"), (0.9, 1, "flat"),
+                                                (0.9, 2, "falling"), (0.9, 2, "close")])
+@pytest.mark.parametrize("x0", [500000.0, -31.0])
+def test_crowded_clouds(owm, oracle, ctx, n, part, spots, heights, x0):
+    """Lanes of one sub-cell that are not neighbours, at the ends of warps, with
+    equal heights, heights that fall with the id and heights that differ in their
+    lower bits alone."""
+    xyz, box = _crowded(n, 120.0, part, spots, n, "none")
+    rng = np.random.default_rng(n)
+    if heights == "flat":
+        xyz[:, 2] = 7.25
+    elif heights == "falling":
+        xyz[:, 2] = 500.0 - np.arange(n) * 1e-6
+    elif heights == "close":
+        xyz[:, 2] = 500.0 + rng.integers(0, 1000, n) * 1e-9
+    xyz[:, 0] += x0 - 500000.0
+    bb = owm.Bbox(x0, box[1], x0 + 120.0, box[3])
+    cfg = owm.run_cfg(10, 0.8, 6, 32)
+    want, _ = oracle.run(xyz, bb, 10, 0.8, 6)
+    cloud = ctx.cloud(xyz, bb)
+    np.testing.assert_array_equal(ctx.run(cloud, cfg), want)
+    cloud.close()
+    np.testing.assert_array_equal(ctx.run_host(xyz, bb, cfg), want)
+    b = owm.Batch(ctx)
+    for got in b.run([(xyz, bb, cfg), (xyz[: n // 3], bb, cfg), (xyz, bb, cfg)])[::2]:
+        np.testing.assert_array_equal(got, want)
+    b.close()
+
+
+def test_crowded_cloud_in_no_order_takes_about_as_long_as_its_scan(owm):
+    """Nine points of ten in one sub-cell: the adds of a warp go as one."""
+    ctx = owm.Context(0)
+    n, side, cfg = 5_000_000, 300.0, owm.run_cfg(10, 0.5, 2, 32)
+    rng = np.random.default_rng(3)
+    xy = rng.random((n, 2)) * side
+    xy[: n // 10 * 9] = 150.5 + rng.random((n // 10 * 9, 2))  # window edges at 150 and 155, cell edges at 150 and 152
+    bb = owm.Bbox(500000.0, 4700000.0, 500000.0 + side, 4700000.0 + side)
+    us = {}
+    for order, at in (("scan", np.lexsort((xy[:, 0], np.floor(xy[:, 1] * 2)))), ("none", rng.permutation(n))):
+        xyz = np.column_stack([500000.0 + xy[at, 0], 4700000.0 + xy[at, 1], np.round(50 + 4 * rng.random(n), 2)])
+        cloud = ctx.cloud(xyz, bb)
+        us[order] = _kernel_us(owm, ctx, lambda: ctx.run(cloud, cfg))["k_grid_fold"]
+        cloud.close()
+    assert us["none"] < 2 * us["scan"], us
+    ctx.close()
