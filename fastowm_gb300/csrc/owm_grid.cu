@@ -439,14 +439,17 @@ __device__ __forceinline__ void fold_stretch(const GridJob& J, Axes axes, const 
   }
 }
 
-// What a warp found out, stored once: a store per point to the one word cost
-// 0.4 ms on 40 M points in whole centimetres.
+// What a warp found out, stored unless another one did: stores to the one word
+// queue.  A store per point cost 0.4 ms on 40 M points in whole centimetres, and
+// one per warp 0.3 ms on 5 M points in no order and in multiples of 2 m (384 -> 78
+// us).
 __device__ __forceinline__ void fold_flags(const GridJob& J, uint32_t flags, uint32_t* __restrict__ status) {
   flags = __reduce_or_sync(0xffffffffu, flags);
   if ((threadIdx.x & 31) == 0 && flags) {
     if (flags & kPointNonFinite) atomicOr(status, kStatusNonFinite);
-    if (flags & kPointOtherX) J.occ[1] = 1;
-    if (flags & kPointOtherY) J.occ[3] = 1;
+    volatile uint32_t* occ = J.occ;
+    if ((flags & kPointOtherX) && !occ[1]) occ[1] = 1;
+    if ((flags & kPointOtherY) && !occ[3]) occ[3] = 1;
   }
 }
 

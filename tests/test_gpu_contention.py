@@ -122,3 +122,23 @@ def test_crowded_cloud_in_no_order_takes_about_as_long_as_its_scan(owm):
         cloud.close()
     assert us["none"] < 2 * us["scan"], us
     ctx.close()
+
+
+def test_points_on_edges_in_no_order(owm, oracle):
+    """Coordinates in whole metres, most of them on window edges: the words that
+    say so are stored once, not by every warp."""
+    ctx = owm.Context(0)
+    n, side, cfg = 300_000, 500.0, owm.run_cfg(10, 0.8, 20, 32)
+    rng = np.random.default_rng(6)
+    xy = rng.random((n, 2)) * side
+    bb = owm.Bbox(500000.0, 4700000.0, 500000.0 + side, 4700000.0 + side)
+    us = {}
+    for step in (0.0, 2.0):
+        p = np.round(xy / step) * step if step else xy
+        xyz = np.column_stack([500000.0 + p[:, 0], 4700000.0 + p[:, 1], np.round(50 + 4 * rng.random(n), 2)])
+        cloud = ctx.cloud(xyz, bb)
+        np.testing.assert_array_equal(ctx.run(cloud, cfg), oracle.run(xyz, bb, 10, 0.8, 20)[0])
+        us[step] = _kernel_us(owm, ctx, lambda: ctx.run(cloud, cfg))["k_grid_fold"]
+        cloud.close()
+    assert us[2.0] < 3 * us[0.0], us
+    ctx.close()
