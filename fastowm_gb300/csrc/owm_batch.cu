@@ -1301,12 +1301,7 @@ int owm_batch_set_leaf_classes(owm_batch* b, int32_t nclass, const int64_t* boun
     b->run.class_bound[k] = bounds[k];
     b->run.class_leaf[k] = leaf[k];
   }
-  if (b->run.graph) {
-    cudaGraphExecDestroy(b->run.graph);
-    b->run.graph = nullptr;
-    b->run.graph_sig.clear();
-  }
-  return OWM_OK;
+  return OWM_OK;  // a graph of the trees names its leaf sizes
 }
 
 // For tests: device bytes that a batch of these tiles takes (0 on_grid: by its

@@ -363,7 +363,8 @@ int owm_batch_run(owm_batch* b, const owm_tile_desc* tiles, int32_t ntiles, int6
  * shapes, and replay it when the same shapes come back (1 = on). */
 int owm_batch_set_graphs(owm_batch* b, int enable);
 /* Leaf size per size class: classes by point count, bounds[k] is the upper
- * bound of class k; leaf[k] in {16,32,64,128}.  nclass <= 8. */
+ * bound of class k; leaf[k] a power of two up to 256.  nclass <= 8.  Of the trees
+ * alone: batches on the window grid have no leaves. */
 int owm_batch_set_leaf_classes(owm_batch* b, int32_t nclass, const int64_t* bounds,
                                const int32_t* leaf);
 
