@@ -507,7 +507,8 @@ def main():
     info = RunInfo()
 
     # leaf size (the reference's maxNumber knob): every choice gives the same
-    # seeds, so the library's tuner picks the fastest unless --leaf fixes it
+    # seeds, so the library's tuner picks the tree path's fastest unless --leaf
+    # fixes it (runs on the window grid do not depend on it)
     leaf_tuning = None
     if args.leaf > 0:
         mn = args.leaf
@@ -517,7 +518,7 @@ def main():
         leaf_tuning = autotune.tune_leaf_single(ctx, cloud, lambda L: F.run_cfg(W, Ov, B, L, stage1_walk=args.stage1_walk))
         mn = leaf_tuning["leaf"]
     cfg = F.run_cfg(W, Ov, B, mn, stage1_walk=args.stage1_walk)
-    # launch shapes (gather block, cell-walk warps): exact for every choice
+    # launch shapes of the tree path (gather block, cell-walk warps): exact for every choice
     from fastowm_gb300 import autotune
 
     shape_tuning = autotune.tune_shapes_single(ctx, cloud, cfg, walk=args.stage1_walk) if args.leaf == 0 else None
@@ -746,14 +747,17 @@ def run_batched(F, torch, ctx, args, local, ws):
     autotune.apply(batch, tuned)
     batch.set_graphs(True)
 
-    def run_once():
+    walk = (TileDesc * len(info))(*(TileDesc(d.xyz, d.n, d.bbox, F.run_cfg(d.cfg.wsize, d.cfg.overlap, d.cfg.bsize,
+                                                                           d.cfg.tree.max_number, stage1_walk=True)) for d in descs))
+
+    def run_once(descs=descs):
         rc = F.lib().owm_batch_run(batch.handle, descs, len(info), out.ctypes.data_as(C.POINTER(C.c_int64)), cap,
                                    offs.ctypes.data_as(C.POINTER(C.c_int64)), None)
         if rc:
             raise F.OwmError(rc, "batch_run")
 
-    # launch shapes of the batch's kernels (one set per launch): coordinate
-    # search on the whole batch, seeds checked against the first candidate
+    # launch shapes of the tree path's kernels (one set per launch): coordinate
+    # search on the whole batch by the tree walk, seeds checked against the grid's
     saved_shapes = ctx.tuning()
     run_once()
     ref_out = out.copy()
@@ -762,13 +766,13 @@ def run_batched(F, torch, ctx, args, local, ws):
         best, best_ms = None, float("inf")
         for v in values:
             ctx.set_tuning(**{name: v})
-            run_once()
-            if not np.array_equal(out, ref_out):
+            run_once(walk)
+            if not np.array_equal(out[:offs[-1]], ref_out[:offs[-1]]):
                 raise RuntimeError(f"batched {name}={v}: seeds differ")
             torch.cuda.synchronize()
             t0 = time.perf_counter()
             for _ in range(3):
-                run_once()
+                run_once(walk)
             ms = 1e3 * (time.perf_counter() - t0) / 3
             shape_ms[f"{name}={v}"] = round(ms, 3)
             if ms < best_ms:

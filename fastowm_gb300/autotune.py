@@ -1,6 +1,7 @@
-"""Autotuner for batched tiles: picks the leaf size (the reference's -s
-maxNumber knob, CPP-TBB-CPU/application/owm_optim3.cpp:27) per tile size
-class by timing real batched runs on the device.
+"""Autotuner of the tree path: picks the leaf size (the reference's -s
+maxNumber knob, CPP-TBB-CPU/application/owm_optim3.cpp:27) and the launch shapes
+by timing real runs on the device that walk the tree (stage1_walk).  Runs on the
+window grid have neither: their time does not depend on the picks.
 
 Size classes are point-count bands; for each band a sample of tiles from the
 batched-tiles generator (config 4) is run with every candidate leaf size and
@@ -19,13 +20,18 @@ DEFAULT_BOUNDS = (150_000, 500_000, 1_000_000, 1 << 40)
 DEFAULT_LEAVES = (16, 32, 64, 128, 256)
 
 
+def _walk(F, cfg):
+    """The same run by the tree walk."""
+    return F.run_cfg(cfg.wsize, cfg.overlap, cfg.bsize, cfg.tree.max_number, cfg.tree.policy, cfg.tree.min_radius, stage1_walk=True)
+
+
 def _class_tiles(F, lo: int, hi: int, want: int, config: int = 4, start: int = 0, limit: int = 4096):
     tiles = []
     for t in range(start, start + limit):
         spec, W, Ov, B, mn, seed = F.synth_config(config, t)
         if lo < spec.n <= hi:
             xyz, bb = F.synth_cloud(spec, seed)
-            tiles.append((xyz, bb, F.run_cfg(W, Ov, B, mn)))
+            tiles.append((xyz, bb, F.run_cfg(W, Ov, B, mn, stage1_walk=True)))
             if len(tiles) >= want:
                 break
     return tiles
@@ -69,8 +75,8 @@ def apply(batch, tuned: dict) -> None:
 
 
 def tune_leaf_single(ctx, cloud, make_cfg, leaves=(32, 64, 128, 256), reps: int = 3) -> dict:
-    """Leaf size for one cloud: times owm_run on the device-resident cloud
-    with each candidate (make_cfg(leaf) -> RunCfg) and returns
+    """Leaf size for one cloud: times owm_run by the tree walk on the
+    device-resident cloud with each candidate (make_cfg(leaf) -> RunCfg) and returns
     {"leaf": best, "ms": {leaf: median ms}}.  Every choice gives the same
     seeds; the tuner checks that too."""
     import torch
@@ -80,7 +86,7 @@ def tune_leaf_single(ctx, cloud, make_cfg, leaves=(32, 64, 128, 256), reps: int 
     stream = torch.cuda.ExternalStream(F.lib().owm_ctx_stream(ctx.handle))
     timings, ref = {}, None
     for leaf in leaves:
-        cfg = make_cfg(leaf)
+        cfg = _walk(F, make_cfg(leaf))
         seeds = ctx.run(cloud, cfg)  # warm-up (buffers)
         if ref is None:
             ref = seeds
@@ -121,8 +127,8 @@ def _timed_median(fn, stream, reps: int) -> float:
 
 def tune_shapes_single(ctx, cloud, cfg, walk: bool = False, reps: int = 3) -> dict:
     """Launch shapes for one cloud and run config: coordinate search over the
-    gather's block size, the stage-3 cell walk's warps per block and (for the
-    tree-walk stage 1) the walk's window patch, each timed by owm_run on the
+    gather's block size, the stage-3 cell walk's warps per block and (with walk)
+    the stage-1 walk's window patch, each timed by owm_run by the tree walk on the
     device-resident cloud, every candidate's seeds checked against the first.
     Leaves the best shapes set on ctx; returns {"tuning": {...}, "ms": {...}}."""
     import torch
@@ -130,6 +136,7 @@ def tune_shapes_single(ctx, cloud, cfg, walk: bool = False, reps: int = 3) -> di
     import fastowm_gb300 as F
 
     stream = torch.cuda.ExternalStream(F.lib().owm_ctx_stream(ctx.handle))
+    cfg = _walk(F, cfg)
     ref = ctx.run(cloud, cfg)
     timings = {}
     knobs = [("gather_block", GATHER_BLOCKS), ("cell_warps", CELL_WARPS)]
@@ -154,9 +161,9 @@ def tune_shapes_classes(ctx, bounds=DEFAULT_BOUNDS, tiles_per_class: int = 8, re
                         config: int = 4) -> dict:
     """Launch shapes per tile size class: for each point-count band a sample
     of tiles (config 4 generator) runs one tile per owm_run, and a coordinate
-    search picks the gather block, the cell-walk warps and -- for the
-    tree-walk stage 1 -- the walk's window patch that minimise the band's
-    total device time; every candidate's seeds are checked against the
+    search picks the gather block, the cell-walk warps and (with walk) the
+    stage-1 walk's window patch that minimise the band's
+    total device time of the tree walk; every candidate's seeds are checked against the
     first's.  Returns {"bounds": [...], "classes": [{"tuning", "ms"}, ...]};
     ctx is left with its shapes from before."""
     import torch
@@ -172,14 +179,12 @@ def tune_shapes_classes(ctx, bounds=DEFAULT_BOUNDS, tiles_per_class: int = 8, re
         if not tiles:
             out.append(None)
             continue
-        clouds = [(ctx.cloud(xyz, bb), cfg) for xyz, bb, cfg in tiles]
-        knobs = [("gather_block", GATHER_BLOCKS, False), ("cell_warps", CELL_WARPS, False)]
+        runs = [(ctx.cloud(xyz, bb), cfg) for xyz, bb, cfg in tiles]
+        knobs = [("gather_block", GATHER_BLOCKS), ("cell_warps", CELL_WARPS)]
         if walk:
-            knobs.append(("walk_patch_x", WALK_PATCHES, True))
+            knobs.append(("walk_patch_x", WALK_PATCHES))
         timings = {}
-        for name, values, use_walk in knobs:
-            runs = [(cl, F.run_cfg(cfg.wsize, cfg.overlap, cfg.bsize, cfg.tree.max_number, stage1_walk=use_walk))
-                    for cl, cfg in clouds]
+        for name, values in knobs:
             refs = [ctx.run(cl, c2) for cl, c2 in runs]
             best, best_ms = None, float("inf")
             for v in values:
@@ -198,7 +203,7 @@ def tune_shapes_classes(ctx, bounds=DEFAULT_BOUNDS, tiles_per_class: int = 8, re
                     best, best_ms = v, ms
             ctx.set_tuning(**{name: best})
         out.append({"tuning": ctx.tuning(), "ms": timings})
-        for cl, _ in clouds:
+        for cl, _ in runs:
             cl.close()
         ctx.set_tuning(**saved)
     return {"bounds": list(bounds), "classes": out}

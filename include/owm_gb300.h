@@ -148,6 +148,7 @@ int owm_ctx_set_walk_limit(owm_ctx* ctx, int32_t limit);
 /* Launch shapes of this context's kernels (owm_run, owm_tree_build,
  * owm_stage1, owm_stage3 and the batches made from the context).  Every
  * choice gives the same results; fastowm_gb300.autotune picks them by timing.
+ * They are the tree path's: runs and batches on the window grid do not read them.
  * A field of 0 keeps its default.  No counterpart in the reference, whose
  * launch knobs are the leaf size (-s, owm_optim3.cpp:27) and the -DAUTOGRID
  * grid (SYCL-CUDA-GPU/ordered/cuda/ordered_builder.inl:306-313). */

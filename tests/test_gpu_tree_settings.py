@@ -1,6 +1,8 @@
 """The tree path's settings act on the tree path: leaf classes leave a batch's
-graph on the window grid alone, and runs by the walk give the oracle's seeds for
-every leaf size and policy."""
+graph on the window grid alone, the tuners time runs that build the tree, and
+runs by the walk give the oracle's seeds for every leaf size and policy."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -34,6 +36,32 @@ def test_leaf_classes_and_the_graph(owm, walk):
     b.run(tiles)
     assert ctx.launches - l0 == 1
     b.close()
+    ctx.close()
+
+
+def _kernels(owm, ctx, fn, cap=128):
+    owm.lib().owm_ctx_set_profiling(ctx.handle, 1)
+    fn()
+    names, ms, calls, n = (C.c_char * 64 * cap)(), (C.c_double * cap)(), (C.c_int64 * cap)(), C.c_int32()
+    owm.lib().owm_ctx_kernel_times(ctx.handle, cap, names, ms, calls, C.byref(n))
+    owm.lib().owm_ctx_set_profiling(ctx.handle, 0)
+    return {names[k].value.decode(): calls[k] for k in range(n.value)}
+
+
+def test_tuners_time_the_tree_path(owm):
+    from fastowm_gb300 import autotune
+
+    ctx = owm.Context(0)
+    xyz, box = _cloud()
+    cloud = ctx.cloud(xyz, owm.Bbox(*box))
+    leaves = (32, 128)
+    runs = {"leaf": lambda: autotune.tune_leaf_single(ctx, cloud, lambda leaf: owm.run_cfg(10, 0.8, 15, leaf), leaves, reps=1),
+            "shapes": lambda: autotune.tune_shapes_single(ctx, cloud, owm.run_cfg(10, 0.8, 15, 32), reps=1),
+            "classes": lambda: autotune.tune_leaf_classes(ctx, bounds=(200_000,), leaves=leaves, tiles_per_class=1, reps=1)}
+    for name, tune in runs.items():
+        seen = _kernels(owm, ctx, tune)
+        assert any("gather" in k for k in seen) and not any("grid" in k for k in seen), (name, seen)
+    cloud.close()
     ctx.close()
 
 
