@@ -317,14 +317,21 @@ int run_pipeline(owm_ctx* c, const PointsView& pts, int64_t n, const owm_bbox& b
   const int64_t nllp = rb.words[kLlpSlot], ns3 = rb.words[kS3Slot];
   const int64_t total = nllp + ns3;
   *n_seeds = total;
+  if (total > 0 && total <= cap) {
+    if (!s64 && !is_device_ptr(seeds)) {
+      std::memcpy(seeds, rb.seeds, (size_t)total * 8);
+    } else {  // the run's time ends with this copy
+      OWM_CUDA_TRY(cudaMemcpyAsync(seeds, s64 ? s64 : rb.seeds, (size_t)total * 8, cudaMemcpyDefault, s));
+      OWM_CUDA_TRY(cudaEventRecord(c->ev[5], s));
+      OWM_CUDA_TRY(cudaStreamSynchronize(s));
+    }
+  }
   if (info) {
     std::memset(info, 0, sizeof(*info));
     info->n_llp = nllp;
     info->n_stage3 = ns3;
     info->n_seeds = total;
     info->params = p;
-  }
-  if (info) {
     if (rb.words[8]) {
       unsigned long long t[kGridStamps];
       std::memcpy(t, rb.words + 16, sizeof(t));
@@ -345,14 +352,7 @@ int run_pipeline(owm_ctx* c, const PointsView& pts, int64_t n, const owm_bbox& b
     cudaEventElapsedTime(&f, c->ev[0], c->ev[5]);
     info->ms_total = f;
   }
-  if (total > cap) return OWM_ERANGE;
-  if (total > 0 && !s64 && !is_device_ptr(seeds)) {
-    std::memcpy(seeds, rb.seeds, (size_t)total * 8);
-  } else if (total > 0) {
-    OWM_CUDA_TRY(cudaMemcpyAsync(seeds, s64 ? s64 : rb.seeds, (size_t)total * 8, cudaMemcpyDefault, s));
-    OWM_CUDA_TRY(cudaStreamSynchronize(s));
-  }
-  return OWM_OK;
+  return total > cap ? OWM_ERANGE : OWM_OK;
 }
 
 }  // namespace owm
