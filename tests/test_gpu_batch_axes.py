@@ -27,8 +27,8 @@ KINDS = {
     "across zero, scan": dict(n=30_001, x0=-31.0, y0=1000.0, side=60.0, W=9, Ov=0.3, B=4, quantum=0.01, order="scan"),
     "negative": dict(n=20_000, x0=-500000.0, y0=-4700000.0, side=50.0, W=10, Ov=0.5, B=15, quantum=0.5),
     "power of two": dict(n=30_000, x0=524250.0, y0=4194280.0, side=60.0, W=10, Ov=0.8, B=20, quantum=0.01),
-    "own cells": dict(n=50_000, x0=500000.0, y0=4700000.0, side=600.0, W=40, Ov=0.5, B=1, quantum=0.25),
-    "own cells, scan": dict(n=50_000, x0=-300.0, y0=4700000.0, side=600.0, W=31, Ov=0.2, B=1, order="scan"),
+    "own cells": dict(n=50_000, x0=500000.0, y0=4700000.0, side=1200.0, W=40, Ov=0.5, B=2, quantum=0.25),
+    "own cells, scan": dict(n=50_000, x0=-600.0, y0=4700000.0, side=1200.0, W=31, Ov=0.2, B=2, order="scan"),
     "outside": dict(n=25_000, x0=100000.0, y0=200000.0, side=40.0, W=7, Ov=0.5, B=6, out=3.7),
     "edges": dict(n=40_000, x0=500000.0, y0=4700000.0, side=80.0, W=10, Ov=0.8, B=20, quantum=1.0),
     "crowded": dict(n=60_000, x0=500000.0, y0=4700000.0, side=80.0, W=10, Ov=0.8, B=5, crowd=0.8),

@@ -6,7 +6,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n,side,B", [(5_000_000, 2000.0, 1), (200_000, 100.0, 20)])
+@pytest.mark.parametrize("n,side,B", [(5_000_000, 3000.0, 2), (200_000, 100.0, 20)])
 @pytest.mark.parametrize("walk", [False, True])
 def test_total_covers_the_copy_of_the_seeds(owm, n, side, B, walk):
     ctx = owm.Context(0)
@@ -18,7 +18,7 @@ def test_total_covers_the_copy_of_the_seeds(owm, n, side, B, walk):
     info = owm.RunInfo()
     seeds = ctx.run(cloud, cfg, info)
     phases = info.ms_tree + info.ms_stage1 + info.ms_stage2 + info.ms_stage3
-    copy = 8 * len(seeds) / 20e9 * 1e3  # pageable memory takes a fifth of that rate
-    assert info.n_seeds == len(seeds) and phases > 0
-    assert info.ms_total > phases + (copy if B == 1 else -0.02), (info.ms_total, phases, copy)
+    copy = 8 * len(seeds) / 250e9 * 1e3  # faster than the link can
+    assert info.n_seeds == len(seeds) and phases > 0 and (B != 2 or len(seeds) > 1_500_000)
+    assert info.ms_total > phases + (copy if B == 2 else -0.02), (info.ms_total, phases, copy)
     ctx.close()
