@@ -661,7 +661,7 @@ __device__ __forceinline__ void window_of(const GridJob& J, int64_t item) {
   if (J.win)
     J.win[(int64_t)ii * J.y.n + jj] = id;
   else
-    s2_mark_id(J.once, J.twice, (uint32_t)J.n, id);
+    s2_mark_id<false>(J.once, J.twice, (uint32_t)J.n, id);
 }
 
 template <bool kMulti>

@@ -344,7 +344,7 @@ __global__ void k_s2_mark(const uint32_t* __restrict__ win, int64_t n, uint32_t 
                           uint32_t* __restrict__ once, uint32_t* __restrict__ twice, const uint32_t* __restrict__ top) {
   if (top && *top > max_id) return;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    s2_mark_id(once, twice, max_id, win[i]);  // kNone (and nothing else: ids are <= max_id) is skipped
+    s2_mark_id<true>(once, twice, max_id, win[i]);  // kNone (and nothing else: ids are <= max_id) is skipped
   }
 }
 

@@ -66,18 +66,20 @@ int run_stage2_bitmap(const uint32_t* d_win, int64_t n, int64_t npoints, double 
 
 // Stage 2's occupancy marks of one window result v (ids 0..max_id; kNone is
 // skipped): the first occurrence sets `once`, a later one `twice`.  One lane marks
-// for the lanes of the warp that have the same id (neighbouring windows mostly
-// do), and the bits only rise, so an id whose second bit is set is done: where few
-// ids repeat often (a sparse cloud under many windows) the atomics on their few
-// words queue in L2.  9 M windows over 2000 points 6.1 -> 0.2 ms, 3 M windows of
-// 430 K ids in runs 39 -> 21 us, of 1000 ids in no order 1468 -> 164 (without the
-// look at the second bit 1440).
+// for the lanes of the warp that have the same id, as neighbouring windows mostly
+// do: where few ids repeat often (a sparse cloud under many windows) the atomics on
+// their few words queue in L2 (9 M windows over 2000 points 6.1 -> 0.2 ms).
+// kLook, for lists in any order: an id whose second bit is set is done (3 M windows
+// of 1000 ids in no order 1440 -> 164 us, of 430 K ids in runs 16 -> 21; 39 by a
+// mark for each lane).  The windows of a run do without: the read before the marks
+// costs their kernel 4 us of 16.
+template <bool kLook>
 __device__ __forceinline__ void s2_mark_id(uint32_t* __restrict__ once, uint32_t* __restrict__ twice, uint32_t max_id,
                                            uint32_t v) {
   if (v > max_id) return;
   const uint32_t bit = 1u << (v & 31u), group = __match_any_sync(__activemask(), v);
   if ((group & (0u - group)) != 1u << (threadIdx.x & 31)) return;
-  if (*(volatile uint32_t*)(twice + (v >> 5)) & bit) return;
+  if (kLook && (*(volatile uint32_t*)(twice + (v >> 5)) & bit)) return;
   if ((atomicOr(once + (v >> 5), bit) & bit) || (group & (group - 1))) atomicOr(twice + (v >> 5), bit);
 }
 // Same with explicit working arrays (n uint32 each; d_llp must not alias
