@@ -1,7 +1,7 @@
 // Batched tiles: many independent clouds (own bbox, Wsize, overlap, Bsize and
 // leaf size) run together with one launch per step instead of one launch
 // sequence per tile.  On the window grid (owm_grid.cuh), or, when a tile asks
-// for the tree walk:
+// for the tree walk or the grid's tables cannot be held:
 //
 //   * all points are sorted once on a (tile, Morton) key, so every tile's
 //     points stay in their own contiguous range;

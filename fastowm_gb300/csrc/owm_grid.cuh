@@ -69,7 +69,10 @@ struct __align__(16) GridAxis {
 // the origin 2.  Places further than the guard from an edge's nominal place
 // are therefore on the same side of the edge as the coordinate is.
 constexpr uint32_t kGridGuard = 16;
-constexpr int32_t kGridMinFrac = 8;  // fewest fraction bits of the fixed-point form (4 guards a step)
+// Fewest fraction bits of the fixed-point form: a step of 256 units, an eighth of
+// which lies within the guard of an edge.
+constexpr int32_t kGridMinFrac = 8;
+static_assert((1u << kGridMinFrac) >= 4 * kGridGuard, "the guards of neighbouring edges do not meet");
 
 __host__ __device__ __forceinline__ double grid_add(double a, double b) {
 #ifdef __CUDA_ARCH__
