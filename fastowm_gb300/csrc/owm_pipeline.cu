@@ -2,7 +2,8 @@
 // runs it per loop iteration (CPP-TBB-CPU/application/owm_optim3.cpp:77-230):
 // index, stage 1, sort + stage 2, LLP grid + stage 3, and the result (stage-3
 // ids followed by the LLPs).  The index is the window grid (owm_grid.cuh), or
-// the tree: with stage1_walk, and for stage 3 while a walk limit is set.
+// the tree: with stage1_walk, for stage 3 while a walk limit is set, and where the
+// grid's tables do not fit.
 // Intermediates never leave the device; the host sees two small count words
 // and the final seed list.
 #include <cuda_runtime.h>
@@ -221,14 +222,19 @@ int run_pipeline_enqueue(owm_ctx* c, const PointsView& pts, int64_t n, const owm
   rc = rb->reserve(room <= direct_max ? room : 0, c->stream);
   if (rc) return rc;
   rb->words[8] = 0;
-  if (!cfg.stage1_walk && c->walk_limit == 0) return run_grid(c, pts, n, p, rb, direct_max, d_seeds);
+  bool walk1 = cfg.stage1_walk;  // stage 1 walks the tree
+  if (!walk1 && c->walk_limit == 0) {
+    rc = run_grid(c, pts, n, p, rb, direct_max, d_seeds);
+    if (rc != OWM_ENOMEM) return rc;
+    walk1 = true;  // no room for the tables, nothing queued: a sparse cloud's trees take less
+  }
   const int64_t nc = p.ncells, ng = std::max<int64_t>(p.ngrid, 0);
   rc = tree_alloc(&c->tree, &c->tree_mem, n, cfg.tree, c->stream);
   if (rc) return rc;
   // With a walk limit alone, stage 1 counts on the window grid, which needs no
   // walk: the limit acts on the cells.
   GridPlan g1;
-  if (!cfg.stage1_walk) rc = grid_plan(p, n, nullptr, &g1, true);
+  rc = walk1 ? OWM_OK : grid_plan(p, n, nullptr, &g1, true);
   if (rc) return rc;
   // scratch = [tree build | stage 1's grid | stage 2 | stage 3]
   const size_t bbytes = (tree_scratch_bytes(n) + 255) & ~(size_t)255;
@@ -269,7 +275,7 @@ int run_pipeline_enqueue(owm_ctx* c, const PointsView& pts, int64_t n, const owm
   void* s3scratch = static_cast<char*>(c->scratch.ptr) + tbytes + s2al;
   const size_t s3cap = c->scratch.cap - tbytes - s2al;
   OWM_CUDA_TRY(cudaEventRecord(c->ev[1], s));
-  if (cfg.stage1_walk) {
+  if (walk1) {
     rc = run_stage1(c, c->tree, p, ex, ey, win);
   } else {
     GridPoints gp;

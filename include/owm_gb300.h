@@ -284,7 +284,8 @@ typedef struct {
    *  0  window grid: every point is folded once into the sub-cell of windows
    *     and cells that contain it (count and minimum), and windows and cells
    *     are rectangles of sub-cells, O(N); no hierarchy is built (`tree` is
-   *     checked, and the seeds do not depend on it);
+   *     checked, and the seeds do not depend on it); as 1 where the grid's
+   *     tables do not fit in device memory;
    *  1  tree build, warp-cooperative stackless tree walk per window with min-z
    *     pruning, tree walk per cell.  In a context with a walk limit
    *     (owm_ctx_set_walk_limit) 0 walks the tree for the cells too, with
