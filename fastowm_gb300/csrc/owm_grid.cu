@@ -33,6 +33,12 @@ constexpr int kFoldBlocks = 6;  // resident fold blocks per SM (40 registers a t
 // tiles: 1.32 ms in order, 1.18 in 16 stripes, 1.20 in 64, 1.25 in 256).
 constexpr int64_t kTileChunk = 4096;
 constexpr int kTileStripes = 16;
+// Points a full sub-cell from which on the fold reduces a warp's sub-cells one
+// after the other (a step for each) instead of all runs of neighbours by a network
+// of shuffles: in scan order a warp then meets some five of them.  Fold of 5 M
+// points in scan order, one after the other / network: 4 points a sub-cell 87 / 65
+// us, 12 69 / 61, 48 54 / 56, 160 49 / 52; 41 M at 48 407 / 416.
+constexpr int64_t kFoldDense = 24;
 
 // Start of a kernel of a chain: lets the next one be set up while this one runs
 // (its launch latency then overlaps this kernel), and waits until everything
@@ -324,7 +330,7 @@ __device__ __noinline__ void raise_own_cells(const GridJob& J, uint64_t x, uint6
 //   its adds queue in L2 (a cloud crowded in a few places, in no order: 20 M
 //   points, half of them within a metre, 3.4 -> 0.6 to 1.0 ms; 1 / r^2 around one
 //   place 1.7 -> 1.0).  Such lanes are found where neighbours share a sub-cell,
-//   and looked for in every group once a warp has met some;
+//   and looked for in every group of 32 once a warp has met some;
 // - points on edges (whole centimetres: 1 in 100): two loads side by side in
 //   place of a call (20 M in no order 0.37 -> 0.24 ms, in scan order 0.28 -> 0.23).
 // One point a thread at 48 warps an SM: two at 40 took 1.05 ms for the 100 M,
@@ -387,7 +393,7 @@ __device__ __forceinline__ void fast_cell(const GridJob& J, Axes axes, uint64_t 
   }
 }
 
-template <int kStride, int kFast, class Axes>
+template <int kStride, int kFast, bool kSparse, class Axes>
 __device__ __forceinline__ void fold_stretch(const GridJob& J, Axes axes, const GridPoints& pts, uint32_t b, uint32_t e,
                                              uint32_t& flags) {
   const int lane = threadIdx.x & 31;
@@ -411,7 +417,8 @@ __device__ __forceinline__ void fold_stretch(const GridJob& J, Axes axes, const 
     const ulonglong2 cur = load_zid(J.zid + cell);
     // neighbouring lanes in one sub-cell (a cloud in scan order)
     const uint32_t before = __shfl_up_sync(0xffffffffu, cell, 1);
-    if (!__any_sync(0xffffffffu, (lane && before == cell) || (flags & kCrowded))) {  // none (a lane past the end would repeat its neighbour)
+    const uint32_t heads = __ballot_sync(0xffffffffu, before != cell) | 1u;
+    if (heads == 0xFFFFFFFFu && !__any_sync(0xffffffffu, flags & kCrowded)) {  // none (a lane past the end would repeat its neighbour)
       atomicAdd(J.count + grid_count_slot(J, cell), 1u);
       if (w >= cur.x) raise_zid(J.zid + cell, cur, w, nid);
       continue;
@@ -422,17 +429,49 @@ __device__ __forceinline__ void fold_stretch(const GridJob& J, Axes axes, const 
     const uint32_t from = group >> lane;
     if (from & (from + 1)) flags |= kCrowded;
     if (!__any_sync(0xffffffffu, w >= cur.x)) continue;
-    // the lane with the highest top half of w in the group raises the entry
+    // the lane with the highest top half of w in its group, or in its run of
+    // neighbours (kFoldDense), raises the entry
     const uint32_t top = (uint32_t)(w >> 32);
-    bool raise = __reduce_max_sync(group, top) == top && w >= cur.x;
-    const uint32_t several = __ballot_sync(0xffffffffu, raise) & group;
-    if (__any_sync(0xffffffffu, (several & (several - 1)) != 0)) {
-      raise = raise && zid_above(w, nid, cur);
-      if (__any_sync(0xffffffffu, raise)) {  // none on flat ground: its ids rise
-        const uint32_t low = __reduce_max_sync(group, raise ? (uint32_t)w : 0u);
-        raise = raise && (uint32_t)w == low;
-        const uint32_t best = __reduce_max_sync(group, raise ? nid : 0u);
-        raise = raise && nid == best;
+    bool raise = w >= cur.x;
+    if (!kSparse) {
+      const uint32_t most = __reduce_max_sync(group, top);  // by every lane, raising or not
+      raise = raise && most == top;
+      const uint32_t several = __ballot_sync(0xffffffffu, raise) & group;
+      if (__any_sync(0xffffffffu, (several & (several - 1)) != 0)) {
+        raise = raise && zid_above(w, nid, cur);
+        if (__any_sync(0xffffffffu, raise)) {  // none on flat ground: its ids rise
+          const uint32_t low = __reduce_max_sync(group, raise ? (uint32_t)w : 0u);
+          raise = raise && (uint32_t)w == low;
+          const uint32_t best = __reduce_max_sync(group, raise ? nid : 0u);
+          raise = raise && nid == best;
+        }
+      }
+    } else {
+      const uint32_t after = heads & (0xFFFFFFFEu << lane);
+      const int end = after ? __ffs(after) - 1 : 32, start = 31 - __clz(heads & (0xFFFFFFFFu >> (31 - lane)));
+      uint32_t most = top;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {  // the run's highest, to its head and from there to all
+        const uint32_t other = __shfl_down_sync(0xffffffffu, most, o);
+        if (lane + o < end) most = max(most, other);
+      }
+      most = __shfl_sync(0xffffffffu, most, start);
+      raise = raise && most == top;
+      const uint32_t several = __ballot_sync(0xffffffffu, raise) & (0xFFFFFFFFu << start) & (0xFFFFFFFFu >> (32 - end));
+      if (__any_sync(0xffffffffu, (several & (several - 1)) != 0)) {
+        raise = raise && zid_above(w, nid, cur);
+        if (__any_sync(0xffffffffu, raise)) {
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {  // the run's minimum, to its head
+            const unsigned long long ow = __shfl_down_sync(0xffffffffu, w, o);
+            const uint32_t on = __shfl_down_sync(0xffffffffu, nid, o);
+            if (lane + o < end && (ow > w || (ow == w && on > nid))) {
+              w = ow;
+              nid = on;
+            }
+          }
+          raise = (heads >> lane) & 1u;
+        }
       }
     }
     if (raise) raise_zid(J.zid + cell, cur, w, nid);
@@ -453,7 +492,7 @@ __device__ __forceinline__ void fold_flags(const GridJob& J, uint32_t flags, uin
   }
 }
 
-template <int kStride, int kFast>
+template <int kStride, int kFast, bool kSparse>
 __global__ void __launch_bounds__(kFoldBlock, kFoldBlocks)
     k_grid_fold(const __grid_constant__ GridJob J, const __grid_constant__ GridPoints pts, uint32_t* __restrict__ status) {
   chain_start();
@@ -461,7 +500,7 @@ __global__ void __launch_bounds__(kFoldBlock, kFoldBlocks)
   uint32_t flags = 0;
   int64_t t0, t1;
   chunk_tiles(((int64_t)J.n + 31) / 32, nwarps, ((int64_t)blockIdx.x * kFoldBlock + threadIdx.x) >> 5, &t0, &t1);
-  fold_stretch<kStride, kFast>(J, ParamAxes{&J}, pts, (uint32_t)(t0 * 32), (uint32_t)(t1 * 32), flags);
+  fold_stretch<kStride, kFast, kSparse>(J, ParamAxes{&J}, pts, (uint32_t)(t0 * 32), (uint32_t)(t1 * 32), flags);
   fold_flags(J, flags, status);
 }
 
@@ -561,12 +600,13 @@ __global__ void __launch_bounds__(kFoldBlock, kFoldBlocks)
   uint32_t flags = 0;
   int64_t t0, t1;
   chunk_tiles((n + 31) / 32, kFoldBlock / 32, threadIdx.x >> 5, &t0, &t1);
+  const uint32_t b = (uint32_t)(c0 + t0 * 32), e = (uint32_t)(c0 + t1 * 32);
   if (J.fast == 2)
-    fold_stretch<3, 2>(J, SharedAxes{&J}, pts, (uint32_t)(c0 + t0 * 32), (uint32_t)(c0 + t1 * 32), flags);
+    J.sparse ? fold_stretch<3, 2, true>(J, SharedAxes{&J}, pts, b, e, flags) : fold_stretch<3, 2, false>(J, SharedAxes{&J}, pts, b, e, flags);
   else if (J.fast)
-    fold_stretch<3, 1>(J, SharedAxes{&J}, pts, (uint32_t)(c0 + t0 * 32), (uint32_t)(c0 + t1 * 32), flags);
+    J.sparse ? fold_stretch<3, 1, true>(J, SharedAxes{&J}, pts, b, e, flags) : fold_stretch<3, 1, false>(J, SharedAxes{&J}, pts, b, e, flags);
   else
-    fold_stretch<3, 0>(J, SharedAxes{&J}, pts, (uint32_t)(c0 + t0 * 32), (uint32_t)(c0 + t1 * 32), flags);
+    fold_stretch<3, 0, true>(J, SharedAxes{&J}, pts, b, e, flags);
   fold_flags(J, flags, status);
 }
 
@@ -1329,8 +1369,8 @@ int grid_sizes(const owm_params& p, int64_t n, GridSizes* z) {
   z->nsub = sx * sy;
   // the sub-cells that points in no order spread over: all, or one quadrant
   const bool tile = steps_tile((uint16_t)p.wsize / 2, p.displace, (uint16_t)p.bsize, z->merged);
-  const int64_t main = tile ? ((sx + 1) / 2) * ((sy + 1) / 2) : z->nsub;
-  z->counts = z->nsub + (main <= kGridSpreadMax ? 3 * main : 0);
+  z->main = tile ? ((sx + 1) / 2) * ((sy + 1) / 2) : z->nsub;
+  z->counts = z->nsub + (z->main <= kGridSpreadMax ? 3 * z->main : 0);
   z->nwin = nc * nr;
   z->ncell = ncg * nrg;
   z->rows = sy * nc;
@@ -1349,6 +1389,7 @@ void grid_job(const owm_params& p, int64_t n, const GridSizes& z, GridJob* j) {
   J.thr = p.min_num_points;
   J.n = (int32_t)n;
   J.need_dup = p.overlap > 0.0;
+  J.sparse = n < kFoldDense * z.main;
   J.base[1] = (uint32_t)J.x.width[0] * (uint32_t)J.y.width[0];
   J.base[2] = J.base[1] + (uint32_t)J.x.width[1] * (uint32_t)J.y.width[0];
   J.base[3] = J.base[2] + (uint32_t)J.x.width[0] * (uint32_t)J.y.width[1];
@@ -1625,8 +1666,7 @@ namespace {
 // 55 and 122, 6200 (20 M) 209 and 904.
 constexpr int64_t kFewCells = 8192;  // 192 KB of tables
 bool fold_few(const GridPlan& g) {
-  const int64_t main = g.z.counts > g.z.nsub ? (g.z.counts - g.z.nsub) / 3 : g.z.nsub;
-  return g.z.nsub <= kFewCells && g.n >= 96 * main;
+  return g.z.nsub <= kFewCells && g.n >= 96 * g.z.main;
 }
 }  // namespace
 
@@ -1644,10 +1684,11 @@ int grid_fold(const GridPlan& g, const GridPoints& pts, uint32_t* status, cudaSt
   }
   const unsigned nb = blocks_for(J.n, 152 * kFoldBlocks, kFoldBlock);
   using Kernel = void (*)(GridJob, GridPoints, uint32_t*);
-  static const Kernel kernels[3][3] = {{k_grid_fold<0, 0>, k_grid_fold<0, 1>, k_grid_fold<0, 2>},
-                                       {k_grid_fold<3, 0>, k_grid_fold<3, 1>, k_grid_fold<3, 2>},
-                                       {k_grid_fold<4, 0>, k_grid_fold<4, 1>, k_grid_fold<4, 2>}};
-  const Kernel kernel = kernels[pts.stride == 4 ? 2 : pts.stride == 3 ? 1 : 0][J.fast];
+  static const Kernel kernels[3][3][2] = {
+      {{k_grid_fold<0, 0, true>, k_grid_fold<0, 0, true>}, {k_grid_fold<0, 1, false>, k_grid_fold<0, 1, true>}, {k_grid_fold<0, 2, false>, k_grid_fold<0, 2, true>}},
+      {{k_grid_fold<3, 0, true>, k_grid_fold<3, 0, true>}, {k_grid_fold<3, 1, false>, k_grid_fold<3, 1, true>}, {k_grid_fold<3, 2, false>, k_grid_fold<3, 2, true>}},
+      {{k_grid_fold<4, 0, true>, k_grid_fold<4, 0, true>}, {k_grid_fold<4, 1, false>, k_grid_fold<4, 1, true>}, {k_grid_fold<4, 2, false>, k_grid_fold<4, 2, true>}}};
+  const Kernel kernel = kernels[pts.stride == 4 ? 2 : pts.stride == 3 ? 1 : 0][J.fast][J.sparse];
   OWM_LAUNCH("k_grid_fold", s, OWM_CUDA_TRY(chain(kernel, nb, kFoldBlock, s, J, pts, status)));
   count_launch(launches);
   OWM_CUDA_TRY(cudaGetLastError());

@@ -326,7 +326,8 @@ struct __align__(16) GridJob {
   uint32_t thr;
   int32_t n;
   const double* rec;     // batches: the tile's points (plain x, y, z)
-  int32_t need_dup;      // overlap > 0: LLPs are ids of two or more windows
+  int16_t need_dup;      // overlap > 0: LLPs are ids of two or more windows
+  int16_t sparse;        // fewer than kFoldDense points a full sub-cell
   unsigned long long* stamps;  // [kGridStamps] nanoseconds at the phases' ends, or null
 };
 // Phase stamps: start, index done, stage 1, stage 2, stage 3 and output done.
@@ -379,6 +380,7 @@ void grid_axis_setup(double lo, double hi, double step, int32_t whalf, int32_t n
 // cannot be numbered in 32 bits), and its job, pointers excepted.
 struct GridSizes {
   int64_t nsub = 0, nwin = 0, ncell = 0, rows = 0, edges = 0;
+  int64_t main = 0;     // sub-cells that points in no order spread over (the full ones)
   int64_t counts = 0;  // words of the counts
   int64_t chunks = 0;  // of a stage-2 bitmap
   bool merged = false;  // cells share the windows' sub-cells

@@ -142,3 +142,37 @@ def test_points_on_edges_in_no_order(owm, oracle):
         cloud.close()
     assert us[2.0] < 3 * us[0.0], us
     ctx.close()
+
+
+@pytest.mark.parametrize("density", [0.6, 2.9, 5.9, 6.1, 30.0])
+@pytest.mark.parametrize("heights", ["rough", "flat", "falling", "close"])
+@pytest.mark.parametrize("W,Ov,B", [(10, 0.8, 20), (9, 0.3, 4)])
+def test_scan_order_by_density(owm, oracle, ctx, density, heights, W, Ov, B):
+    """Runs of neighbours in a sub-cell, short and long, on both sides of the
+    density from which on they are reduced another way; two tiles of a batch on
+    different sides."""
+    n = 40_003
+    side = float(np.ceil(np.sqrt(n / density)))
+    rng = np.random.default_rng(int(10 * density))
+    xy = rng.random((n, 2)) * side
+    xy = xy[np.lexsort((xy[:, 0], np.floor(xy[:, 1] * 2)))]
+    z = {"rough": np.round(50 + 4 * rng.random(n), 2), "flat": np.full(n, 7.25), "falling": 500.0 - np.arange(n) * 1e-6,
+         "close": 500.0 + rng.integers(0, 1000, n) * 1e-9}[heights]
+    xyz = np.column_stack([500000.0 + xy[:, 0], 4700000.0 + xy[:, 1], z])
+    bb = owm.Bbox(500000.0, 4700000.0, 500000.0 + side, 4700000.0 + side)
+    cfg = owm.run_cfg(W, Ov, B, 32)
+    want, _ = oracle.run(xyz, bb, W, Ov, B)
+    cloud = ctx.cloud(xyz, bb)
+    np.testing.assert_array_equal(ctx.run(cloud, cfg), want)
+    tree = ctx.tree(cloud)
+    p = owm.params(bb, n, W, Ov, B)
+    np.testing.assert_array_equal(ctx.stage1(tree, p), oracle.stage1(xyz, oracle.params(bb, n, W, Ov, B)))
+    tree.close()
+    cloud.close()
+    dense = xyz * [0.1, 0.1, 1.0] + [450000.0, 4230000.0, 0.0]
+    db = owm.Bbox(500000.0, 4700000.0, 500000.0 + side / 10 + 1, 4700000.0 + side / 10 + 1)
+    b = owm.Batch(ctx)
+    got = b.run([(xyz, bb, cfg), (dense, db, cfg)])
+    np.testing.assert_array_equal(got[0], want)
+    np.testing.assert_array_equal(got[1], oracle.run(dense, db, W, Ov, B)[0])
+    b.close()
